@@ -85,6 +85,22 @@ def lib():
     return _lib
 
 
+_binding = None
+
+
+def binding():
+    """The native host path (_binding.so, csrc/sb_torch.cpp); raises if it has not been built."""
+    global _binding
+    if _binding is None:
+        lib()  # libsbattn.so first: its absence has the clearer message, and _binding.so refers to it
+        if not os.path.exists(os.path.join(HERE, "_binding.so")):
+            raise RuntimeError(f"{HERE}/_binding.so is missing: the CUDA library has not been built "
+                               "(python -m stickbreaking_attention_b200.build). There is no fallback implementation.")
+        from . import _binding as mod
+        _binding = mod
+    return _binding
+
+
 def check(code, where):
     if code != 0:
         raise SbAttnError(code, where)

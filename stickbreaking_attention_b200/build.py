@@ -1,4 +1,5 @@
-"""Builds libsbattn.so (sm_100a only) next to this file with nvcc.  Usage: python -m stickbreaking_attention_b200.build"""
+"""Builds libsbattn.so (sm_100a only, nvcc) and _binding.so (the PyTorch layer's native host path, g++) next to this file.
+Usage: python -m stickbreaking_attention_b200.build"""
 import glob
 import os
 import shutil
@@ -7,6 +8,8 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libsbattn.so")
+BINDING = os.path.join(HERE, "_binding.so")
+BINDING_SRC = os.path.join(HERE, "csrc", "sb_torch.cpp")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
          "-Xcompiler", "-fPIC"]
 # files that must keep IEEE division/exp (the float32-arithmetic kernels): compiled without --use_fast_math
@@ -26,9 +29,41 @@ def stale():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def binding_stale():
+    if not os.path.exists(BINDING):
+        return True
+    t = os.path.getmtime(BINDING)
+    return any(os.path.getmtime(d) > t for d in [BINDING_SRC] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
+
+
+def start_binding():
+    """The compiler process of _binding.so; it refers to libsbattn.so by name and finds it beside itself ($ORIGIN)."""
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import CUDA_HOME, include_paths
+    libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = CUDA_HOME or "/usr/local/cuda"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_binding",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f"-isystem{d}" for d in include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]]
+    cmd += [BINDING_SRC, "-o", BINDING, f"-L{libdir}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+            "-L" + HERE, "-l:libsbattn.so", "-Wl,-rpath,$ORIGIN"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
 def build(force=False, verbose=False):
-    if not force and not stale():
-        return LIB
+    if force or stale():
+        build_library(verbose)
+    if force or binding_stale():
+        pr = start_binding()
+        out, _ = pr.communicate()
+        if pr.returncode != 0:
+            sys.stderr.write(out)
+            raise RuntimeError("g++ failed")
+    return LIB
+
+
+def build_library(verbose):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         raise RuntimeError("nvcc not found: cannot build libsbattn.so")
@@ -50,8 +85,7 @@ def build(force=False, verbose=False):
         failed |= pr.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
-    subprocess.check_call([nvcc, "-shared", "-o", LIB] + objs)
-    return LIB
+    subprocess.check_call([nvcc, "-shared", "-Xlinker", "-soname=libsbattn.so", "-o", LIB] + objs)
 
 
 if __name__ == "__main__":

@@ -16,7 +16,6 @@ from ._lib import SbMat, SbParams, SbVec
 
 _DTYPES = {torch.bfloat16: _lib.SBATTN_BF16, torch.float32: _lib.SBATTN_F32, torch.float16: _lib.SBATTN_F16}
 _PATHS = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tensor": _lib.PATH_TENSOR}
-_status_words = {}
 _forced_path = os.environ.get("SBATTN_PATH", "auto")
 
 
@@ -57,10 +56,8 @@ def get_path():
 
 def status_word(device):
     """int32 device word the kernels OR their SBATTN_ST_* bits into (one per device, never reset by the library)."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    if key not in _status_words:
-        _status_words[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-    return _status_words[key]
+    index = torch.device(device).index
+    return _lib.binding().status_word(torch.cuda.current_device() if index is None else index)
 
 
 def check_status(device=None, reset=True):
@@ -278,10 +275,9 @@ def _register_ops():
 OP_NAMESPACE, _OPS = _register_ops()
 
 
-def _forward(q, k, v, batched, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, fused=False):
-    compiling = torch.compiler.is_compiling()
-    if not compiling:
-        _require_cuda(q, k, v)
+def _forward_traced(q, k, v, batched, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, fused=False):
+    """The forward while torch.compile is tracing: buffers allocated here, one opaque operator (eager calls go to
+    _lib.binding())."""
     q, k, v = _unit_inner(q), _unit_inner(k), _unit_inner(v)
     o = _empty_like_rows(q)
     # no zero-fill: the library writes every row of rem and neg_log_acc (zeros for tokens outside every sequence, which is
@@ -294,57 +290,45 @@ def _forward(q, k, v, batched, cu_seqlens, max_seqlens, logit_scale, attend_curr
         n_seqs, heads, tokens = cu_seqlens.numel(), q.size(0), q.size(1)
     fwd_bytes, _ = workspace_bytes(batched, n_seqs, heads, tokens, max_seqlens, not no_grad)
     ws = torch.empty(fwd_bytes, dtype=torch.uint8, device=q.device)
-    if compiling:  # the traced program sees one opaque operator
-        if batched:
-            _OPS["attn_fwd"](q, k, v, float(logit_scale), bool(attend_current), bool(no_grad), bool(fused), o, rem,
-                             neg_log_acc, ws)
-        else:
-            _OPS["varlen_fwd"](q, k, v, cu_seqlens, int(max_seqlens), float(logit_scale), bool(attend_current),
-                               bool(no_grad), bool(fused), o, rem, neg_log_acc, ws)
+    if batched:
+        _OPS["attn_fwd"](q, k, v, float(logit_scale), bool(attend_current), bool(no_grad), bool(fused), o, rem, neg_log_acc, ws)
     else:
-        _forward_into(q, k, v, batched, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, o, rem, neg_log_acc,
-                      ws, fused)
+        _OPS["varlen_fwd"](q, k, v, cu_seqlens, int(max_seqlens), float(logit_scale), bool(attend_current), bool(no_grad),
+                           bool(fused), o, rem, neg_log_acc, ws)
     return o, rem, neg_log_acc, ws
 
 
-def _backward(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logit_scale, attend_current, phases=0,
-              out=None, bwd_ws=None, fused=False, rem=None):
+def _backward_traced(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logit_scale, attend_current, fused=False, rem=None):
+    """The backward while torch.compile is tracing."""
     if rem is None:
         rem = dr  # placeholder of the right shape: only read when fused
-    compiling = torch.compiler.is_compiling()
-    if not compiling:
-        _require_cuda(q, k, v, do, dr, ws)
     q, k, v, do = _unit_inner(q), _unit_inner(k), _unit_inner(v), _unit_inner(do)
     if do.dtype != q.dtype:
         do = do.to(q.dtype)
-    if fused and not compiling and not _tma_ok(do):
-        do = do.contiguous().clone()  # the fused backward exists in the tensor-core kernels only: give them an aligned copy
     if dr.dtype != q.dtype:
         dr = dr.to(q.dtype)
-    if out is not None:
-        dq, dk, dv = out
-    else:
-        # no zero-fill: the library writes every row (rows outside all sequences are cleared by a small kernel)
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        if dq.stride(-1) != 1:
-            dq, dk, dv = (torch.empty(q.shape, dtype=q.dtype, device=q.device) for _ in range(3))
+    # no zero-fill: the library writes every row (rows outside all sequences are cleared by a small kernel)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    if dq.stride(-1) != 1:
+        dq, dk, dv = (torch.empty(q.shape, dtype=q.dtype, device=q.device) for _ in range(3))
     if batched:
         n_seqs, heads, tokens = q.size(0), q.size(1), q.size(2)
     else:
         n_seqs, heads, tokens = cu_seqlens.numel(), q.size(0), q.size(1)
     _, bwd_bytes = workspace_bytes(batched, n_seqs, heads, tokens, max_seqlens)
-    bws = bwd_ws if bwd_ws is not None else torch.empty(bwd_bytes, dtype=torch.uint8, device=q.device)
-    if compiling:
-        if batched:
-            _OPS["attn_bwd"](do, dr, q, k, v, ws, float(logit_scale), bool(attend_current), bool(fused), rem, dq, dk, dv,
-                             bws)
-        else:
-            _OPS["varlen_bwd"](do, dr, q, k, v, cu_seqlens, int(max_seqlens), ws, float(logit_scale), bool(attend_current),
-                               bool(fused), rem, dq, dk, dv, bws)
+    bws = torch.empty(bwd_bytes, dtype=torch.uint8, device=q.device)
+    if batched:
+        _OPS["attn_bwd"](do, dr, q, k, v, ws, float(logit_scale), bool(attend_current), bool(fused), rem, dq, dk, dv, bws)
     else:
-        _backward_into(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logit_scale, attend_current, phases, dq, dk,
-                       dv, bws, fused, rem)
+        _OPS["varlen_bwd"](do, dr, q, k, v, cu_seqlens, int(max_seqlens), ws, float(logit_scale), bool(attend_current),
+                           bool(fused), rem, dq, dk, dv, bws)
     return dq, dk, dv
+
+
+def attend(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, fuse_remainder):
+    """(o, rem) with an autograd node, through the native host path; cu_seqlens None: batched layout."""
+    return _lib.binding().attend(q, k, v, cu_seqlens, max_seqlens, logit_scale, bool(attend_current), bool(fuse_remainder),
+                                 _carry_policy == "recompute", _PATHS[_forced_path])
 
 
 def _tma_ok(t):
@@ -393,9 +377,13 @@ def varlen_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current=Fal
 
     Returns (o, rem, neg_log_acc, workspace) and, with ``return_attention``, the float32 attention matrix [H, T, T] after
     them.  Mirrors varlen_fwd of the reference (sb_varlen_fwd.py:411-452)."""
-    _check_qkv(q, k, v, 3)
-    cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
-    out = _forward(q, k, v, False, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, fuse_remainder)
+    if torch.compiler.is_compiling():
+        _check_qkv(q, k, v, 3)
+        cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
+        out = _forward_traced(q, k, v, False, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, fuse_remainder)
+    else:
+        out = _lib.binding().fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, bool(attend_current), bool(no_grad),
+                                 bool(fuse_remainder), _PATHS[_forced_path])
     if return_attention:
         return out + (attention_weights(q, k, cu_seqlens, logit_scale, attend_current),)
     return out
@@ -406,17 +394,24 @@ def varlen_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, workspace, logit_scale,
     """Returns (dq, dk, dv).  Mirrors varlen_bwd of the reference (sb_varlen_bwd.py:483-539); ``workspace`` takes
     the place of its ``neg_log_acc`` argument.  ``phases`` (1: dq kernel only, 2: dk/dv kernel only), ``out`` and
     ``bwd_workspace`` exist for benchmarking the two backward kernels apart; leave them at their defaults."""
-    _check_qkv(q, k, v, 3)
-    cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
-    return _backward(do, dr, q, k, v, False, cu_seqlens, max_seqlens, workspace, logit_scale, attend_current, phases,
-                     out, bwd_workspace, fuse_remainder, rem)
+    if torch.compiler.is_compiling():
+        _check_qkv(q, k, v, 3)
+        cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
+        return _backward_traced(do, dr, q, k, v, False, cu_seqlens, max_seqlens, workspace, logit_scale, attend_current,
+                                fuse_remainder, rem)
+    return tuple(_lib.binding().bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, workspace, logit_scale, bool(attend_current), phases,
+                                    bool(fuse_remainder), rem, _PATHS[_forced_path], list(out) if out is not None else [], bwd_workspace))
 
 
 def attn_fwd(q, k, v, logit_scale, attend_current=False, no_grad=False, fuse_remainder=False, return_attention=False):
     """Batched layout: q, k, v [B, H, T, D].  Mirrors _fwd of the reference (sb_attn/sb_fwd.py:137-173); with
     ``return_attention`` the float32 attention matrix [B, H, T, T] follows the other results."""
-    _check_qkv(q, k, v, 4)
-    out = _forward(q, k, v, True, None, q.size(2), logit_scale, attend_current, no_grad, fuse_remainder)
+    if torch.compiler.is_compiling():
+        _check_qkv(q, k, v, 4)
+        out = _forward_traced(q, k, v, True, None, q.size(2), logit_scale, attend_current, no_grad, fuse_remainder)
+    else:
+        out = _lib.binding().fwd(q, k, v, None, None, logit_scale, bool(attend_current), bool(no_grad), bool(fuse_remainder),
+                                 _PATHS[_forced_path])
     if return_attention:
         return out + (attention_weights(q, k, None, logit_scale, attend_current),)
     return out
@@ -424,6 +419,8 @@ def attn_fwd(q, k, v, logit_scale, attend_current=False, no_grad=False, fuse_rem
 
 def attn_bwd(do, dr, q, k, v, workspace, logit_scale, attend_current=False, fuse_remainder=False, rem=None):
     """Mirrors _bwd of the reference (sb_attn/sb_bwd.py:162-204)."""
-    _check_qkv(q, k, v, 4)
-    return _backward(do, dr, q, k, v, True, None, q.size(2), workspace, logit_scale, attend_current, 0, None, None,
-                     fuse_remainder, rem)
+    if torch.compiler.is_compiling():
+        _check_qkv(q, k, v, 4)
+        return _backward_traced(do, dr, q, k, v, True, None, q.size(2), workspace, logit_scale, attend_current, fuse_remainder, rem)
+    return tuple(_lib.binding().bwd(do, dr, q, k, v, None, None, workspace, logit_scale, bool(attend_current), 0, bool(fuse_remainder),
+                                    rem, _PATHS[_forced_path], [], None))

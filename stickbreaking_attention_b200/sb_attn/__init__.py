@@ -4,7 +4,7 @@ import math
 
 import torch
 
-from ..ops import attn_bwd, attn_fwd, fusable, get_carry_policy
+from ..ops import attend, attn_bwd, attn_fwd, fusable, get_carry_policy
 
 
 class StickBreakingAttention(torch.autograd.Function):
@@ -41,6 +41,8 @@ def sb_attn(q, k, v, inv_temp=None, zero_start=True, attend_current=False, fuse_
     ``fuse_remainder=True`` (no counterpart in the reference) returns ``o + rem[..., None] * v`` as the first result."""
     if inv_temp is None:
         inv_temp = 1 / math.sqrt(q.size(-1))
+    if not torch.compiler.is_compiling():
+        return attend(q, k, v, None, None, inv_temp, attend_current, fuse_remainder)
     if fuse_remainder and not fusable(q, k, v):  # fp32-arithmetic kernels: the same sum, formed here
         o, rem = sb_attn_(q, k, v, inv_temp, attend_current=attend_current)
         return o + rem[..., None] * v, rem

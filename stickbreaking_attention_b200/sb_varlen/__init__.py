@@ -4,7 +4,8 @@ import math
 
 import torch
 
-from ..ops import fusable, get_carry_policy, varlen_bwd, varlen_fwd
+from .. import _lib
+from ..ops import attend, fusable, get_carry_policy, varlen_bwd, varlen_fwd
 
 
 class StickBreakingAttention(torch.autograd.Function):
@@ -47,11 +48,20 @@ def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_st
     which costs one synchronisation.  Returns (o, rem); callers usually form ``o + rem[..., None] * v``
     (tests/test_varlen.py:103 of the reference): with ``fuse_remainder=True`` (no counterpart in the reference) the first
     result is that sum already, computed in the kernels' epilogues, and the backward accounts for it."""
-    if zero_start:
-        assert cu_seqlens[0] == 0
-        cu_seqlens = cu_seqlens[1:]
     if inv_temp is None:
         inv_temp = 1 / math.sqrt(q.size(-1))
+    traced = torch.compiler.is_compiling()
+    if zero_start:
+        if not traced and cu_seqlens.dtype in (torch.int32, torch.int64) and cu_seqlens.dim() == 1 and cu_seqlens.numel() > 0:
+            # one device-to-host copy answers both questions: is the first entry zero, how long is the longest sequence
+            first, longest = _lib.binding().seq_bounds(cu_seqlens, True, max_seqlens is None)
+            assert first == 0
+            max_seqlens = longest if max_seqlens is None else max_seqlens
+        else:
+            assert cu_seqlens[0] == 0
+        cu_seqlens = cu_seqlens[1:]
+    if not traced:
+        return attend(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, fuse_remainder)
     if fuse_remainder and not fusable(q, k, v):  # fp32-arithmetic kernels: the same sum, formed here
         o, rem = sb_attn_varlen_(q, k, v, inv_temp, cu_seqlens, max_seqlens, attend_current)
         return o + rem[..., None] * v, rem
