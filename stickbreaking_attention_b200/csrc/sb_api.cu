@@ -51,6 +51,7 @@ KArgs make_args(const SbParams& p, const WsLayout& L) {
     a.drem_eff = p.bwd_workspace ? (float*)((char*)p.bwd_workspace + L.off_drem) : nullptr;
     a.fused = (p.flags & SBATTN_FLAG_FUSED_REMAINDER) ? 1 : 0;
     a.tokens = p.tokens;
+    a.zero_tail = p.batch == 0 && p.bwd_phases == SBATTN_BWD_ALL;  // the batched layout covers every token
     a.drem_rows = (int64_t)p.tokens * (p.batch > 0 ? p.batch : 1);
     a.slot_cap = 2 * L.slot_cap;  // 32-key slots
     a.heads = p.heads;
@@ -142,7 +143,6 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     cudaStream_t st = (cudaStream_t)p->stream;
     if (launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
     const KArgs a = make_args(*p, L);
-    if (launch_zero_tail_rows(*p, a, st) != 0) return SBATTN_ECUDA;
     int e = path == 1 ? launch_tensor_fwd(*p, L, a, st) : launch_simt_fwd(*p, L, a, st);
     // a layout the tensor-map encoder refuses (nothing has been launched yet): the other kernels take any strides
     if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER))
@@ -172,7 +172,6 @@ extern "C" int sbattn_bwd(const SbParams* p) {
     }
     cudaStream_t st = (cudaStream_t)p->stream;
     const KArgs a = make_args(*p, L);
-    if (p->bwd_phases == SBATTN_BWD_ALL && launch_zero_tail(*p, a, st) != 0) return SBATTN_ECUDA;
     int e = path == 1 ? launch_tensor_bwd(*p, L, a, st) : launch_simt_bwd(*p, L, a, st);
     if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER))
         e = launch_simt_bwd(*p, L, a, st);

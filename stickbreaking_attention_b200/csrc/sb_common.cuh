@@ -7,6 +7,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/sbattn.h"
 
 namespace sb {
@@ -111,6 +113,7 @@ struct KArgs {
     int64_t drem_rows;      // batch * tokens (tokens for the packed layout)
     int32_t head_group;     // heads whose work is interleaved (sized so that their K and V stay in L2)
     int32_t defer_fwd, defer_dq, defer_dkdv;  // tensor-core kernels: store an item's result one step into the next item
+    int32_t zero_tail;      // packed layout: clear the result rows of tokens behind the last sequence
     int32_t* sched;         // WsHeader::sched
     float inv_temp;
     MatView q, k, v, o, d_o, dq, dk, dv;
@@ -142,12 +145,61 @@ template <> __device__ inline __half from_f32<__half>(float x) { return __float2
 extern unsigned long long g_launch_count;
 inline void count_launch() { __atomic_fetch_add(&g_launch_count, 1ull, __ATOMIC_RELAXED); }
 
+// Programmatic dependent launch: every kernel of the library may start while the kernel before it in the stream drains, sets up
+// what needs no global memory, and then waits here for that kernel's completion (and with it, since every kernel of
+// the library waits, for everything before).  A kernel that lets its successor start early calls pdl_launch_dependents().
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgsT, typename... ArgsT>
+inline int launch_kernel(void (*kernel)(KArgsT...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, ArgsT&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<ArgsT>(args)...);
+    count_launch();
+    return (int)(e == cudaSuccess ? cudaGetLastError() : e);
+}
+
+// Result rows of tokens that belong to no sequence (a pack whose last end is below T), shared out over all threads of the grid:
+// every other row is written by the attention kernels, so the caller need not clear anything.  rem and neg_log_acc are
+// zero there (what the reference's zero-initialised outputs hold, sb_varlen_fwd.py:418-419), and so are the gradients.
+template <typename T>
+__device__ inline void zero_tail_rows(const KArgs& a, int first, int64_t thread, int64_t n_threads) {
+    const int64_t total = (int64_t)(a.tokens - first) * a.heads;
+    for (int64_t i = thread; i < total; i += n_threads) {
+        const int h = (int)(i % a.heads);
+        const int64_t t = first + i / a.heads;
+        ((T*)a.rem.ptr)[h * a.rem.sh + t * a.rem.st] = T(0.f);
+        ((float*)a.nla.ptr)[h * a.nla.sh + t * a.nla.st] = 0.f;
+    }
+}
+template <typename T>
+__device__ inline void zero_tail_grads(const KArgs& a, int first, int64_t thread, int64_t n_threads) {
+    const int D = a.head_dim;
+    const int64_t total = (int64_t)(a.tokens - first) * a.heads * D;
+    for (int64_t i = thread; i < total; i += n_threads) {
+        const int d = (int)(i % D);
+        const int64_t rh = i / D;
+        const int h = (int)(rh % a.heads);
+        const int64_t t = first + rh / a.heads;
+        ((T*)a.dq.ptr)[h * a.dq.sh + t * a.dq.st + d] = T(0.f);
+        ((T*)a.dk.ptr)[h * a.dk.sh + t * a.dk.st + d] = T(0.f);
+        ((T*)a.dv.ptr)[h * a.dv.sh + t * a.dv.st + d] = T(0.f);
+    }
+}
+
 // launchers implemented in the .cu files (each returns a cudaError_t as int; the tensor-core launchers return
 // kMapEncodeFailed when a tensor map could not be encoded, before anything has been launched)
 constexpr int kMapEncodeFailed = -1000;
 int launch_prep(const SbParams& p, const WsLayout& L, cudaStream_t st);
-int launch_zero_tail(const SbParams& p, const KArgs& a, cudaStream_t st);
-int launch_zero_tail_rows(const SbParams& p, const KArgs& a, cudaStream_t st);
 int launch_simt_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 int launch_simt_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 bool tensor_path_eligible(const SbParams& p, bool backward, int* why);

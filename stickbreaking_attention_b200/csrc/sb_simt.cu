@@ -181,6 +181,10 @@ __device__ inline bool fetch_item(const KArgs& a, int item, ItemCtx& c) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1) simt_fwd_kernel(const KArgs a) {
     extern __shared__ float smem[];
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
+        const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+        zero_tail_rows<T>(a, a.hdr->covered_end, block * kThreads + threadIdx.x, (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads);
+    }
     ItemCtx c;
     if (!fetch_item(a, blockIdx.x, c)) return;
     const int h = blockIdx.y;
@@ -255,6 +259,10 @@ __global__ void __launch_bounds__(kThreads, 1) simt_fwd_kernel(const KArgs a) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1) simt_bwd_dq_kernel(const KArgs a) {
     extern __shared__ float smem[];
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
+        const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+        zero_tail_grads<T>(a, a.hdr->covered_end, block * kThreads + threadIdx.x, (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads);
+    }
     ItemCtx c;
     if (!fetch_item(a, blockIdx.x, c)) return;
     const int h = blockIdx.y;

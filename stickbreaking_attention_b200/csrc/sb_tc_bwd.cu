@@ -191,6 +191,13 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
+        const int64_t me = (int64_t)blockIdx.x * kDqThreads + tid, all = (int64_t)gridDim.x * kDqThreads;
+        if (kF16) zero_tail_grads<__half>(a, a.hdr->covered_end, me, all);
+        else zero_tail_grads<__nv_bfloat16>(a, a.hdr->covered_end, me, all);
+    }
     const int n_items = a.hdr->n_items;
     const int n_work = *abort_flag ? 0 : n_items * a.heads;
     // G counts 128-key steps over all items of this block: step G uses K stage G % 3, V stage G % 2 and S buffer G % 2;
@@ -675,6 +682,8 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
     const int n_items = a.hdr->n_items;
     const int n_work = *abort_flag ? 0 : n_items * a.heads;
     // G counts query-tile steps over all items of this block; a barrier that completes once per step is in phase G & 1.
@@ -997,20 +1006,16 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 template <int D, bool kF16, bool kFused>
 int launch_bwd_kernels(const SbParams& p, const KArgs& a, cudaStream_t st, const CUtensorMap& mq, const CUtensorMap& mk128,
                        const CUtensorMap& mv128, const CUtensorMap& mdo, const CUtensorMap& mq64, const CUtensorMap& mdo64,
-                       int smem_a, int smem_b) {
+                       int smem_a, int smem_b, dim3 grid) {
     const auto launch_dq = [&](auto kernel) {
         const int e = ensure_kernel_attrs((const void*)kernel, smem_a, true);
         if (e != 0) return e;
-        kernel<<<sm_count(), kDqThreads, smem_a, st>>>(mq, mk128, mv128, mdo, a);
-        count_launch();
-        return (int)cudaGetLastError();
+        return launch_kernel(kernel, grid, dim3(kDqThreads), smem_a, st, mq, mk128, mv128, mdo, a);
     };
     const auto launch_dkdv = [&](auto kernel) {
         const int e = ensure_kernel_attrs((const void*)kernel, smem_b, true);
         if (e != 0) return e;
-        kernel<<<sm_count(), kKvThreads, smem_b, st>>>(mq, mk128, mv128, mdo, mq64, mdo64, a);
-        count_launch();
-        return (int)cudaGetLastError();
+        return launch_kernel(kernel, grid, dim3(kKvThreads), smem_b, st, mq, mk128, mv128, mdo, mq64, mdo64, a);
     };
     if (p.bwd_phases != SBATTN_BWD_DKDV) {
         const int e = a.defer_dq ? launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, true>) : launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, false>);
@@ -1025,7 +1030,7 @@ int launch_bwd_kernels(const SbParams& p, const KArgs& a, cudaStream_t st, const
 }
 
 template <int D, bool kF16>
-int launch_bwd_t(const SbParams& p, const KArgs& a, cudaStream_t st) {
+int launch_bwd_t(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
     // Q, dO, K, V as 128-row tiles; the dk/dv kernel loads Q and dO also as 64-row halves
     CUtensorMap mq, mdo, mk128, mv128, mq64, mdo64;
     const int kind = kF16 ? 2 : 0;
@@ -1043,16 +1048,17 @@ int launch_bwd_t(const SbParams& p, const KArgs& a, cudaStream_t st) {
     constexpr int need_b = 6 * kBM * D * 2 + 2 * 2 * 64 * 128 + 3072;
     constexpr int smem_a = need > 120 * 1024 ? need : 120 * 1024;  // one block per SM: it owns all 512 tensor-memory columns
     constexpr int smem_b = need_b > 120 * 1024 ? need_b : 120 * 1024;  // one block per SM: it owns all 512 tensor-memory columns
-    return a.fused ? launch_bwd_kernels<D, kF16, true>(p, a, st, mq, mk128, mv128, mdo, mq64, mdo64, smem_a, smem_b)
-                   : launch_bwd_kernels<D, kF16, false>(p, a, st, mq, mk128, mv128, mdo, mq64, mdo64, smem_a, smem_b);
+    const dim3 grid(persistent_grid((int64_t)L.max_items * p.heads));
+    return a.fused ? launch_bwd_kernels<D, kF16, true>(p, a, st, mq, mk128, mv128, mdo, mq64, mdo64, smem_a, smem_b, grid)
+                   : launch_bwd_kernels<D, kF16, false>(p, a, st, mq, mk128, mv128, mdo, mq64, mdo64, smem_a, smem_b, grid);
 }
 
 }  // namespace
 
-int launch_tensor_bwd(const SbParams& p, const WsLayout&, const KArgs& a, cudaStream_t st) {
+int launch_tensor_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
     const bool f16 = p.dtype == SBATTN_F16;
-    if (p.head_dim > 64) return f16 ? launch_bwd_t<128, true>(p, a, st) : launch_bwd_t<128, false>(p, a, st);
-    return f16 ? launch_bwd_t<64, true>(p, a, st) : launch_bwd_t<64, false>(p, a, st);
+    if (p.head_dim > 64) return f16 ? launch_bwd_t<128, true>(p, L, a, st) : launch_bwd_t<128, false>(p, L, a, st);
+    return f16 ? launch_bwd_t<64, true>(p, L, a, st) : launch_bwd_t<64, false>(p, L, a, st);
 }
 
 }  // namespace sb

@@ -167,7 +167,8 @@ struct SchedProducer {
         ++i;
         if (!sm100::mbar_wait(&empty[sl], ph[sl], abort_flag)) return -1;
         ph[sl] ^= 1;
-        int w = atomicAdd(counter, 1);
+        // the first item of a block is fixed, the counter deals out the rest
+        int w = i == 1 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(counter, 1);
         if (w >= n_work) w = -1;
         if (w >= 0) {
             out = fetch(w);
@@ -224,6 +225,13 @@ __device__ __forceinline__ void tc_teardown(volatile uint32_t* abort_flag, uint3
         sm100::tc_fence_after();
         sm100::tmem_dealloc(tmem, ncols);
     }
+}
+
+// persistent blocks for at most `n_work` items: one per SM
+inline int sm_count();
+inline int persistent_grid(int64_t n_work) {
+    const int n = sm_count();
+    return (int)(n_work < 1 ? 1 : (n_work < n ? n_work : n));
 }
 
 inline int sm_count() {

@@ -147,6 +147,13 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
+        const int64_t me = (int64_t)blockIdx.x * kFwdThreads + tid, all = (int64_t)gridDim.x * kFwdThreads;
+        if (kF16) zero_tail_rows<__half>(a, a.hdr->covered_end, me, all);
+        else zero_tail_rows<__nv_bfloat16>(a, a.hdr->covered_end, me, all);
+    }
     const int n_items = a.hdr->n_items;
     const int n_work = *abort_flag ? 0 : n_items * a.heads;
 
@@ -421,7 +428,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 }
 
 template <int D, bool kF16>
-int launch_fwd_t(const SbParams& p, const KArgs& a, cudaStream_t st) {
+int launch_fwd_t(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
     // D is the padded head dim (64 or 128); the tensor maps carry the true one, and TMA fills the columns beyond it with zeros
     CUtensorMap mq, mk, mv;
     const int kind = kF16 ? 2 : 0;
@@ -437,9 +444,7 @@ int launch_fwd_t(const SbParams& p, const KArgs& a, cudaStream_t st) {
     const auto launch = [&](auto kernel) {
         const int e = ensure_kernel_attrs((const void*)kernel, smem, false);
         if (e != 0) return e;
-        kernel<<<sm_count(), kFwdThreads, smem, st>>>(mq, mk, mv, a);
-        count_launch();
-        return (int)cudaGetLastError();
+        return launch_kernel(kernel, dim3(persistent_grid((int64_t)L.max_items * p.heads)), dim3(kFwdThreads), smem, st, mq, mk, mv, a);
     };
     if (a.fused) return a.defer_fwd ? launch(tc_fwd_kernel<D, kF16, true, true>) : launch(tc_fwd_kernel<D, kF16, true, false>);
     return a.defer_fwd ? launch(tc_fwd_kernel<D, kF16, false, true>) : launch(tc_fwd_kernel<D, kF16, false, false>);
@@ -467,10 +472,10 @@ bool tensor_path_eligible(const SbParams& p, bool backward, int* why) {
     return true;
 }
 
-int launch_tensor_fwd(const SbParams& p, const WsLayout&, const KArgs& a, cudaStream_t st) {
+int launch_tensor_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
     const bool f16 = p.dtype == SBATTN_F16;
-    if (p.head_dim > 64) return f16 ? launch_fwd_t<128, true>(p, a, st) : launch_fwd_t<128, false>(p, a, st);
-    return f16 ? launch_fwd_t<64, true>(p, a, st) : launch_fwd_t<64, false>(p, a, st);
+    if (p.head_dim > 64) return f16 ? launch_fwd_t<128, true>(p, L, a, st) : launch_fwd_t<128, false>(p, L, a, st);
+    return f16 ? launch_fwd_t<64, true>(p, L, a, st) : launch_fwd_t<64, false>(p, L, a, st);
 }
 
 }  // namespace sb
