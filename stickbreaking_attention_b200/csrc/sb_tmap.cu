@@ -35,9 +35,14 @@ int encode_tile_map(CUtensorMap* map, const void* ptr, int elem_kind, int64_t D,
     const cuuint32_t box[4] = {64u, (cuuint32_t)box_rows, 1u, 1u};
     const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     const CUtensorMapDataType dt = elem_kind == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const CUresult r = g_encode(map, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const auto encode = [&]() {
+        return g_encode(map, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    // The driver call wants a current context, which a thread that has made no runtime call yet does not have (the first backward
+    // on an autograd thread): any runtime call binds the device's primary context.
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaFree(nullptr) == cudaSuccess) r = encode();
     return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
