@@ -7,6 +7,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <mutex>
+#include <unordered_map>
 #include <utility>
 
 #include "../../include/sbattn.h"
@@ -166,6 +168,29 @@ inline int launch_kernel(void (*kernel)(KArgsT...), dim3 grid, dim3 block, size_
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<ArgsT>(args)...);
     count_launch();
     return (int)(e == cudaSuccess ? cudaGetLastError() : e);
+}
+
+// Dynamic shared memory size (and the carve-out preference) of a kernel, set once per kernel and device instead of on
+// every launch: the two driver calls cost more than the launch itself for small problems.
+inline int ensure_kernel_attrs(const void* kernel, int smem_bytes, bool prefer_shared) {
+    static std::mutex mu;
+    static std::unordered_map<const void*, uint64_t> done;  // bit d: set on device d
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return (int)cudaErrorInvalidDevice;
+    const bool tracked = dev >= 0 && dev < 64;
+    if (tracked) {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = done.find(kernel);
+        if (it != done.end() && ((it->second >> dev) & 1)) return 0;
+    }
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e != cudaSuccess) return (int)e;
+    if (prefer_shared) cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (tracked) {
+        std::lock_guard<std::mutex> lock(mu);
+        done[kernel] |= 1ull << dev;
+    }
+    return 0;
 }
 
 // Result rows of tokens that belong to no sequence (a pack whose last end is below T), shared out over all threads of the grid:

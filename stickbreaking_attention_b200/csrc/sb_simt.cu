@@ -2,116 +2,206 @@
 //
 // They serve float32 inputs (where products must not be rounded to bf16/tf32), head dims other than 32, 64 and
 // 128, and tensors whose strides the TMA path cannot take.  Structure mirrors the tensor-core kernels:
-//   * forward walks the key tiles of one 64-row query block right to left and carries, per row, the running
+//   * forward walks the key tiles of one query block right to left and carries, per row, the running
 //     product W = prod(1 - beta) of everything to the right (the reference carries its log,
 //     stickbreaking_attention/sb_varlen/sb_varlen_fwd.py:53-66,155-193);
-//   * the value of W at every 64-key boundary is saved ("carry_w") so that the backward can enter any tile
+//   * the value of W at every 32-key boundary is saved ("carry_w") so that the backward can enter any tile
 //     directly instead of subtracting from the row total as the reference does (sb_varlen_bwd.py:396-445);
 //   * backward-dq walks left to right carrying the prefix sum of g = A * dA (sb_varlen_bwd.py:438-449) and saves
 //     it at every boundary ("carry_c");
 //   * backward-dk/dv keeps one 64-key tile stationary and walks the query blocks below it, entering each
 //     tile with the two saved carries; dk and dv are accumulated in registers and stored once, so there is no
 //     atomic or lock on the data (the reference uses a spin lock per key tile, sb_varlen_bwd.py:11-53).
+//
+// What bounds them is the FMA pipes (128 per clock and SM), so everything else is kept out of their way: a thread owns a
+// register tile of 8 (or 4) rows x 4 columns of every product, operands come from shared memory in 16-byte pieces (3 loads per 16
+// packed fp32x2 multiply-adds), scores never leave the registers (the 16 lanes of a row exchange their products and sums by
+// shuffles), and only the weights pass through shared memory on their way into the second product.  With one 4 x 4 tile per
+// thread, scalar shared loads and the scores in shared memory, 4096 float32 tokens (8 heads, head dim 64) took 0.64 / 0.82 /
+// 1.03 ms in the three kernels, 7 TFLOP/s.
 #include "sb_common.cuh"
 
 namespace sb {
 
 namespace {
 
-constexpr int kBM = 64;         // query rows per block
-constexpr int kBN = 64;         // keys per tile
-constexpr int kThreads = 256;   // 16 x 16 thread grid, 4 x 4 outputs each
-constexpr int kSP = kBN + 1;    // padded row length of the score tiles
+constexpr int kBN = 64;         // keys per tile (and query rows per tile of the dk/dv kernel)
+constexpr int kThreads = 128;   // 8 row groups x 16 column groups
 
+// An operand tile in shared memory, transposed: [DP][kW] floats, element (row, d) in row d of the tile.  The 16-byte pieces of
+// a row are permuted by a function of d so that neither the transposing stores (lanes along d) nor the loads (lanes along the
+// piece index, or along d with a fixed piece) pile up on a bank: (d ^ d / 4) is a permutation of 0 ... 15 both over
+// 16 consecutive d and over 16 d that are 4 apart.
+template <int kW>
+__device__ __forceinline__ int piece(int d, int c) {
+    return d * kW + (((c ^ d ^ (d >> 2)) & (kW / 4 - 1)) << 2);
+}
+
+template <typename T> struct Quad;  // four consecutive elements as they lie in global memory
+template <> struct Quad<float> { typedef float4 type; };
+template <> struct Quad<__nv_bfloat16> { typedef uint2 type; };
+template <> struct Quad<__half> { typedef uint2 type; };
+__device__ __forceinline__ float4 quad_f32(const float4& x, float) { return x; }
+__device__ __forceinline__ float4 quad_f32(const uint2& x, __nv_bfloat16) {
+    return make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
+}
+__device__ __forceinline__ float4 quad_f32(const uint2& x, __half) {
+    const float2 a = __half22float2(*(const __half2*)&x.x), b = __half22float2(*(const __half2*)&x.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 template <typename T>
-__device__ inline void load_rows(float* dst, int DP, int D, const MatView& m, int b, int h, int row0, int rows_valid) {
-    const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh;
-    for (int idx = threadIdx.x; idx < kBM * D; idx += kThreads) {
-        const int r = idx / D, d = idx - r * D;
-        float x = 0.f;
-        if (r < rows_valid) x = to_f32<T>(base[(int64_t)(row0 + r) * m.st + d]);
-        dst[r * DP + d] = x;
+__device__ __forceinline__ bool quads_ok(const MatView& m, int D) {
+    return (D & 3) == 0 && ((uintptr_t)m.ptr % (4 * sizeof(T))) == 0 && (m.st & 3) == 0 && (m.sh & 3) == 0 && (m.sb & 3) == 0;
+}
+
+// kRows rows of a [.., T, D] tensor into shared memory as float32, zeros behind the valid rows and columns.
+// kT: transposed tile (see piece); otherwise rows of DP floats.
+template <typename T, int DP, int kRows, bool kT>
+__device__ __forceinline__ void load_tile(float* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
+    const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
+    const auto put = [&](int r, int d, float x) {
+        if (kT) dst[piece<kRows>(d, r >> 2) + (r & 3)] = x;
+        else dst[r * DP + d] = x;
+    };
+    if (quads_ok<T>(m, D)) {
+        constexpr int kPer = DP / 4, kN = (kRows * kPer + kThreads - 1) / kThreads;
+        constexpr int kBatch = kN < 8 ? kN : 8;  // loads in flight per thread
+#pragma unroll 1
+        for (int i0 = 0; i0 < kN; i0 += kBatch) {
+            float4 x[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / kPer, d = 4 * (idx % kPer);
+                x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < rows_valid && r < kRows && d < D) x[i] = quad_f32(*(const typename Quad<T>::type*)(base + (int64_t)r * m.st + d), T());
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / kPer, d = 4 * (idx % kPer);
+                if (r >= kRows) continue;
+                if (kT) {
+                    put(r, d, x[i].x);
+                    put(r, d + 1, x[i].y);
+                    put(r, d + 2, x[i].z);
+                    put(r, d + 3, x[i].w);
+                } else {
+                    *(float4*)(dst + r * DP + d) = x[i];
+                }
+            }
+        }
+    } else {
+        constexpr int kN = kRows * DP / kThreads, kBatch = kN < 16 ? kN : 16;
+#pragma unroll 1
+        for (int i0 = 0; i0 < kN; i0 += kBatch) {
+            float x[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / DP, d = idx % DP;
+                x[i] = (r < rows_valid && d < D) ? to_f32<T>(base[(int64_t)r * m.st + d]) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int idx = (i0 + i) * kThreads + threadIdx.x;
+                put(idx / DP, idx % DP, x[i]);
+            }
+        }
     }
 }
 
-// C[64x64] = A[64xD] * B[64xD]^T ; thread (ty,tx) owns rows ty+16r, cols tx+16c
-__device__ inline void gemm_nt(float* C, const float* A, const float* B, int DP, int D) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4] = {};
+__device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
+
+// column of the head dim that accumulator column c of lane group tx stands for
+template <int DP>
+__device__ __forceinline__ int col_of(int c, int tx) {
+    return DP >= 64 ? (c >> 2) * 64 + 4 * tx + (c & 3) : (DP / 16) * tx + c;
+}
+
+// s[rows of ty x 4 keys of tx] = A (kR rows per thread, tile width kWA) * B^T (64 keys), both transposed tiles
+template <int DP, int kR, int kWA>
+__device__ __forceinline__ void product_nt(float2 (&s)[kR / 2][4], const float* A, const float* B, int ty, int tx, int D) {
+#pragma unroll
+    for (int i = 0; i < kR / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = make_float2(0.f, 0.f);
+#pragma unroll 4
     for (int d = 0; d < D; ++d) {
-        float a[4], bb[4];
+        float4 x[kR / 4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = A[(ty + 16 * r) * DP + d];
+        for (int i = 0; i < kR / 4; ++i) x[i] = *(const float4*)(A + piece<kWA>(d, ty * (kR / 4) + i));
+        const float4 k = *(const float4*)(B + piece<64>(d, tx));
+        const float2 kk[4] = {dup(k.x), dup(k.y), dup(k.z), dup(k.w)};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) bb[c] = B[(tx + 16 * c) * DP + d];
+        for (int i = 0; i < kR / 4; ++i)
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r], bb[c], acc[r][c]);
+            for (int j = 0; j < 4; ++j) {
+                s[2 * i][j] = __ffma2_rn(make_float2(x[i].x, x[i].y), kk[j], s[2 * i][j]);
+                s[2 * i + 1][j] = __ffma2_rn(make_float2(x[i].z, x[i].w), kk[j], s[2 * i + 1][j]);
+            }
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) C[(ty + 16 * r) * kSP + tx + 16 * c] = acc[r][c];
 }
 
-// acc[64 x D] += P[64 x 64] * V[64 x D] ; thread owns rows ty+16r, cols tx+16c (c < 8)
-__device__ inline void gemm_pv(float (&acc)[4][8], const float* P, const float* V, int DP, int D) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int nc = (D + 15) >> 4;
-    for (int j = 0; j < kBN; ++j) {
-        float p[4];
+// acc[kR rows x DP/16 columns] += P * X: P in shared memory with the contracted index along its rows (row j: 16-byte pieces of
+// rows, permuted by kSwz ? j / 4 : 0), X a transposed tile [d][contracted index]; four contracted indices at a time
+template <int DP, int kR, int kWP, bool kSwz>
+__device__ __forceinline__ void product_px(float2 (&acc)[kR / 2][DP / 16], const float* P, const float* X, int ty, int tx) {
+    constexpr int kNC = DP / 16;
+#pragma unroll 2
+    for (int j4 = 0; j4 < 16; ++j4) {
+        float4 x[kNC];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) p[r] = P[(ty + 16 * r) * kSP + j];
+        for (int c = 0; c < kNC; ++c) x[c] = *(const float4*)(X + piece<64>(col_of<DP>(c, tx), j4));
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if (c < nc) {
-                const float vv = V[j * DP + tx + 16 * c];  // columns beyond D read the zero padding
+        for (int jj = 0; jj < 4; ++jj) {
+            float4 p[kR / 4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) acc[r][c] = fmaf(p[r], vv, acc[r][c]);
+            for (int i = 0; i < kR / 4; ++i) {
+                const int c = ty * (kR / 4) + i;
+                p[i] = *(const float4*)(P + (4 * j4 + jj) * kWP + ((kSwz ? ((c ^ j4) & (kWP / 4 - 1)) : c) << 2));
+            }
+#pragma unroll
+            for (int c = 0; c < kNC; ++c) {
+                const float2 xx = dup(jj == 0 ? x[c].x : jj == 1 ? x[c].y : jj == 2 ? x[c].z : x[c].w);
+#pragma unroll
+                for (int i = 0; i < kR / 4; ++i) {
+                    acc[2 * i][c] = __ffma2_rn(make_float2(p[i].x, p[i].y), xx, acc[2 * i][c]);
+                    acc[2 * i + 1][c] = __ffma2_rn(make_float2(p[i].z, p[i].w), xx, acc[2 * i + 1][c]);
+                }
             }
         }
     }
 }
 
-// acc[64 keys x D] += P[64 q x 64 keys]^T * X[64 q x D]
-__device__ inline void gemm_ptx(float (&acc)[4][8], const float* P, const float* X, int DP, int D) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int nc = (D + 15) >> 4;
-    for (int i = 0; i < kBM; ++i) {
-        float p[4];
+// four keys of kR rows into the [key][row] tile that product_px<kSwz> reads
+template <int kR, int kW>
+__device__ __forceinline__ void put_weights(float* P, const float2 (&p)[kR / 2][4], int ty, int tx) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) p[r] = P[i * kSP + ty + 16 * r];
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if (c < nc) {
-                const float xv = X[i * DP + tx + 16 * c];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) acc[r][c] = fmaf(p[r], xv, acc[r][c]);
-            }
-        }
-    }
+        for (int i = 0; i < kR / 4; ++i)
+            *(float4*)(P + (4 * tx + j) * kW + (((ty * (kR / 4) + i) ^ tx) & (kW / 4 - 1)) * 4) =
+                make_float4(p[2 * i][j].x, p[2 * i][j].y, p[2 * i + 1][j].x, p[2 * i + 1][j].y);
 }
 
-template <typename T>
-__device__ inline void store_acc(const float (&acc)[4][8], float scale, const MatView& m, int b, int h, int row0,
-                                 int rows_valid, int D) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    T* base = (T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh;
+template <typename T, int DP, int kR>
+__device__ __forceinline__ void store_acc(const float2 (&acc)[kR / 2][DP / 16], float scale, const MatView& m, int D, int b, int h, int row0,
+                                          int rows_valid, int ty, int tx) {
+    constexpr int kNC = DP / 16;
+    T* base = (T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int row = ty + 16 * r;
+    for (int r = 0; r < kR; ++r) {
+        const int row = ty * kR + r;
         if (row >= rows_valid) continue;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const int d = tx + 16 * c;
-            if (d < D) base[(int64_t)(row0 + row) * m.st + d] = from_f32<T>(acc[r][c] * scale);
+        for (int c = 0; c < kNC; ++c) {
+            const int d = col_of<DP>(c, tx);
+            const float x = (r & 1) ? acc[r >> 1][c].y : acc[r >> 1][c].x;
+            if (d < D) base[(int64_t)row * m.st + d] = from_f32<T>(x * scale);
         }
     }
 }
 
 // sigmoid pieces with full relative accuracy on both sides: beta = sigmoid(s), r = 1 - beta
-__device__ inline void sigmoid_pair(float s, float& beta, float& r) {
+__device__ __forceinline__ void sigmoid_pair(float s, float& beta, float& r) {
     const float e = expf(-fabsf(s));
     const float inv = 1.0f / (1.0f + e);
     const float big = inv, small = e * inv;
@@ -119,52 +209,33 @@ __device__ inline void sigmoid_pair(float s, float& beta, float& r) {
     r = s >= 0.f ? small : big;
 }
 
-// The 4 threads of a row (consecutive lanes) each own 16 consecutive keys of the 64-key tile.
-struct RowPart {
-    int row, part, lane_base;
-};
-__device__ inline RowPart row_part() {
-    RowPart rp;
-    rp.row = threadIdx.x >> 2;
-    rp.part = threadIdx.x & 3;
-    rp.lane_base = (threadIdx.x & 31) & ~3;
-    return rp;
-}
-// product / sum over the 4 threads of a row, identical bits on all of them
-__device__ inline float quad_prod(float x) {
-    x *= __shfl_xor_sync(0xffffffffu, x, 1);
-    x *= __shfl_xor_sync(0xffffffffu, x, 2);
+// A row's 64 keys lie in 16 consecutive lanes, four each.  Inclusive product (sum) over this lane and those to its right (left).
+__device__ __forceinline__ float right_prod(float x, int tx) {
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+        const float y = __shfl_down_sync(0xffffffffu, x, off, 16);
+        x *= tx + off < 16 ? y : 1.f;
+    }
     return x;
 }
-__device__ inline float quad_sum(float x) {
-    x += __shfl_xor_sync(0xffffffffu, x, 1);
-    x += __shfl_xor_sync(0xffffffffu, x, 2);
+__device__ __forceinline__ float right_sum(float x, int tx) {
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+        const float y = __shfl_down_sync(0xffffffffu, x, off, 16);
+        x += tx + off < 16 ? y : 0.f;
+    }
     return x;
 }
-// product (sum) of the values held by the parts to the right (left) of this one
-__device__ inline float quad_right_prod(float x, int part) {
-    const float a = __shfl_down_sync(0xffffffffu, x, 1);
-    const float b = __shfl_down_sync(0xffffffffu, x, 2);
-    const float c = __shfl_down_sync(0xffffffffu, x, 3);
-    return (part < 3 ? a : 1.f) * (part < 2 ? b : 1.f) * (part < 1 ? c : 1.f);
-}
-__device__ inline float quad_right_sum(float x, int part) {
-    const float a = __shfl_down_sync(0xffffffffu, x, 1);
-    const float b = __shfl_down_sync(0xffffffffu, x, 2);
-    const float c = __shfl_down_sync(0xffffffffu, x, 3);
-    return (part < 3 ? a : 0.f) + (part < 2 ? b : 0.f) + (part < 1 ? c : 0.f);
-}
-__device__ inline float quad_left_sum(float x, int part) {
-    const float a = __shfl_up_sync(0xffffffffu, x, 1);
-    const float b = __shfl_up_sync(0xffffffffu, x, 2);
-    const float c = __shfl_up_sync(0xffffffffu, x, 3);
-    return (part > 0 ? a : 0.f) + (part > 1 ? b : 0.f) + (part > 2 ? c : 0.f);
+__device__ __forceinline__ float left_sum(float x, int tx) {
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, x, off, 16);
+        x += tx >= off ? y : 0.f;
+    }
+    return x;
 }
 
-// key j (index inside the sequence) visible from query i?
-__device__ inline bool visible(int i, int j, int len, int attend_current) {
-    return j < len && (attend_current ? j <= i : j < i);
-}
+__device__ __forceinline__ float& pick(float2& v, int odd) { return odd ? v.y : v.x; }
 
 struct ItemCtx {
     int seq, qt, b, start, len, slot_base;
@@ -177,299 +248,347 @@ __device__ inline bool fetch_item(const KArgs& a, int item, ItemCtx& c) {
     return true;
 }
 
+__device__ __forceinline__ int64_t linear_thread() {
+    return (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kThreads + threadIdx.x;
+}
+__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads; }
+
 // ------------------------------------------------------------------------------------------ forward
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) simt_fwd_kernel(const KArgs a) {
-    extern __shared__ float smem[];
-    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
-        const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-        zero_tail_rows<T>(a, a.hdr->covered_end, block * kThreads + threadIdx.x, (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads);
-    }
+// kR rows per thread: blocks of 8 * kR query rows.  64-row blocks need fewer loads per product, 32-row ones spread a small
+// problem over twice as many SMs (the host chooses).
+template <typename T, int DP, int kR>
+__global__ void __launch_bounds__(kThreads, DP > 64 ? 2 : 3) simt_fwd_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kBM = 8 * kR;
+    extern __shared__ __align__(16) float smem[];
+    float* Qt = smem;             // [DP][kBM]
+    float* Kt = Qt + DP * kBM;    // [DP][64]
+    float* Vt = Kt + DP * kBN;    // [DP][64]
+    float* Ps = Vt + DP * kBN;    // [64 keys][kBM]
+    pdl_wait();
+    pdl_launch_dependents();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_rows<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
     if (!fetch_item(a, blockIdx.x, c)) return;
-    const int h = blockIdx.y;
-    const int qb = 2 * c.qt + blockIdx.z;  // 64-row block inside the sequence
-    const int row0 = qb * kBM;
+    const int h = blockIdx.y, D = a.head_dim;
+    const int sub = blockIdx.z * kBM;  // first row inside the 128-row tile
+    const int row0 = c.qt * kTileQ + sub;
     if (row0 >= c.len) return;
-    // row pitch: odd (no bank conflicts) and with zero padding so that column reads up to 16*ceil(D/16) stay inside
-    const int D = a.head_dim, DPP = (D | 1) + 16;
-    float* Qs = smem;
-    float* Ks = Qs + kBM * DPP;
-    float* Vs = Ks + kBN * DPP;
-    float* Ss = Vs + kBN * DPP;
-    for (int idx = threadIdx.x; idx < 3 * kBM * DPP; idx += kThreads) smem[idx] = 0.f;
-    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int rows_valid = min(kBM, c.len - row0);
-    load_rows<T>(Qs, DPP, D, a.q, c.b, h, c.start + row0, rows_valid);
+    load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+    float W[kR];
+    float2 o[kR / 2][DP / 16];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) W[r] = 1.f;
+#pragma unroll
+    for (int i = 0; i < kR / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < DP / 16; ++j) o[i][j] = make_float2(0.f, 0.f);
+    float* cw = a.carry_w ? a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ + sub + ty * kR : nullptr;
+    const int last = (min(row0 + kBM, c.len) - 1) / kBN;
+    // key tiles of the 128-key diagonal tile that lie right of these rows: a tensor-core backward may follow, and it reads the
+    // carry of every quarter of its tile
+    if (cw && tx == 0)
+        for (int kh = last + 1; kh <= 2 * c.qt + 1 && kh * kBN < c.len; ++kh)
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                cw[carry_slot(c.slot_base, c.qt, kh) * kTileQ + r] = 1.f;
+                cw[carry_slot32(c.slot_base, c.qt, 2 * kh) * kTileQ + r] = 1.f;
+            }
 
-    const RowPart rp = row_part();
-    const int qi = row0 + rp.row;
-    float W = 1.f;
-    float acc[4][8] = {};
-    float* cw = a.carry_w ? a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ : nullptr;
-    const int rloc = (qb & 1) * kBM + rp.row;  // row inside the 128-row tile
-
-    for (int kh = qb; kh >= 0; --kh) {
+    for (int kh = last; kh >= 0; --kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_rows<T>(Ks, DPP, D, a.k, c.b, h, c.start + key0, keys_valid);
-        load_rows<T>(Vs, DPP, D, a.v, c.b, h, c.start + key0, keys_valid);
+        load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
         __syncthreads();
-        gemm_nt(Ss, Qs, Ks, DPP, D);
-        __syncthreads();
-        // element-wise part: 4 threads per row, 16 keys each
-        if (cw && rp.part == 0) cw[carry_slot(c.slot_base, c.qt, kh) * kTileQ + rloc] = W;  // right edge of the half
-        float beta[16], r[16];
-        float prod = 1.f;
+        float2 s[kR / 2][4];
+        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
+        const bool edge = key0 + kBN > row0 || keys_valid < kBN;  // some pair of the tile is not visible
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-            const int j = rp.part * 16 + jj;
-            const float s = Ss[rp.row * kSP + j] * a.inv_temp;
-            float bt, rr;
-            sigmoid_pair(s, bt, rr);
-            const bool vis = visible(qi, key0 + j, c.len, a.attend_current);
-            beta[jj] = vis ? bt : 0.f;
-            r[jj] = vis ? rr : 1.f;
-            prod *= r[jj];
-        }
-        const float win = W * quad_right_prod(prod, rp.part);
-        // the carry in the middle of the half as well: a tensor-core backward may follow this forward (the two are
-        // chosen independently, by the alignment of their own operands), and it enters every 32-key quarter directly
-        if (cw && rp.part == 1) cw[carry_slot32(c.slot_base, c.qt, 2 * kh) * kTileQ + rloc] = win;
-        float run = win;
+        for (int r = 0; r < kR; ++r) {
+            const int lim = edge ? min(keys_valid, row0 + ty * kR + r + a.attend_current - key0) : kBN;  // keys < lim are visible
+            float beta[4], om[4];
 #pragma unroll
-        for (int jj = 15; jj >= 0; --jj) {
-            Ss[rp.row * kSP + rp.part * 16 + jj] = beta[jj] * run;
-            run *= r[jj];
+            for (int j = 0; j < 4; ++j) {
+                sigmoid_pair(pick(s[r >> 1][j], r & 1) * a.inv_temp, beta[j], om[j]);
+                if (4 * tx + j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
+            }
+            const float incl = right_prod((om[0] * om[1]) * (om[2] * om[3]), tx);
+            float right = __shfl_down_sync(0xffffffffu, incl, 1, 16);
+            if (tx == 15) right = 1.f;
+            float run = W[r] * right;
+            if (cw) {  // W at the right edges of the two 32-key quarters
+                if (tx == 15) cw[carry_slot(c.slot_base, c.qt, kh) * kTileQ + r] = run;
+                if (tx == 7) cw[carry_slot32(c.slot_base, c.qt, 2 * kh) * kTileQ + r] = run;
+            }
+            W[r] *= __shfl_sync(0xffffffffu, incl, 0, 16);
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                pick(s[r >> 1][j], r & 1) = beta[j] * run;
+                run *= om[j];
+            }
         }
-        W *= quad_prod(prod);
+        put_weights<kR, kBM>(Ps, s, ty, tx);
         __syncthreads();
-        gemm_pv(acc, Ss, Vs, DPP, D);
+        product_px<DP, kR, kBM, true>(o, Ps, Vt, ty, tx);
     }
-    store_acc<T>(acc, 1.f, a.o, c.b, h, c.start + row0, rows_valid, D);
-    if (rp.part == 0 && rp.row < rows_valid) {
-        const int64_t t = c.start + qi;
-        ((T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + t * a.rem.st] = from_f32<T>(W);
-        ((float*)a.nla.ptr)[(int64_t)c.b * a.nla.sb + (int64_t)h * a.nla.sh + t * a.nla.st] = log2f(W);
+    store_acc<T, DP, kR>(o, 1.f, a.o, D, c.b, h, c.start + row0, rows_valid, ty, tx);
+    if (tx == 0) {
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            if (ty * kR + r >= rows_valid) continue;
+            const int64_t t = c.start + row0 + ty * kR + r;
+            ((T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + t * a.rem.st] = from_f32<T>(W[r]);
+            ((float*)a.nla.ptr)[(int64_t)c.b * a.nla.sb + (int64_t)h * a.nla.sh + t * a.nla.st] = log2f(W[r]);
+        }
     }
 }
 
 // ------------------------------------------------------------------------------------------ backward: dq
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) simt_bwd_dq_kernel(const KArgs a) {
-    extern __shared__ float smem[];
-    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
-        const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-        zero_tail_grads<T>(a, a.hdr->covered_end, block * kThreads + threadIdx.x, (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads);
-    }
+template <typename T, int DP, int kR>
+__global__ void __launch_bounds__(kThreads, 2) simt_bwd_dq_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kBM = 8 * kR;
+    extern __shared__ __align__(16) float smem[];
+    float* Qt = smem;
+    float* Gt = Qt + DP * kBM;  // dO
+    float* Kt = Gt + DP * kBM;
+    float* Vt = Kt + DP * kBN;
+    float* Ss = Vt + DP * kBN;  // dS, [64 keys][kBM]
+    pdl_wait();
+    pdl_launch_dependents();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
     if (!fetch_item(a, blockIdx.x, c)) return;
-    const int h = blockIdx.y;
-    const int qb = 2 * c.qt + blockIdx.z;
-    const int row0 = qb * kBM;
+    const int h = blockIdx.y, D = a.head_dim;
+    const int sub = blockIdx.z * kBM;
+    const int row0 = c.qt * kTileQ + sub;
     if (row0 >= c.len) return;
-    const int D = a.head_dim, DPP = (D | 1) + 16;
-    float* Qs = smem;
-    float* Gs = Qs + kBM * DPP;  // dO
-    float* Ks = Gs + kBM * DPP;
-    float* Vs = Ks + kBN * DPP;
-    float* Ss = Vs + kBN * DPP;
-    float* Ps = Ss + kBM * kSP;
-    for (int idx = threadIdx.x; idx < 4 * kBM * DPP; idx += kThreads) smem[idx] = 0.f;
-    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int rows_valid = min(kBM, c.len - row0);
-    load_rows<T>(Qs, DPP, D, a.q, c.b, h, c.start + row0, rows_valid);
-    load_rows<T>(Gs, DPP, D, a.d_o, c.b, h, c.start + row0, rows_valid);
+    load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+    load_tile<T, DP, kBM, true>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+    float drem[kR], prefix[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+        const int64_t t = c.start + row0 + ty * kR + r;
+        drem[r] = ty * kR + r < rows_valid ? to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + t * a.d_rem.st]) : 0.f;
+        prefix[r] = 0.f;  // sum of g over all keys left of the current tile
+    }
+    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ + sub + ty * kR;
+    float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ + sub + ty * kR;
+    float2 o[kR / 2][DP / 16];
+#pragma unroll
+    for (int i = 0; i < kR / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < DP / 16; ++j) o[i][j] = make_float2(0.f, 0.f);
+    const int last = (min(row0 + kBM, c.len) - 1) / kBN;
 
-    const RowPart rp = row_part();
-    const int qi = row0 + rp.row;
-    const bool row_ok = rp.row < rows_valid;
-    float drem = 0.f;
-    if (row_ok)
-        drem = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh +
-                                                 (int64_t)(c.start + qi) * a.d_rem.st]);
-    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
-    float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    const int rloc = (qb & 1) * kBM + rp.row;
-    float cprefix = 0.f;  // sum of g over all keys left of the current tile
-    float acc[4][8] = {};
-
-    for (int kh = 0; kh <= qb; ++kh) {
+    for (int kh = 0; kh <= last; ++kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_rows<T>(Ks, DPP, D, a.k, c.b, h, c.start + key0, keys_valid);
-        load_rows<T>(Vs, DPP, D, a.v, c.b, h, c.start + key0, keys_valid);
-        __syncthreads();
-        gemm_nt(Ss, Qs, Ks, DPP, D);
-        gemm_nt(Ps, Gs, Vs, DPP, D);
-        __syncthreads();
-        const int64_t slot = carry_slot(c.slot_base, c.qt, kh) * kTileQ + rloc;
-        const float W = row_ok ? cw[slot] : 0.f;
-        float beta[16], g[16];
-        float prod = 1.f;
+        load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
+        const int64_t slot = carry_slot(c.slot_base, c.qt, kh) * kTileQ;
+        float Win[kR];
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-            const int j = rp.part * 16 + jj;
-            float bt, rr;
-            sigmoid_pair(Ss[rp.row * kSP + j] * a.inv_temp, bt, rr);
-            const bool vis = row_ok && visible(qi, key0 + j, c.len, a.attend_current);
-            beta[jj] = vis ? bt : 0.f;
-            g[jj] = vis ? rr : 1.f;  // holds r until the suffix pass below
-            prod *= g[jj];
-        }
-        float run = W * quad_right_prod(prod, rp.part);
-        float gsum = 0.f;
-#pragma unroll
-        for (int jj = 15; jj >= 0; --jj) {
-            const float rr = g[jj];
-            const float p = beta[jj] * run;
-            g[jj] = p * (Ps[rp.row * kSP + rp.part * 16 + jj] - drem);
-            gsum += g[jj];
-            run *= rr;
-        }
-        float cin = cprefix + quad_left_sum(gsum, rp.part);
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-            cin += g[jj];
-            Ss[rp.row * kSP + rp.part * 16 + jj] = g[jj] - beta[jj] * cin;
-        }
-        cprefix += quad_sum(gsum);
-        if (rp.part == 0 && row_ok) cc[slot] = cprefix;  // prefix including this tile
+        for (int r = 0; r < kR; ++r) Win[r] = ty * kR + r < rows_valid ? cw[slot + r] : 0.f;
         __syncthreads();
-        gemm_pv(acc, Ss, Ks, DPP, D);
+        float2 s[kR / 2][4], dp[kR / 2][4];
+        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
+        product_nt<DP, kR, kBM>(dp, Gt, Vt, ty, tx, D);
+        const bool edge = key0 + kBN > row0 || keys_valid < kBN;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const int lim = edge ? min(keys_valid, row0 + ty * kR + r + a.attend_current - key0) : kBN;
+            float beta[4], om[4], g[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                sigmoid_pair(pick(s[r >> 1][j], r & 1) * a.inv_temp, beta[j], om[j]);
+                if (4 * tx + j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
+            }
+            const float incl = right_prod((om[0] * om[1]) * (om[2] * om[3]), tx);
+            float right = __shfl_down_sync(0xffffffffu, incl, 1, 16);
+            if (tx == 15) right = 1.f;
+            float run = Win[r] * right;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                g[j] = beta[j] * run * (pick(dp[r >> 1][j], r & 1) - drem[r]);
+                run *= om[j];
+            }
+            const float mine = (g[0] + g[1]) + (g[2] + g[3]);
+            const float upto = left_sum(mine, tx);  // through this lane's keys
+            float cin = prefix[r] + (upto - mine);
+            prefix[r] += __shfl_sync(0xffffffffu, upto, 15, 16);
+            if (tx == 15 && ty * kR + r < rows_valid) cc[slot + r] = prefix[r];  // prefix including this tile
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                cin += g[j];
+                pick(s[r >> 1][j], r & 1) = g[j] - beta[j] * cin;
+            }
+        }
+        put_weights<kR, kBM>(Ss, s, ty, tx);
+        __syncthreads();
+        product_px<DP, kR, kBM, true>(o, Ss, Kt, ty, tx);
     }
-    store_acc<T>(acc, a.inv_temp, a.dq, c.b, h, c.start + row0, rows_valid, D);
+    store_acc<T, DP, kR>(o, a.inv_temp, a.dq, D, c.b, h, c.start + row0, rows_valid, ty, tx);
 }
 
 // ------------------------------------------------------------------------------------------ backward: dk, dv
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) simt_bwd_dkdv_kernel(const KArgs a) {
-    extern __shared__ float smem[];
+template <typename T, int DP>
+__global__ void __launch_bounds__(kThreads, 2) simt_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kR = 8, kBM = 64;
+    extern __shared__ __align__(16) float smem[];
+    float* Qt = smem;
+    float* Gt = Qt + DP * kBM;
+    float* Kt = Gt + DP * kBM;
+    float* Vt = Kt + DP * kBN;
+    float* Ps = Vt + DP * kBN;   // P, [64 queries][64 keys]
+    float* Ss = Ps + kBM * kBN;  // dS
+    pdl_wait();
+    pdl_launch_dependents();
     ItemCtx c;
     const int n_items = a.hdr->n_items;
     if ((int)blockIdx.x >= n_items) return;
     // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
     if (!fetch_item(a, n_items - 1 - (int)blockIdx.x, c)) return;
-    const int h = blockIdx.y;
+    const int h = blockIdx.y, D = a.head_dim;
     const int kh = 2 * c.qt + blockIdx.z;
     const int key0 = kh * kBN;
     if (key0 >= c.len) return;
-    const int D = a.head_dim, DPP = (D | 1) + 16;
-    float* Qs = smem;
-    float* Gs = Qs + kBM * DPP;
-    float* Ks = Gs + kBM * DPP;
-    float* Vs = Ks + kBN * DPP;
-    float* Ss = Vs + kBN * DPP;
-    float* Ps = Ss + kBM * kSP;
-    for (int idx = threadIdx.x; idx < 4 * kBM * DPP; idx += kThreads) smem[idx] = 0.f;
-    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int keys_valid = min(kBN, c.len - key0);
-    load_rows<T>(Ks, DPP, D, a.k, c.b, h, c.start + key0, keys_valid);
-    load_rows<T>(Vs, DPP, D, a.v, c.b, h, c.start + key0, keys_valid);
-
-    const RowPart rp = row_part();
+    load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+    load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    float acc_k[4][8] = {}, acc_v[4][8] = {};
+    float2 ok[kR / 2][DP / 16], ov[kR / 2][DP / 16];
+#pragma unroll
+    for (int i = 0; i < kR / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < DP / 16; ++j) ok[i][j] = ov[i][j] = make_float2(0.f, 0.f);
     const int n_qb = (c.len + kBM - 1) / kBM;
 
     for (int qb = kh; qb < n_qb; ++qb) {
         const int row0 = qb * kBM;
         const int rows_valid = min(kBM, c.len - row0);
         __syncthreads();
-        load_rows<T>(Qs, DPP, D, a.q, c.b, h, c.start + row0, rows_valid);
-        load_rows<T>(Gs, DPP, D, a.d_o, c.b, h, c.start + row0, rows_valid);
-        __syncthreads();
-        gemm_nt(Ss, Qs, Ks, DPP, D);
-        gemm_nt(Ps, Gs, Vs, DPP, D);
-        __syncthreads();
-        const int qi = row0 + rp.row;
-        const bool row_ok = rp.row < rows_valid;
-        float drem = 0.f, W = 0.f, cright = 0.f;
-        if (row_ok) {
-            drem = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh +
-                                                     (int64_t)(c.start + qi) * a.d_rem.st]);
-            const int64_t slot = carry_slot(c.slot_base, qb >> 1, kh) * kTileQ + (qb & 1) * kBM + rp.row;
-            W = cw[slot];
-            cright = cc[slot];
-        }
-        float beta[16], g[16];
-        float prod = 1.f;
+        load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<T, DP, kBM, true>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        const int64_t slot = carry_slot(c.slot_base, qb >> 1, kh) * kTileQ + (qb & 1) * kBM + ty * kR;
+        float Win[kR], cright[kR], drem[kR];
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-            const int j = rp.part * 16 + jj;
-            float bt, rr;
-            sigmoid_pair(Ss[rp.row * kSP + j] * a.inv_temp, bt, rr);
-            const bool vis = row_ok && visible(qi, key0 + j, c.len, a.attend_current);
-            beta[jj] = vis ? bt : 0.f;
-            g[jj] = vis ? rr : 1.f;
-            prod *= g[jj];
-        }
-        float run = W * quad_right_prod(prod, rp.part);
-        float gsum = 0.f;
-        float pv[16];
-#pragma unroll
-        for (int jj = 15; jj >= 0; --jj) {
-            const float rr = g[jj];
-            pv[jj] = beta[jj] * run;
-            g[jj] = pv[jj] * (Ps[rp.row * kSP + rp.part * 16 + jj] - drem);
-            gsum += g[jj];
-            run *= rr;
-        }
-        // inclusive prefix at key j = (prefix through the tile's right edge) - (sum of g right of j)
-        float right = quad_right_sum(gsum, rp.part);
-#pragma unroll
-        for (int jj = 15; jj >= 0; --jj) {
-            const float cin = cright - right;
-            Ss[rp.row * kSP + rp.part * 16 + jj] = pv[jj];
-            Ps[rp.row * kSP + rp.part * 16 + jj] = g[jj] - beta[jj] * cin;
-            right += g[jj];
+        for (int r = 0; r < kR; ++r) {
+            const bool row_ok = ty * kR + r < rows_valid;
+            const int64_t t = c.start + row0 + ty * kR + r;
+            Win[r] = row_ok ? cw[slot + r] : 0.f;
+            cright[r] = row_ok ? cc[slot + r] : 0.f;
+            drem[r] = row_ok ? to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + t * a.d_rem.st]) : 0.f;
         }
         __syncthreads();
-        gemm_ptx(acc_v, Ss, Gs, DPP, D);
-        gemm_ptx(acc_k, Ps, Qs, DPP, D);
+        float2 s[kR / 2][4], dp[kR / 2][4];
+        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
+        product_nt<DP, kR, kBM>(dp, Gt, Vt, ty, tx, D);
+        const bool edge = qb == kh || keys_valid < kBN;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const int lim = edge ? min(keys_valid, row0 + ty * kR + r + a.attend_current - key0) : kBN;
+            float beta[4], om[4], g[4], p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                sigmoid_pair(pick(s[r >> 1][j], r & 1) * a.inv_temp, beta[j], om[j]);
+                if (4 * tx + j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
+            }
+            const float incl = right_prod((om[0] * om[1]) * (om[2] * om[3]), tx);
+            float right = __shfl_down_sync(0xffffffffu, incl, 1, 16);
+            if (tx == 15) right = 1.f;
+            float run = Win[r] * right;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                p[j] = beta[j] * run;
+                g[j] = p[j] * (pick(dp[r >> 1][j], r & 1) - drem[r]);
+                run *= om[j];
+            }
+            const float from = right_sum((g[0] + g[1]) + (g[2] + g[3]), tx);
+            float behind = __shfl_down_sync(0xffffffffu, from, 1, 16);  // sum of g right of this lane's keys
+            if (tx == 15) behind = 0.f;
+            // inclusive prefix at key j = (prefix through the tile's right edge) - (sum of g right of j)
+            float cin = cright[r] - behind;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                pick(s[r >> 1][j], r & 1) = p[j];
+                pick(dp[r >> 1][j], r & 1) = g[j] - beta[j] * cin;
+                cin -= g[j];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const int q = ty * kR + r;
+            *(float4*)(Ps + q * kBN + 4 * tx) = make_float4(pick(s[r >> 1][0], r & 1), pick(s[r >> 1][1], r & 1), pick(s[r >> 1][2], r & 1), pick(s[r >> 1][3], r & 1));
+            *(float4*)(Ss + q * kBN + 4 * tx) = make_float4(pick(dp[r >> 1][0], r & 1), pick(dp[r >> 1][1], r & 1), pick(dp[r >> 1][2], r & 1), pick(dp[r >> 1][3], r & 1));
+        }
+        __syncthreads();
+        product_px<DP, kR, kBN, false>(ov, Ps, Gt, ty, tx);
+        product_px<DP, kR, kBN, false>(ok, Ss, Qt, ty, tx);
     }
-    store_acc<T>(acc_k, a.inv_temp, a.dk, c.b, h, c.start + key0, keys_valid, D);
-    store_acc<T>(acc_v, 1.f, a.dv, c.b, h, c.start + key0, keys_valid, D);
+    store_acc<T, DP, kR>(ok, a.inv_temp, a.dk, D, c.b, h, c.start + key0, keys_valid, ty, tx);
+    store_acc<T, DP, kR>(ov, 1.f, a.dv, D, c.b, h, c.start + key0, keys_valid, ty, tx);
 }
 
-size_t simt_smem_bytes(int D, bool bwd) {
-    const int DPP = (D | 1) + 16;
-    return sizeof(float) * (size_t)((bwd ? 4 : 3) * kBM * DPP + (bwd ? 2 : 1) * kBM * kSP);
+// Blocks of 32 query rows where 64-row blocks (`heads * items * 2`, an upper bound) would leave SMs without any
+bool small_problem(const WsLayout& L, const KArgs& a) { return (int64_t)L.max_items * a.heads * 2 <= 2 * 148; }
+
+template <typename T, int DP, int kR>
+int launch_fwd_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    const int smem = (int)sizeof(float) * (DP * 8 * kR + 2 * DP * kBN + kBN * 8 * kR);
+    const auto kernel = simt_fwd_kernel<T, DP, kR>;
+    const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
+    if (e != 0) return e;
+    return launch_kernel(kernel, dim3(L.max_items, a.heads, 16 / kR), dim3(kThreads), smem, st, a);
+}
+template <typename T, int DP, int kR>
+int launch_dq_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    const int smem = (int)sizeof(float) * (2 * DP * 8 * kR + 2 * DP * kBN + kBN * 8 * kR);
+    const auto kernel = simt_bwd_dq_kernel<T, DP, kR>;
+    const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
+    if (e != 0) return e;
+    return launch_kernel(kernel, dim3(L.max_items, a.heads, 16 / kR), dim3(kThreads), smem, st, a);
+}
+template <typename T, int DP>
+int launch_dkdv_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    const int smem = (int)sizeof(float) * (4 * DP * kBN + 2 * kBN * kBN);
+    const auto kernel = simt_bwd_dkdv_kernel<T, DP>;
+    const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
+    if (e != 0) return e;
+    return launch_kernel(kernel, dim3(L.max_items, a.heads, 2), dim3(kThreads), smem, st, a);
+}
+
+template <typename T, int DP>
+int launch_fwd_d(const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    return small_problem(L, a) ? launch_fwd_k<T, DP, 4>(L, a, st) : launch_fwd_k<T, DP, 8>(L, a, st);
+}
+template <typename T, int DP>
+int launch_bwd_d(const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
+    if (phases != SBATTN_BWD_DKDV) {
+        const int e = small_problem(L, a) ? launch_dq_k<T, DP, 4>(L, a, st) : launch_dq_k<T, DP, 8>(L, a, st);
+        if (e != 0) return e;
+    }
+    return phases != SBATTN_BWD_DQ ? launch_dkdv_k<T, DP>(L, a, st) : 0;
 }
 
 template <typename T>
 int launch_fwd_t(const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    const size_t smem = simt_smem_bytes(a.head_dim, false);
-    cudaError_t e = cudaFuncSetAttribute(simt_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    dim3 grid(L.max_items, a.heads, 2);
-    simt_fwd_kernel<T><<<grid, kThreads, smem, st>>>(a);
-    count_launch();
-    return (int)cudaGetLastError();
+    if (a.head_dim > 64) return launch_fwd_d<T, 128>(L, a, st);
+    if (a.head_dim > 32) return launch_fwd_d<T, 64>(L, a, st);
+    return a.head_dim > 16 ? launch_fwd_d<T, 32>(L, a, st) : launch_fwd_d<T, 16>(L, a, st);
 }
-
 template <typename T>
 int launch_bwd_t(const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
-    const size_t smem = simt_smem_bytes(a.head_dim, true);
-    cudaError_t e = cudaFuncSetAttribute(simt_bwd_dq_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(simt_bwd_dkdv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    dim3 grid(L.max_items, a.heads, 2);
-    if (phases != SBATTN_BWD_DKDV) {
-        simt_bwd_dq_kernel<T><<<grid, kThreads, smem, st>>>(a);
-        count_launch();
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    if (phases != SBATTN_BWD_DQ) {
-        simt_bwd_dkdv_kernel<T><<<grid, kThreads, smem, st>>>(a);
-        count_launch();
-    }
-    return (int)cudaGetLastError();
+    if (a.head_dim > 64) return launch_bwd_d<T, 128>(L, a, phases, st);
+    if (a.head_dim > 32) return launch_bwd_d<T, 64>(L, a, phases, st);
+    return a.head_dim > 16 ? launch_bwd_d<T, 32>(L, a, phases, st) : launch_bwd_d<T, 16>(L, a, phases, st);
 }
 
 }  // namespace
