@@ -14,11 +14,14 @@
 //     atomic or lock on the data (the reference uses a spin lock per key tile, sb_varlen_bwd.py:11-53).
 //
 // What bounds them is the FMA pipes (128 per clock and SM), so everything else is kept out of their way: a thread owns a
-// register tile of 8 (or 4) rows x 4 columns of every product, operands come from shared memory in 16-byte pieces (3 loads per 16
-// packed fp32x2 multiply-adds), scores never leave the registers (the 16 lanes of a row exchange their products and sums by
-// shuffles), and only the weights pass through shared memory on their way into the second product.  With one 4 x 4 tile per
-// thread, scalar shared loads and the scores in shared memory, 4096 float32 tokens (8 heads, head dim 64) took 0.64 / 0.82 /
-// 1.03 ms in the three kernels, 7 TFLOP/s.
+// register tile of 4 rows x 4 columns of every product in packed fp32x2 multiply-adds, operands come from shared memory in 16-byte
+// pieces, scores never leave the registers (the 16 lanes of a row exchange their products and sums by shuffles), and only
+// the weights pass through shared memory on their way into the second product.  us per kernel, forward / dq / dk,dv, with scalar
+// loads and the scores in shared memory -> now (tiles of 8 x 4 need a quarter fewer instructions but leave 8 to 12 warps per SM,
+// too few to hide their latencies: 255 / 378 / 388 in the first line):
+//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:   642 / 825 / 1028 -> 201 / 297 / 363
+//   4 x 8 heads x 500 tokens, bf16, head dim 50:                186 / 235 / 280  ->  76 / 106 / 119
+//   4 heads, 512 float32 tokens, head dim 64:                    53 / 72 / 82    ->  27 / 37 / 31
 #include "sb_common.cuh"
 
 namespace sb {
@@ -26,7 +29,6 @@ namespace sb {
 namespace {
 
 constexpr int kBN = 64;         // keys per tile (and query rows per tile of the dk/dv kernel)
-constexpr int kThreads = 128;   // 8 row groups x 16 column groups
 
 // An operand tile in shared memory, transposed: [DP][kW] floats, element (row, d) in row d of the tile.  The 16-byte pieces of
 // a row are permuted by a function of d so that neither the transposing stores (lanes along d) nor the loads (lanes along the
@@ -37,75 +39,70 @@ __device__ __forceinline__ int piece(int d, int c) {
     return d * kW + (((c ^ d ^ (d >> 2)) & (kW / 4 - 1)) << 2);
 }
 
-template <typename T> struct Quad;  // four consecutive elements as they lie in global memory
-template <> struct Quad<float> { typedef float4 type; };
-template <> struct Quad<__nv_bfloat16> { typedef uint2 type; };
-template <> struct Quad<__half> { typedef uint2 type; };
-__device__ __forceinline__ float4 quad_f32(const float4& x, float) { return x; }
-__device__ __forceinline__ float4 quad_f32(const uint2& x, __nv_bfloat16) {
-    return make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
-}
-__device__ __forceinline__ float4 quad_f32(const uint2& x, __half) {
-    const float2 a = __half22float2(*(const __half2*)&x.x), b = __half22float2(*(const __half2*)&x.y);
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-template <typename T>
-__device__ __forceinline__ bool quads_ok(const MatView& m, int D) {
-    return (D & 3) == 0 && ((uintptr_t)m.ptr % (4 * sizeof(T))) == 0 && (m.st & 3) == 0 && (m.sh & 3) == 0 && (m.sb & 3) == 0;
-}
-
-// kRows rows of a [.., T, D] tensor into shared memory as float32, zeros behind the valid rows and columns.
-// kT: transposed tile (see piece); otherwise rows of DP floats.
-template <typename T, int DP, int kRows, bool kT>
-__device__ __forceinline__ void load_tile(float* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
-    const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
-    const auto put = [&](int r, int d, float x) {
-        if (kT) dst[piece<kRows>(d, r >> 2) + (r & 3)] = x;
-        else dst[r * DP + d] = x;
-    };
-    if (quads_ok<T>(m, D)) {
-        constexpr int kPer = DP / 4, kN = (kRows * kPer + kThreads - 1) / kThreads;
-        constexpr int kBatch = kN < 8 ? kN : 8;  // loads in flight per thread
-#pragma unroll 1
-        for (int i0 = 0; i0 < kN; i0 += kBatch) {
-            float4 x[kBatch];
-#pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / kPer, d = 4 * (idx % kPer);
-                x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (r < rows_valid && r < kRows && d < D) x[i] = quad_f32(*(const typename Quad<T>::type*)(base + (int64_t)r * m.st + d), T());
-            }
-#pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / kPer, d = 4 * (idx % kPer);
-                if (r >= kRows) continue;
-                if (kT) {
-                    put(r, d, x[i].x);
-                    put(r, d + 1, x[i].y);
-                    put(r, d + 2, x[i].z);
-                    put(r, d + 3, x[i].w);
-                } else {
-                    *(float4*)(dst + r * DP + d) = x[i];
-                }
-            }
+// kU consecutive elements as float32
+template <typename T, int kU>
+__device__ __forceinline__ void load_unit(const T* src, float (&x)[kU]) {
+    if constexpr (sizeof(T) == 4) {
+        if constexpr (kU == 4) {
+            const float4 v = *(const float4*)src;
+            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        } else if constexpr (kU == 2) {
+            const float2 v = *(const float2*)src;
+            x[0] = v.x; x[1] = v.y;
+        } else {
+            x[0] = to_f32<T>(*src);
         }
     } else {
-        constexpr int kN = kRows * DP / kThreads, kBatch = kN < 16 ? kN : 16;
+        T v[kU];
+        if constexpr (kU == 4) *(uint2*)v = *(const uint2*)src;
+        else if constexpr (kU == 2) *(uint32_t*)v = *(const uint32_t*)src;
+        else v[0] = *src;
+#pragma unroll
+        for (int i = 0; i < kU; ++i) x[i] = to_f32<T>(v[i]);
+    }
+}
+// whether rows can be read in units of u elements
+template <typename T>
+__device__ __forceinline__ bool units_ok(const MatView& m, int D, int u) {
+    return ((D | m.st | m.sh | m.sb) & (u - 1)) == 0 && ((uintptr_t)m.ptr & (u * sizeof(T) - 1)) == 0;
+}
+
+// kRows rows of a [.., T, D] tensor into a transposed tile (see piece) as float32, zeros behind the valid rows and columns.
+// A thread keeps its columns and walks the rows, several loads in flight.
+template <int kT, typename T, int DP, int kRows, int kU>
+__device__ __forceinline__ void load_tile_u(float* dst, const T* base, int64_t st, int D, int rows_valid) {
+    constexpr int kPer = DP / kU;                   // threads per row
+    constexpr int kStep = kT / kPer;                // rows per pass
+    constexpr int kN = kRows / kStep > 0 ? kRows / kStep : 1;
+    constexpr int kMax = 32 / kU < 8 ? 8 : 32 / kU, kBatch = kN < kMax ? kN : kMax;
+    const int d = kU * ((int)threadIdx.x % kPer), r0 = (int)threadIdx.x / kPer;
+    const T* src = base + r0 * st + d;
+    const bool col_ok = d < D;
 #pragma unroll 1
-        for (int i0 = 0; i0 < kN; i0 += kBatch) {
-            float x[kBatch];
+    for (int i0 = 0; i0 < kN; i0 += kBatch) {
+        float x[kBatch][kU];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int idx = (i0 + i) * kThreads + threadIdx.x, r = idx / DP, d = idx % DP;
-                x[i] = (r < rows_valid && d < D) ? to_f32<T>(base[(int64_t)r * m.st + d]) : 0.f;
-            }
+        for (int i = 0; i < kBatch; ++i) {
+            const int r = r0 + (i0 + i) * kStep;
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int idx = (i0 + i) * kThreads + threadIdx.x;
-                put(idx / DP, idx % DP, x[i]);
-            }
+            for (int u = 0; u < kU; ++u) x[i][u] = 0.f;
+            if (col_ok && r < rows_valid) load_unit<T, kU>(src + (int64_t)(i0 + i) * kStep * st, x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            const int r = r0 + (i0 + i) * kStep;
+            if (kRows < kStep && r >= kRows) continue;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) dst[piece<kRows>(d + u, r >> 2) + (r & 3)] = x[i][u];
         }
     }
+}
+template <int kT, typename T, int DP, int kRows>
+__device__ __forceinline__ void load_tile(float* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
+    const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
+    if (units_ok<T>(m, D, 4)) load_tile_u<kT, T, DP, kRows, 4>(dst, base, m.st, D, rows_valid);
+    else if (units_ok<T>(m, D, 2)) load_tile_u<kT, T, DP, kRows, 2>(dst, base, m.st, D, rows_valid);
+    else load_tile_u<kT, T, DP, kRows, 1>(dst, base, m.st, D, rows_valid);
 }
 
 __device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
@@ -116,24 +113,30 @@ __device__ __forceinline__ int col_of(int c, int tx) {
     return DP >= 64 ? (c >> 2) * 64 + 4 * tx + (c & 3) : (DP / 16) * tx + c;
 }
 
-// s[rows of ty x 4 keys of tx] = A (kR rows per thread, tile width kWA) * B^T (64 keys), both transposed tiles
-template <int DP, int kR, int kWA>
-__device__ __forceinline__ void product_nt(float2 (&s)[kR / 2][4], const float* A, const float* B, int ty, int tx, int D) {
+// s[rows of ty x kJ keys of tx] = A (kR rows per thread, tile width kWA) * B^T (16 * kJ keys), both transposed tiles
+template <int kR, int kWA, int kJ>
+__device__ __forceinline__ void product_nt(float2 (&s)[kR / 2][kJ], const float* A, const float* B, int ty, int tx, int D) {
 #pragma unroll
     for (int i = 0; i < kR / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = make_float2(0.f, 0.f);
+        for (int j = 0; j < kJ; ++j) s[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 4
     for (int d = 0; d < D; ++d) {
         float4 x[kR / 4];
 #pragma unroll
         for (int i = 0; i < kR / 4; ++i) x[i] = *(const float4*)(A + piece<kWA>(d, ty * (kR / 4) + i));
-        const float4 k = *(const float4*)(B + piece<64>(d, tx));
-        const float2 kk[4] = {dup(k.x), dup(k.y), dup(k.z), dup(k.w)};
+        float2 kk[kJ];
+        if constexpr (kJ == 4) {
+            const float4 k = *(const float4*)(B + piece<64>(d, tx));
+            kk[0] = dup(k.x); kk[1] = dup(k.y); kk[2] = dup(k.z); kk[3] = dup(k.w);
+        } else {
+            const float2 k = *(const float2*)(B + piece<32>(d, tx >> 1) + 2 * (tx & 1));
+            kk[0] = dup(k.x); kk[1] = dup(k.y);
+        }
 #pragma unroll
         for (int i = 0; i < kR / 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kJ; ++j) {
                 s[2 * i][j] = __ffma2_rn(make_float2(x[i].x, x[i].y), kk[j], s[2 * i][j]);
                 s[2 * i + 1][j] = __ffma2_rn(make_float2(x[i].z, x[i].w), kk[j], s[2 * i + 1][j]);
             }
@@ -152,20 +155,23 @@ __device__ __forceinline__ void product_px(float2 (&acc)[kR / 2][DP / 16], const
         for (int c = 0; c < kNC; ++c) x[c] = *(const float4*)(X + piece<64>(col_of<DP>(c, tx), j4));
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-            float4 p[kR / 4];
+            float2 p[kR / 2];
+            if constexpr (kR == 2) {
+                p[0] = *(const float2*)(P + (4 * j4 + jj) * kWP + 2 * ty);
+            } else {
 #pragma unroll
-            for (int i = 0; i < kR / 4; ++i) {
-                const int c = ty * (kR / 4) + i;
-                p[i] = *(const float4*)(P + (4 * j4 + jj) * kWP + ((kSwz ? ((c ^ j4) & (kWP / 4 - 1)) : c) << 2));
+                for (int i = 0; i < kR / 4; ++i) {
+                    const int c = ty * (kR / 4) + i;
+                    const float4 q = *(const float4*)(P + (4 * j4 + jj) * kWP + ((kSwz ? ((c ^ j4) & (kWP / 4 - 1)) : c) << 2));
+                    p[2 * i] = make_float2(q.x, q.y);
+                    p[2 * i + 1] = make_float2(q.z, q.w);
+                }
             }
 #pragma unroll
             for (int c = 0; c < kNC; ++c) {
                 const float2 xx = dup(jj == 0 ? x[c].x : jj == 1 ? x[c].y : jj == 2 ? x[c].z : x[c].w);
 #pragma unroll
-                for (int i = 0; i < kR / 4; ++i) {
-                    acc[2 * i][c] = __ffma2_rn(make_float2(p[i].x, p[i].y), xx, acc[2 * i][c]);
-                    acc[2 * i + 1][c] = __ffma2_rn(make_float2(p[i].z, p[i].w), xx, acc[2 * i + 1][c]);
-                }
+                for (int i = 0; i < kR / 2; ++i) acc[i][c] = __ffma2_rn(p[i], xx, acc[i][c]);
             }
         }
     }
@@ -248,17 +254,23 @@ __device__ inline bool fetch_item(const KArgs& a, int item, ItemCtx& c) {
     return true;
 }
 
-__device__ __forceinline__ int64_t linear_thread() {
-    return (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kThreads + threadIdx.x;
+// Blocks in the order of the item table (heaviest first), the heads and the parts of a 128-row tile innermost: the hardware
+// deals blocks out in this order, so the heavy ones of all heads start first.
+struct BlockIdx {
+    int item, h, part;
+};
+__device__ __forceinline__ BlockIdx block_idx(int heads, int parts) {
+    const int per = heads * parts, item = (int)blockIdx.x / per, rest = (int)blockIdx.x - item * per;
+    return BlockIdx{item, rest / parts, rest % parts};
 }
-__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * gridDim.y * gridDim.z * kThreads; }
+__device__ __forceinline__ int64_t linear_thread() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * blockDim.x; }
 
 // ------------------------------------------------------------------------------------------ forward
-// kR rows per thread: blocks of 8 * kR query rows.  64-row blocks need fewer loads per product, 32-row ones spread a small
-// problem over twice as many SMs (the host chooses).
-template <typename T, int DP, int kR>
-__global__ void __launch_bounds__(kThreads, DP > 64 ? 2 : 3) simt_fwd_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kBM = 8 * kR;
+// kT / 16 groups of 4 query rows: blocks of 64 rows, or 32 where the problem is small (the host chooses)
+template <typename T, int DP, int kT>
+__global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 4) simt_fwd_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kR = 4, kBM = kT / 16 * kR;
     extern __shared__ __align__(16) float smem[];
     float* Qt = smem;             // [DP][kBM]
     float* Kt = Qt + DP * kBM;    // [DP][64]
@@ -268,14 +280,15 @@ __global__ void __launch_bounds__(kThreads, DP > 64 ? 2 : 3) simt_fwd_kernel(con
     pdl_launch_dependents();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_rows<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
-    if (!fetch_item(a, blockIdx.x, c)) return;
-    const int h = blockIdx.y, D = a.head_dim;
-    const int sub = blockIdx.z * kBM;  // first row inside the 128-row tile
+    const BlockIdx bi = block_idx(a.heads, kTileQ / kBM);
+    if (!fetch_item(a, bi.item, c)) return;
+    const int h = bi.h, D = a.head_dim;
+    const int sub = bi.part * kBM;  // first row inside the 128-row tile
     const int row0 = c.qt * kTileQ + sub;
     if (row0 >= c.len) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int rows_valid = min(kBM, c.len - row0);
-    load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+    load_tile<kT, T, DP, kBM>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
     float W[kR];
     float2 o[kR / 2][DP / 16];
 #pragma unroll
@@ -300,11 +313,11 @@ __global__ void __launch_bounds__(kThreads, DP > 64 ? 2 : 3) simt_fwd_kernel(con
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
-        load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kBN>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kBN>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
         __syncthreads();
         float2 s[kR / 2][4];
-        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
+        product_nt<kR, kBM>(s, Qt, Kt, ty, tx, D);
         const bool edge = key0 + kBN > row0 || keys_valid < kBN;  // some pair of the tile is not visible
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
@@ -347,28 +360,30 @@ __global__ void __launch_bounds__(kThreads, DP > 64 ? 2 : 3) simt_fwd_kernel(con
 }
 
 // ------------------------------------------------------------------------------------------ backward: dq
-template <typename T, int DP, int kR>
-__global__ void __launch_bounds__(kThreads, 2) simt_bwd_dq_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kBM = 8 * kR;
+template <typename T, int DP, int kT>
+__global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 3) simt_bwd_dq_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kR = 4, kBM = kT / 16 * kR;
+    constexpr bool kShare = DP >= kBM;  // dS takes the place of V, which is done with
     extern __shared__ __align__(16) float smem[];
     float* Qt = smem;
     float* Gt = Qt + DP * kBM;  // dO
     float* Kt = Gt + DP * kBM;
     float* Vt = Kt + DP * kBN;
-    float* Ss = Vt + DP * kBN;  // dS, [64 keys][kBM]
+    float* Ss = kShare ? Vt : Vt + DP * kBN;  // dS, [64 keys][kBM]
     pdl_wait();
     pdl_launch_dependents();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
-    if (!fetch_item(a, blockIdx.x, c)) return;
-    const int h = blockIdx.y, D = a.head_dim;
-    const int sub = blockIdx.z * kBM;
+    const BlockIdx bi = block_idx(a.heads, kTileQ / kBM);
+    if (!fetch_item(a, bi.item, c)) return;
+    const int h = bi.h, D = a.head_dim;
+    const int sub = bi.part * kBM;
     const int row0 = c.qt * kTileQ + sub;
     if (row0 >= c.len) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int rows_valid = min(kBM, c.len - row0);
-    load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
-    load_tile<T, DP, kBM, true>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+    load_tile<kT, T, DP, kBM>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+    load_tile<kT, T, DP, kBM>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
     float drem[kR], prefix[kR];
 #pragma unroll
     for (int r = 0; r < kR; ++r) {
@@ -389,16 +404,16 @@ __global__ void __launch_bounds__(kThreads, 2) simt_bwd_dq_kernel(const __grid_c
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
-        load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kBN>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kBN>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
         const int64_t slot = carry_slot(c.slot_base, c.qt, kh) * kTileQ;
         float Win[kR];
 #pragma unroll
         for (int r = 0; r < kR; ++r) Win[r] = ty * kR + r < rows_valid ? cw[slot + r] : 0.f;
         __syncthreads();
         float2 s[kR / 2][4], dp[kR / 2][4];
-        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
-        product_nt<DP, kR, kBM>(dp, Gt, Vt, ty, tx, D);
+        product_nt<kR, kBM>(s, Qt, Kt, ty, tx, D);
+        product_nt<kR, kBM>(dp, Gt, Vt, ty, tx, D);
         const bool edge = key0 + kBN > row0 || keys_valid < kBN;
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
@@ -422,13 +437,17 @@ __global__ void __launch_bounds__(kThreads, 2) simt_bwd_dq_kernel(const __grid_c
             const float upto = left_sum(mine, tx);  // through this lane's keys
             float cin = prefix[r] + (upto - mine);
             prefix[r] += __shfl_sync(0xffffffffu, upto, 15, 16);
-            if (tx == 15 && ty * kR + r < rows_valid) cc[slot + r] = prefix[r];  // prefix including this tile
+            if (ty * kR + r < rows_valid) {  // prefixes through the right edges of the two 32-key quarters
+                if (tx == 15) cc[slot + r] = prefix[r];
+                if (tx == 7) cc[slot - kTileQ + r] = cin + mine;
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 cin += g[j];
                 pick(s[r >> 1][j], r & 1) = g[j] - beta[j] * cin;
             }
         }
+        if (kShare) __syncthreads();  // everybody has read V
         put_weights<kR, kBM>(Ss, s, ty, tx);
         __syncthreads();
         product_px<DP, kR, kBM, true>(o, Ss, Kt, ty, tx);
@@ -437,47 +456,49 @@ __global__ void __launch_bounds__(kThreads, 2) simt_bwd_dq_kernel(const __grid_c
 }
 
 // ------------------------------------------------------------------------------------------ backward: dk, dv
-template <typename T, int DP>
-__global__ void __launch_bounds__(kThreads, 2) simt_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kR = 8, kBM = 64;
+// kJ keys per lane: stationary tiles of 16 * kJ keys (64, or 32 for small problems)
+template <typename T, int DP, int kJ>
+__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) simt_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 256, kR = 4, kBM = 64, kKeys = 16 * kJ, kRK = kKeys / 16;
     extern __shared__ __align__(16) float smem[];
     float* Qt = smem;
     float* Gt = Qt + DP * kBM;
     float* Kt = Gt + DP * kBM;
-    float* Vt = Kt + DP * kBN;
-    float* Ps = Vt + DP * kBN;   // P, [64 queries][64 keys]
-    float* Ss = Ps + kBM * kBN;  // dS
+    float* Vt = Kt + DP * kKeys;
+    float* Ps = Vt + DP * kKeys;   // P, [64 queries][kKeys]
+    float* Ss = Ps + kBM * kKeys;  // dS
     pdl_wait();
     pdl_launch_dependents();
     ItemCtx c;
     const int n_items = a.hdr->n_items;
-    if ((int)blockIdx.x >= n_items) return;
+    const BlockIdx bi = block_idx(a.heads, kTileQ / kKeys);
+    if (bi.item >= n_items) return;
     // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
-    if (!fetch_item(a, n_items - 1 - (int)blockIdx.x, c)) return;
-    const int h = blockIdx.y, D = a.head_dim;
-    const int kh = 2 * c.qt + blockIdx.z;
-    const int key0 = kh * kBN;
+    if (!fetch_item(a, n_items - 1 - bi.item, c)) return;
+    const int h = bi.h, D = a.head_dim;
+    const int key0 = c.qt * kTileQ + bi.part * kKeys;
+    const int edge_slot = key0 / 32 + kKeys / 32 - 1;  // the 32-key quarter at the tile's right edge
     if (key0 >= c.len) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int keys_valid = min(kBN, c.len - key0);
-    load_tile<T, DP, kBN, true>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
-    load_tile<T, DP, kBN, true>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
+    const int keys_valid = min(kKeys, c.len - key0);
+    load_tile<kT, T, DP, kKeys>(Kt, a.k, D, c.b, h, c.start + key0, keys_valid);
+    load_tile<kT, T, DP, kKeys>(Vt, a.v, D, c.b, h, c.start + key0, keys_valid);
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    float2 ok[kR / 2][DP / 16], ov[kR / 2][DP / 16];
+    float2 ok[kRK / 2][DP / 16], ov[kRK / 2][DP / 16];
 #pragma unroll
-    for (int i = 0; i < kR / 2; ++i)
+    for (int i = 0; i < kRK / 2; ++i)
 #pragma unroll
         for (int j = 0; j < DP / 16; ++j) ok[i][j] = ov[i][j] = make_float2(0.f, 0.f);
     const int n_qb = (c.len + kBM - 1) / kBM;
 
-    for (int qb = kh; qb < n_qb; ++qb) {
+    for (int qb = key0 / kBM; qb < n_qb; ++qb) {
         const int row0 = qb * kBM;
         const int rows_valid = min(kBM, c.len - row0);
         __syncthreads();
-        load_tile<T, DP, kBM, true>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
-        load_tile<T, DP, kBM, true>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
-        const int64_t slot = carry_slot(c.slot_base, qb >> 1, kh) * kTileQ + (qb & 1) * kBM + ty * kR;
+        load_tile<kT, T, DP, kBM>(Qt, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<kT, T, DP, kBM>(Gt, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        const int64_t slot = carry_slot32(c.slot_base, qb >> 1, edge_slot) * kTileQ + (qb & 1) * kBM + ty * kR;
         float Win[kR], cright[kR], drem[kR];
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
@@ -488,36 +509,36 @@ __global__ void __launch_bounds__(kThreads, 2) simt_bwd_dkdv_kernel(const __grid
             drem[r] = row_ok ? to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + t * a.d_rem.st]) : 0.f;
         }
         __syncthreads();
-        float2 s[kR / 2][4], dp[kR / 2][4];
-        product_nt<DP, kR, kBM>(s, Qt, Kt, ty, tx, D);
-        product_nt<DP, kR, kBM>(dp, Gt, Vt, ty, tx, D);
-        const bool edge = qb == kh || keys_valid < kBN;
+        float2 s[kR / 2][kJ], dp[kR / 2][kJ];
+        product_nt<kR, kBM>(s, Qt, Kt, ty, tx, D);
+        product_nt<kR, kBM>(dp, Gt, Vt, ty, tx, D);
+        const bool edge = qb == key0 / kBM || keys_valid < kKeys;
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
-            const int lim = edge ? min(keys_valid, row0 + ty * kR + r + a.attend_current - key0) : kBN;
-            float beta[4], om[4], g[4], p[4];
+            const int lim = edge ? min(keys_valid, row0 + ty * kR + r + a.attend_current - key0) : kKeys;
+            float beta[kJ], om[kJ], g[kJ], p[kJ];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kJ; ++j) {
                 sigmoid_pair(pick(s[r >> 1][j], r & 1) * a.inv_temp, beta[j], om[j]);
-                if (4 * tx + j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
+                if (kJ * tx + j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
             }
-            const float incl = right_prod((om[0] * om[1]) * (om[2] * om[3]), tx);
+            const float incl = right_prod(kJ == 4 ? (om[0] * om[1]) * (om[kJ - 2] * om[kJ - 1]) : om[0] * om[1], tx);
             float right = __shfl_down_sync(0xffffffffu, incl, 1, 16);
             if (tx == 15) right = 1.f;
             float run = Win[r] * right;
 #pragma unroll
-            for (int j = 3; j >= 0; --j) {
+            for (int j = kJ - 1; j >= 0; --j) {
                 p[j] = beta[j] * run;
                 g[j] = p[j] * (pick(dp[r >> 1][j], r & 1) - drem[r]);
                 run *= om[j];
             }
-            const float from = right_sum((g[0] + g[1]) + (g[2] + g[3]), tx);
+            const float from = right_sum(kJ == 4 ? (g[0] + g[1]) + (g[kJ - 2] + g[kJ - 1]) : g[0] + g[1], tx);
             float behind = __shfl_down_sync(0xffffffffu, from, 1, 16);  // sum of g right of this lane's keys
             if (tx == 15) behind = 0.f;
             // inclusive prefix at key j = (prefix through the tile's right edge) - (sum of g right of j)
             float cin = cright[r] - behind;
 #pragma unroll
-            for (int j = 3; j >= 0; --j) {
+            for (int j = kJ - 1; j >= 0; --j) {
                 pick(s[r >> 1][j], r & 1) = p[j];
                 pick(dp[r >> 1][j], r & 1) = g[j] - beta[j] * cin;
                 cin -= g[j];
@@ -526,56 +547,66 @@ __global__ void __launch_bounds__(kThreads, 2) simt_bwd_dkdv_kernel(const __grid
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
             const int q = ty * kR + r;
-            *(float4*)(Ps + q * kBN + 4 * tx) = make_float4(pick(s[r >> 1][0], r & 1), pick(s[r >> 1][1], r & 1), pick(s[r >> 1][2], r & 1), pick(s[r >> 1][3], r & 1));
-            *(float4*)(Ss + q * kBN + 4 * tx) = make_float4(pick(dp[r >> 1][0], r & 1), pick(dp[r >> 1][1], r & 1), pick(dp[r >> 1][2], r & 1), pick(dp[r >> 1][3], r & 1));
+            if constexpr (kJ == 4) {
+                *(float4*)(Ps + q * kKeys + 4 * tx) = make_float4(pick(s[r >> 1][0], r & 1), pick(s[r >> 1][1], r & 1), pick(s[r >> 1][2], r & 1), pick(s[r >> 1][3], r & 1));
+                *(float4*)(Ss + q * kKeys + 4 * tx) = make_float4(pick(dp[r >> 1][0], r & 1), pick(dp[r >> 1][1], r & 1), pick(dp[r >> 1][2], r & 1), pick(dp[r >> 1][3], r & 1));
+            } else {
+                *(float2*)(Ps + q * kKeys + 2 * tx) = make_float2(pick(s[r >> 1][0], r & 1), pick(s[r >> 1][1], r & 1));
+                *(float2*)(Ss + q * kKeys + 2 * tx) = make_float2(pick(dp[r >> 1][0], r & 1), pick(dp[r >> 1][1], r & 1));
+            }
         }
         __syncthreads();
-        product_px<DP, kR, kBN, false>(ov, Ps, Gt, ty, tx);
-        product_px<DP, kR, kBN, false>(ok, Ss, Qt, ty, tx);
+        product_px<DP, kRK, kKeys, false>(ov, Ps, Gt, ty, tx);
+        product_px<DP, kRK, kKeys, false>(ok, Ss, Qt, ty, tx);
     }
-    store_acc<T, DP, kR>(ok, a.inv_temp, a.dk, D, c.b, h, c.start + key0, keys_valid, ty, tx);
-    store_acc<T, DP, kR>(ov, 1.f, a.dv, D, c.b, h, c.start + key0, keys_valid, ty, tx);
+    store_acc<T, DP, kRK>(ok, a.inv_temp, a.dk, D, c.b, h, c.start + key0, keys_valid, ty, tx);
+    store_acc<T, DP, kRK>(ov, 1.f, a.dv, D, c.b, h, c.start + key0, keys_valid, ty, tx);
 }
 
-// Blocks of 32 query rows where 64-row blocks (`heads * items * 2`, an upper bound) would leave SMs without any
-bool small_problem(const WsLayout& L, const KArgs& a) { return (int64_t)L.max_items * a.heads * 2 <= 2 * 148; }
+// Blocks of 32 query rows (key tiles of 32) where 64-row ones, `items * heads * 2` at most, would not give every SM one: half the
+// work per block, at the price of loading every key (query) tile for half as many rows.  float32, 4 heads, 512 tokens: 96.7 -> 88
+// us per step; from two blocks per SM on, 64 rows are faster in each kernel (below: 76 / 106 / 119 against 90 / 114 / 132).
+bool small_problem(const WsLayout& L, const KArgs& a) { return (int64_t)L.max_items * a.heads * 2 <= 148; }
 
-template <typename T, int DP, int kR>
+template <typename T, int DP, int kT>
 int launch_fwd_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    const int smem = (int)sizeof(float) * (DP * 8 * kR + 2 * DP * kBN + kBN * 8 * kR);
-    const auto kernel = simt_fwd_kernel<T, DP, kR>;
+    constexpr int kBM = kT / 4;
+    const int smem = (int)sizeof(float) * (DP * kBM + 2 * DP * kBN + kBN * kBM);
+    const auto kernel = simt_fwd_kernel<T, DP, kT>;
     const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
     if (e != 0) return e;
-    return launch_kernel(kernel, dim3(L.max_items, a.heads, 16 / kR), dim3(kThreads), smem, st, a);
+    return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * (kTileQ / kBM)), dim3(kT), smem, st, a);
 }
-template <typename T, int DP, int kR>
+template <typename T, int DP, int kT>
 int launch_dq_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    const int smem = (int)sizeof(float) * (2 * DP * 8 * kR + 2 * DP * kBN + kBN * 8 * kR);
-    const auto kernel = simt_bwd_dq_kernel<T, DP, kR>;
+    constexpr int kBM = kT / 4;
+    const int smem = (int)sizeof(float) * (2 * DP * kBM + 2 * DP * kBN + (DP >= kBM ? 0 : kBN * kBM));
+    const auto kernel = simt_bwd_dq_kernel<T, DP, kT>;
     const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
     if (e != 0) return e;
-    return launch_kernel(kernel, dim3(L.max_items, a.heads, 16 / kR), dim3(kThreads), smem, st, a);
+    return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * (kTileQ / kBM)), dim3(kT), smem, st, a);
 }
-template <typename T, int DP>
+template <typename T, int DP, int kJ>
 int launch_dkdv_k(const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    const int smem = (int)sizeof(float) * (4 * DP * kBN + 2 * kBN * kBN);
-    const auto kernel = simt_bwd_dkdv_kernel<T, DP>;
+    const int smem = (int)sizeof(float) * (2 * DP * (64 + 16 * kJ) + 2 * 64 * 16 * kJ);
+    const auto kernel = simt_bwd_dkdv_kernel<T, DP, kJ>;
     const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
     if (e != 0) return e;
-    return launch_kernel(kernel, dim3(L.max_items, a.heads, 2), dim3(kThreads), smem, st, a);
+    return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * (8 / kJ)), dim3(256), smem, st, a);
 }
 
 template <typename T, int DP>
 int launch_fwd_d(const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    return small_problem(L, a) ? launch_fwd_k<T, DP, 4>(L, a, st) : launch_fwd_k<T, DP, 8>(L, a, st);
+    return small_problem(L, a) ? launch_fwd_k<T, DP, 128>(L, a, st) : launch_fwd_k<T, DP, 256>(L, a, st);
 }
 template <typename T, int DP>
 int launch_bwd_d(const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
     if (phases != SBATTN_BWD_DKDV) {
-        const int e = small_problem(L, a) ? launch_dq_k<T, DP, 4>(L, a, st) : launch_dq_k<T, DP, 8>(L, a, st);
+        const int e = small_problem(L, a) ? launch_dq_k<T, DP, 128>(L, a, st) : launch_dq_k<T, DP, 256>(L, a, st);
         if (e != 0) return e;
     }
-    return phases != SBATTN_BWD_DQ ? launch_dkdv_k<T, DP>(L, a, st) : 0;
+    if (phases == SBATTN_BWD_DQ) return 0;
+    return small_problem(L, a) ? launch_dkdv_k<T, DP, 2>(L, a, st) : launch_dkdv_k<T, DP, 4>(L, a, st);
 }
 
 template <typename T>
