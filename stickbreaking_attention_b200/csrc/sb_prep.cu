@@ -62,9 +62,9 @@ prep_kernel(WsHeader* hdr, SeqInfo* seqs, int2* items, int32_t* bins, const void
     const int t = threadIdx.x;
     int* cursor = n_max <= kSharedBins ? sh_bins : bins;  // [n_max+2]: sequences per tile count, then write position per cost class
     if (t == 0) sh_bad = 0;
-    for (int i = t; i < n_max + 2; i += kPrepThreads) cursor[i] = 0;
-    pdl_wait();
+    pdl_wait();  // before anything is written to the workspace, whose memory an earlier kernel may still be reading
     pdl_launch_dependents();
+    for (int i = t; i < n_max + 2; i += kPrepThreads) cursor[i] = 0;
     if (t < 8) hdr->sched[t] = 0;
     __syncthreads();
 

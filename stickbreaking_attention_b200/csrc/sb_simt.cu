@@ -277,7 +277,6 @@ __global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 4) simt_fwd_k
     float* Vt = Kt + DP * kBN;    // [DP][64]
     float* Ps = Vt + DP * kBN;    // [64 keys][kBM]
     pdl_wait();
-    pdl_launch_dependents();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_rows<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
     const BlockIdx bi = block_idx(a.heads, kTileQ / kBM);
@@ -347,6 +346,7 @@ __global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 4) simt_fwd_k
         __syncthreads();
         product_px<DP, kR, kBM, true>(o, Ps, Vt, ty, tx);
     }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     store_acc<T, DP, kR>(o, 1.f, a.o, D, c.b, h, c.start + row0, rows_valid, ty, tx);
     if (tx == 0) {
 #pragma unroll
@@ -371,7 +371,6 @@ __global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 3) simt_bwd_d
     float* Vt = Kt + DP * kBN;
     float* Ss = kShare ? Vt : Vt + DP * kBN;  // dS, [64 keys][kBM]
     pdl_wait();
-    pdl_launch_dependents();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
     ItemCtx c;
     const BlockIdx bi = block_idx(a.heads, kTileQ / kBM);
@@ -452,6 +451,7 @@ __global__ void __launch_bounds__(kT, DP > 64 ? 1 : kT > 128 ? 2 : 3) simt_bwd_d
         __syncthreads();
         product_px<DP, kR, kBM, true>(o, Ss, Kt, ty, tx);
     }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     store_acc<T, DP, kR>(o, a.inv_temp, a.dq, D, c.b, h, c.start + row0, rows_valid, ty, tx);
 }
 
@@ -468,7 +468,6 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) simt_bwd_dkdv_kernel(con
     float* Ps = Vt + DP * kKeys;   // P, [64 queries][kKeys]
     float* Ss = Ps + kBM * kKeys;  // dS
     pdl_wait();
-    pdl_launch_dependents();
     ItemCtx c;
     const int n_items = a.hdr->n_items;
     const BlockIdx bi = block_idx(a.heads, kTileQ / kKeys);
@@ -559,6 +558,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) simt_bwd_dkdv_kernel(con
         product_px<DP, kRK, kKeys, false>(ov, Ps, Gt, ty, tx);
         product_px<DP, kRK, kKeys, false>(ok, Ss, Qt, ty, tx);
     }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     store_acc<T, DP, kRK>(ok, a.inv_temp, a.dk, D, c.b, h, c.start + key0, keys_valid, ty, tx);
     store_acc<T, DP, kRK>(ov, 1.f, a.dv, D, c.b, h, c.start + key0, keys_valid, ty, tx);
 }
