@@ -111,7 +111,7 @@ struct KArgs {
     int32_t heads, head_dim, attend_current;
     int32_t fused;          // SBATTN_FLAG_FUSED_REMAINDER
     int32_t tokens;         // tokens per batch entry (row index of drem_eff: batch * tokens + token)
-    float* drem_eff;        // [heads][drem_rows]: drem + do . v, written by the dq kernel when fused
+    float* drem_eff;        // [heads][drem_rows]: drem + do . v (fused-remainder backward)
     int64_t drem_rows;      // batch * tokens (tokens for the packed layout)
     int32_t head_group;     // heads whose work is interleaved (sized so that their K and V stay in L2)
     int32_t defer_fwd, defer_dq, defer_dkdv;  // tensor-core kernels: store an item's result one step into the next item
@@ -225,6 +225,7 @@ __device__ inline void zero_tail_grads(const KArgs& a, int first, int64_t thread
 // kMapEncodeFailed when a tensor map could not be encoded, before anything has been launched)
 constexpr int kMapEncodeFailed = -1000;
 int launch_prep(const SbParams& p, const WsLayout& L, cudaStream_t st);
+int launch_drem(const SbParams& p, const KArgs& a, cudaStream_t st);
 int launch_simt_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 int launch_simt_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 bool tensor_path_eligible(const SbParams& p, bool backward, int* why);

@@ -401,25 +401,12 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             const int64_t tok = wk.start + qi;
             float drem = 0.f;
             if (row_ok) {
-                const char* dp = a.d_rem.ptr + 2 * ((int64_t)wk.b * a.d_rem.sb + (int64_t)wk.h * a.d_rem.sh + tok * a.d_rem.st);
-                drem = kF16 ? __half2float(*(const __half*)dp) : __bfloat162float(*(const __nv_bfloat16*)dp);
-            }
-            if (kFused && row_ok) {
-                // rem also receives do . v; the sum is left for the dk/dv kernel
-                const char* dorow = a.d_o.ptr + 2 * ((int64_t)wk.b * a.d_o.sb + (int64_t)wk.h * a.d_o.sh + tok * a.d_o.st);
-                const char* vrow = a.v.ptr + 2 * ((int64_t)wk.b * a.v.sb + (int64_t)wk.h * a.v.sh + tok * a.v.st);
-                float dot = 0.f;
-#pragma unroll 1
-                for (int cidx = 0; cidx < D / 32; ++cidx) {
-                    float x[32], y[32];
-                    if (D == 64 && a.head_dim <= 32 * cidx) break;  // D == 64 serves head dim 32 as well
-                    load_row32<kF16>(dorow + cidx * 64, x);
-                    load_row32<kF16>(vrow + cidx * 64, y);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) dot = fmaf(x[i], y[i], dot);
+                if (kFused) {  // drem + do . v
+                    drem = __ldg(a.drem_eff + (int64_t)wk.h * a.drem_rows + (int64_t)wk.b * a.tokens + tok);
+                } else {
+                    const char* dp = a.d_rem.ptr + 2 * ((int64_t)wk.b * a.d_rem.sb + (int64_t)wk.h * a.d_rem.sh + tok * a.d_rem.st);
+                    drem = kF16 ? __half2float(*(const __half*)dp) : __bfloat162float(*(const __nv_bfloat16*)dp);
                 }
-                drem += dot;
-                if (kq == 3) a.drem_eff[(int64_t)wk.h * a.drem_rows + (int64_t)wk.b * a.tokens + wk.start + qi] = drem;
             }
             const float* cw = a.carry_w + ((int64_t)wk.h * a.slot_cap) * kTileQ + r;
             float* cc = a.carry_c + ((int64_t)wk.h * a.slot_cap) * kTileQ + r;
@@ -921,7 +908,7 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                         W = __ldg(cw + slot);
                         c = __ldg(cc + slot);  // loses every g it passes
                     }
-                    if (kFused) {  // drem + do . v (float32), left behind by the dq kernel
+                    if (kFused) {  // drem + do . v (float32)
                         drem = __ldg((const uint32_t*)a.drem_eff + (int64_t)wk.h * a.drem_rows + (int64_t)wk.b * a.tokens + wk.start + qi);
                     } else {
                         const char* dp = a.d_rem.ptr + 2 * ((int64_t)wk.b * a.d_rem.sb + (int64_t)wk.h * a.d_rem.sh +
@@ -1018,6 +1005,10 @@ int launch_bwd_kernels(const SbParams& p, const KArgs& a, cudaStream_t st, const
         return launch_kernel(kernel, grid, dim3(kKvThreads), smem_b, st, mq, mk128, mv128, mdo, mq64, mdo64, a);
     };
     if (p.bwd_phases != SBATTN_BWD_DKDV) {
+        if (kFused) {
+            const int e = launch_drem(p, a, st);
+            if (e != 0) return e;
+        }
         const int e = a.defer_dq ? launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, true>) : launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, false>);
         if (e != 0) return e;
     }
