@@ -13,24 +13,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 2^x for two values at once on the FMA pipes instead of the special-function unit (which delivers 16 results per clock
-// and SM against 128 fused multiply-adds): x = n + f with n the nearest integer (the magic-number addition leaves n in
-// the low mantissa bits of t), 2^f by a degree-4 polynomial on [-0.5, 0.5] (relative error 3.5e-6, far below the 16-bit
-// rounding of the weights), and n added to the exponent field.  The caller keeps x within [-125, 15].
-// Every multiply-add is a packed fp32x2 instruction.
-__device__ __forceinline__ float2 ex2_fma2(float2 x) {
-    const float kMagic = 12582912.f;  // 1.5 * 2^23
-    const float2 t = __fadd2_rn(x, make_float2(kMagic, kMagic));
-    const float2 n = __fadd2_rn(t, make_float2(-kMagic, -kMagic));
-    const float2 f = __fadd2_rn(x, make_float2(-n.x, -n.y));
-    // Chebyshev interpolant of 2^f on [-0.5, 0.5]
-    float2 p = __ffma2_rn(f, make_float2(9.666368515e-3f, 9.666368515e-3f), make_float2(5.592197584e-2f, 5.592197584e-2f));
-    p = __ffma2_rn(p, f, make_float2(2.402234904e-1f, 2.402234904e-1f));
-    p = __ffma2_rn(p, f, make_float2(6.931210452e-1f, 6.931210452e-1f));
-    p = __ffma2_rn(p, f, make_float2(1.f, 1.f));
-    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
-                       __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
-}
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -36,11 +36,6 @@ constexpr int kBM = 128, kBN = 128;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColS0 = 0, kColO = 384, kColPOff = 64;  // S buffer i at 128*i (i = step mod 3), its P at +64
 constexpr int kKStages = 3, kVStages = 2;
-// Eighths of every 32-key chunk whose exponential is computed on the FMA pipes (ex2_fma2) instead of the special-function
-// unit.  Measured on the 16384-token benchmark pack (forward, one B200): 0 -> 0.4316 ms, 1 -> 0.4342 ms, 2 -> 0.4455 ms.
-// The special-function unit is not what bounds the sweep (it is ~50 % busy), and the polynomial costs five more issue
-// slots per score than ex2.approx, so the share stays at zero; the path is kept for shapes where that changes.
-constexpr int kFmaExpEighths = 0;
 enum FwdBar { Q_FULL, Q_EMPTY, K_FULL0, K_FULL1, K_FULL2, K_EMPTY0, K_EMPTY1, K_EMPTY2, V_FULL0, V_FULL1, V_EMPTY0, V_EMPTY1, S_READY0, S_READY1,
               S_READY2, P_READY0, P_READY1, P_READY2, O_READY, O_FREE, WORK_FULL0, WORK_FULL1, WORK_EMPTY0, WORK_EMPTY1,
               X_W0,  // 32 barriers for the carry chain: [quarter][tile parity][warp & 3]
@@ -52,51 +47,55 @@ enum FwdBar { Q_FULL, Q_EMPTY, K_FULL0, K_FULL1, K_FULL2, K_EMPTY0, K_EMPTY1, K_
 // which needs one reciprocal per GROUP instead of one per key.  Scores are clamped at 2^15 (beta = 1 - 3e-5 there)
 // so that the product of 8 factors stays below 2^127.  Masked keys get e = 0: weight 0 and no stick broken.
 //
-// First pass over a chunk of 32 keys: s[idx] <- e * (product of d over the keys of its group to the LEFT);
-// run[g] <- product of d over group g.  The four groups are swept side by side so that their chains overlap.
+// First pass over a chunk of 32 keys: p <- e * (product of d over the keys of its group to the LEFT); run <- product of d over
+// the group.  The four groups are swept side by side so that their chains overlap, and in pairs: p[h][m] holds key m of groups 2h
+// and 2h + 1, so that every multiplication of the chains is one packed fp32x2 instruction for two keys (the exponentials deliver
+// their results into whatever register the pairing wants).
 template <bool kMasked>
-__device__ __forceinline__ void fwd_sweep(uint32_t (&s)[32], float scale, int col0, int lim, float (&run)[4]) {
-#pragma unroll
-    for (int g = 0; g < 4; ++g) run[g] = 1.f;
+__device__ __forceinline__ void fwd_sweep(const uint32_t (&s)[32], float scale, int col0, int lim, float2 (&p)[2][8], float2 (&run)[2]) {
+    run[0] = run[1] = make_float2(1.f, 1.f);
 #pragma unroll
     for (int m = 0; m < 8; m += 2) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const int idx = g * 8 + m;  // two adjacent keys: the scaling is one packed fp32x2 multiply
-            const float2 x = __fmul2_rn(make_float2(__uint_as_float(s[idx]), __uint_as_float(s[idx + 1])), make_float2(scale, scale));
-            float e0, e1;
-            if (kFmaExpEighths > 0 && g == 3 && (kFmaExpEighths >= 2 || (m & 2))) {  // this share of the exponentials on the FMA pipes
-                const float2 e = ex2_fma2(make_float2(fmaxf(fminf(x.x, 15.f), -125.f), fmaxf(fminf(x.y, 15.f), -125.f)));
-                e0 = e.x;
-                e1 = e.y;
-            } else {
-                e0 = ex2_approx(fminf(x.x, 15.f));
-                e1 = ex2_approx(fminf(x.y, 15.f));
+        for (int h = 0; h < 2; ++h) {
+            const int i0 = 16 * h + m, i1 = i0 + 8;  // two adjacent keys of either group: the scaling is a packed multiply too
+            const float2 x0 = __fmul2_rn(make_float2(__uint_as_float(s[i0]), __uint_as_float(s[i0 + 1])), make_float2(scale, scale));
+            const float2 x1 = __fmul2_rn(make_float2(__uint_as_float(s[i1]), __uint_as_float(s[i1 + 1])), make_float2(scale, scale));
+            float2 ea = make_float2(ex2_approx(fminf(x0.x, 15.f)), ex2_approx(fminf(x1.x, 15.f)));
+            float2 eb = make_float2(ex2_approx(fminf(x0.y, 15.f)), ex2_approx(fminf(x1.y, 15.f)));
+            if (kMasked) {
+                if (col0 + i0 >= lim) ea.x = 0.f;
+                if (col0 + i1 >= lim) ea.y = 0.f;
+                if (col0 + i0 + 1 >= lim) eb.x = 0.f;
+                if (col0 + i1 + 1 >= lim) eb.y = 0.f;
             }
-            if (kMasked && col0 + idx >= lim) e0 = 0.f;
-            if (kMasked && col0 + idx + 1 >= lim) e1 = 0.f;
-            s[idx] = __float_as_uint(e0 * run[g]);
-            run[g] = fmaf(run[g], e0, run[g]);
-            s[idx + 1] = __float_as_uint(e1 * run[g]);
-            run[g] = fmaf(run[g], e1, run[g]);
+            p[h][m] = __fmul2_rn(ea, run[h]);
+            run[h] = __ffma2_rn(run[h], ea, run[h]);
+            p[h][m + 1] = __fmul2_rn(eb, run[h]);
+            run[h] = __ffma2_rn(run[h], eb, run[h]);
         }
     }
 }
-// carry entering each group from the right: f[g] = W / (product of d over groups g..3); W <- the chunk's exit carry
-__device__ __forceinline__ void fwd_carries(const float (&run)[4], float& W, float* f) {
-    f[3] = W * rcp_approx(run[3]);
-    f[2] = f[3] * rcp_approx(run[2]);
-    f[1] = f[2] * rcp_approx(run[1]);
-    f[0] = f[1] * rcp_approx(run[0]);
-    W = f[0];
+// carry entering each group from the right: f[h] = (W / (product of d over groups 2h..3), W / (product over groups 2h+1..3));
+// W <- the chunk's exit carry
+__device__ __forceinline__ void fwd_carries(const float2 (&run)[2], float& W, float2 (&f)[2]) {
+    f[1].y = W * rcp_approx(run[1].y);
+    f[1].x = f[1].y * rcp_approx(run[1].x);
+    f[0].y = f[1].x * rcp_approx(run[0].y);
+    f[0].x = f[0].y * rcp_approx(run[0].x);
+    W = f[0].x;
 }
 template <bool kF16>
-__device__ __forceinline__ void fwd_finish(const uint32_t (&s)[32], const float* f, float mul, uint32_t (&packed)[16]) {
+__device__ __forceinline__ void fwd_finish(const float2 (&p)[2][8], const float2 (&f)[2], float mul, uint32_t (&packed)[16]) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float fj = f[j >> 2] * mul;
-        const float2 p = __fmul2_rn(make_float2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), make_float2(fj, fj));
-        packed[j] = pack16<kF16>(p.x, p.y);
+    for (int h = 0; h < 2; ++h) {
+        const float2 fm = __fmul2_rn(f[h], make_float2(mul, mul));
+#pragma unroll
+        for (int m = 0; m < 8; m += 2) {
+            const float2 a = __fmul2_rn(p[h][m], fm), b = __fmul2_rn(p[h][m + 1], fm);
+            packed[8 * h + m / 2] = pack16<kF16>(a.x, b.x);
+            packed[8 * h + 4 + m / 2] = pack16<kF16>(a.y, b.y);
+        }
     }
 }
 
@@ -367,12 +366,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 tc_fence_after();
                 // sweep the quarter right to left relative to an entering carry of 1
                 uint32_t u[32], packed[16];
-                float run[4], f[4];
+                float2 pw[2][8], run[2], f[2];
                 float Wl = 1.f;
                 tmem_ld32(s_base + 32 * kq, u);
                 tmem_wait_ld(u);
-                if (j == 0) fwd_sweep<true>(u, scale, 32 * kq, lim, run);
-                else fwd_sweep<false>(u, scale, 32 * kq, lim, run);
+                if (j == 0) fwd_sweep<true>(u, scale, 32 * kq, lim, pw, run);
+                else fwd_sweep<false>(u, scale, 32 * kq, lim, pw, run);
                 fwd_carries(run, Wl, f);
                 // The true entering carry travels along the row as a chain through shared memory: a thread takes it from
                 // the quarter to its right (the rightmost quarter from the leftmost one of the previous tile), multiplies
@@ -394,7 +393,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 mbar_arrive(&bars[X_W0 + 8 * kq + 4 * (g & 1) + (warp & 3)]);
                 if (kFused && kq == 0 && j + 1 == n) wfin[(items % 3) * 128 + r] = W;  // visible to all once O_READY has completed
                 if (cw) cw[carry_slot32(wk.slot_base, wk.qt, 4 * kt + kq) * kTileQ] = Win;  // the carry at the quarter's right edge
-                fwd_finish<kF16>(u, f, Win, packed);
+                fwd_finish<kF16>(pw, f, Win, packed);
                 tmem_st16(s_base + kColPOff + 16 * kq, packed);
                 tmem_wait_st();
                 tc_fence_before();
