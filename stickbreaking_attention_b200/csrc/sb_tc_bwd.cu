@@ -17,55 +17,14 @@
 // Both kernels: one persistent block of 608 threads per SM (warps 0-15: one thread per query row and 32-key quarter of
 // a step; warps 16 and 18: TMA producers; warp 17 issues tcgen05.mma), all 512 tensor-memory columns, work drawn from a
 // global counter.
-#include "sb_tc_common.cuh"
-
+#include "sb_tc_bwd_common.cuh"
 
 namespace sb {
 
 using namespace sm100;
+using namespace bwd;
 
 namespace {
-
-constexpr int kBM = 128;  // query rows per tile
-constexpr int kBK = 64;   // keys per half of a step: the unit of masking and a 128-byte row of the p / ds buffers
-constexpr int kQBox = 128 * 128;  // bytes of one TMA box of a 128-row tile (64 elements wide)
-constexpr int kKBox = 64 * 128;   // bytes of one TMA box of a 64-row tile
-
-// Element-wise core shared by both kernels, four adjacent scores at a time: om = 1 - beta = 1 / (1 + 2^(s * scale));
-// masked keys get om = 1 (no stick broken, weight 0).  The operations without a dependency along the row are packed
-// fp32x2 instructions, and the four reciprocals cost one MUFU operation: with d_i = 1 + e_i,
-// 1 / d_i = (product of the other three) / (d_0 d_1 d_2 d_3).  The exponent is clamped at 30 so that the product of four
-// stays finite (om = 2^-30 instead of something smaller: no visible difference).
-template <bool kMasked, bool kGrouped = true>
-__device__ __forceinline__ void stick4(float s0, float s1, float s2, float s3, float scale, int col, int lim, float2& om01,
-                                       float2& om23) {
-    float2 x01 = __fmul2_rn(make_float2(s0, s1), make_float2(scale, scale));
-    float2 x23 = __fmul2_rn(make_float2(s2, s3), make_float2(scale, scale));
-    if (kGrouped) {
-        x01.x = fminf(x01.x, 30.f);
-        x01.y = fminf(x01.y, 30.f);
-        x23.x = fminf(x23.x, 30.f);
-        x23.y = fminf(x23.y, 30.f);
-    }
-    if (kMasked) {
-        if (col >= lim) x01.x = -INFINITY;
-        if (col + 1 >= lim) x01.y = -INFINITY;
-        if (col + 2 >= lim) x23.x = -INFINITY;
-        if (col + 3 >= lim) x23.y = -INFINITY;
-    }
-    const float2 d01 = __fadd2_rn(make_float2(ex2_approx(x01.x), ex2_approx(x01.y)), make_float2(1.f, 1.f));
-    const float2 d23 = __fadd2_rn(make_float2(ex2_approx(x23.x), ex2_approx(x23.y)), make_float2(1.f, 1.f));
-    if (!kGrouped) {
-        om01 = make_float2(rcp_approx(d01.x), rcp_approx(d01.y));
-        om23 = make_float2(rcp_approx(d23.x), rcp_approx(d23.y));
-        return;
-    }
-    const float2 m = __fmul2_rn(d01, d23);  // (d0 d2, d1 d3)
-    const float r = rcp_approx(m.x * m.y);
-    const float2 rm = make_float2(r * m.y, r * m.x);  // (1 / (d0 d2), 1 / (d1 d3))
-    om01 = __fmul2_rn(rm, d23);
-    om23 = __fmul2_rn(rm, d01);
-}
 
 // ================================================================================================ dq kernel
 // One block per SM (608 threads: 19 warps put five on one scheduler, which caps a thread at 96 registers), one work item = (head, sequence, 128-row query tile) at a
@@ -511,30 +470,9 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 // latency is covered.  Warp 16 loads K, V (once per item) and the early Q, dO tiles, warp 18 the late halves, warp 17
 // issues every tcgen05.mma.
 constexpr int kKvThreads = 608;
-constexpr int kKT = 128;  // keys per stationary tile
 enum KvBar { B_KV_FULL, B_KV_EMPTY, B_E_FULL, B_E_EMPTY, B_L_FULL0, B_L_FULL1, B_L_EMPTY0, B_L_EMPTY1, B_SDP_READY, B_LOADED,
              B_PDS_READY0, B_PDS_READY1, B_PDS_FREE0, B_PDS_FREE1, B_PDS_FREE2, B_PDS_FREE3, B_DKV_READY, B_DKV_FREE, B_WORK_FULL0,
              B_WORK_FULL1, B_WORK_EMPTY0, B_WORK_EMPTY1, kNumKvBars };
-
-struct KvWork {
-    int h, b, start, len, kt, slot_base, n_qt;
-};
-__device__ __forceinline__ KvWork fetch_kv_work(const KArgs& a, int n_items, int w) {
-    // groups of head_group heads; inside a group the 128-key tiles heaviest first (key tiles are heaviest where
-    // query tiles are lightest: the item table is walked backwards), the heads of the group innermost
-    const int per_group = n_items * a.head_group;
-    const int g = w / per_group, rest = w - g * per_group;
-    const int hg = min(a.head_group, a.heads - g * a.head_group);
-    const int idx = rest / hg;
-    const int2 it = a.items[n_items - 1 - idx];
-    const SeqInfo s = a.seqs[it.x];
-    KvWork k;
-    k.h = g * a.head_group + rest - idx * hg;
-    k.b = s.batch; k.start = s.start; k.len = s.len; k.slot_base = s.slot_base;
-    k.kt = it.y;
-    k.n_qt = (s.len + kBM - 1) / kBM;
-    return k;
-}
 
 template <bool kMasked, bool kF16>
 __device__ __forceinline__ void kv_chunk(const uint32_t (&s)[32], const uint32_t (&dp)[32], float scale, int col0, int lim,
@@ -564,54 +502,6 @@ __device__ __forceinline__ void kv_chunk(const uint32_t (&s)[32], const uint32_t
             ps[jj] = pack16<kF16>(ds0, ds1);
         }
     }
-}
-
-// dk or dv of a finished item out of tensor memory: a thread holds one key row and D / 2 columns of the head dim, from
-// chunk0 * 32 on.
-// Not inlined: it runs once per item, and inside the step loop it would only dilute the instruction cache.
-// With the fused remainder dv also receives rem * do of its own row: the direct path of out = o + rem * v.
-template <int D, bool kF16, bool kFused>
-__device__ __forceinline__ void kv_store_rows_inl(const KArgs& a, bool is_dv, const KvWork e, int r, uint32_t taddr, int chunk0,
-                                                  int n_chunks) {
-    tc_fence_after();
-    const MatView m = is_dv ? a.dv : a.dk;
-    const float sc = is_dv ? 1.f : a.inv_temp;
-    const bool key_ok = e.kt * kKT + r < e.len;
-    const int64_t tok = e.start + e.kt * kKT + r;
-    char* orow = m.ptr + 2 * ((int64_t)e.b * m.sb + (int64_t)e.h * m.sh + tok * m.st);
-    const char* add = nullptr;
-    float mul = 0.f;
-    if (kFused && is_dv && key_ok) {
-        add = a.d_o.ptr + 2 * ((int64_t)e.b * a.d_o.sb + (int64_t)e.h * a.d_o.sh + tok * a.d_o.st);
-        const char* rp = a.rem.ptr + 2 * ((int64_t)e.b * a.rem.sb + (int64_t)e.h * a.rem.sh + tok * a.rem.st);
-        mul = kF16 ? __half2float(*(const __half*)rp) : __bfloat162float(*(const __nv_bfloat16*)rp);
-    }
-#pragma unroll
-    for (int cc = 0; cc < D / 64; ++cc) {  // this thread's half of the head dim, 32 columns at a time
-        const int cidx = chunk0 + cc;
-        uint32_t v[32];
-        tmem_ld32(taddr + cidx * 32, v);
-        tmem_wait_ld(v);
-        if (!(kFused && is_dv)) {  // two rows per lane pair: -7 % on a pack of 128-token sequences, -0.6 % on long ones
-            // (the same in the forward and the dq kernel, whose threads store half as much, cost 1-5 %)
-            store_row32_pairs<kF16>(orow + cidx * 64, v, sc, (int64_t)m.st * 2, key_ok && (D == 128 || cc < n_chunks), (int)(threadIdx.x & 31));
-        } else if (key_ok && (D == 128 || cc < n_chunks)) {  // D == 64 serves head dim 32 as well: then fewer chunks exist
-            if (kFused && add) {
-                float x[32];
-                load_row32<kF16>(add + cidx * 64, x);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(fmaf(mul, x[i], __uint_as_float(v[i])));
-                store_row32<kF16>(orow + cidx * 64, v, 1.f);
-            } else {
-                store_row32<kF16>(orow + cidx * 64, v, sc);
-            }
-        }
-    }
-    tc_fence_before();
-}
-template <int D, bool kF16, bool kFused>
-__device__ __noinline__ void kv_store_rows(const KArgs& a, bool is_dv, const KvWork e, int r, uint32_t taddr, int chunk0, int n_chunks) {
-    kv_store_rows_inl<D, kF16, kFused>(a, is_dv, e, r, taddr, chunk0, n_chunks);
 }
 
 template <int D, bool kF16, bool kFused, bool kDefer>
@@ -1047,6 +937,9 @@ int launch_bwd_t(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStrea
 }  // namespace
 
 int launch_tensor_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    // sequences of at most one tile (max_seqlen <= 128): nothing crosses tiles, one kernel forms everything once (-36 % of the backward
+    // of 512 sequences of 128 tokens)
+    if (L.n_max == 1 && p.bwd_phases == SBATTN_BWD_ALL) return launch_tensor_bwd_tile(p, L, a, st);
     const bool f16 = p.dtype == SBATTN_F16;
     if (p.head_dim > 64) return f16 ? launch_bwd_t<128, true>(p, L, a, st) : launch_bwd_t<128, false>(p, L, a, st);
     return f16 ? launch_bwd_t<64, true>(p, L, a, st) : launch_bwd_t<64, false>(p, L, a, st);
