@@ -143,10 +143,10 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     cudaStream_t st = (cudaStream_t)p->stream;
     if (launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
     const KArgs a = make_args(*p, L);
-    int e = path == 1 ? launch_tensor_fwd(*p, L, a, st) : launch_simt_fwd(*p, L, a, st);
+    int e = path == 1 ? launch_tensor_fwd(*p, L, a, st) : launch_f32_fwd(*p, L, a, st);
     // a layout the tensor-map encoder refuses (nothing has been launched yet): the other kernels take any strides
     if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER))
-        e = launch_simt_fwd(*p, L, a, st);
+        e = launch_f32_fwd(*p, L, a, st);
     return e == 0 ? SBATTN_OK : (e == kMapEncodeFailed ? SBATTN_EUNSUPPORTED : SBATTN_ECUDA);
 }
 
@@ -172,9 +172,9 @@ extern "C" int sbattn_bwd(const SbParams* p) {
     }
     cudaStream_t st = (cudaStream_t)p->stream;
     const KArgs a = make_args(*p, L);
-    int e = path == 1 ? launch_tensor_bwd(*p, L, a, st) : launch_simt_bwd(*p, L, a, st);
+    int e = path == 1 ? launch_tensor_bwd(*p, L, a, st) : launch_f32_bwd(*p, L, a, st);
     if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER))
-        e = launch_simt_bwd(*p, L, a, st);
+        e = launch_f32_bwd(*p, L, a, st);
     return e == 0 ? SBATTN_OK : (e == kMapEncodeFailed ? SBATTN_EUNSUPPORTED : SBATTN_ECUDA);
 }
 

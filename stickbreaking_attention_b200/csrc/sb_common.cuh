@@ -226,8 +226,8 @@ __device__ inline void zero_tail_grads(const KArgs& a, int first, int64_t thread
 constexpr int kMapEncodeFailed = -1000;
 int launch_prep(const SbParams& p, const WsLayout& L, cudaStream_t st);
 int launch_drem(const SbParams& p, const KArgs& a, cudaStream_t st);
-int launch_simt_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
-int launch_simt_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
+int launch_f32_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
+int launch_f32_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 bool tensor_path_eligible(const SbParams& p, bool backward, int* why);
 int launch_tensor_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 int launch_tensor_bwd_tile(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);  // sequences of one tile

@@ -1,0 +1,773 @@
+// Kernels of float32 precision: forward, backward-dq and backward-dk/dv.
+//
+// They serve float32 inputs (whose products must not be rounded to bf16/tf32), head dims other than 32, 64 and
+// 128, and tensors whose strides the TMA path cannot take.  Structure mirrors the tensor-core kernels:
+//   * forward walks the key tiles of one query block right to left and carries, per row, the running
+//     product W = prod(1 - beta) of everything to the right (the reference carries its log,
+//     stickbreaking_attention/sb_varlen/sb_varlen_fwd.py:53-66,155-193);
+//   * the value of W at every 32-key boundary is saved ("carry_w") so that the backward can enter any quarter
+//     directly instead of subtracting from the row total as the reference does (sb_varlen_bwd.py:396-445);
+//   * backward-dq walks left to right carrying the prefix sum of g = A * dA (sb_varlen_bwd.py:438-449) and saves
+//     it at every boundary ("carry_c");
+//   * backward-dk/dv keeps one 64-key tile stationary and walks the query blocks below it, entering each
+//     32-key quarter with the two saved carries; dk and dv are accumulated in registers and stored once, so there is no
+//     atomic or lock on the data (the reference uses a spin lock per key tile, sb_varlen_bwd.py:11-53).
+//
+// Arithmetic.  A value is written as a sum of bf16 terms: x = x0 + x1 + x2 with x0 = bf16(x), x1 = bf16(x - x0), x2 = bf16(x - x0 - x1).
+// One term holds a bf16 value, two an f16 value, three the 24 bits of a float32, all exactly.  Every product runs on the tensor
+// cores as the sum of the term products x_i y_j with i + j <= 2, accumulated in float32: what is left out, x1 y2 and smaller, is
+// below 2^-25 |x y|, a unit of which float32 multiply-adds lose as much in every addition.  Weights and score gradients are
+// float32 values and enter the second products in three terms.  exp and division are the accurate ones (no fast math here).
+//
+// What bounds them: the latency of the chain load -> scores -> scan -> second product of a tile, with the issue slots of the per-score
+// arithmetic behind it.  (warp-level mma takes 1024 multiply-adds per clock and SM, measured: a 64 x 64 x 64 product costs 256
+// clocks for bf16 inputs, 768 where one side is float32 and 1536 where both are, against 2048 on the FMA pipes at their peak.
+// tcgen05 would take an eighth, but its operands would have to pass through shared memory, three tiles each, where here P and dS
+// stay in registers from the scores to the second product.)  So a block has eight warps where registers allow it, and the keys of
+// a tile are stored in an order that makes the keys of a thread neighbours: the scan along a row is a serial one in registers
+// and one over four lanes.
+// us per kernel, forward / dq / dk,dv:                          scalar FMA kernels   FMA register tiles   now
+//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    642 / 825 / 1028     201 / 297 / 363      145 / 191 / 311
+//   4 x 8 heads x 500 tokens, bf16, head dim 50:                 186 / 235 / 280       76 / 106 / 119       47 /  58 / 107
+//   4 heads, 512 float32 tokens, head dim 64:                     53 /  72 /  82       27 /  37 /  31       24 /  35 /  61
+#include "sb_common.cuh"
+
+namespace sb {
+
+namespace {
+
+constexpr int kBM = 64;   // query rows per block
+constexpr int kBN = 64;   // keys per tile
+
+template <typename T> struct Terms;
+template <> struct Terms<__nv_bfloat16> { static constexpr int n = 1; };
+template <> struct Terms<__half> { static constexpr int n = 2; };
+template <> struct Terms<float> { static constexpr int n = 3; };
+constexpr int kWTerms = 3;  // weights and score gradients
+
+// An operand tile in shared memory: N planes (terms) of 64 rows of DP bf16 values; rows are 16 bytes longer, which spreads the
+// eight rows of a matrix load over all banks.
+template <int DP> constexpr int kPitch = DP + 8;
+template <int DP> constexpr int kPlane = 64 * kPitch<DP>;
+template <typename T, int DP> constexpr int kTileElems = Terms<T>::n * kPlane<DP>;
+
+// Where row r of a tile is stored.  A lane = 4 g + t holds of a 16 x 8 accumulator block the elements (g, 2t), (g, 2t + 1), (g + 8, 2t),
+// (g + 8, 2t + 1).
+enum Order { kPlain, kKeyColumns, kKeyRows };
+template <int kOrder>
+__device__ __forceinline__ int stored_row(int r) {
+    const int k = r & 31;
+    // keys along the columns of four blocks (32 keys): key 8 t + 2 n + e in block n, column 2 t + e: a thread has eight neighbours
+    if (kOrder == kKeyColumns) return (r & 32) + 8 * ((k >> 1) & 3) + 2 * (k >> 3) + (k & 1);
+    // keys along the rows of two blocks: key 4 g + 2 m + h in block m, row 8 h + g: a thread has four neighbours
+    if (kOrder == kKeyRows) return (r & 32) + 16 * ((k >> 1) & 1) + 8 * (k & 1) + (k >> 2);
+    return r;
+}
+
+// two values -> N packed terms
+template <int N>
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&t)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        t[i] = *(const uint32_t*)&h;
+        if (i + 1 < N) {
+            const float a = __uint_as_float(t[i] << 16), b = __uint_as_float(t[i] & 0xffff0000u);
+            x = a == x ? 0.f : x - a;  // the comparison keeps an infinity out of the later terms
+            y = b == y ? 0.f : y - b;
+        }
+    }
+}
+
+// kU consecutive elements as float32
+template <typename T, int kU>
+__device__ __forceinline__ void load_unit(const T* src, float (&x)[kU]) {
+    if constexpr (sizeof(T) == 4) {
+        if constexpr (kU == 4) {
+            const float4 v = *(const float4*)src;
+            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        } else if constexpr (kU == 2) {
+            const float2 v = *(const float2*)src;
+            x[0] = v.x; x[1] = v.y;
+        } else {
+            x[0] = to_f32<T>(*src);
+        }
+    } else {
+        T v[kU];
+        if constexpr (kU == 4) *(uint2*)v = *(const uint2*)src;
+        else if constexpr (kU == 2) *(uint32_t*)v = *(const uint32_t*)src;
+        else v[0] = *src;
+#pragma unroll
+        for (int i = 0; i < kU; ++i) x[i] = to_f32<T>(v[i]);
+    }
+}
+// whether rows can be read or written in units of u elements
+template <typename T>
+__device__ __forceinline__ bool units_ok(const MatView& m, int D, int u) {
+    return ((D | m.st | m.sh | m.sb) & (u - 1)) == 0 && ((uintptr_t)m.ptr & (u * sizeof(T) - 1)) == 0;
+}
+
+// 64 rows of a [.., T, D] tensor into a tile, zeros behind the valid rows and columns.  A thread keeps its columns and walks the rows.
+template <int kT, typename T, int DP, int kOrder, int kU>
+__device__ __forceinline__ void load_tile_u(__nv_bfloat16* dst, const T* base, int64_t st, int D, int rows_valid) {
+    constexpr int kN = Terms<T>::n;
+    constexpr int kPer = DP / kU;                      // threads per row
+    constexpr int kStep = kT / kPer;                   // rows per pass
+    constexpr int kPasses = 64 / kStep > 0 ? 64 / kStep : 1;
+    constexpr int kBatch = kPasses < 8 ? kPasses : 8;  // loads in flight
+    const int d = kU * ((int)threadIdx.x % kPer), r0 = (int)threadIdx.x / kPer;
+    const T* src = base + r0 * st + d;
+    const bool col_ok = d < D;
+#pragma unroll 1
+    for (int i0 = 0; i0 < kPasses; i0 += kBatch) {
+        float x[kBatch][kU];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+#pragma unroll
+            for (int u = 0; u < kU; ++u) x[i][u] = 0.f;
+            if (col_ok && r0 + (i0 + i) * kStep < rows_valid) load_unit<T, kU>(src + (int64_t)(i0 + i) * kStep * st, x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            const int r = r0 + (i0 + i) * kStep;
+            if (kStep > 64 && r >= 64) continue;
+            __nv_bfloat16* p = dst + stored_row<kOrder>(r) * kPitch<DP> + d;
+            uint32_t a[kN], b[kN];
+            split_pair<kN>(x[i][0], kU > 1 ? x[i][kU > 1 ? 1 : 0] : 0.f, a);
+            if constexpr (kU == 4) split_pair<kN>(x[i][2], x[i][3], b);
+#pragma unroll
+            for (int n = 0; n < kN; ++n) {
+                if constexpr (kU == 4) *(uint2*)(p + n * kPlane<DP>) = make_uint2(a[n], b[n]);
+                else if constexpr (kU == 2) *(uint32_t*)(p + n * kPlane<DP>) = a[n];
+                else *(unsigned short*)(p + n * kPlane<DP>) = (unsigned short)a[n];
+            }
+        }
+    }
+}
+template <int kT, typename T, int DP, int kOrder>
+__device__ __forceinline__ void load_tile(__nv_bfloat16* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
+    const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
+    if (units_ok<T>(m, D, 4)) load_tile_u<kT, T, DP, kOrder, 4>(dst, base, m.st, D, rows_valid);
+    else if (units_ok<T>(m, D, 2)) load_tile_u<kT, T, DP, kOrder, 2>(dst, base, m.st, D, rows_valid);
+    else load_tile_u<kT, T, DP, kOrder, 1>(dst, base, m.st, D, rows_valid);
+}
+
+// ------------------------------------------------------------------------------------------ warp-level matrix instructions
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The tensor cores round every accumulation towards zero, so sums are kept short: the leading products x0 y0 of at most 64 indices
+// are accumulated from zero, all smaller ones (whose rounding does not matter) in a second accumulator, and the two are added
+// with ordinary float32 additions.  Longer sums are float32 additions of such pieces.  Independent accumulators are innermost
+// in the loops: a chain of dependent mma runs at a fraction of the rate.
+
+// c[mb][nb] = A[16 kMB rows] * B[8 kNB rows]^T over D columns; A and B tiles, `a` and `b` at their first rows
+template <int kN, int DP, int kMB, int kNB>
+__device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_bfloat16* a, const __nv_bfloat16* b, int D, int lane) {
+    const __nv_bfloat16* pa = a + (lane & 15) * kPitch<DP> + (lane >> 4) * 8;
+    const __nv_bfloat16* pb = b + ((lane & 7) + ((lane >> 4) << 3)) * kPitch<DP> + ((lane >> 3) & 1) * 8;
+    float small[kMB][kNB][4], first[kMB][kNB][4];  // first: the leading products of the first 64 indices, D > 64
+#pragma unroll
+    for (int m = 0; m < kMB; ++m)
+#pragma unroll
+        for (int n = 0; n < kNB; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[m][n][i] = small[m][n][i] = first[m][n][i] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < D; k += 16) {
+        uint32_t fa[kMB][kN][4];
+#pragma unroll
+        for (int m = 0; m < kMB; ++m)
+#pragma unroll
+            for (int i = 0; i < kN; ++i) ldsm4(fa[m][i], pa + i * kPlane<DP> + m * 16 * kPitch<DP> + k);
+#pragma unroll
+        for (int j = 0; j < kN; ++j) {
+            uint32_t fb[kNB / 2][4];
+#pragma unroll
+            for (int n2 = 0; n2 < kNB / 2; ++n2) ldsm4(fb[n2], pb + j * kPlane<DP> + n2 * 16 * kPitch<DP> + k);
+#pragma unroll
+            for (int i = 0; i < kN; ++i) {
+                if (i + j > 2) continue;
+#pragma unroll
+                for (int n = 0; n < kNB; ++n)
+#pragma unroll
+                    for (int m = 0; m < kMB; ++m)
+                        mma(i + j == 0 ? c[m][n] : small[m][n], fa[m][i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+            }
+        }
+        if (DP > 64 && k + 16 == 64) {  // 64 indices are the longest sum: the second 64 start anew
+#pragma unroll
+            for (int m = 0; m < kMB; ++m)
+#pragma unroll
+                for (int n = 0; n < kNB; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        first[m][n][i] = c[m][n][i];
+                        c[m][n][i] = 0.f;
+                    }
+        }
+    }
+    if (kN > 1 || DP > 64)
+#pragma unroll
+        for (int m = 0; m < kMB; ++m)
+#pragma unroll
+            for (int n = 0; n < kNB; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) c[m][n][i] += DP > 64 ? first[m][n][i] + small[m][n][i] : small[m][n][i];
+}
+
+// acc[mb][DC / 8] += P * X: P = kMB x kNB accumulator blocks in registers (float32, three terms), X a tile whose rows are the contracted
+// index (`x` at the first row and column), DC columns of it, 32 at a time
+template <int kN, int DP, int DC, int kMB, int kNB>
+__device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const float (&p)[kMB][kNB][4], const __nv_bfloat16* x, int lane) {
+    constexpr int kNC = DC < 32 ? DC / 8 : 4;  // column blocks at a time
+    const __nv_bfloat16* px = x + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8;
+    uint32_t fa[kNB / 2][kMB][kWTerms][4];
+#pragma unroll
+    for (int k = 0; k < kNB / 2; ++k)
+#pragma unroll
+        for (int m = 0; m < kMB; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* v = p[m][2 * k + (e >> 1)];
+                uint32_t t[kWTerms];
+                split_pair<kWTerms>(v[2 * (e & 1)], v[2 * (e & 1) + 1], t);
+#pragma unroll
+                for (int i = 0; i < kWTerms; ++i) fa[k][m][i][e] = t[i];
+            }
+#pragma unroll
+    for (int n0 = 0; n0 < DC / 8; n0 += kNC) {
+        float big[kMB][kNC][4] = {}, small[kMB][kNC][4] = {};
+#pragma unroll
+        for (int k = 0; k < kNB / 2; ++k) {
+#pragma unroll
+            for (int j = 0; j < kN; ++j) {
+                uint32_t fb[kNC / 2][4];
+#pragma unroll
+                for (int n2 = 0; n2 < kNC / 2; ++n2) ldsm4_t(fb[n2], px + j * kPlane<DP> + k * 16 * kPitch<DP> + n0 * 8 + n2 * 16);
+#pragma unroll
+                for (int i = 0; i < kWTerms; ++i) {
+                    if (i + j > 2) continue;
+#pragma unroll
+                    for (int n = 0; n < kNC; ++n)
+#pragma unroll
+                        for (int m = 0; m < kMB; ++m)
+                            mma(i + j == 0 ? big[m][n] : small[m][n], fa[k][m][i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < kMB; ++m)
+#pragma unroll
+            for (int n = 0; n < kNC; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[m][n0 + n][i] += big[m][n][i] + small[m][n][i];
+    }
+}
+
+// a row of accumulator blocks (elements i0, i0 + 1 of each) into row `row` of a [.., T, D] tensor
+template <typename T, int DC>
+__device__ __forceinline__ void store_row(const float (&acc)[DC / 8][4], int i0, float scale, const MatView& m, bool pairs, int D, int col0, T* base,
+                                          int row, int t) {
+    T* dst = base + (int64_t)row * m.st;
+#pragma unroll
+    for (int n = 0; n < DC / 8; ++n) {
+        const int d = col0 + 8 * n + 2 * t;
+        T v[2] = {from_f32<T>(acc[n][i0] * scale), from_f32<T>(acc[n][i0 + 1] * scale)};
+        if (pairs) {
+            if (d < D) {
+                if constexpr (sizeof(T) == 4) *(float2*)(dst + d) = make_float2(v[0], v[1]);
+                else *(uint32_t*)(dst + d) = *(const uint32_t*)v;
+            }
+        } else {
+            if (d < D) dst[d] = v[0];
+            if (d + 1 < D) dst[d + 1] = v[1];
+        }
+    }
+}
+
+// sigmoid pieces with full relative accuracy on both sides: beta = sigmoid(s), r = 1 - beta
+__device__ __forceinline__ void sigmoid_pair(float s, float& beta, float& r) {
+    const float e = expf(-fabsf(s));
+    const float inv = 1.0f / (1.0f + e);
+    const float big = inv, small = e * inv;
+    beta = s >= 0.f ? big : small;
+    r = s >= 0.f ? small : big;
+}
+
+// One step of a scan over lanes: combine with the value `off` lanes to the right (left) where there is one.  kSeg: clamp and segment
+// operand of the shuffle (0x1c1f: four lanes, towards larger; 0x1c00: four lanes, towards smaller; 0x1f: the warp).
+template <int kSeg>
+__device__ __forceinline__ float mul_right(float x, int off) {
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 y;\n\t"
+        "shfl.sync.down.b32 y|p, %0, %1, %2, 0xffffffff;\n\t"
+        "@p mul.rn.f32 %0, %0, y;\n\t}" : "+f"(x) : "r"(off), "n"(kSeg));
+    return x;
+}
+template <int kSeg>
+__device__ __forceinline__ float add_right(float x, int off) {
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 y;\n\t"
+        "shfl.sync.down.b32 y|p, %0, %1, %2, 0xffffffff;\n\t"
+        "@p add.rn.f32 %0, %0, y;\n\t}" : "+f"(x) : "r"(off), "n"(kSeg));
+    return x;
+}
+template <int kSeg>
+__device__ __forceinline__ float add_left(float x, int off) {
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 y;\n\t"
+        "shfl.sync.up.b32 y|p, %0, %1, %2, 0xffffffff;\n\t"
+        "@p add.rn.f32 %0, %0, y;\n\t}" : "+f"(x) : "r"(off), "n"(kSeg));
+    return x;
+}
+constexpr int kQuadRight = 0x1c1f, kQuadLeft = 0x1c00, kWarpRight = 0x1f;
+
+// the two warps that share 16 query rows
+__device__ __forceinline__ void pair_sync(int group) { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); }
+
+struct ItemCtx {
+    int qt, b, start, len, slot_base;
+};
+__device__ inline ItemCtx item_ctx(const KArgs& a, int item) {
+    const int2 it = a.items[item];
+    const SeqInfo s = a.seqs[it.x];
+    return ItemCtx{it.y, s.batch, s.start, s.len, s.slot_base};
+}
+// Blocks in the order of the item table (heaviest first), the heads and the halves of a 128-row tile innermost: the hardware
+// deals blocks out in this order, so the heavy ones of all heads start first.
+struct BlockIdx {
+    int item, h, part;
+};
+__device__ __forceinline__ BlockIdx block_idx(int heads) {
+    const int per = heads * 2, item = (int)blockIdx.x / per, rest = (int)blockIdx.x - item * per;
+    return BlockIdx{item, rest >> 1, rest & 1};
+}
+__device__ __forceinline__ int64_t linear_thread() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * blockDim.x; }
+
+// ------------------------------------------------------------------------------------------ forward
+// Eight warps: four groups of 16 query rows x the two 32-key halves of a tile.  The halves exchange their products once per tile; o
+// is summed over the halves at the end.
+template <typename T, int DP>
+__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 256, kN = Terms<T>::n;
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __shared__ float xs[2][kBM];  // product of 1 - beta over a half, per row
+    __nv_bfloat16* sQ = tiles;
+    __nv_bfloat16* sK = sQ + kTileElems<T, DP>;
+    __nv_bfloat16* sV = sK + kTileElems<T, DP>;
+    pdl_wait();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_rows<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
+    const BlockIdx bi = block_idx(a.heads);
+    if (bi.item >= a.hdr->n_items) return;
+    const ItemCtx c = item_ctx(a, bi.item);
+    const int h = bi.h, D = a.head_dim;
+    const int row0 = c.qt * kTileQ + bi.part * kBM;
+    if (row0 >= c.len) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int rg = warp & 3, hf = warp >> 2;  // hf 0: the left 32 keys, 1: the right
+    const int rows_valid = min(kBM, c.len - row0);
+    load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+    const int wrow = 16 * rg + g;  // this lane's rows of the block: wrow, wrow + 8
+    float W[2] = {1.f, 1.f};
+    float o[1][DP / 8][4] = {};
+    float* cw = a.carry_w ? a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ + bi.part * kBM + wrow : nullptr;
+    const int last = (row0 + rows_valid - 1) / kBN;
+    // key tiles of the 128-key diagonal tile that lie right of these rows: a tensor-core backward may follow, and it reads the
+    // carry of every quarter of its tile
+    if (cw && t == 0)
+        for (int kh = last + 1; kh <= 2 * c.qt + 1 && kh * kBN < c.len; ++kh)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) cw[carry_slot32(c.slot_base, c.qt, 2 * kh + hf) * kTileQ + 8 * r] = 1.f;
+
+    for (int kh = last; kh >= 0; --kh) {
+        const int key0 = kh * kBN;
+        const int keys_valid = min(kBN, c.len - key0);
+        __syncthreads();
+        load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        __syncthreads();
+        float s[1][4][4], om[2][8], excl[2];
+        product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
+        const bool edge = kh == last || keys_valid < kBN;  // some pair of the tile is not visible
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float beta[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sigmoid_pair(s[0][j >> 1][2 * r + (j & 1)] * a.inv_temp, beta[j], om[r][j]);
+            if (edge) {
+                const int lim = min(keys_valid, row0 + wrow + 8 * r + a.attend_current - key0) - 32 * hf - 8 * t;  // keys < lim of this lane are visible
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j >= lim) { beta[j] = 0.f; om[r][j] = 1.f; }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[0][j >> 1][2 * r + (j & 1)] = beta[j];
+            float incl = ((om[r][0] * om[r][1]) * (om[r][2] * om[r][3])) * ((om[r][4] * om[r][5]) * (om[r][6] * om[r][7]));
+            incl = mul_right<kQuadRight>(incl, 1);
+            incl = mul_right<kQuadRight>(incl, 2);
+            const float y = __shfl_down_sync(0xffffffffu, incl, 1, 4);
+            excl[r] = t == 3 ? 1.f : y;
+            if (t == 0) xs[hf][wrow + 8 * r] = incl;  // over the whole half
+        }
+        pair_sync(rg);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float right = xs[1][wrow + 8 * r], left = xs[0][wrow + 8 * r];
+            const float win = hf ? W[r] : W[r] * right;  // at the right edge of this half
+            if (cw && t == 0) cw[carry_slot32(c.slot_base, c.qt, 2 * kh + hf) * kTileQ + 8 * r] = win;
+            float run = win * excl[r];
+#pragma unroll
+            for (int j = 7; j >= 0; --j) {
+                s[0][j >> 1][2 * r + (j & 1)] *= run;
+                run *= om[r][j];
+            }
+            W[r] = W[r] * right * left;
+        }
+        product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
+    }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    float* x = (float*)tiles;
+    __syncthreads();
+    if (hf == 1) {
+#pragma unroll
+        for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
+    }
+    __syncthreads();
+    if (hf == 1) return;
+#pragma unroll
+    for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+    const bool pairs = units_ok<T>(a.o, D, 2);
+    T* base = (T*)a.o.ptr + (int64_t)c.b * a.o.sb + (int64_t)h * a.o.sh + (int64_t)(c.start + row0) * a.o.st;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        if (wrow + 8 * r >= rows_valid) continue;
+        store_row<T, DP>(o[0], 2 * r, 1.f, a.o, pairs, D, 0, base, wrow + 8 * r, t);
+        if (t == 0) {
+            const int64_t tok = c.start + row0 + wrow + 8 * r;
+            ((T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + tok * a.rem.st] = from_f32<T>(W[r]);
+            ((float*)a.nla.ptr)[(int64_t)c.b * a.nla.sb + (int64_t)h * a.nla.sh + tok * a.nla.st] = log2f(W[r]);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------ backward: dq
+// Warps as in the forward; W comes from the forward's carries, the halves exchange their sums of g.
+template <typename T, int DP>
+__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 256, kN = Terms<T>::n;
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __shared__ float xs[2][kBM];  // sum of g over a half, per row
+    __nv_bfloat16* sQ = tiles;
+    __nv_bfloat16* sG = sQ + kTileElems<T, DP>;  // dO
+    __nv_bfloat16* sK = sG + kTileElems<T, DP>;
+    __nv_bfloat16* sV = sK + kTileElems<T, DP>;
+    pdl_wait();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
+    const BlockIdx bi = block_idx(a.heads);
+    if (bi.item >= a.hdr->n_items) return;
+    const ItemCtx c = item_ctx(a, bi.item);
+    const int h = bi.h, D = a.head_dim;
+    const int row0 = c.qt * kTileQ + bi.part * kBM;
+    if (row0 >= c.len) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int rg = warp & 3, hf = warp >> 2;
+    const int rows_valid = min(kBM, c.len - row0);
+    load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+    load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+    const int wrow = 16 * rg + g;
+    float drem[2], prefix[2] = {0.f, 0.f};  // prefix: sum of g over all keys left of the current tile
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int64_t tok = c.start + row0 + wrow + 8 * r;
+        drem[r] = wrow + 8 * r < rows_valid ? to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + tok * a.d_rem.st]) : 0.f;
+    }
+    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ + bi.part * kBM + wrow;
+    float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ + bi.part * kBM + wrow;
+    float o[1][DP / 8][4] = {};
+    const int last = (row0 + rows_valid - 1) / kBN;
+
+    for (int kh = 0; kh <= last; ++kh) {
+        const int key0 = kh * kBN;
+        const int keys_valid = min(kBN, c.len - key0);
+        __syncthreads();
+        load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+        load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        const int64_t slot = carry_slot32(c.slot_base, c.qt, 2 * kh + hf) * kTileQ;
+        float W[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) W[r] = wrow + 8 * r < rows_valid ? cw[slot + 8 * r] : 0.f;
+        __syncthreads();
+        float s[1][4][4], dp[1][4][4], excl[2];
+        product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
+        product_nt<kN, DP, 1, 4>(dp, sG + 16 * rg * kPitch<DP>, sV + 32 * hf * kPitch<DP>, D, lane);
+        const bool edge = kh == last || keys_valid < kBN;
+        // right to left: s <- beta, dp <- g
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float beta[8], om[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sigmoid_pair(s[0][j >> 1][2 * r + (j & 1)] * a.inv_temp, beta[j], om[j]);
+            if (edge) {
+                const int lim = min(keys_valid, row0 + wrow + 8 * r + a.attend_current - key0) - 32 * hf - 8 * t;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j >= lim) { beta[j] = 0.f; om[j] = 1.f; }
+            }
+            float incl = ((om[0] * om[1]) * (om[2] * om[3])) * ((om[4] * om[5]) * (om[6] * om[7]));
+            incl = mul_right<kQuadRight>(incl, 1);
+            incl = mul_right<kQuadRight>(incl, 2);
+            const float y = __shfl_down_sync(0xffffffffu, incl, 1, 4);
+            float run = W[r] * (t == 3 ? 1.f : y);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 7; j >= 0; --j) {
+                float& d = dp[0][j >> 1][2 * r + (j & 1)];
+                d = beta[j] * run * (d - drem[r]);
+                sum += d;
+                run *= om[j];
+                s[0][j >> 1][2 * r + (j & 1)] = beta[j];
+            }
+            float upto = add_left<kQuadLeft>(sum, 1);
+            upto = add_left<kQuadLeft>(upto, 2);
+            const float z = __shfl_up_sync(0xffffffffu, upto, 1, 4);
+            excl[r] = t == 0 ? 0.f : z;
+            if (t == 3) xs[hf][wrow + 8 * r] = upto;  // over the whole half
+        }
+        pair_sync(rg);
+        // left to right: s <- ds = g - beta * (prefix of g including the key)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float right = xs[1][wrow + 8 * r], left = xs[0][wrow + 8 * r];
+            const float base = hf ? prefix[r] + left : prefix[r];  // at the left edge of this half
+            if (t == 0 && wrow + 8 * r < rows_valid) cc[slot + 8 * r] = base + (hf ? right : left);  // prefix through the half's right edge
+            float cin = base + excl[r];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float gj = dp[0][j >> 1][2 * r + (j & 1)];
+                float& sj = s[0][j >> 1][2 * r + (j & 1)];
+                cin += gj;
+                sj = gj - sj * cin;
+            }
+            prefix[r] = prefix[r] + left + right;
+        }
+        product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
+    }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    float* x = (float*)tiles;
+    __syncthreads();
+    if (hf == 1) {
+#pragma unroll
+        for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
+    }
+    __syncthreads();
+    if (hf == 1) return;
+#pragma unroll
+    for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+    const bool pairs = units_ok<T>(a.dq, D, 2);
+    T* base = (T*)a.dq.ptr + (int64_t)c.b * a.dq.sb + (int64_t)h * a.dq.sh + (int64_t)(c.start + row0) * a.dq.st;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        if (wrow + 8 * r < rows_valid) store_row<T, DP>(o[0], 2 * r, a.inv_temp, a.dq, pairs, D, 0, base, wrow + 8 * r, t);
+}
+
+// ------------------------------------------------------------------------------------------ backward: dk, dv
+// Scores transposed (rows = keys), so that P^T and dS^T come out of the first products in the form in which the second ones take
+// them.  Four warps: the two 32-key quarters (each entered with its own carries) x the halves of the 64 queries for D <= 64, whose
+// dk, dv are added at the end, or the halves of the columns of dk, dv for D > 64 (two accumulators of 32 x 128 do not fit a
+// thread's registers), whose scores are formed twice.
+template <typename T, int DP>
+__global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 128, kN = Terms<T>::n;
+    constexpr bool kSplitCols = DP > 64;
+    constexpr int kDC = kSplitCols ? DP / 2 : DP;  // columns of dk, dv per warp
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __nv_bfloat16* sK = tiles;
+    __nv_bfloat16* sV = sK + kTileElems<T, DP>;
+    __nv_bfloat16* sQ = sV + kTileElems<T, DP>;
+    __nv_bfloat16* sG = sQ + kTileElems<T, DP>;
+    pdl_wait();
+    const BlockIdx bi = block_idx(a.heads);
+    const int n_items = a.hdr->n_items;
+    if (bi.item >= n_items) return;
+    // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
+    const ItemCtx c = item_ctx(a, n_items - 1 - bi.item);
+    const int h = bi.h, D = a.head_dim;
+    const int key0 = c.qt * kTileQ + bi.part * kBN;
+    if (key0 >= c.len) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int kq = warp & 1, part = warp >> 1;
+    const int keys_valid = min(kBN, c.len - key0);
+    load_tile<kT, T, DP, kKeyRows>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+    load_tile<kT, T, DP, kKeyRows>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+    const int col0 = kSplitCols ? part * kDC : 0;
+    const int quarter = key0 / 32 + kq;            // of the sequence
+    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
+    const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
+    float ok[2][kDC / 8][4] = {}, ov[2][kDC / 8][4] = {};
+    const int n_qb = (c.len + kBM - 1) / kBM;
+
+    for (int qb = key0 / kBM; qb < n_qb; ++qb) {
+        const int row0 = qb * kBM;
+        const int rows_valid = min(kBM, c.len - row0);
+        __syncthreads();
+        load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        __syncthreads();
+        const int64_t slot = carry_slot32(c.slot_base, qb >> 1, quarter) * kTileQ + (qb & 1) * kBM;
+        const bool edge = qb == key0 / kBM || keys_valid < kBN;
+#pragma unroll 1
+        for (int half = kSplitCols ? 0 : part; half < (kSplitCols ? 2 : part + 1); ++half) {
+            float s[2][4][4], dp[2][4][4];
+            product_nt<kN, DP, 2, 4>(s, sK + 32 * kq * kPitch<DP>, sQ + 32 * half * kPitch<DP>, D, lane);
+            product_nt<kN, DP, 2, 4>(dp, sV + 32 * kq * kPitch<DP>, sG + 32 * half * kPitch<DP>, D, lane);
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {  // a query column of this lane: keys 32 kq + 4 g + (0 ... 3)
+                    const int q = 32 * half + 8 * n + 2 * t + e;
+                    float W = 0.f, cr = 0.f, drem = 0.f;
+                    if (q < rows_valid) {
+                        W = cw[slot + q];
+                        cr = cc[slot + q];
+                        drem = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
+                    }
+                    float beta[4], om[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) sigmoid_pair(s[k >> 1][n][2 * (k & 1) + e] * a.inv_temp, beta[k], om[k]);
+                    if (edge) {
+                        const int lim = min(keys_valid, row0 + q + a.attend_current - key0) - 32 * kq - 4 * g;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k >= lim) { beta[k] = 0.f; om[k] = 1.f; }
+                    }
+                    float incl = (om[0] * om[1]) * (om[2] * om[3]);
+#pragma unroll
+                    for (int off = 4; off < 32; off <<= 1) incl = mul_right<kWarpRight>(incl, off);
+                    const float y = __shfl_down_sync(0xffffffffu, incl, 4);
+                    float run = W * (g == 7 ? 1.f : y);
+                    float gk[4];
+#pragma unroll
+                    for (int k = 3; k >= 0; --k) {
+                        const float p = beta[k] * run;
+                        run *= om[k];
+                        gk[k] = p * (dp[k >> 1][n][2 * (k & 1) + e] - drem);
+                        s[k >> 1][n][2 * (k & 1) + e] = p;
+                    }
+                    float from = (gk[0] + gk[1]) + (gk[2] + gk[3]);
+#pragma unroll
+                    for (int off = 4; off < 32; off <<= 1) from = add_right<kWarpRight>(from, off);
+                    const float z = __shfl_down_sync(0xffffffffu, from, 4);
+                    // inclusive prefix at a key = (prefix through the quarter's right edge) - (sum of g right of it)
+                    float cin = cr - (g == 7 ? 0.f : z);
+#pragma unroll
+                    for (int k = 3; k >= 0; --k) {
+                        dp[k >> 1][n][2 * (k & 1) + e] = gk[k] - beta[k] * cin;
+                        cin -= gk[k];
+                    }
+                }
+            product_px<kN, DP, kDC, 2, 4>(ov, s, sG + 32 * half * kPitch<DP> + col0, lane);
+            product_px<kN, DP, kDC, 2, 4>(ok, dp, sQ + 32 * half * kPitch<DP> + col0, lane);
+        }
+    }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    if (!kSplitCols) {  // add the two query halves: warps 2, 3 hand theirs over through shared memory
+        float* x = (float*)tiles;
+        __syncthreads();
+        if (part == 1) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int idx = ((m * (kDC / 8) + n) * 4 + e) * 64 + kq * 32 + lane;
+                        x[idx] = ok[m][n][e];
+                        x[idx + 64 * kDC] = ov[m][n][e];
+                    }
+        }
+        __syncthreads();
+        if (part == 1) return;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int idx = ((m * (kDC / 8) + n) * 4 + e) * 64 + kq * 32 + lane;
+                    ok[m][n][e] += x[idx];
+                    ov[m][n][e] += x[idx + 64 * kDC];
+                }
+    }
+    const bool pk = units_ok<T>(a.dk, D, 2), pv = units_ok<T>(a.dv, D, 2);
+    T* bk = (T*)a.dk.ptr + (int64_t)c.b * a.dk.sb + (int64_t)h * a.dk.sh + (int64_t)(c.start + key0) * a.dk.st;
+    T* bv = (T*)a.dv.ptr + (int64_t)c.b * a.dv.sb + (int64_t)h * a.dv.sh + (int64_t)(c.start + key0) * a.dv.st;
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int row = 32 * kq + 4 * g + 2 * m + hh;
+            if (row >= keys_valid) continue;
+            store_row<T, kDC>(ok[m], 2 * hh, a.inv_temp, a.dk, pk, D, col0, bk, row, t);
+            store_row<T, kDC>(ov[m], 2 * hh, 1.f, a.dv, pv, D, col0, bv, row, t);
+        }
+}
+
+template <typename T, int DP>
+int launch_one(void (*kernel)(KArgs), int threads, int tiles, const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    const int smem = tiles * kTileElems<T, DP> * 2;
+    const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
+    if (e != 0) return e;
+    return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * 2), dim3(threads), smem, st, a);
+}
+template <typename T, int DP>
+int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
+    if (!backward) return launch_one<T, DP>(f32_fwd_kernel<T, DP>, 256, 3, L, a, st);
+    if (phases != SBATTN_BWD_DKDV) {
+        const int e = launch_one<T, DP>(f32_bwd_dq_kernel<T, DP>, 256, 4, L, a, st);
+        if (e != 0) return e;
+    }
+    return phases != SBATTN_BWD_DQ ? launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP>, 128, 4, L, a, st) : 0;
+}
+template <typename T>
+int launch_t(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
+    if (a.head_dim > 64) return launch_d<T, 128>(backward, L, a, phases, st);
+    if (a.head_dim > 32) return launch_d<T, 64>(backward, L, a, phases, st);
+    return a.head_dim > 16 ? launch_d<T, 32>(backward, L, a, phases, st) : launch_d<T, 16>(backward, L, a, phases, st);
+}
+int launch_any(const SbParams& p, bool backward, const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    if (L.max_items <= 0) return 0;
+    switch (p.dtype) {
+        case SBATTN_BF16: return launch_t<__nv_bfloat16>(backward, L, a, p.bwd_phases, st);
+        case SBATTN_F16: return launch_t<__half>(backward, L, a, p.bwd_phases, st);
+        default: return launch_t<float>(backward, L, a, p.bwd_phases, st);
+    }
+}
+
+}  // namespace
+
+int launch_f32_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) { return launch_any(p, false, L, a, st); }
+int launch_f32_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) { return launch_any(p, true, L, a, st); }
+
+}  // namespace sb
