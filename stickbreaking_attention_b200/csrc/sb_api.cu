@@ -78,7 +78,21 @@ KArgs make_args(const SbParams& p, const WsLayout& L) {
     a.d_o = view(p.d_o); a.dq = view(p.dq); a.dk = view(p.dk); a.dv = view(p.dv);
     a.rem = view(p.rem); a.nla = view(p.neg_log_acc); a.d_rem = view(p.d_rem);
     a.status = p.status;
+    a.cu_seqlens = p.cu_seqlens;
+    a.cu_width = p.cu_width;
+    a.n_seqs = L.n_seqs;
+    a.batch = p.batch;
+    a.max_len = p.batch > 0 ? p.tokens : (p.max_seqlen > 0 ? p.max_seqlen : p.tokens);
+    a.n_max = L.n_max;
+    a.max_items = L.max_items;
     return a;
+}
+
+// Small forwards do without the prep kernel: its launch costs the host ~2.5 us and the GPU ~3 us of the 13 us of a forward over a
+// few short sequences.  Up to two items per SM, which then are dealt out in turn: beyond that the blocks should draw their
+// items from the counter, which only a kernel before this one can set to zero.
+bool forward_builds_tables(const SbParams& p, const WsLayout& L) {
+    return L.n_seqs <= 32 && L.max_items <= 256 && (int64_t)L.max_items * p.heads <= 2 * 148;
 }
 
 // 0: SIMT, 1: tensor, <0: error
@@ -141,12 +155,15 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     if (path < 0) return path;
     if ((p->flags & SBATTN_FLAG_FUSED_REMAINDER) && path != 1) return SBATTN_EUNSUPPORTED;  // tensor-core kernels only
     cudaStream_t st = (cudaStream_t)p->stream;
-    if (launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
-    const KArgs a = make_args(*p, L);
+    KArgs a = make_args(*p, L);
+    a.own_tables = path == 1 && forward_builds_tables(*p, L);
+    if (!a.own_tables && launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
     int e = path == 1 ? launch_tensor_fwd(*p, L, a, st) : launch_f32_fwd(*p, L, a, st);
     // a layout the tensor-map encoder refuses (nothing has been launched yet): the other kernels take any strides
-    if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER))
+    if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER)) {
+        if (a.own_tables && launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
         e = launch_f32_fwd(*p, L, a, st);
+    }
     return e == 0 ? SBATTN_OK : (e == kMapEncodeFailed ? SBATTN_EUNSUPPORTED : SBATTN_ECUDA);
 }
 

@@ -118,6 +118,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     uint32_t* tmem_slot = (uint32_t*)(ring + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     float* xw = (float*)(tmem_slot + 4);  // [quarter][128 rows]: carry leaving the quarter its thread has just swept
+    OwnTables* own = (OwnTables*)(xw + 512 + 384);
     float* wfin = xw + 512;               // [item mod 3][128 rows]: remainder of the row, for the fused epilogue (read one item late)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -148,12 +149,17 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const uint32_t tmem = *tmem_slot;
     pdl_wait();
     pdl_launch_dependents();
-    if (a.zero_tail && a.hdr->covered_end < a.tokens) {
-        const int64_t me = (int64_t)blockIdx.x * kFwdThreads + tid, all = (int64_t)gridDim.x * kFwdThreads;
-        if (kF16) zero_tail_rows<__half>(a, a.hdr->covered_end, me, all);
-        else zero_tail_rows<__nv_bfloat16>(a, a.hdr->covered_end, me, all);
+    if (a.own_tables) {
+        if (warp == 0) build_own_tables(a, own, lane);
+        __syncthreads();
     }
-    const int n_items = a.hdr->n_items;
+    const int covered_end = a.own_tables ? own->covered_end : a.hdr->covered_end;
+    if (a.zero_tail && covered_end < a.tokens) {
+        const int64_t me = (int64_t)blockIdx.x * kFwdThreads + tid, all = (int64_t)gridDim.x * kFwdThreads;
+        if (kF16) zero_tail_rows<__half>(a, covered_end, me, all);
+        else zero_tail_rows<__nv_bfloat16>(a, covered_end, me, all);
+    }
+    const int n_items = a.own_tables ? own->n_items : a.hdr->n_items;
     const int n_work = *abort_flag ? 0 : n_items * a.heads;
 
     if (warp == 16) {
@@ -165,8 +171,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
             SchedProducer sched;
             int w;
             Work wk;
-            const auto fetch = [&](int w_) { return fetch_work(a, n_items, w_); };
-            while (ok && (w = sched.next(a.sched + 0, n_work, ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, fetch, wk)) >= 0) {
+            const int2* items = a.own_tables ? own->items : a.items;
+            const SeqInfo* seqs = a.own_tables ? own->seqs : a.seqs;
+            const auto fetch = [&](int w_) { return fetch_work(a, items, seqs, n_items, w_); };
+            while (ok && (w = sched.next(a.own_tables ? nullptr : a.sched + 0, n_work, ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, fetch, wk)) >= 0) {
                 ok = mbar_wait_idle(&bars[Q_EMPTY], ph_qe, abort_flag);
                 ph_qe ^= 1;
                 if (!ok) break;
@@ -423,7 +431,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         if (kDefer && ok && have_pend) store_item();  // the block's last item
     }
     tc_teardown(abort_flag, a.status, tmem, kTmemCols, 17);
-    sched_finish(a.sched + 0);
+    if (!a.own_tables) sched_finish(a.sched + 0);
 }
 
 template <int D, bool kF16>
@@ -438,7 +446,7 @@ int launch_fwd_t(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStrea
         encode_tile_map(&mv, p.v.ptr, kind, hd, p.tokens, p.heads, B, p.v.stride_t, p.v.stride_h, p.v.stride_b, kBN))
         return kMapEncodeFailed;
     // Q + three K stages + two V stages; at least 120 KB so that one block owns the SM and its tensor memory
-    constexpr int need = (1 + kKStages + kVStages) * kBM * D * 2 + 1024 + 5120;  // tiles, alignment, barriers and exchange slots
+    constexpr int need = (1 + kKStages + kVStages) * kBM * D * 2 + 1024 + 5120 + (int)sizeof(OwnTables);  // tiles, alignment, barriers and exchange slots
     constexpr int smem = need > 120 * 1024 ? need : 120 * 1024;
     const auto launch = [&](auto kernel) {
         const int e = ensure_kernel_attrs((const void*)kernel, smem, false);

@@ -6,6 +6,7 @@
 // Reference counterparts: StickBreakingAttention (stickbreaking_attention/sb_varlen/__init__.py:23-67,
 // sb_attn/__init__.py:15-53), varlen_fwd / varlen_bwd (sb_varlen/sb_varlen_fwd.py:411-452, sb_varlen_bwd.py:483-539).
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -122,7 +123,10 @@ Tensor prep_cu(const Tensor& cu, const Tensor& q, std::optional<int64_t>& max_se
 }
 
 Tensor unit_inner(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+// Allocations past the dispatcher (~0.5 us each less): the caching allocator's memory all the same
+Tensor empty_like_dtype(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype) { return at::detail::empty_cuda(sizes, dtype, t.device(), std::nullopt); }
 Tensor empty_rows(const Tensor& t) {
+    if (t.is_non_overlapping_and_dense() && t.stride(-1) == 1) return at::detail::empty_strided_cuda(t.sizes(), t.strides(), t.scalar_type(), t.device());
     Tensor out = at::empty_like(t);
     return out.stride(-1) == 1 ? out : at::empty(t.sizes(), t.options());
 }
@@ -171,12 +175,13 @@ SbParams base_params(const Tensor& q, const Tensor& cu, const Opts& o, bool save
     return p;
 }
 
-Tensor bytes(size_t n, const Tensor& like) { return at::empty({(int64_t)n}, like.options().dtype(at::kByte)); }
+Tensor bytes(size_t n, const Tensor& like) { return empty_like_dtype(like, {(int64_t)n}, at::kByte); }
 
 struct FwdOut {
     Tensor o, rem, nla, ws;
 };
-FwdOut forward(Tensor q, Tensor k, Tensor v, const Tensor& cu, const Opts& opt, bool save) {
+// want_nla: neg_log_acc as a tensor of its own; otherwise it lies behind the workspace, where nobody reads it
+FwdOut forward(Tensor q, Tensor k, Tensor v, const Tensor& cu, const Opts& opt, bool save, bool want_nla) {
     require_cuda(q);
     c10::cuda::OptionalCUDAGuard guard(q.device());
     q = unit_inner(q);
@@ -186,18 +191,23 @@ FwdOut forward(Tensor q, Tensor k, Tensor v, const Tensor& cu, const Opts& opt, 
     out.o = empty_rows(q);
     const auto rows = q.sizes().slice(0, q.dim() - 1);
     // no zero-fill: the library writes every row of rem and neg_log_acc
-    out.rem = at::empty(rows, q.options());
-    out.nla = at::empty(rows, q.options().dtype(at::kFloat));
+    out.rem = empty_like_dtype(q, rows, q.scalar_type());
+    if (want_nla) out.nla = empty_like_dtype(q, rows, at::kFloat);
     SbParams p = base_params(q, cu, opt, save);
     size_t fb = 0;
     check(sbattn_workspace_bytes(&p, &fb, nullptr), "sbattn_workspace_bytes");
-    out.ws = bytes(fb, q);
+    out.ws = bytes(fb + (want_nla ? 0 : 4 * (size_t)out.rem.numel()), q);  // fb is a multiple of 4
     p.q = mat(q, opt.batched);
     p.k = mat(k, opt.batched);
     p.v = mat(v, opt.batched);
     p.o = mat(out.o, opt.batched);
     p.rem = vec(out.rem, opt.batched);
-    p.neg_log_acc = vec(out.nla, opt.batched);
+    if (want_nla) {
+        p.neg_log_acc = vec(out.nla, opt.batched);
+    } else {
+        p.neg_log_acc = vec(out.rem, opt.batched);  // same shape, contiguous as well
+        p.neg_log_acc.ptr = (char*)out.ws.data_ptr() + fb;
+    }
     p.fwd_workspace = out.ws.data_ptr();
     p.fwd_workspace_bytes = fb;
     check(sbattn_fwd(&p), "sbattn_fwd");
@@ -272,7 +282,7 @@ struct StickBreaking : public torch::autograd::Function<StickBreaking> {
                                                   bool fused, bool recompute, int64_t path) {
         const Opts opt{batched, max_seqlens, scale, attend_current, fused, (int)path};
         const Tensor cu = cu_seqlens.value_or(Tensor());
-        FwdOut r = ::forward(q, k, v, cu, opt, !recompute);
+        FwdOut r = ::forward(q, k, v, cu, opt, !recompute, false);
         ctx->save_for_backward({q, k, v, cu, recompute ? Tensor() : r.ws, r.rem});
         ctx->saved_data["o"] = c10::ivalue::Tuple::create({batched, max_seqlens, scale, attend_current, fused, recompute, path});
         return {r.o, r.rem};
@@ -283,7 +293,7 @@ struct StickBreaking : public torch::autograd::Function<StickBreaking> {
         const auto& e = tuple->elements();
         const Opts opt{e[0].toBool(), e[1].toInt(), e[2].toDouble(), e[3].toBool(), e[4].toBool(), (int)e[6].toInt()};
         const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &cu = saved[3];
-        const Tensor ws = e[5].toBool() ? ::forward(q, k, v, cu, opt, true).ws : saved[4];
+        const Tensor ws = e[5].toBool() ? ::forward(q, k, v, cu, opt, true, false).ws : saved[4];
         const auto g = ::backward(grads[0], grads[1], q, k, v, cu, ws, saved[5], opt, 0, {}, std::nullopt);
         Tensor none;
         return {g[0], g[1], g[2], none, none, none, none, none, none, none, none};
@@ -309,7 +319,7 @@ std::pair<Tensor, Tensor> attend(const Tensor& q, const Tensor& k, const Tensor&
         auto r = StickBreaking::apply(q, k, v, batched ? OptTensor() : OptTensor(cu), batched, *max_seqlens, scale, attend_current, fused, recompute, (int64_t)path);
         return done(r[0], r[1]);
     }
-    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path}, false);
+    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path}, false, false);
     return done(r.o, r.rem);
 }
 
@@ -323,7 +333,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> fwd(const Tensor& q, const Tensor& k,
     Tensor cu;
     if (batched) max_seqlens = q.size(2);
     else cu = prep_cu(*cu_seqlens, q, max_seqlens);
-    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path}, !no_grad);
+    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path}, !no_grad, true);
     return {r.o, r.rem, r.nla, r.ws};
 }
 // varlen_bwd / attn_bwd: (dq, dk, dv)

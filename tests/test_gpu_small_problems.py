@@ -1,0 +1,57 @@
+"""Small forwards build the table of work items inside the kernel; larger ones take it from a kernel of its own."""
+import numpy as np
+import pytest
+import torch
+
+from util import synth
+
+pytestmark = pytest.mark.gpu
+
+PACKS = {
+    "one": [1],
+    "ragged": [130, 0, 257, 64, 1, 0, 128],
+    "most_sequences": [(37 * i) % 200 for i in range(32)],   # 32 sequences: the last count that builds its own table
+    "too_many": [(37 * i) % 200 for i in range(33)],
+    "one_long": [128 * 96 + 5],
+}
+
+
+def _run(q, k, v, do, dr, cu, m):
+    from stickbreaking_attention_b200 import launch_count, sb_attn_varlen
+    q, k, v = (x.clone().requires_grad_() for x in (q, k, v))
+    before = launch_count()
+    o, rem = sb_attn_varlen(q, k, v, cu, m, zero_start=False)
+    torch.cuda.synchronize()
+    launches = launch_count() - before
+    return launches, (o.detach(), rem.detach()) + torch.autograd.grad([o, rem], [q, k, v], [do, dr])
+
+
+@pytest.mark.parametrize("cu_dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("name", sorted(PACKS))
+def test_own_tables_give_the_same_bits(name, cu_dtype):
+    """The first head alone (own table) against the same head among so many that the table kernel runs; tokens behind the last
+    sequence included."""
+    lengths, pad, D = PACKS[name], 7, 64
+    T = sum(lengths) + pad
+    H = 296 // (T // 128 + len(lengths)) + 1  # one head more than the rule allows
+    q, k, v, do, dr = (torch.from_numpy(x).to("cuda", torch.bfloat16) for x in synth(H, T, D, 41))
+    cu = torch.tensor(np.cumsum(lengths), dtype=cu_dtype, device="cuda")
+    m = max(lengths)
+    n_all, want = _run(q, k, v, do, dr, cu, m)
+    n_one, got = _run(q[:1], k[:1], v[:1], do[:1], dr[:1], cu, m)
+    assert n_all == 2 and n_one == (2 if name == "too_many" else 1)
+    covered = T - pad
+    assert torch.equal(got[0][:, :covered], want[0][:1, :covered])  # rows of o behind the last sequence are left alone
+    for a, b in zip(got[1:], want[1:]):
+        assert torch.equal(a, b[:1])
+
+
+def test_own_tables_report_bad_sequence_ends():
+    import stickbreaking_attention_b200 as sb
+    q = torch.randn(1, 256, 64, device="cuda", dtype=torch.bfloat16)
+    sb.check_status()
+    for ends, m in ([200, 100], 256), ([100, 300], 256), ([100, 256], 120):
+        with pytest.raises(ValueError):
+            sb.sb_attn_varlen(q, q, q, torch.tensor(ends, device="cuda"), m, zero_start=False)
+            sb.check_status()
+    assert sb.check_status() == 0
