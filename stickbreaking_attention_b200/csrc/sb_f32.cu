@@ -159,6 +159,12 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) 
                  : "r"((uint32_t)__cvta_generic_to_shared(p))
                  : "memory");
 }
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];"
+                 : "=r"(r[0]), "=r"(r[1])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p))
+                 : "memory");
+}
 __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const __nv_bfloat16* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -197,7 +203,8 @@ __device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_b
             for (int i = 0; i < kN; ++i) ldsm4(fa[m][i], pa + i * kPlane<DP> + m * 16 * kPitch<DP> + k);
 #pragma unroll
         for (int j = 0; j < kN; ++j) {
-            uint32_t fb[kNB / 2][4];
+            uint32_t fb[(kNB + 1) / 2][4];
+            if constexpr (kNB == 1) ldsm2(fb[0], pb + j * kPlane<DP> + k);
 #pragma unroll
             for (int n2 = 0; n2 < kNB / 2; ++n2) ldsm4(fb[n2], pb + j * kPlane<DP> + n2 * 16 * kPitch<DP> + k);
 #pragma unroll
@@ -593,15 +600,169 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
 }
 
 // ------------------------------------------------------------------------------------------ backward: dk, dv
-// Scores transposed (rows = keys), so that P^T and dS^T come out of the first products in the form in which the second ones take
-// them.  Four warps: the two 32-key quarters (each entered with its own carries) x the halves of the 64 queries for D <= 64, whose
-// dk, dv are added at the end, or the halves of the columns of dk, dv for D > 64 (two accumulators of 32 x 128 do not fit a
-// thread's registers), whose scores are formed twice.
+// One query column of a block of transposed scores, keys 4 g ... 4 g + 3 of a quarter: s <- weights, dp <- ds.  W and cr enter at the
+// quarter's right edge (product of 1 - beta to the right, sum of g through it); keys >= lim of the lane's four are not visible.
+__device__ __forceinline__ void column(float* const (&s)[4], float* const (&dp)[4], float inv_temp, bool edge, int lim, float W, float cr, float drem, int g) {
+    float beta[4], om[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sigmoid_pair(*s[k] * inv_temp, beta[k], om[k]);
+    if (edge) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k >= lim) { beta[k] = 0.f; om[k] = 1.f; }
+    }
+    float incl = (om[0] * om[1]) * (om[2] * om[3]);
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) incl = mul_right<kWarpRight>(incl, off);
+    const float y = __shfl_down_sync(0xffffffffu, incl, 4);
+    float run = W * (g == 7 ? 1.f : y);
+    float gk[4];
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+        const float p = beta[k] * run;
+        run *= om[k];
+        gk[k] = p * (*dp[k] - drem);
+        *s[k] = p;
+    }
+    float from = (gk[0] + gk[1]) + (gk[2] + gk[3]);
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) from = add_right<kWarpRight>(from, off);
+    const float z = __shfl_down_sync(0xffffffffu, from, 4);
+    // inclusive prefix at a key = (prefix through the quarter's right edge) - (sum of g right of it)
+    float cin = cr - (g == 7 ? 0.f : z);
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+        *dp[k] = gk[k] - beta[k] * cin;
+        cin -= gk[k];
+    }
+}
+
+// Scores transposed (rows = keys).  Sixteen warps.  First half of a step: two 32-key quarters (each entered with its own carries) x eight
+// groups of 8 queries; P^T and dS^T go to shared memory as three terms each.  Second half: four groups of 16 keys x {dv, dk} x
+// the two halves of the columns, so that a thread accumulates 16 or 32 values only.  (With P^T and dS^T kept in registers four
+// warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 107 and 311 us in the lines above.)
 template <typename T, int DP>
-__global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kT = 128, kN = Terms<T>::n;
-    constexpr bool kSplitCols = DP > 64;
-    constexpr int kDC = kSplitCols ? DP / 2 : DP;  // columns of dk, dv per warp
+__global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 512, kN = Terms<T>::n;
+    constexpr int kDC = DP >= 32 ? DP / 2 : DP;     // columns of dk or dv per warp
+    constexpr int kPP = kPitch<64>, kPPlane = kPlane<64>;  // P^T, dS^T: [64 keys][64 queries], three planes each
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __nv_bfloat16* sK = tiles;
+    __nv_bfloat16* sV = sK + kTileElems<T, DP>;
+    __nv_bfloat16* sQ = sV + kTileElems<T, DP>;
+    __nv_bfloat16* sG = sQ + kTileElems<T, DP>;
+    __nv_bfloat16* sP = sG + kTileElems<T, DP>;
+    __nv_bfloat16* sS = sP + kWTerms * kPPlane;
+    pdl_wait();
+    const BlockIdx bi = block_idx(a.heads);
+    const int n_items = a.hdr->n_items;
+    if (bi.item >= n_items) return;
+    // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
+    const ItemCtx c = item_ctx(a, n_items - 1 - bi.item);
+    const int h = bi.h, D = a.head_dim;
+    const int key0 = c.qt * kTileQ + bi.part * kBN;
+    if (key0 >= c.len) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int kq = warp & 1, q0 = 8 * (warp >> 1);                                     // first half of a step
+    const int kg = warp & 3, col0 = (warp >> 3) * kDC;                                 // second half
+    const bool is_dk = (warp >> 2) & 1, second = col0 < DP;                            // (head dim 16: the columns are not split)
+    const int keys_valid = min(kBN, c.len - key0);
+    load_tile<kT, T, DP, kKeyRows>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+    load_tile<kT, T, DP, kKeyRows>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+    const int quarter = key0 / 32 + kq;            // of the sequence
+    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
+    const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
+    float acc[kDC / 8][4] = {};
+    const int n_qb = (c.len + kBM - 1) / kBM;
+
+    for (int qb = key0 / kBM; qb < n_qb; ++qb) {
+        const int row0 = qb * kBM;
+        const int rows_valid = min(kBM, c.len - row0);
+        __syncthreads();
+        load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        const int64_t slot = carry_slot32(c.slot_base, qb >> 1, quarter) * kTileQ + (qb & 1) * kBM;
+        float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int q = q0 + 2 * t + e;
+            if (q < rows_valid) {
+                W[e] = cw[slot + q];
+                cr[e] = cc[slot + q];
+                drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
+            }
+        }
+        __syncthreads();
+        const bool edge = qb == key0 / kBM || keys_valid < kBN;
+        float s[2][1][4], dp[2][1][4];
+        product_nt<kN, DP, 2, 1>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
+        product_nt<kN, DP, 2, 1>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
+            float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
+            column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q0 + 2 * t + e + a.attend_current - key0) - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                uint32_t tp[kWTerms], ts[kWTerms];
+                split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
+                split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
+                const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
+#pragma unroll
+                for (int i = 0; i < kWTerms; ++i) {
+                    *(uint32_t*)(sP + i * kPPlane + at) = tp[i];
+                    *(uint32_t*)(sS + i * kPPlane + at) = ts[i];
+                }
+            }
+        __syncthreads();
+        if (second) {
+            const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
+            const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
+            float big[kDC / 8][4] = {}, small[kDC / 8][4] = {};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                uint32_t fa[kWTerms][4];
+#pragma unroll
+                for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
+#pragma unroll
+                for (int j = 0; j < kN; ++j) {
+                    uint32_t fb[kDC / 16][4];
+#pragma unroll
+                    for (int n2 = 0; n2 < kDC / 16; ++n2) ldsm4_t(fb[n2], px + j * kPlane<DP> + k * 16 * kPitch<DP> + n2 * 16);
+#pragma unroll
+                    for (int i = 0; i < kWTerms; ++i) {
+                        if (i + j > 2) continue;
+#pragma unroll
+                        for (int n = 0; n < kDC / 8; ++n) mma(i + j == 0 ? big[n] : small[n], fa[i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[n][i] += big[n][i] + small[n][i];
+        }
+    }
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    if (!second) return;
+    const MatView m = is_dk ? a.dk : a.dv;
+    const bool pairs = units_ok<T>(m, D, 2);
+    T* base = (T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + key0) * m.st;
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int row = 32 * (kg >> 1) + 4 * g + 2 * (kg & 1) + hh;
+        if (row < keys_valid) store_row<T, kDC>(acc, 2 * hh, is_dk ? a.inv_temp : 1.f, m, pairs, D, col0, base, row, t);
+    }
+}
+
+// float32 at D > 64, where the operand tiles leave no room for P^T and dS^T: four warps, the two 32-key quarters x the halves of the
+// columns of dk, dv, both scored by the warp itself and kept in registers.
+template <typename T, int DP>
+__global__ void __launch_bounds__(128, 1) f32_bwd_dkdv_wide_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 128, kN = Terms<T>::n, kDC = DP / 2;
     extern __shared__ __align__(16) __nv_bfloat16 tiles[];
     __nv_bfloat16* sK = tiles;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
@@ -621,7 +782,7 @@ __global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(cons
     const int keys_valid = min(kBN, c.len - key0);
     load_tile<kT, T, DP, kKeyRows>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
     load_tile<kT, T, DP, kKeyRows>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
-    const int col0 = kSplitCols ? part * kDC : 0;
+    const int col0 = part * kDC;
     const int quarter = key0 / 32 + kq;            // of the sequence
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
@@ -638,7 +799,7 @@ __global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(cons
         const int64_t slot = carry_slot32(c.slot_base, qb >> 1, quarter) * kTileQ + (qb & 1) * kBM;
         const bool edge = qb == key0 / kBM || keys_valid < kBN;
 #pragma unroll 1
-        for (int half = kSplitCols ? 0 : part; half < (kSplitCols ? 2 : part + 1); ++half) {
+        for (int half = 0; half < 2; ++half) {
             float s[2][4][4], dp[2][4][4];
             product_nt<kN, DP, 2, 4>(s, sK + 32 * kq * kPitch<DP>, sQ + 32 * half * kPitch<DP>, D, lane);
             product_nt<kN, DP, 2, 4>(dp, sV + 32 * kq * kPitch<DP>, sG + 32 * half * kPitch<DP>, D, lane);
@@ -653,73 +814,15 @@ __global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(cons
                         cr = cc[slot + q];
                         drem = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
                     }
-                    float beta[4], om[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) sigmoid_pair(s[k >> 1][n][2 * (k & 1) + e] * a.inv_temp, beta[k], om[k]);
-                    if (edge) {
-                        const int lim = min(keys_valid, row0 + q + a.attend_current - key0) - 32 * kq - 4 * g;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k >= lim) { beta[k] = 0.f; om[k] = 1.f; }
-                    }
-                    float incl = (om[0] * om[1]) * (om[2] * om[3]);
-#pragma unroll
-                    for (int off = 4; off < 32; off <<= 1) incl = mul_right<kWarpRight>(incl, off);
-                    const float y = __shfl_down_sync(0xffffffffu, incl, 4);
-                    float run = W * (g == 7 ? 1.f : y);
-                    float gk[4];
-#pragma unroll
-                    for (int k = 3; k >= 0; --k) {
-                        const float p = beta[k] * run;
-                        run *= om[k];
-                        gk[k] = p * (dp[k >> 1][n][2 * (k & 1) + e] - drem);
-                        s[k >> 1][n][2 * (k & 1) + e] = p;
-                    }
-                    float from = (gk[0] + gk[1]) + (gk[2] + gk[3]);
-#pragma unroll
-                    for (int off = 4; off < 32; off <<= 1) from = add_right<kWarpRight>(from, off);
-                    const float z = __shfl_down_sync(0xffffffffu, from, 4);
-                    // inclusive prefix at a key = (prefix through the quarter's right edge) - (sum of g right of it)
-                    float cin = cr - (g == 7 ? 0.f : z);
-#pragma unroll
-                    for (int k = 3; k >= 0; --k) {
-                        dp[k >> 1][n][2 * (k & 1) + e] = gk[k] - beta[k] * cin;
-                        cin -= gk[k];
-                    }
+                    float* const ps[4] = {&s[0][n][e], &s[0][n][2 + e], &s[1][n][e], &s[1][n][2 + e]};
+                    float* const pd[4] = {&dp[0][n][e], &dp[0][n][2 + e], &dp[1][n][e], &dp[1][n][2 + e]};
+                    column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q + a.attend_current - key0) - 32 * kq - 4 * g, W, cr, drem, g);
                 }
             product_px<kN, DP, kDC, 2, 4>(ov, s, sG + 32 * half * kPitch<DP> + col0, lane);
             product_px<kN, DP, kDC, 2, 4>(ok, dp, sQ + 32 * half * kPitch<DP> + col0, lane);
         }
     }
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
-    if (!kSplitCols) {  // add the two query halves: warps 2, 3 hand theirs over through shared memory
-        float* x = (float*)tiles;
-        __syncthreads();
-        if (part == 1) {
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int n = 0; n < kDC / 8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int idx = ((m * (kDC / 8) + n) * 4 + e) * 64 + kq * 32 + lane;
-                        x[idx] = ok[m][n][e];
-                        x[idx + 64 * kDC] = ov[m][n][e];
-                    }
-        }
-        __syncthreads();
-        if (part == 1) return;
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int n = 0; n < kDC / 8; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int idx = ((m * (kDC / 8) + n) * 4 + e) * 64 + kq * 32 + lane;
-                    ok[m][n][e] += x[idx];
-                    ov[m][n][e] += x[idx + 64 * kDC];
-                }
-    }
     const bool pk = units_ok<T>(a.dk, D, 2), pv = units_ok<T>(a.dv, D, 2);
     T* bk = (T*)a.dk.ptr + (int64_t)c.b * a.dk.sb + (int64_t)h * a.dk.sh + (int64_t)(c.start + key0) * a.dk.st;
     T* bv = (T*)a.dv.ptr + (int64_t)c.b * a.dv.sb + (int64_t)h * a.dv.sh + (int64_t)(c.start + key0) * a.dv.st;
@@ -735,20 +838,22 @@ __global__ void __launch_bounds__(128, DP > 64 ? 1 : 2) f32_bwd_dkdv_kernel(cons
 }
 
 template <typename T, int DP>
-int launch_one(void (*kernel)(KArgs), int threads, int tiles, const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    const int smem = tiles * kTileElems<T, DP> * 2;
+int launch_one(void (*kernel)(KArgs), int threads, int tiles, int more, const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    const int smem = tiles * kTileElems<T, DP> * 2 + more;
     const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
     if (e != 0) return e;
     return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * 2), dim3(threads), smem, st, a);
 }
 template <typename T, int DP>
 int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
-    if (!backward) return launch_one<T, DP>(f32_fwd_kernel<T, DP>, 256, 3, L, a, st);
+    if (!backward) return launch_one<T, DP>(f32_fwd_kernel<T, DP>, 256, 3, 0, L, a, st);
     if (phases != SBATTN_BWD_DKDV) {
-        const int e = launch_one<T, DP>(f32_bwd_dq_kernel<T, DP>, 256, 4, L, a, st);
+        const int e = launch_one<T, DP>(f32_bwd_dq_kernel<T, DP>, 256, 4, 0, L, a, st);
         if (e != 0) return e;
     }
-    return phases != SBATTN_BWD_DQ ? launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP>, 128, 4, L, a, st) : 0;
+    if (phases == SBATTN_BWD_DQ) return 0;
+    if constexpr (DP > 64 && Terms<T>::n == 3) return launch_one<T, DP>(f32_bwd_dkdv_wide_kernel<T, DP>, 128, 4, 0, L, a, st);
+    else return launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP>, 512, 4, 2 * kWTerms * kPlane<64> * 2, L, a, st);
 }
 template <typename T>
 int launch_t(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
