@@ -27,9 +27,9 @@
 // a tile are stored in an order that makes the keys of a thread neighbours: the scan along a row is a serial one in registers
 // and one over four lanes.
 // us per kernel, forward / dq / dk,dv:                          scalar FMA kernels   FMA register tiles   now
-//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    642 / 825 / 1028     201 / 297 / 363      145 / 191 / 311
-//   4 x 8 heads x 500 tokens, bf16, head dim 50:                 186 / 235 / 280       76 / 106 / 119       47 /  58 / 107
-//   4 heads, 512 float32 tokens, head dim 64:                     53 /  72 /  82       27 /  37 /  31       24 /  35 /  61
+//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    642 / 825 / 1028     201 / 297 / 363      143 / 193 / 282
+//   4 x 8 heads x 500 tokens, bf16, head dim 50:                 186 / 235 / 280       76 / 106 / 119       47 /  57 /  60
+//   4 heads, 512 float32 tokens, head dim 64:                     53 /  72 /  82       27 /  37 /  31       25 /  35 /  30
 #include "sb_common.cuh"
 
 namespace sb {
@@ -107,13 +107,13 @@ __device__ __forceinline__ bool units_ok(const MatView& m, int D, int u) {
     return ((D | m.st | m.sh | m.sb) & (u - 1)) == 0 && ((uintptr_t)m.ptr & (u * sizeof(T) - 1)) == 0;
 }
 
-// 64 rows of a [.., T, D] tensor into a tile, zeros behind the valid rows and columns.  A thread keeps its columns and walks the rows.
-template <int kT, typename T, int DP, int kOrder, int kU>
+// kRows rows of a [.., T, D] tensor into a tile, zeros behind the valid rows and columns.  A thread keeps its columns and walks the rows.
+template <int kT, typename T, int DP, int kOrder, int kRows, int kU>
 __device__ __forceinline__ void load_tile_u(__nv_bfloat16* dst, const T* base, int64_t st, int D, int rows_valid) {
     constexpr int kN = Terms<T>::n;
     constexpr int kPer = DP / kU;                      // threads per row
     constexpr int kStep = kT / kPer;                   // rows per pass
-    constexpr int kPasses = 64 / kStep > 0 ? 64 / kStep : 1;
+    constexpr int kPasses = kRows / kStep > 0 ? kRows / kStep : 1;
     constexpr int kBatch = kPasses < 8 ? kPasses : 8;  // loads in flight
     const int d = kU * ((int)threadIdx.x % kPer), r0 = (int)threadIdx.x / kPer;
     const T* src = base + r0 * st + d;
@@ -130,26 +130,26 @@ __device__ __forceinline__ void load_tile_u(__nv_bfloat16* dst, const T* base, i
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
             const int r = r0 + (i0 + i) * kStep;
-            if (kStep > 64 && r >= 64) continue;
+            if (kStep > kRows && r >= kRows) continue;
             __nv_bfloat16* p = dst + stored_row<kOrder>(r) * kPitch<DP> + d;
             uint32_t a[kN], b[kN];
             split_pair<kN>(x[i][0], kU > 1 ? x[i][kU > 1 ? 1 : 0] : 0.f, a);
             if constexpr (kU == 4) split_pair<kN>(x[i][2], x[i][3], b);
 #pragma unroll
             for (int n = 0; n < kN; ++n) {
-                if constexpr (kU == 4) *(uint2*)(p + n * kPlane<DP>) = make_uint2(a[n], b[n]);
-                else if constexpr (kU == 2) *(uint32_t*)(p + n * kPlane<DP>) = a[n];
-                else *(unsigned short*)(p + n * kPlane<DP>) = (unsigned short)a[n];
+                if constexpr (kU == 4) *(uint2*)(p + n * kRows * kPitch<DP>) = make_uint2(a[n], b[n]);
+                else if constexpr (kU == 2) *(uint32_t*)(p + n * kRows * kPitch<DP>) = a[n];
+                else *(unsigned short*)(p + n * kRows * kPitch<DP>) = (unsigned short)a[n];
             }
         }
     }
 }
-template <int kT, typename T, int DP, int kOrder>
+template <int kT, typename T, int DP, int kOrder, int kRows = 64>
 __device__ __forceinline__ void load_tile(__nv_bfloat16* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
     const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
-    if (units_ok<T>(m, D, 4)) load_tile_u<kT, T, DP, kOrder, 4>(dst, base, m.st, D, rows_valid);
-    else if (units_ok<T>(m, D, 2)) load_tile_u<kT, T, DP, kOrder, 2>(dst, base, m.st, D, rows_valid);
-    else load_tile_u<kT, T, DP, kOrder, 1>(dst, base, m.st, D, rows_valid);
+    if (units_ok<T>(m, D, 4)) load_tile_u<kT, T, DP, kOrder, kRows, 4>(dst, base, m.st, D, rows_valid);
+    else if (units_ok<T>(m, D, 2)) load_tile_u<kT, T, DP, kOrder, kRows, 2>(dst, base, m.st, D, rows_valid);
+    else load_tile_u<kT, T, DP, kOrder, kRows, 1>(dst, base, m.st, D, rows_valid);
 }
 
 // ------------------------------------------------------------------------------------------ warp-level matrix instructions
@@ -182,8 +182,8 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
 // with ordinary float32 additions.  Longer sums are float32 additions of such pieces.  Independent accumulators are innermost
 // in the loops: a chain of dependent mma runs at a fraction of the rate.
 
-// c[mb][nb] = A[16 kMB rows] * B[8 kNB rows]^T over D columns; A and B tiles, `a` and `b` at their first rows
-template <int kN, int DP, int kMB, int kNB>
+// c[mb][nb] = A[16 kMB rows] * B[8 kNB rows]^T over D columns; A and B tiles, `a` and `b` at their first rows, B of kRowsB rows
+template <int kN, int DP, int kMB, int kNB, int kRowsB = 64>
 __device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_bfloat16* a, const __nv_bfloat16* b, int D, int lane) {
     const __nv_bfloat16* pa = a + (lane & 15) * kPitch<DP> + (lane >> 4) * 8;
     const __nv_bfloat16* pb = b + ((lane & 7) + ((lane >> 4) << 3)) * kPitch<DP> + ((lane >> 3) & 1) * 8;
@@ -204,9 +204,9 @@ __device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_b
 #pragma unroll
         for (int j = 0; j < kN; ++j) {
             uint32_t fb[(kNB + 1) / 2][4];
-            if constexpr (kNB == 1) ldsm2(fb[0], pb + j * kPlane<DP> + k);
+            if constexpr (kNB == 1) ldsm2(fb[0], pb + j * kRowsB * kPitch<DP> + k);
 #pragma unroll
-            for (int n2 = 0; n2 < kNB / 2; ++n2) ldsm4(fb[n2], pb + j * kPlane<DP> + n2 * 16 * kPitch<DP> + k);
+            for (int n2 = 0; n2 < kNB / 2; ++n2) ldsm4(fb[n2], pb + j * kRowsB * kPitch<DP> + n2 * 16 * kPitch<DP> + k);
 #pragma unroll
             for (int i = 0; i < kN; ++i) {
                 if (i + j > 2) continue;
@@ -640,18 +640,22 @@ __device__ __forceinline__ void column(float* const (&s)[4], float* const (&dp)[
 // Scores transposed (rows = keys).  Sixteen warps.  First half of a step: two 32-key quarters (each entered with its own carries) x eight
 // groups of 8 queries; P^T and dS^T go to shared memory as three terms each.  Second half: four groups of 16 keys x {dv, dk} x
 // the two halves of the columns, so that a thread accumulates 16 or 32 values only.  (With P^T and dS^T kept in registers four
-// warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 107 and 311 us in the lines above.)
-template <typename T, int DP>
+// warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 311 and 107 us in the first two lines at the top.)
+// kQ: queries per step, 64, or 32 where the tiles would not fit otherwise (float32 at D > 64; eight of the warps then sit out the
+// first half; forward + backward of 8 heads, 4096 tokens, head dim 128: 1638 us with four warps that kept P^T and dS^T in registers,
+// 1163 us so)
+template <typename T, int DP, int kQ>
 __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
     constexpr int kT = 512, kN = Terms<T>::n;
     constexpr int kDC = DP >= 32 ? DP / 2 : DP;     // columns of dk or dv per warp
-    constexpr int kPP = kPitch<64>, kPPlane = kPlane<64>;  // P^T, dS^T: [64 keys][64 queries], three planes each
+    constexpr int kPP = kQ + 8, kPPlane = 64 * kPP;  // P^T, dS^T: [64 keys][kQ queries], three planes each
+    constexpr int kQTile = kN * kQ * kPitch<DP>;     // Q, dO: kQ rows
     extern __shared__ __align__(16) __nv_bfloat16 tiles[];
     __nv_bfloat16* sK = tiles;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
     __nv_bfloat16* sQ = sV + kTileElems<T, DP>;
-    __nv_bfloat16* sG = sQ + kTileElems<T, DP>;
-    __nv_bfloat16* sP = sG + kTileElems<T, DP>;
+    __nv_bfloat16* sG = sQ + kQTile;
+    __nv_bfloat16* sP = sG + kQTile;
     __nv_bfloat16* sS = sP + kWTerms * kPPlane;
     pdl_wait();
     const BlockIdx bi = block_idx(a.heads);
@@ -673,15 +677,13 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
     float acc[kDC / 8][4] = {};
-    const int n_qb = (c.len + kBM - 1) / kBM;
 
-    for (int qb = key0 / kBM; qb < n_qb; ++qb) {
-        const int row0 = qb * kBM;
-        const int rows_valid = min(kBM, c.len - row0);
+    for (int row0 = key0; row0 < c.len; row0 += kQ) {
+        const int rows_valid = min(kQ, c.len - row0);
         __syncthreads();
-        load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
-        load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
-        const int64_t slot = carry_slot32(c.slot_base, qb >> 1, quarter) * kTileQ + (qb & 1) * kBM;
+        load_tile<kT, T, DP, kPlain, kQ>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<kT, T, DP, kPlain, kQ>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, quarter) * kTileQ + row0 % kTileQ;
         float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -693,37 +695,39 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
             }
         }
         __syncthreads();
-        const bool edge = qb == key0 / kBM || keys_valid < kBN;
-        float s[2][1][4], dp[2][1][4];
-        product_nt<kN, DP, 2, 1>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
-        product_nt<kN, DP, 2, 1>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+        const bool edge = row0 < key0 + kBN || keys_valid < kBN;
+        if (q0 < kQ) {
+            float s[2][1][4], dp[2][1][4];
+            product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
+            product_nt<kN, DP, 2, 1, kQ>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
-            float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
-            column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q0 + 2 * t + e + a.attend_current - key0) - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
-        }
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                uint32_t tp[kWTerms], ts[kWTerms];
-                split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
-                split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
-                const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
-#pragma unroll
-                for (int i = 0; i < kWTerms; ++i) {
-                    *(uint32_t*)(sP + i * kPPlane + at) = tp[i];
-                    *(uint32_t*)(sS + i * kPPlane + at) = ts[i];
-                }
+            for (int e = 0; e < 2; ++e) {
+                float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
+                float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
+                column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q0 + 2 * t + e + a.attend_current - key0) - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
             }
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    uint32_t tp[kWTerms], ts[kWTerms];
+                    split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
+                    split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
+                    const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
+#pragma unroll
+                    for (int i = 0; i < kWTerms; ++i) {
+                        *(uint32_t*)(sP + i * kPPlane + at) = tp[i];
+                        *(uint32_t*)(sS + i * kPPlane + at) = ts[i];
+                    }
+                }
+        }
         __syncthreads();
         if (second) {
             const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
             const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
             float big[kDC / 8][4] = {}, small[kDC / 8][4] = {};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < kQ / 16; ++k) {
                 uint32_t fa[kWTerms][4];
 #pragma unroll
                 for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
                 for (int j = 0; j < kN; ++j) {
                     uint32_t fb[kDC / 16][4];
 #pragma unroll
-                    for (int n2 = 0; n2 < kDC / 16; ++n2) ldsm4_t(fb[n2], px + j * kPlane<DP> + k * 16 * kPitch<DP> + n2 * 16);
+                    for (int n2 = 0; n2 < kDC / 16; ++n2) ldsm4_t(fb[n2], px + j * kQ * kPitch<DP> + k * 16 * kPitch<DP> + n2 * 16);
 #pragma unroll
                     for (int i = 0; i < kWTerms; ++i) {
                         if (i + j > 2) continue;
@@ -758,85 +762,6 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
     }
 }
 
-// float32 at D > 64, where the operand tiles leave no room for P^T and dS^T: four warps, the two 32-key quarters x the halves of the
-// columns of dk, dv, both scored by the warp itself and kept in registers.
-template <typename T, int DP>
-__global__ void __launch_bounds__(128, 1) f32_bwd_dkdv_wide_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kT = 128, kN = Terms<T>::n, kDC = DP / 2;
-    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
-    __nv_bfloat16* sK = tiles;
-    __nv_bfloat16* sV = sK + kTileElems<T, DP>;
-    __nv_bfloat16* sQ = sV + kTileElems<T, DP>;
-    __nv_bfloat16* sG = sQ + kTileElems<T, DP>;
-    pdl_wait();
-    const BlockIdx bi = block_idx(a.heads);
-    const int n_items = a.hdr->n_items;
-    if (bi.item >= n_items) return;
-    // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
-    const ItemCtx c = item_ctx(a, n_items - 1 - bi.item);
-    const int h = bi.h, D = a.head_dim;
-    const int key0 = c.qt * kTileQ + bi.part * kBN;
-    if (key0 >= c.len) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int kq = warp & 1, part = warp >> 1;
-    const int keys_valid = min(kBN, c.len - key0);
-    load_tile<kT, T, DP, kKeyRows>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
-    load_tile<kT, T, DP, kKeyRows>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
-    const int col0 = part * kDC;
-    const int quarter = key0 / 32 + kq;            // of the sequence
-    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
-    const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    float ok[2][kDC / 8][4] = {}, ov[2][kDC / 8][4] = {};
-    const int n_qb = (c.len + kBM - 1) / kBM;
-
-    for (int qb = key0 / kBM; qb < n_qb; ++qb) {
-        const int row0 = qb * kBM;
-        const int rows_valid = min(kBM, c.len - row0);
-        __syncthreads();
-        load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
-        load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
-        __syncthreads();
-        const int64_t slot = carry_slot32(c.slot_base, qb >> 1, quarter) * kTileQ + (qb & 1) * kBM;
-        const bool edge = qb == key0 / kBM || keys_valid < kBN;
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-            float s[2][4][4], dp[2][4][4];
-            product_nt<kN, DP, 2, 4>(s, sK + 32 * kq * kPitch<DP>, sQ + 32 * half * kPitch<DP>, D, lane);
-            product_nt<kN, DP, 2, 4>(dp, sV + 32 * kq * kPitch<DP>, sG + 32 * half * kPitch<DP>, D, lane);
-#pragma unroll
-            for (int n = 0; n < 4; ++n)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {  // a query column of this lane: keys 32 kq + 4 g + (0 ... 3)
-                    const int q = 32 * half + 8 * n + 2 * t + e;
-                    float W = 0.f, cr = 0.f, drem = 0.f;
-                    if (q < rows_valid) {
-                        W = cw[slot + q];
-                        cr = cc[slot + q];
-                        drem = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
-                    }
-                    float* const ps[4] = {&s[0][n][e], &s[0][n][2 + e], &s[1][n][e], &s[1][n][2 + e]};
-                    float* const pd[4] = {&dp[0][n][e], &dp[0][n][2 + e], &dp[1][n][e], &dp[1][n][2 + e]};
-                    column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q + a.attend_current - key0) - 32 * kq - 4 * g, W, cr, drem, g);
-                }
-            product_px<kN, DP, kDC, 2, 4>(ov, s, sG + 32 * half * kPitch<DP> + col0, lane);
-            product_px<kN, DP, kDC, 2, 4>(ok, dp, sQ + 32 * half * kPitch<DP> + col0, lane);
-        }
-    }
-    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
-    const bool pk = units_ok<T>(a.dk, D, 2), pv = units_ok<T>(a.dv, D, 2);
-    T* bk = (T*)a.dk.ptr + (int64_t)c.b * a.dk.sb + (int64_t)h * a.dk.sh + (int64_t)(c.start + key0) * a.dk.st;
-    T* bv = (T*)a.dv.ptr + (int64_t)c.b * a.dv.sb + (int64_t)h * a.dv.sh + (int64_t)(c.start + key0) * a.dv.st;
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int row = 32 * kq + 4 * g + 2 * m + hh;
-            if (row >= keys_valid) continue;
-            store_row<T, kDC>(ok[m], 2 * hh, a.inv_temp, a.dk, pk, D, col0, bk, row, t);
-            store_row<T, kDC>(ov[m], 2 * hh, 1.f, a.dv, pv, D, col0, bv, row, t);
-        }
-}
-
 template <typename T, int DP>
 int launch_one(void (*kernel)(KArgs), int threads, int tiles, int more, const WsLayout& L, const KArgs& a, cudaStream_t st) {
     const int smem = tiles * kTileElems<T, DP> * 2 + more;
@@ -852,8 +777,8 @@ int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaS
         if (e != 0) return e;
     }
     if (phases == SBATTN_BWD_DQ) return 0;
-    if constexpr (DP > 64 && Terms<T>::n == 3) return launch_one<T, DP>(f32_bwd_dkdv_wide_kernel<T, DP>, 128, 4, 0, L, a, st);
-    else return launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP>, 512, 4, 2 * kWTerms * kPlane<64> * 2, L, a, st);
+    constexpr int kQ = DP > 64 && Terms<T>::n == 3 ? 32 : 64;
+    return launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP, kQ>, 512, 2, 2 * (2 * Terms<T>::n * kQ * kPitch<DP> + 2 * kWTerms * 64 * (kQ + 8)), L, a, st);
 }
 template <typename T>
 int launch_t(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
