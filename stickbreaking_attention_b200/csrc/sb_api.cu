@@ -89,10 +89,11 @@ KArgs make_args(const SbParams& p, const WsLayout& L) {
 }
 
 // Small forwards do without the prep kernel: its launch costs the host ~2.5 us and the GPU ~3 us of the 13 us of a forward over a
-// few short sequences.  Up to two items per SM, which then are dealt out in turn: beyond that the blocks should draw their
-// items from the counter, which only a kernel before this one can set to zero.
-bool forward_builds_tables(const SbParams& p, const WsLayout& L) {
-    return L.n_seqs <= 32 && L.max_items <= 256 && (int64_t)L.max_items * p.heads <= 2 * 148;
+// few short sequences.  Tensor-core kernel: up to two items per SM, which then are dealt out in turn: beyond that the blocks
+// should draw their items from the counter, which only a kernel before this one can set to zero.  Float32-precision kernel (two
+// blocks per item): while all blocks fit the GPU at once, since each pays for the table.
+bool forward_builds_tables(const SbParams& p, const WsLayout& L, bool tensor) {
+    return L.n_seqs <= kOwnSeqs && L.max_items <= kOwnItems && (int64_t)L.max_items * p.heads <= (tensor ? 2 : 1) * 148;
 }
 
 // 0: SIMT, 1: tensor, <0: error
@@ -156,12 +157,13 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     if ((p->flags & SBATTN_FLAG_FUSED_REMAINDER) && path != 1) return SBATTN_EUNSUPPORTED;  // tensor-core kernels only
     cudaStream_t st = (cudaStream_t)p->stream;
     KArgs a = make_args(*p, L);
-    a.own_tables = path == 1 && forward_builds_tables(*p, L);
+    a.own_tables = forward_builds_tables(*p, L, path == 1);
     if (!a.own_tables && launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
     int e = path == 1 ? launch_tensor_fwd(*p, L, a, st) : launch_f32_fwd(*p, L, a, st);
     // a layout the tensor-map encoder refuses (nothing has been launched yet): the other kernels take any strides
     if (e == kMapEncodeFailed && p->path == SBATTN_PATH_AUTO && !(p->flags & SBATTN_FLAG_FUSED_REMAINDER)) {
         if (a.own_tables && launch_prep(*p, L, st) != 0) return SBATTN_ECUDA;
+        a.own_tables = 0;
         e = launch_f32_fwd(*p, L, a, st);
     }
     return e == 0 ? SBATTN_OK : (e == kMapEncodeFailed ? SBATTN_EUNSUPPORTED : SBATTN_ECUDA);

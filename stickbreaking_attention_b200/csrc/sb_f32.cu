@@ -348,11 +348,12 @@ __device__ __forceinline__ void pair_sync(int group) { asm volatile("bar.sync %0
 struct ItemCtx {
     int qt, b, start, len, slot_base;
 };
-__device__ inline ItemCtx item_ctx(const KArgs& a, int item) {
-    const int2 it = a.items[item];
-    const SeqInfo s = a.seqs[it.x];
+__device__ inline ItemCtx item_ctx(const int2* items, const SeqInfo* seqs, int item) {
+    const int2 it = items[item];
+    const SeqInfo s = seqs[it.x];
     return ItemCtx{it.y, s.batch, s.start, s.len, s.slot_base};
 }
+__device__ inline ItemCtx item_ctx(const KArgs& a, int item) { return item_ctx(a.items, a.seqs, item); }
 // Blocks in the order of the item table (heaviest first), the heads and the halves of a 128-row tile innermost: the hardware
 // deals blocks out in this order, so the heavy ones of all heads start first.
 struct BlockIdx {
@@ -376,11 +377,17 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
     __nv_bfloat16* sQ = tiles;
     __nv_bfloat16* sK = sQ + kTileElems<T, DP>;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
+    __shared__ OwnTables own;
     pdl_wait();
-    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_rows<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
+    if (a.own_tables) {
+        if (threadIdx.x < 32) build_own_tables(a, &own, threadIdx.x);
+        __syncthreads();
+    }
+    const int covered_end = a.own_tables ? own.covered_end : a.hdr->covered_end;
+    if (a.zero_tail && covered_end < a.tokens) zero_tail_rows<T>(a, covered_end, linear_thread(), all_threads());
     const BlockIdx bi = block_idx(a.heads);
-    if (bi.item >= a.hdr->n_items) return;
-    const ItemCtx c = item_ctx(a, bi.item);
+    if (bi.item >= (a.own_tables ? own.n_items : a.hdr->n_items)) return;
+    const ItemCtx c = a.own_tables ? item_ctx(own.items, own.seqs, bi.item) : item_ctx(a, bi.item);
     const int h = bi.h, D = a.head_dim;
     const int row0 = c.qt * kTileQ + bi.part * kBM;
     if (row0 >= c.len) return;

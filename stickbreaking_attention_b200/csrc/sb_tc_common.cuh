@@ -124,77 +124,6 @@ __device__ __forceinline__ Work fetch_work(const KArgs& a, const int2* items, co
 }
 __device__ __forceinline__ Work fetch_work(const KArgs& a, int n_items, int w) { return fetch_work(a, a.items, a.seqs, n_items, w); }
 
-// The tables of prep_kernel for at most 32 sequences and kOwnItems items, built by one warp in shared memory; the launch of that
-// kernel is a quarter of a small forward.  Every block comes to the same order (heaviest first; inside a class by sequence).
-// Block 0 leaves the tables in the workspace for the backward.
-constexpr int kOwnSeqs = 32, kOwnItems = 256;
-struct OwnTables {
-    SeqInfo seqs[kOwnSeqs];
-    int2 items[kOwnItems];
-    int n_items, covered_end;
-};
-__device__ inline void build_own_tables(const KArgs& a, OwnTables* t, int lane) {
-    const auto end_of = [&](int s) { return a.cu_width == 8 ? ((const int64_t*)a.cu_seqlens)[s] : (int64_t)((const int32_t*)a.cu_seqlens)[s]; };
-    int b = 0, start = 0, len = 0, end = 0;
-    bool bad = false;
-    if (lane < a.n_seqs) {
-        if (a.batch > 0) {
-            b = lane;
-            len = a.tokens;
-        } else {
-            const int64_t e1 = end_of(lane), e0 = lane > 0 ? end_of(lane - 1) : 0;
-            bad = e0 < 0 || e1 < e0 || e1 > a.tokens || e1 - e0 > a.max_len;
-            start = (int)e0;
-            len = bad ? 0 : (int)(e1 - e0);
-            end = (int)e1;
-        }
-    }
-    const int n = (len + kTileQ - 1) / kTileQ;
-    int slots = n * (n + 1), total = n;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, slots, off), y = __shfl_up_sync(0xffffffffu, total, off);
-        if (lane >= off) {
-            slots += x;
-            total += y;
-        }
-    }
-    const int total_slots = __shfl_sync(0xffffffffu, slots, 31);
-    total = __shfl_sync(0xffffffffu, total, 31);
-    bad = __any_sync(0xffffffffu, bad) || total > a.max_items || 2 * (int64_t)total_slots > a.slot_cap;
-    const SeqInfo mine{b, start, len, slots - n * (n + 1)};
-    if (lane < a.n_seqs) t->seqs[lane] = mine;
-    end = __shfl_sync(0xffffffffu, end, max(a.n_seqs - 1, 0));
-    const bool out = blockIdx.x == 0;
-    int pos = 0;
-    for (int c = bad ? 0 : a.n_max; c >= 1; --c) {  // sequences with at least c tiles have a tile c - 1
-        const unsigned has = __ballot_sync(0xffffffffu, n >= c);
-        if (n >= c) {
-            const int at = pos + __popc(has & ((1u << lane) - 1u));
-            t->items[at] = make_int2(lane, c - 1);
-            if (out) const_cast<int2*>(a.items)[at] = make_int2(lane, c - 1);
-        }
-        pos += __popc(has);
-    }
-    if (lane == 0) {
-        t->n_items = bad ? 0 : total;
-        t->covered_end = a.batch > 0 ? a.tokens : bad ? 0 : end;
-    }
-    if (out) {
-        WsHeader* hdr = const_cast<WsHeader*>(a.hdr);
-        if (lane < a.n_seqs) const_cast<SeqInfo*>(a.seqs)[lane] = mine;
-        if (lane < 8) hdr->sched[lane] = 0;
-        if (lane == 0) {
-            hdr->n_items = bad ? 0 : total;
-            hdr->n_seqs = a.n_seqs;
-            hdr->total_slots = total_slots;
-            hdr->bad = bad ? 1 : 0;
-            hdr->covered_end = a.batch > 0 ? a.tokens : bad ? 0 : end;
-            if (bad) atomicOr(a.status, SBATTN_ST_BAD_SEQLENS);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------------------------- work scheduler
 // One thread of the block (a TMA producer) draws work indices from a global counter, looks the item up (two dependent
 // global loads) and hands index and item to the other roles through a two-slot ring in shared memory, so that nobody

@@ -26,15 +26,15 @@ def _run(q, k, v, do, dr, cu, m):
     return launches, (o.detach(), rem.detach()) + torch.autograd.grad([o, rem], [q, k, v], [do, dr])
 
 
-@pytest.mark.parametrize("cu_dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("dtype,cu_dtype", [(torch.bfloat16, torch.int32), (torch.bfloat16, torch.int64), (torch.float32, torch.int32)])
 @pytest.mark.parametrize("name", sorted(PACKS))
-def test_own_tables_give_the_same_bits(name, cu_dtype):
+def test_own_tables_give_the_same_bits(name, dtype, cu_dtype):
     """The first head alone (own table) against the same head among so many that the table kernel runs; tokens behind the last
     sequence included."""
     lengths, pad, D = PACKS[name], 7, 64
     T = sum(lengths) + pad
     H = 296 // (T // 128 + len(lengths)) + 1  # one head more than the rule allows
-    q, k, v, do, dr = (torch.from_numpy(x).to("cuda", torch.bfloat16) for x in synth(H, T, D, 41))
+    q, k, v, do, dr = (torch.from_numpy(x).to("cuda", dtype) for x in synth(H, T, D, 41))
     cu = torch.tensor(np.cumsum(lengths), dtype=cu_dtype, device="cuda")
     m = max(lengths)
     n_all, want = _run(q, k, v, do, dr, cu, m)
