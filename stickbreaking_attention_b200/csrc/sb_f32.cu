@@ -30,12 +30,16 @@
 //   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    642 / 825 / 1028     201 / 297 / 363      143 / 193 / 282
 //   4 x 8 heads x 500 tokens, bf16, head dim 50:                 186 / 235 / 280       76 / 106 / 119       47 /  57 /  60
 //   4 heads, 512 float32 tokens, head dim 64:                     53 /  72 /  82       27 /  37 /  31       25 /  35 /  30
+// Back to back (no gaps between launches), before and after loads a tile ahead, two buffers in dk/dv and the cheaper split:
+// 137 / 171 / 265 -> 135 / 168 / 249; 44 / 46 / 48 -> 39 / 42 / 44; 18 / 22 / 25 -> 18 / 22 / 24.
+// 16 heads, 4096 float32 tokens: tensor pipe 49 %, issue slots 47 %, shared memory 56 % busy in dk/dv, 45 / 52 / 37 % in the forward.
 #include "sb_common.cuh"
 
 namespace sb {
 
 namespace {
 
+constexpr int kMaxSmem = 227 * 1024;
 constexpr int kBM = 64;   // query rows per block
 constexpr int kBN = 64;   // keys per tile
 
@@ -64,8 +68,9 @@ __device__ __forceinline__ int stored_row(int r) {
     return r;
 }
 
-// two values -> N packed terms
-template <int N>
+// two values -> N packed terms.  kFinite: the values are known to be (weights are); otherwise an infinity, also one that the
+// rounding to bf16 makes, stays out of the later terms.
+template <int N, bool kFinite = false>
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&t)[N]) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -73,83 +78,123 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&t)[N]) {
         t[i] = *(const uint32_t*)&h;
         if (i + 1 < N) {
             const float a = __uint_as_float(t[i] << 16), b = __uint_as_float(t[i] & 0xffff0000u);
-            x = a == x ? 0.f : x - a;  // the comparison keeps an infinity out of the later terms
-            y = b == y ? 0.f : y - b;
+            x = !kFinite && i == 0 && fabsf(a) == INFINITY ? 0.f : x - a;
+            y = !kFinite && i == 0 && fabsf(b) == INFINITY ? 0.f : y - b;
         }
     }
 }
 
-// kU consecutive elements as float32
-template <typename T, int kU>
-__device__ __forceinline__ void load_unit(const T* src, float (&x)[kU]) {
-    if constexpr (sizeof(T) == 4) {
-        if constexpr (kU == 4) {
-            const float4 v = *(const float4*)src;
-            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-        } else if constexpr (kU == 2) {
-            const float2 v = *(const float2*)src;
-            x[0] = v.x; x[1] = v.y;
-        } else {
-            x[0] = to_f32<T>(*src);
-        }
-    } else {
-        T v[kU];
-        if constexpr (kU == 4) *(uint2*)v = *(const uint2*)src;
-        else if constexpr (kU == 2) *(uint32_t*)v = *(const uint32_t*)src;
-        else v[0] = *src;
-#pragma unroll
-        for (int i = 0; i < kU; ++i) x[i] = to_f32<T>(v[i]);
-    }
-}
 // whether rows can be read or written in units of u elements
 template <typename T>
 __device__ __forceinline__ bool units_ok(const MatView& m, int D, int u) {
     return ((D | m.st | m.sh | m.sb) & (u - 1)) == 0 && ((uintptr_t)m.ptr & (u * sizeof(T) - 1)) == 0;
 }
 
-// kRows rows of a [.., T, D] tensor into a tile, zeros behind the valid rows and columns.  A thread keeps its columns and walks the rows.
-template <int kT, typename T, int DP, int kOrder, int kRows, int kU>
-__device__ __forceinline__ void load_tile_u(__nv_bfloat16* dst, const T* base, int64_t st, int D, int rows_valid) {
-    constexpr int kN = Terms<T>::n;
-    constexpr int kPer = DP / kU;                      // threads per row
-    constexpr int kStep = kT / kPer;                   // rows per pass
-    constexpr int kPasses = kRows / kStep > 0 ? kRows / kStep : 1;
-    constexpr int kBatch = kPasses < 8 ? kPasses : 8;  // loads in flight
-    const int d = kU * ((int)threadIdx.x % kPer), r0 = (int)threadIdx.x / kPer;
-    const T* src = base + r0 * st + d;
-    const bool col_ok = d < D;
-#pragma unroll 1
-    for (int i0 = 0; i0 < kPasses; i0 += kBatch) {
-        float x[kBatch][kU];
+// kRows rows of a [.., T, D] tensor on their way into a tile: fetch() issues the loads, put() splits and stores them, with zeros
+// behind the valid rows and columns.  Between the two lie a barrier and, where registers allow, the work on the tile before.  A
+// thread keeps its columns and walks the rows.
+template <int kT, typename T, int DP, int kRows = 64, int kTileRows = kRows>
+struct Rows {
+    uint32_t w[kRows * DP / kT > 4 ? kRows * DP / kT : 4];
+
+    template <int kU>  // elements per load
+    struct Map {
+        static constexpr int kPer = DP / kU;                      // threads per row
+        static constexpr int kStep = kT / kPer;                   // rows per pass
+        static constexpr int kPasses = kRows / kStep > 0 ? kRows / kStep : 1;
+        static constexpr int kWords = sizeof(T) == 4 ? kU : (kU + 1) / 2;
+    };
+    template <int kU>
+    __device__ __forceinline__ void fetch_u(const T* base, int64_t st, int D, int rows_valid) {
+        using M = Map<kU>;
+        const int d = kU * ((int)threadIdx.x % M::kPer), r0 = (int)threadIdx.x / M::kPer;
+        const T* src = base + r0 * st + d;
+        const bool col_ok = d < D;
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
+        for (int i = 0; i < M::kPasses; ++i) {
+            uint32_t* x = w + i * M::kWords;
 #pragma unroll
-            for (int u = 0; u < kU; ++u) x[i][u] = 0.f;
-            if (col_ok && r0 + (i0 + i) * kStep < rows_valid) load_unit<T, kU>(src + (int64_t)(i0 + i) * kStep * st, x[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-            const int r = r0 + (i0 + i) * kStep;
-            if (kStep > kRows && r >= kRows) continue;
-            __nv_bfloat16* p = dst + stored_row<kOrder>(r) * kPitch<DP> + d;
-            uint32_t a[kN], b[kN];
-            split_pair<kN>(x[i][0], kU > 1 ? x[i][kU > 1 ? 1 : 0] : 0.f, a);
-            if constexpr (kU == 4) split_pair<kN>(x[i][2], x[i][3], b);
-#pragma unroll
-            for (int n = 0; n < kN; ++n) {
-                if constexpr (kU == 4) *(uint2*)(p + n * kRows * kPitch<DP>) = make_uint2(a[n], b[n]);
-                else if constexpr (kU == 2) *(uint32_t*)(p + n * kRows * kPitch<DP>) = a[n];
-                else *(unsigned short*)(p + n * kRows * kPitch<DP>) = (unsigned short)a[n];
+            for (int u = 0; u < M::kWords; ++u) x[u] = 0;
+            if (!col_ok || r0 + i * M::kStep >= rows_valid) continue;
+            const T* p = src + (int64_t)i * M::kStep * st;
+            if constexpr (M::kWords == 4) {
+                const uint4 v = *(const uint4*)p;
+                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+            } else if constexpr (M::kWords == 2) {
+                const uint2 v = *(const uint2*)p;
+                x[0] = v.x; x[1] = v.y;
+            } else if constexpr (sizeof(T) * kU == 4) {
+                x[0] = *(const uint32_t*)p;
+            } else {
+                x[0] = *(const unsigned short*)p;
             }
         }
     }
-}
-template <int kT, typename T, int DP, int kOrder, int kRows = 64>
+    template <int kOrder, int kU>
+    __device__ __forceinline__ void put_u(__nv_bfloat16* dst, int first = 0) const {
+        using M = Map<kU>;
+        constexpr int kN = Terms<T>::n;
+        const int d = kU * ((int)threadIdx.x % M::kPer), r0 = (int)threadIdx.x / M::kPer;
+#pragma unroll
+        for (int i = 0; i < M::kPasses; ++i) {
+            const uint32_t* x = w + i * M::kWords;
+            const int r = r0 + i * M::kStep;
+            if (M::kStep > kRows && r >= kRows) continue;
+            uint32_t t[kU > 1 ? kU / 2 : 1][kN];
+#pragma unroll
+            for (int u = 0; u < (kU > 1 ? kU / 2 : 1); ++u) {
+                if constexpr (kN == 1) {
+                    t[u][0] = x[u];
+                } else if constexpr (sizeof(T) == 4) {
+                    split_pair<kN>(__uint_as_float(x[kU > 1 ? 2 * u : 0]), kU > 1 ? __uint_as_float(x[kU > 1 ? 2 * u + 1 : 0]) : 0.f, t[u]);
+                } else {
+                    const float2 v = __half22float2(*(const __half2*)&x[u]);
+                    split_pair<kN>(v.x, v.y, t[u]);
+                }
+            }
+            __nv_bfloat16* p = dst + stored_row<kOrder>(first + r) * kPitch<DP> + d;
+#pragma unroll
+            for (int n = 0; n < kN; ++n) {
+                if constexpr (kU == 4) *(uint2*)(p + n * kTileRows * kPitch<DP>) = make_uint2(t[0][n], t[1][n]);
+                else if constexpr (kU == 2) *(uint32_t*)(p + n * kTileRows * kPitch<DP>) = t[0][n];
+                else *(unsigned short*)(p + n * kTileRows * kPitch<DP>) = (unsigned short)t[0][n];
+            }
+        }
+    }
+    // u: what unit() says of the tensor
+    __device__ __forceinline__ void fetch(const MatView& m, int u, int D, int b, int h, int row0, int rows_valid) {
+        const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
+        if (u == 4) fetch_u<4>(base, m.st, D, rows_valid);
+        else if (u == 2) fetch_u<2>(base, m.st, D, rows_valid);
+        else fetch_u<1>(base, m.st, D, rows_valid);
+    }
+    template <int kOrder>
+    __device__ __forceinline__ void put(__nv_bfloat16* dst, int u) const {
+        if (u == 4) put_u<kOrder, 4>(dst);
+        else if (u == 2) put_u<kOrder, 2>(dst);
+        else put_u<kOrder, 1>(dst);
+    }
+};
+template <typename T>
+__device__ __forceinline__ int unit(const MatView& m, int D) { return units_ok<T>(m, D, 4) ? 4 : units_ok<T>(m, D, 2) ? 2 : 1; }
+template <int kT, typename T, int DP, int kOrder>
 __device__ __forceinline__ void load_tile(__nv_bfloat16* dst, const MatView& m, int D, int b, int h, int row0, int rows_valid) {
     const T* base = (const T*)m.ptr + (int64_t)b * m.sb + (int64_t)h * m.sh + (int64_t)row0 * m.st;
-    if (units_ok<T>(m, D, 4)) load_tile_u<kT, T, DP, kOrder, kRows, 4>(dst, base, m.st, D, rows_valid);
-    else if (units_ok<T>(m, D, 2)) load_tile_u<kT, T, DP, kOrder, kRows, 2>(dst, base, m.st, D, rows_valid);
-    else load_tile_u<kT, T, DP, kOrder, kRows, 1>(dst, base, m.st, D, rows_valid);
+    Rows<kT, T, DP> x;
+    if (units_ok<T>(m, D, 4)) {
+        x.template fetch_u<4>(base, m.st, D, rows_valid);
+        x.template put_u<kOrder, 4>(dst);
+    } else if (units_ok<T>(m, D, 2)) {
+        x.template fetch_u<2>(base, m.st, D, rows_valid);
+        x.template put_u<kOrder, 2>(dst);
+    } else {
+        Rows<kT, T, DP, 32, 64> y;
+#pragma unroll 1
+        for (int r = 0; r < 64; r += 32) {
+            y.template fetch_u<1>(base + r * m.st, m.st, D, rows_valid - r);
+            y.template put_u<kOrder, 1>(dst, r);
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------ warp-level matrix instructions
@@ -240,7 +285,7 @@ __device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_b
 
 // acc[mb][DC / 8] += P * X: P = kMB x kNB accumulator blocks in registers (float32, three terms), X a tile whose rows are the contracted
 // index (`x` at the first row and column), DC columns of it, 32 at a time
-template <int kN, int DP, int DC, int kMB, int kNB>
+template <int kN, int DP, int DC, int kMB, int kNB, bool kFinite = false>
 __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const float (&p)[kMB][kNB][4], const __nv_bfloat16* x, int lane) {
     constexpr int kNC = DC < 32 ? DC / 8 : 4;  // column blocks at a time
     const __nv_bfloat16* px = x + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8;
@@ -253,7 +298,7 @@ __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const f
             for (int e = 0; e < 4; ++e) {
                 const float* v = p[m][2 * k + (e >> 1)];
                 uint32_t t[kWTerms];
-                split_pair<kWTerms>(v[2 * (e & 1)], v[2 * (e & 1) + 1], t);
+                split_pair<kWTerms, kFinite>(v[2 * (e & 1)], v[2 * (e & 1) + 1], t);
 #pragma unroll
                 for (int i = 0; i < kWTerms; ++i) fa[k][m][i][e] = t[i];
             }
@@ -372,6 +417,7 @@ __device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * b
 template <typename T, int DP>
 __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __grid_constant__ KArgs a) {
     constexpr int kT = 256, kN = Terms<T>::n;
+    constexpr bool kEarly = sizeof(T) == 2;  // loads a tile ahead; the 32 words of two float32 tiles cost more registers than they gain
     extern __shared__ __align__(16) __nv_bfloat16 tiles[];
     __shared__ float xs[2][kBM];  // product of 1 - beta over a half, per row
     __nv_bfloat16* sQ = tiles;
@@ -407,12 +453,25 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
 #pragma unroll
             for (int r = 0; r < 2; ++r) cw[carry_slot32(c.slot_base, c.qt, 2 * kh + hf) * kTileQ + 8 * r] = 1.f;
 
+    const int uk = unit<T>(a.k, D), uv = unit<T>(a.v, D);
+    Rows<kT, T, DP> rk, rv;
+    auto fetch = [&](int kh) {
+        const int n = min(kBN, c.len - kh * kBN);
+        rk.fetch(a.k, uk, D, c.b, h, c.start + kh * kBN, n);
+        rv.fetch(a.v, uv, D, c.b, h, c.start + kh * kBN, n);
+    };
+    if (kEarly) fetch(last);
     for (int kh = last; kh >= 0; --kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
-        load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        if (kEarly) {
+            rk.template put<kKeyColumns>(sK, uk);
+            rv.template put<kKeyColumns>(sV, uv);
+        } else {
+            load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+            load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        }
         __syncthreads();
         float s[1][4][4], om[2][8], excl[2];
         product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
@@ -451,7 +510,8 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
             }
             W[r] = W[r] * right * left;
         }
-        product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
+        if (kEarly && kh > 0) fetch(kh - 1);
+        product_px<kN, DP, DP, 1, 4, true>(o, s, sV + 32 * hf * kPitch<DP>, lane);
     }
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     float* x = (float*)tiles;
@@ -487,6 +547,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
 template <typename T, int DP>
 __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const __grid_constant__ KArgs a) {
     constexpr int kT = 256, kN = Terms<T>::n;
+    constexpr bool kEarly = kN == 1 || (kN == 2 && DP < 64);  // loads a tile ahead, where registers allow
     extern __shared__ __align__(16) __nv_bfloat16 tiles[];
     __shared__ float xs[2][kBM];  // sum of g over a half, per row
     __nv_bfloat16* sQ = tiles;
@@ -518,12 +579,25 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
     float o[1][DP / 8][4] = {};
     const int last = (row0 + rows_valid - 1) / kBN;
 
+    const int uk = unit<T>(a.k, D), uv = unit<T>(a.v, D);
+    Rows<kT, T, DP> rk, rv;
+    auto fetch = [&](int kh) {
+        const int n = min(kBN, c.len - kh * kBN);
+        rk.fetch(a.k, uk, D, c.b, h, c.start + kh * kBN, n);
+        rv.fetch(a.v, uv, D, c.b, h, c.start + kh * kBN, n);
+    };
+    if (kEarly) fetch(0);
     for (int kh = 0; kh <= last; ++kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
-        load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        if (kEarly) {
+            rk.template put<kKeyColumns>(sK, uk);
+            rv.template put<kKeyColumns>(sV, uv);
+        } else {
+            load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
+            load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
+        }
         const int64_t slot = carry_slot32(c.slot_base, c.qt, 2 * kh + hf) * kTileQ;
         float W[2];
 #pragma unroll
@@ -582,6 +656,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
             }
             prefix[r] = prefix[r] + left + right;
         }
+        if (kEarly && kh < last) fetch(kh + 1);
         product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
     }
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
@@ -644,25 +719,33 @@ __device__ __forceinline__ void column(float* const (&s)[4], float* const (&dp)[
     }
 }
 
-// Scores transposed (rows = keys).  Sixteen warps.  First half of a step: two 32-key quarters (each entered with its own carries) x eight
-// groups of 8 queries; P^T and dS^T go to shared memory as three terms each.  Second half: four groups of 16 keys x {dv, dk} x
-// the two halves of the columns, so that a thread accumulates 16 or 32 values only.  (With P^T and dS^T kept in registers four
-// warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 311 and 107 us in the first two lines at the top.)
-// kQ: queries per step, 64, or 32 where the tiles would not fit otherwise (float32 at D > 64; eight of the warps then sit out the
-// first half; forward + backward of 8 heads, 4096 tokens, head dim 128: 1638 us with four warps that kept P^T and dS^T in registers,
-// 1163 us so)
-template <typename T, int DP, int kQ>
-__global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
-    constexpr int kT = 512, kN = Terms<T>::n;
-    constexpr int kDC = DP >= 32 ? DP / 2 : DP;     // columns of dk or dv per warp
+// Scores transposed (rows = keys).  kQ queries per step.  First half of a step: two 32-key quarters (each entered with its own carries) x
+// groups of 8 queries; P^T and dS^T go to shared memory as three terms each.  Second half: four groups of 16 keys x {dv, dk} (x the
+// two halves of the columns with sixteen warps, so that a thread accumulates 16 or 32 values only).  (With P^T and dS^T kept in
+// registers four warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 311 and 107 us in the first two
+// lines at the top.)
+// Sixteen warps, one block per SM, take steps of 64 queries, or of 32 where the tiles would not fit otherwise (float32 at D > 64; eight
+// of the warps then sit out the first half; forward + backward of 8 heads, 4096 tokens, head dim 128: 1638 us with four warps
+// that kept P^T and dS^T in registers, 1163 us so).  kBuf = 2, where shared memory has the room: the next step's Q and dO travel during
+// the second half and go to the other buffer at its end, which takes a barrier and the whole load out of the step (265 -> 255 us in the first
+// line at the top).
+// Eight warps, two blocks per SM, take steps of 32: one block's loads and scans run under the other's products.  Better from six blocks
+// for each SM on, where a short last wave does not matter (64 sequences of 64 float32 tokens, 8 heads: 42 -> 36 us; 16 heads, 4096
+// tokens, bf16, head dim 50: 300 -> 289 us), worse below (4 x 8 heads x 500 tokens: 45 -> 61 us).
+template <typename T, int DP, int kWarps, int kQ, int kBuf>
+__global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
+    constexpr int kT = 32 * kWarps, kN = Terms<T>::n;
+    constexpr int kDC = kWarps == 16 && DP >= 32 ? DP / 2 : DP;  // columns of dk or dv per warp
+    constexpr int kNC = kDC < 32 ? kDC / 8 : 4;                  // column blocks at a time
     constexpr int kPP = kQ + 8, kPPlane = 64 * kPP;  // P^T, dS^T: [64 keys][kQ queries], three planes each
     constexpr int kQTile = kN * kQ * kPitch<DP>;     // Q, dO: kQ rows
+    constexpr bool kEarly = kBuf == 2 || (kWarps == 8 && sizeof(T) == 2);  // loads a step ahead; float32 lacks the registers otherwise
     extern __shared__ __align__(16) __nv_bfloat16 tiles[];
     __nv_bfloat16* sK = tiles;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
-    __nv_bfloat16* sQ = sV + kTileElems<T, DP>;
-    __nv_bfloat16* sG = sQ + kQTile;
-    __nv_bfloat16* sP = sG + kQTile;
+    __nv_bfloat16* const tiles_q = sV + kTileElems<T, DP>;
+    __nv_bfloat16 *sQ = tiles_q, *sG = sQ + kQTile;
+    __nv_bfloat16* sP = sQ + 2 * kBuf * kQTile;
     __nv_bfloat16* sS = sP + kWTerms * kPPlane;
     pdl_wait();
     const BlockIdx bi = block_idx(a.heads);
@@ -685,11 +768,26 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
     float acc[kDC / 8][4] = {};
 
+    const int uq = unit<T>(a.q, D), ug = unit<T>(a.d_o, D);
+    Rows<kT, T, DP, kQ> rq, rg;
+    auto fetch = [&](int row0) {
+        const int n = min(kQ, c.len - row0);
+        rq.fetch(a.q, uq, D, c.b, h, c.start + row0, n);
+        rg.fetch(a.d_o, ug, D, c.b, h, c.start + row0, n);
+    };
+    if (kEarly) fetch(key0);
+    if (kBuf == 2) {
+        rq.template put<kPlain>(sQ, uq);
+        rg.template put<kPlain>(sG, ug);
+    }
     for (int row0 = key0; row0 < c.len; row0 += kQ) {
         const int rows_valid = min(kQ, c.len - row0);
-        __syncthreads();
-        load_tile<kT, T, DP, kPlain, kQ>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
-        load_tile<kT, T, DP, kPlain, kQ>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+        if (kBuf == 1) {
+            if (!kEarly) fetch(row0);
+            __syncthreads();
+            rq.template put<kPlain>(sQ, uq);
+            rg.template put<kPlain>(sG, ug);
+        }
         const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, quarter) * kTileQ + row0 % kTileQ;
         float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
 #pragma unroll
@@ -718,7 +816,7 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     uint32_t tp[kWTerms], ts[kWTerms];
-                    split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
+                    split_pair<kWTerms, true>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
                     split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
                     const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
 #pragma unroll
@@ -729,32 +827,43 @@ __global__ void __launch_bounds__(512, 1) f32_bwd_dkdv_kernel(const __grid_const
                 }
         }
         __syncthreads();
+        if (kEarly && row0 + kQ < c.len) fetch(row0 + kQ);
         if (second) {
             const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
             const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
-            float big[kDC / 8][4] = {}, small[kDC / 8][4] = {};
 #pragma unroll
-            for (int k = 0; k < kQ / 16; ++k) {
-                uint32_t fa[kWTerms][4];
+            for (int n0 = 0; n0 < kDC / 8; n0 += kNC) {
+                float big[kNC][4] = {}, small[kNC][4] = {};
 #pragma unroll
-                for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
+                for (int k = 0; k < kQ / 16; ++k) {
+                    uint32_t fa[kWTerms][4];
 #pragma unroll
-                for (int j = 0; j < kN; ++j) {
-                    uint32_t fb[kDC / 16][4];
+                    for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
 #pragma unroll
-                    for (int n2 = 0; n2 < kDC / 16; ++n2) ldsm4_t(fb[n2], px + j * kQ * kPitch<DP> + k * 16 * kPitch<DP> + n2 * 16);
+                    for (int j = 0; j < kN; ++j) {
+                        uint32_t fb[kNC / 2][4];
 #pragma unroll
-                    for (int i = 0; i < kWTerms; ++i) {
-                        if (i + j > 2) continue;
+                        for (int n2 = 0; n2 < kNC / 2; ++n2)
+                            ldsm4_t(fb[n2], px + j * kQ * kPitch<DP> + k * 16 * kPitch<DP> + n0 * 8 + n2 * 16);
 #pragma unroll
-                        for (int n = 0; n < kDC / 8; ++n) mma(i + j == 0 ? big[n] : small[n], fa[i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                        for (int i = 0; i < kWTerms; ++i) {
+                            if (i + j > 2) continue;
+#pragma unroll
+                            for (int n = 0; n < kNC; ++n) mma(i + j == 0 ? big[n] : small[n], fa[i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                        }
                     }
                 }
+#pragma unroll
+                for (int n = 0; n < kNC; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[n0 + n][i] += big[n][i] + small[n][i];
             }
-#pragma unroll
-            for (int n = 0; n < kDC / 8; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[n][i] += big[n][i] + small[n][i];
+        }
+        if (kBuf == 2 && row0 + kQ < c.len) {
+            sQ = tiles_q + (sQ == tiles_q ? 2 * kQTile : 0);
+            sG = sQ + kQTile;
+            rq.template put<kPlain>(sQ, uq);
+            rg.template put<kPlain>(sG, ug);
         }
     }
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
@@ -776,6 +885,14 @@ int launch_one(void (*kernel)(KArgs), int threads, int tiles, int more, const Ws
     if (e != 0) return e;
     return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * 2), dim3(threads), smem, st, a);
 }
+template <typename T, int DP, int kQ, int kBuf>
+constexpr int dkdv_smem() {
+    return 2 * (2 * kTileElems<T, DP> + kBuf * 2 * Terms<T>::n * kQ * kPitch<DP> + 2 * kWTerms * 64 * (kQ + 8));
+}
+template <typename T, int DP, int kWarps, int kQ, int kBuf>
+int launch_dkdv(const WsLayout& L, const KArgs& a, cudaStream_t st) {
+    return launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP, kWarps, kQ, kBuf>, 32 * kWarps, 2, dkdv_smem<T, DP, kQ, kBuf>() - 4 * kTileElems<T, DP>, L, a, st);
+}
 template <typename T, int DP>
 int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {
     if (!backward) return launch_one<T, DP>(f32_fwd_kernel<T, DP>, 256, 3, 0, L, a, st);
@@ -784,8 +901,11 @@ int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaS
         if (e != 0) return e;
     }
     if (phases == SBATTN_BWD_DQ) return 0;
+    if constexpr (DP <= 64) {  // six blocks for each SM: see the kernel
+        if ((int64_t)L.max_items * a.heads * 2 >= 6 * 148) return launch_dkdv<T, DP, 8, 32, 1>(L, a, st);
+    }
     constexpr int kQ = DP > 64 && Terms<T>::n == 3 ? 32 : 64;
-    return launch_one<T, DP>(f32_bwd_dkdv_kernel<T, DP, kQ>, 512, 2, 2 * (2 * Terms<T>::n * kQ * kPitch<DP> + 2 * kWTerms * 64 * (kQ + 8)), L, a, st);
+    return launch_dkdv<T, DP, 16, kQ, dkdv_smem<T, DP, kQ, 2>() <= kMaxSmem ? 2 : 1>(L, a, st);
 }
 template <typename T>
 int launch_t(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaStream_t st) {

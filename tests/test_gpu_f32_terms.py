@@ -20,3 +20,13 @@ def test_edges_against_oracle(dtype, D, attend_current):
     want = oracle_varlen(*ins, lengths, 1 / math.sqrt(D), attend_current)
     # float32: a few units of 2^-24 of sums that reach 5; 16-bit types: the output format
     assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_F32 if dtype == torch.float32 else TOL_BF16, f"{dtype} {D}")
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 20), (torch.bfloat16, 50), (torch.bfloat16, 16), (torch.float16, 33)])
+def test_many_blocks_against_oracle(dtype, D):
+    """Enough (sequence, tile, head) blocks for the dk/dv form with two blocks per SM: lengths on both sides of its steps of 32 queries."""
+    lengths = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 161, 193] * 2
+    ins = [rounded(x, dtype) for x in synth(16, sum(lengths), D, seed=52)]
+    got = run_varlen(*ins, lengths, 1 / math.sqrt(D), False, dtype)
+    want = oracle_varlen(*ins, lengths, 1 / math.sqrt(D), False)
+    assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_F32 if dtype == torch.float32 else TOL_BF16, f"{dtype} {D}")
