@@ -27,8 +27,8 @@ Workloads (seeded synthetic data, N(0,1) inputs rounded to bf16, inv_temp = 1/sq
   c4      8 heads, head_dim 128, one sequence of 65536 tokens, inputs 0.5*N(0,1)
   c5     64 heads, head_dim 128, 131072 tokens packed from log-normal lengths; heads are SPLIT over the ranks
   short  32 heads, head_dim 128, 512 sequences of 128 tokens
-  c1     4 heads, head_dim 64, 512 tokens in sequences of 128/192/192, float32 (the fp32-arithmetic kernels)
-  b500   batched layout of the reference's tests: 4 x 8 heads x 500 tokens x head_dim 50, bf16 (fp32-arithmetic kernels)
+  c1     4 heads, head_dim 64, 512 tokens in sequences of 128/192/192, float32 (the kernels of float32 precision)
+  b500   batched layout of the reference's tests: 4 x 8 heads x 500 tokens x head_dim 50, bf16 (kernels of float32 precision)
 """
 import argparse
 import json
