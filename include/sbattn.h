@@ -169,6 +169,12 @@ size_t sbattn_params_size(void);
  * No counterpart in the reference. */
 unsigned long long sbattn_launch_count(void);
 
+/* First entry and longest sequence of n >= 1 cumulative ends on the device (int32 or int64: cu_width 4 or 8), for callers that do not know
+ * the longest sequence.  `leading`: 1 if the first entry is a leading zero and not an end.  `out`: three int64 of pinned host
+ * memory, out[2] = 0 before the call; the kernel writes the first entry, the longest sequence, and last out[2] = 1, so that the host can
+ * wait for this word: a few microseconds sooner than for a copy and a stream synchronisation. */
+int sbattn_seq_bounds(const void* cu, int cu_width, int64_t n, int leading, int64_t* out, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

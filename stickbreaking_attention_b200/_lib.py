@@ -40,7 +40,7 @@ FLAG_FUSED_REMAINDER = 1
 
 EXPORTS = ("sbattn_workspace_bytes", "sbattn_fwd", "sbattn_bwd", "sbattn_strerror", "sbattn_version",
            "sbattn_params_size", "sbattn_fwd_static", "sbattn_static_scratch_bytes", "sbattn_attention_weights",
-           "sbattn_launch_count")
+           "sbattn_launch_count", "sbattn_seq_bounds")
 
 _lib = None
 

@@ -13,6 +13,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -86,30 +87,35 @@ void require_cuda(const Tensor& t) {
     TORCH_CHECK(t.is_cuda(), "stick-breaking attention runs on CUDA tensors only (there is no CPU implementation)");
 }
 
-// (smallest cu_seqlens[0], longest sequence) of cumulative ends, one device-to-host copy; `leading`: the first entry is the leading
-// zero, not an end
+// (cu_seqlens[0], longest sequence) of cumulative ends; `leading`: the first entry is the leading zero, not an end.  On a GPU one small
+// kernel writes both to pinned memory and the host waits for its last word, not for a copy and the stream (us a call, 8 heads, 2048
+// tokens in 6 documents, nothing but cu_seqlens given: forward 31 -> 25, forward and backward 110 -> 100).  When the stream has
+// much to do before, waiting goes over to a stream synchronisation.
 std::pair<int64_t, int64_t> seq_bounds(const Tensor& cu, bool leading, bool want_longest) {
-    Tensor part = want_longest ? cu : cu.narrow(0, 0, 1);
-    Tensor host;
-    if (part.is_cuda()) {
-        c10::cuda::CUDAGuard guard(part.device());
-        host = at::empty(part.sizes(), part.options().device(at::kCPU).pinned_memory(true));
-        host.copy_(part, /*non_blocking=*/true);
-        c10::cuda::getCurrentCUDAStream().synchronize();
-    } else {
-        host = part.contiguous();
-    }
-    const auto at_ = [&](int64_t i) { return host.scalar_type() == at::kLong ? host.const_data_ptr<int64_t>()[i] : (int64_t)host.const_data_ptr<int32_t>()[i]; };
-    int64_t longest = 0;
-    if (want_longest) {
-        int64_t prev = leading ? at_(0) : 0;
-        bool any = false;
-        for (int64_t i = leading ? 1 : 0; i < host.numel(); ++i) {
-            const int64_t e = at_(i);
-            longest = any ? std::max(longest, e - prev) : e - prev;
-            any = true;
-            prev = e;
+    const Tensor c = cu.contiguous();
+    const int64_t n = want_longest ? c.numel() : 1;
+    if (c.is_cuda()) {
+        c10::cuda::CUDAGuard guard(c.device());
+        const auto st = c10::cuda::getCurrentCUDAStream();
+        const Tensor host = at::empty({3}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+        volatile int64_t* out = host.data_ptr<int64_t>();
+        out[2] = 0;
+        check(sbattn_seq_bounds(c.const_data_ptr(), (int)c.element_size(), n, leading, (int64_t*)out, st.stream()), "sbattn_seq_bounds");
+        for (int polls = 1; out[2] == 0; ++polls) {
+            if (polls % 1024 != 0) continue;
+            const cudaError_t e = polls < 64 * 1024 ? cudaStreamQuery(st) : cudaStreamSynchronize(st);
+            if (e == cudaSuccess) break;  // the kernel is done, its writes are visible
+            if (e != cudaErrorNotReady) C10_CUDA_CHECK(e);
         }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return {out[0], out[1]};
+    }
+    const bool wide = c.scalar_type() == at::kLong;
+    const auto at_ = [&](int64_t i) { return wide ? c.const_data_ptr<int64_t>()[i] : (int64_t)c.const_data_ptr<int32_t>()[i]; };
+    int64_t longest = 0;
+    for (int64_t i = leading ? 1 : 0; i < n; ++i) {
+        const int64_t d = at_(i) - (i > 0 ? at_(i - 1) : 0);
+        longest = i == (leading ? 1 : 0) ? d : std::max(longest, d);
     }
     return {at_(0), longest};
 }

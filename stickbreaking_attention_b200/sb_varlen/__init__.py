@@ -53,7 +53,7 @@ def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_st
     traced = torch.compiler.is_compiling()
     if zero_start:
         if not traced and cu_seqlens.dtype in (torch.int32, torch.int64) and cu_seqlens.dim() == 1 and cu_seqlens.numel() > 0:
-            # one device-to-host copy answers both questions: is the first entry zero, how long is the longest sequence
+            # one small kernel answers both questions: is the first entry zero, how long is the longest sequence
             first, longest = _lib.binding().seq_bounds(cu_seqlens, True, max_seqlens is None)
             assert first == 0
             max_seqlens = longest if max_seqlens is None else max_seqlens

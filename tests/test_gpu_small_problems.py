@@ -55,3 +55,19 @@ def test_own_tables_report_bad_sequence_ends():
             sb.sb_attn_varlen(q, q, q, torch.tensor(ends, device="cuda"), m, zero_start=False)
             sb.check_status()
     assert sb.check_status() == 0
+
+
+@pytest.mark.parametrize("cu_dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1000])
+def test_sequence_bounds_read_from_the_device(n, cu_dtype):
+    """First entry and longest sequence, exact, at both sides of the kernel's 256 threads; strided ends as well."""
+    from stickbreaking_attention_b200 import _lib
+    ends = np.cumsum(np.random.default_rng(n).integers(0, 90, n))
+    cu = torch.from_numpy(ends).to("cuda", cu_dtype)
+    strided = torch.stack([cu, cu], 1)[:, 0]
+    for leading in (False, True):
+        gaps = np.diff(ends) if leading else np.diff(ends, prepend=0)
+        want = (int(ends[0]), int(gaps.max()) if len(gaps) else 0)
+        assert _lib.binding().seq_bounds(cu, leading, True) == want
+        assert _lib.binding().seq_bounds(strided, leading, True) == want
+        assert _lib.binding().seq_bounds(cu, leading, False)[0] == want[0]
