@@ -49,7 +49,7 @@ KArgs make_args(const SbParams& p, const WsLayout& L) {
     a.carry_w = p.save_carries ? (float*)(ws + L.off_carry) : nullptr;
     a.carry_c = (float*)p.bwd_workspace;
     a.drem_eff = p.bwd_workspace ? (float*)((char*)p.bwd_workspace + L.off_drem) : nullptr;
-    a.fused = (p.flags & SBATTN_FLAG_FUSED_REMAINDER) ? 1 : 0;
+    a.fused = (p.flags & (SBATTN_FLAG_FUSED_REMAINDER | SBATTN_FLAG_REMAINDER_IN_DV)) ? 1 : 0;
     a.tokens = p.tokens;
     a.zero_tail = p.batch == 0 && p.bwd_phases == SBATTN_BWD_ALL;  // the batched layout covers every token
     a.drem_rows = (int64_t)p.tokens * (p.batch > 0 ? p.batch : 1);
@@ -154,7 +154,7 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     if (((uintptr_t)p->fwd_workspace & 255) != 0) return SBATTN_EWORKSPACE;
     const int path = choose_path(*p, false);
     if (path < 0) return path;
-    if ((p->flags & SBATTN_FLAG_FUSED_REMAINDER) && path != 1) return SBATTN_EUNSUPPORTED;  // tensor-core kernels only
+    if (p->flags & SBATTN_FLAG_REMAINDER_IN_DV) return SBATTN_EINVAL;  // a flag of the backward
     cudaStream_t st = (cudaStream_t)p->stream;
     KArgs a = make_args(*p, L);
     a.own_tables = forward_builds_tables(*p, L, path == 1);
@@ -188,6 +188,10 @@ extern "C" int sbattn_bwd(const SbParams* p) {
     if (p->flags & SBATTN_FLAG_FUSED_REMAINDER) {
         if (path != 1) return SBATTN_EUNSUPPORTED;
         if ((rc = check_vec(p->rem, true))) return rc;  // the forward's rem: dv includes rem * d_o
+    }
+    if (p->flags & SBATTN_FLAG_REMAINDER_IN_DV) {
+        if (path != 0) return SBATTN_EUNSUPPORTED;
+        if ((rc = check_vec(p->rem, true))) return rc;
     }
     cudaStream_t st = (cudaStream_t)p->stream;
     const KArgs a = make_args(*p, L);

@@ -109,7 +109,7 @@ struct KArgs {
     float* carry_c;         // backward carries [heads][slot_cap][128]
     int64_t slot_cap;
     int32_t heads, head_dim, attend_current;
-    int32_t fused;          // SBATTN_FLAG_FUSED_REMAINDER
+    int32_t fused;          // SBATTN_FLAG_FUSED_REMAINDER, SBATTN_FLAG_REMAINDER_IN_DV
     int32_t tokens;         // tokens per batch entry (row index of drem_eff: batch * tokens + token)
     float* drem_eff;        // [heads][drem_rows]: drem + do . v (fused-remainder backward)
     int64_t drem_rows;      // batch * tokens (tokens for the packed layout)

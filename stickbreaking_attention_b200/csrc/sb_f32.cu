@@ -353,6 +353,18 @@ __device__ __forceinline__ void store_row(const float (&acc)[DC / 8][4], int i0,
     }
 }
 
+// the same elements += f * x
+template <typename T, int DC>
+__device__ __forceinline__ void add_row(float (&acc)[DC / 8][4], int i0, float f, const T* x, int D, int col0, int t) {
+#pragma unroll
+    for (int n = 0; n < DC / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int d = col0 + 8 * n + 2 * t + e;
+            if (d < D) acc[n][i0 + e] = __fadd_rn(acc[n][i0 + e], __fmul_rn(f, to_f32<T>(x[d])));
+        }
+}
+
 // sigmoid pieces with full relative accuracy on both sides: beta = sigmoid(s), r = 1 - beta
 __device__ __forceinline__ void sigmoid_pair(float s, float& beta, float& r) {
     const float e = expf(-fabsf(s));
@@ -528,6 +540,12 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
     for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+    if (a.fused) {  // out = o + rem * v, each operation rounded by itself: the same bits as the expression outside for float32
+        const T* v = (const T*)a.v.ptr + (int64_t)c.b * a.v.sb + (int64_t)h * a.v.sh + (int64_t)(c.start + row0) * a.v.st;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            if (wrow + 8 * r < rows_valid) add_row<T, DP>(o[0], 2 * r, to_f32<T>(from_f32<T>(W[r])), v + (int64_t)(wrow + 8 * r) * a.v.st, D, 0, t);
+    }
     const bool pairs = units_ok<T>(a.o, D, 2);
     T* base = (T*)a.o.ptr + (int64_t)c.b * a.o.sb + (int64_t)h * a.o.sh + (int64_t)(c.start + row0) * a.o.st;
 #pragma unroll
@@ -868,6 +886,15 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
     }
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     if (!second) return;
+    if (a.fused && !is_dk) {  // dv += rem * do
+        const T* d_o = (const T*)a.d_o.ptr + (int64_t)c.b * a.d_o.sb + (int64_t)h * a.d_o.sh + (int64_t)(c.start + key0) * a.d_o.st;
+        const T* rem = (const T*)a.rem.ptr + (int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0) * a.rem.st;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int row = 32 * (kg >> 1) + 4 * g + 2 * (kg & 1) + hh;
+            if (row < keys_valid) add_row<T, kDC>(acc, 2 * hh, to_f32<T>(rem[(int64_t)row * a.rem.st]), d_o + (int64_t)row * a.d_o.st, D, col0, t);
+        }
+    }
     const MatView m = is_dk ? a.dk : a.dv;
     const bool pairs = units_ok<T>(m, D, 2);
     T* base = (T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + key0) * m.st;

@@ -153,6 +153,7 @@ struct Opts {
     double scale;
     bool attend_current, fused;
     int path;
+    bool f32_fused = false;  // out = o + rem * v in the kernels of float32 precision
 };
 
 SbParams base_params(const Tensor& q, const Tensor& cu, const Opts& o, bool save) {
@@ -175,7 +176,7 @@ SbParams base_params(const Tensor& q, const Tensor& cu, const Opts& o, bool save
     p.attend_current = o.attend_current;
     p.inv_temp = (float)o.scale;
     p.save_carries = save;
-    p.flags = o.fused ? SBATTN_FLAG_FUSED_REMAINDER : 0;
+    p.flags = o.fused || o.f32_fused ? SBATTN_FLAG_FUSED_REMAINDER : 0;
     p.status = status_ptr(q.get_device());
     p.stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
     return p;
@@ -228,10 +229,13 @@ bool tma_ok(const Tensor& t) {
     return true;
 }
 
-bool fusable(const Tensor& q, const Tensor& k, const Tensor& v, int path) {
+// a type and a head dim of the tensor-core kernels
+bool tensor_type(const Tensor& q, int path) {
     const int64_t d = q.size(-1);
-    return (q.scalar_type() == at::kBFloat16 || q.scalar_type() == at::kHalf) && (d == 32 || d == 64 || d == 128) &&
-           path != SBATTN_PATH_SIMT && tma_ok(q) && tma_ok(k) && tma_ok(v);
+    return (q.scalar_type() == at::kBFloat16 || q.scalar_type() == at::kHalf) && (d == 32 || d == 64 || d == 128) && path != SBATTN_PATH_SIMT;
+}
+bool fusable(const Tensor& q, const Tensor& k, const Tensor& v, int path) {
+    return tensor_type(q, path) && tma_ok(q) && tma_ok(k) && tma_ok(v);
 }
 
 std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Tensor v, const Tensor& cu, const Tensor& ws,
@@ -258,6 +262,10 @@ std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Ten
     }
     SbParams p = base_params(q, cu, opt, true);
     p.bwd_phases = phases;
+    if (opt.f32_fused) {
+        p.flags = SBATTN_FLAG_REMAINDER_IN_DV;
+        d_rem = d_rem + (d_o * v).sum(-1);  // as autograd of o + rem * v forms it
+    }
     size_t fb = 0, bb = 0;
     check(sbattn_workspace_bytes(&p, &fb, &bb), "sbattn_workspace_bytes");
     TORCH_CHECK_VALUE((size_t)ws.numel() >= fb, "the forward workspace does not belong to this problem (was the forward run with no_grad?)");
@@ -268,7 +276,7 @@ std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Ten
     p.v = mat(v, opt.batched);
     p.d_o = mat(d_o, opt.batched);
     p.d_rem = vec(d_rem, opt.batched);
-    if (opt.fused) p.rem = vec(rem.defined() ? rem : d_rem, opt.batched);
+    if (opt.fused || opt.f32_fused) p.rem = vec(rem.defined() ? rem : d_rem, opt.batched);
     p.dq = mat(g[0], opt.batched);
     p.dk = mat(g[1], opt.batched);
     p.dv = mat(g[2], opt.batched);
@@ -285,24 +293,24 @@ std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Ten
 struct StickBreaking : public torch::autograd::Function<StickBreaking> {
     static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v,
                                                   const OptTensor& cu_seqlens, bool batched, int64_t max_seqlens, double scale, bool attend_current,
-                                                  bool fused, bool recompute, int64_t path) {
-        const Opts opt{batched, max_seqlens, scale, attend_current, fused, (int)path};
+                                                  bool fused, bool recompute, int64_t path, bool f32_fused) {
+        const Opts opt{batched, max_seqlens, scale, attend_current, fused, (int)path, f32_fused};
         const Tensor cu = cu_seqlens.value_or(Tensor());
         FwdOut r = ::forward(q, k, v, cu, opt, !recompute, false);
         ctx->save_for_backward({q, k, v, cu, recompute ? Tensor() : r.ws, r.rem});
-        ctx->saved_data["o"] = c10::ivalue::Tuple::create({batched, max_seqlens, scale, attend_current, fused, recompute, path});
+        ctx->saved_data["o"] = c10::ivalue::Tuple::create({batched, max_seqlens, scale, attend_current, fused, recompute, path, f32_fused});
         return {r.o, r.rem};
     }
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
         const auto saved = ctx->get_saved_variables();
         const auto tuple = ctx->saved_data["o"].toTuple();
         const auto& e = tuple->elements();
-        const Opts opt{e[0].toBool(), e[1].toInt(), e[2].toDouble(), e[3].toBool(), e[4].toBool(), (int)e[6].toInt()};
+        const Opts opt{e[0].toBool(), e[1].toInt(), e[2].toDouble(), e[3].toBool(), e[4].toBool(), (int)e[6].toInt(), e[7].toBool()};
         const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &cu = saved[3];
         const Tensor ws = e[5].toBool() ? ::forward(q, k, v, cu, opt, true, false).ws : saved[4];
         const auto g = ::backward(grads[0], grads[1], q, k, v, cu, ws, saved[5], opt, 0, {}, std::nullopt);
         Tensor none;
-        return {g[0], g[1], g[2], none, none, none, none, none, none, none, none};
+        return {g[0], g[1], g[2], none, none, none, none, none, none, none, none, none};
     }
 };
 
@@ -314,18 +322,19 @@ std::pair<Tensor, Tensor> attend(const Tensor& q, const Tensor& k, const Tensor&
     Tensor cu;
     if (batched) max_seqlens = q.size(2);
     else cu = prep_cu(*cu_seqlens, q, max_seqlens);
-    // the fused remainder exists in the tensor-core kernels only; elsewhere the same sum is formed here
-    const bool compose = fused && !fusable(q, k, v, path);
-    if (compose) fused = false;
+    // Operands that could go to the tensor-core kernels but for their strides: the sum is formed here.  (Formed here it costs ten small
+    // operations of autograd: forward and backward of 4 heads, 512 float32 tokens 135 -> 96 us with the sum in the kernels.)
+    const bool other = fused && !fusable(q, k, v, path), f32_fused = other && !tensor_type(q, path), compose = other && !f32_fused;
+    if (other) fused = false;
     const auto done = [&](const Tensor& o, const Tensor& rem) {
         return std::pair<Tensor, Tensor>{compose ? o + rem.unsqueeze(-1) * v : o, rem};
     };
     if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
         require_cuda(q);
-        auto r = StickBreaking::apply(q, k, v, batched ? OptTensor() : OptTensor(cu), batched, *max_seqlens, scale, attend_current, fused, recompute, (int64_t)path);
+        auto r = StickBreaking::apply(q, k, v, batched ? OptTensor() : OptTensor(cu), batched, *max_seqlens, scale, attend_current, fused, recompute, (int64_t)path, f32_fused);
         return done(r[0], r[1]);
     }
-    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path}, false, false);
+    FwdOut r = forward(q, k, v, cu, Opts{batched, *max_seqlens, scale, attend_current, fused, path, f32_fused}, false, false);
     return done(r.o, r.rem);
 }
 

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from util import TOL_BF16, assert_close, rounded, synth
+from util import TOL_BF16, TOL_F32, assert_close, rounded, synth
 from oracle import sb_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -135,3 +135,21 @@ def test_fused_falls_back_for_float32_inputs():
                q, k, v, dout, dr)
     for a_, b_ in zip(got, want):
         assert torch.equal(a_, b_)
+
+
+@pytest.mark.parametrize("D,dtype", [(64, torch.float32), (128, torch.float32), (50, torch.bfloat16), (33, torch.float16), (16, torch.bfloat16)])
+@pytest.mark.parametrize("heads", [2, 30])
+def test_varlen_fused_at_float32_precision_against_oracle(D, dtype, heads):
+    """out = o + rem * v in the epilogues of the kernels of float32 precision (both forms of dk/dv), tokens behind the last sequence."""
+    from stickbreaking_attention_b200 import check_status, sb_attn_varlen
+    lengths = [300, 1, 129, 31, 77, 128, 65, 33]
+    T, used = sum(lengths) + 20, sum(lengths)
+    ins = [rounded(x, dtype) for x in synth(heads, T, D, 22)]
+    q, k, v, dout, dr = (torch.from_numpy(x).to("cuda", dtype) for x in ins)
+    cu = torch.tensor(np.cumsum(lengths), dtype=torch.int32, device="cuda")
+    got = _run(lambda q, k, v: sb_attn_varlen(q, k, v, cu, max(lengths), zero_start=False, fuse_remainder=True), q, k, v, dout, dr)
+    check_status()
+    want = _oracle_fused(*[x[:, :used] for x in ins], lengths, 1 / math.sqrt(D), False)
+    got = [x.double().cpu().numpy()[:, :used] for x in got]
+    # float32: rounding of sums that reach 5; 16-bit types: the output format
+    assert_close(NAMES, got, want, TOL_F32 if dtype == torch.float32 else TOL_BF16, f"fused float32 precision D={D}")
