@@ -275,7 +275,6 @@ tc_bwd_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         uint8_t* prow = sP + hf * kQBox + r * 128;
         uint8_t* srow = sDS + hf * kQBox + r * 128;
         const int kv_chunks = max(0, min(D / 64, a.head_dim / 32 - hf * (D / 64)));  // 32-column chunks of dk / dv this thread stores
-        const int lim = r + a.attend_current - 32 * kq;                             // columns < lim of the quarter are visible
         bool ok = true;
         SchedConsumer sched;
         int w;
@@ -284,6 +283,9 @@ tc_bwd_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const uint32_t ph = i & 1;
             const bool row_ok = r < wk.len;
             const int64_t tok = wk.start + r;
+            // Columns < lim of the quarter are visible.  None to a row behind the end of the sequence: its zero query against an infinite
+            // or NaN key would make a NaN of every weight to the left, and dk, dv contract over such rows up to a multiple of 16.
+            const int lim = row_ok ? r + a.attend_current - 32 * kq : 0;
             float W = 0.f, drem = 0.f;
             if (row_ok) {
                 // a quarter behind the end of the sequence (in a half whose carry slots do not exist) has no visible key: any W does

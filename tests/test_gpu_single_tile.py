@@ -44,3 +44,26 @@ def test_sequences_of_one_tile(D, dtype, attend_current, fused):
     got = [x[:, :T].detach().double().cpu().numpy() for x in (o, rem, dq, dk, dv)]
     half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11  # what storing the exact result in the output type costs
     assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_BF16, f"one tile {D} {dtype} {fused}", out_half_ulp=half_ulp)
+
+
+@pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (64, torch.float16), (32, torch.bfloat16)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_rows_behind_a_sequence_see_no_key(D, dtype, bad):
+    """The last key of every sequence is visible to no query: whatever its k holds, o, rem, dk and dv are the same bits.  (The rows of a
+    tile between the end of the sequence and the next multiple of 16 lie behind that key and are part of the contractions.)"""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    lengths = [n for n in LENGTHS if n % 16]
+    ends = np.cumsum(lengths)
+    ins = [to_dev(rounded(x, dtype), dtype) for x in synth(2, ends[-1], D, seed=33)]
+    cu = torch.tensor(ends, dtype=torch.int32, device="cuda")
+    results = []
+    for value in (0.0, bad):
+        q, k, v, do, dr = (x.clone() for x in ins)
+        k[:, ends - 1] = value
+        for x in (q, k, v):
+            x.requires_grad_()
+        o, rem = sb_attn_varlen(q, k, v, cu, max(lengths), zero_start=False)
+        _, dk, dv = torch.autograd.grad([o, rem], [q, k, v], [do, dr])
+        results.append((o, rem, dk, dv))
+    for name, want, got in zip(("o", "rem", "dk", "dv"), *results):
+        assert torch.equal(got, want), name
