@@ -818,7 +818,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
             }
         }
         __syncthreads();
-        const bool edge = row0 < key0 + kBN || keys_valid < kBN;
+        const bool edge = row0 < key0 + kBN || keys_valid < kBN || rows_valid < kQ;
         if (q0 < kQ) {
             float s[2][1][4], dp[2][1][4];
             product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
@@ -827,7 +827,10 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
             for (int e = 0; e < 2; ++e) {
                 float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
                 float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
-                column(ps, pd, a.inv_temp, edge, min(keys_valid, row0 + q0 + 2 * t + e + a.attend_current - key0) - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
+                const int q = q0 + 2 * t + e;
+                // a query behind the end of the sequence sees no key: its zeros against an infinite or NaN key would make NaNs
+                const int lim = q < rows_valid ? min(keys_valid, row0 + q + a.attend_current - key0) : 0;
+                column(ps, pd, a.inv_temp, edge, lim - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
             }
 #pragma unroll
             for (int m = 0; m < 2; ++m)

@@ -2,10 +2,11 @@
 elements, head dims on both sides of the tile widths, sequence ends on both sides of 32 and 64."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
-from util import TOL_BF16, TOL_F32, assert_close, oracle_varlen, rounded, run_varlen, synth
+from util import TOL_BF16, TOL_F32, assert_close, oracle_varlen, rounded, run_varlen, synth, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +31,27 @@ def test_many_blocks_against_oracle(dtype, D):
     got = run_varlen(*ins, lengths, 1 / math.sqrt(D), False, dtype)
     want = oracle_varlen(*ins, lengths, 1 / math.sqrt(D), False)
     assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_F32 if dtype == torch.float32 else TOL_BF16, f"{dtype} {D}")
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 100), (torch.bfloat16, 50), (torch.float16, 16)])
+@pytest.mark.parametrize("copies", [1, 24])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_rows_behind_a_sequence_see_no_key(dtype, D, copies, bad):
+    """The last key of every sequence is visible to no query: whatever its k holds, o, rem, dk and dv are the same bits, in both forms
+    of dk/dv (`copies`: enough blocks for the one with two blocks per SM)."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    lengths = [1, 31, 33, 63, 65, 100, 129] * copies
+    ends = np.cumsum(lengths)
+    ins = [to_dev(rounded(x, dtype), dtype) for x in synth(2, ends[-1], D, seed=53)]
+    cu = torch.tensor(ends, dtype=torch.int32, device="cuda")
+    results = []
+    for value in (0.0, bad):
+        q, k, v, do, dr = (x.clone() for x in ins)
+        k[:, ends - 1] = value
+        for x in (q, k, v):
+            x.requires_grad_()
+        o, rem = sb_attn_varlen(q, k, v, cu, max(lengths), zero_start=False)
+        _, dk, dv = torch.autograd.grad([o, rem], [q, k, v], [do, dr])
+        results.append((o, rem, dk, dv))
+    for name, want, got in zip(("o", "rem", "dk", "dv"), *results):
+        assert torch.equal(got, want), name
