@@ -18,6 +18,10 @@
 // cores as the sum of the term products x_i y_j with i + j <= 2, accumulated in float32: what is left out, x1 y2 and smaller, is
 // below 2^-25 |x y|, a unit of which float32 multiply-adds lose as much in every addition.  Weights and score gradients are
 // float32 values and enter the second products in three terms.  exp and division are the accurate ones (no fast math here).
+// Three kinds of values do not divide into terms: infinities, magnitudes that round to one in bf16, and magnitudes below 2^-100, whose
+// later terms lie below the smallest bf16.  They show in a block's results, which then are NaN (terms of the first two kinds are), or
+// all tiny: such a block starts over and forms its sums with ordinary multiply-adds on the values as they are ("direct" below;
+// several times slower; a block that does not need it looks at its results and no more).
 //
 // What bounds them: the latency of the chain load -> scores -> scan -> second product of a tile, with the issue slots of the per-score
 // arithmetic behind it.  (warp-level mma takes 1024 multiply-adds per clock and SM, measured: a 64 x 64 x 64 product costs 256
@@ -33,6 +37,8 @@
 // Back to back (no gaps between launches), before and after loads a tile ahead, two buffers in dk/dv and the cheaper split:
 // 137 / 171 / 265 -> 135 / 168 / 249; 44 / 46 / 48 -> 39 / 42 / 44; 18 / 22 / 25 -> 18 / 22 / 24.
 // 16 heads, 4096 float32 tokens: tensor pipe 49 %, issue slots 47 %, shared memory 56 % busy in dk/dv, 45 / 52 / 37 % in the forward.
+#include <type_traits>
+
 #include "sb_common.cuh"
 
 namespace sb {
@@ -68,18 +74,16 @@ __device__ __forceinline__ int stored_row(int r) {
     return r;
 }
 
-// two values -> N packed terms.  kFinite: the values are known to be (weights are); otherwise an infinity, also one that the
-// rounding to bf16 makes, stays out of the later terms.
-template <int N, bool kFinite = false>
+// two values -> N packed terms.  An infinity, or a value that rounds to one, leaves a NaN in a later term.
+template <int N>
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&t)[N]) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
         t[i] = *(const uint32_t*)&h;
         if (i + 1 < N) {
-            const float a = __uint_as_float(t[i] << 16), b = __uint_as_float(t[i] & 0xffff0000u);
-            x = !kFinite && i == 0 && fabsf(a) == INFINITY ? 0.f : x - a;
-            y = !kFinite && i == 0 && fabsf(b) == INFINITY ? 0.f : y - b;
+            x -= __uint_as_float(t[i] << 16);
+            y -= __uint_as_float(t[i] & 0xffff0000u);
         }
     }
 }
@@ -285,7 +289,7 @@ __device__ __forceinline__ void product_nt(float (&c)[kMB][kNB][4], const __nv_b
 
 // acc[mb][DC / 8] += P * X: P = kMB x kNB accumulator blocks in registers (float32, three terms), X a tile whose rows are the contracted
 // index (`x` at the first row and column), DC columns of it, 32 at a time
-template <int kN, int DP, int DC, int kMB, int kNB, bool kFinite = false>
+template <int kN, int DP, int DC, int kMB, int kNB>
 __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const float (&p)[kMB][kNB][4], const __nv_bfloat16* x, int lane) {
     constexpr int kNC = DC < 32 ? DC / 8 : 4;  // column blocks at a time
     const __nv_bfloat16* px = x + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8;
@@ -298,7 +302,7 @@ __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const f
             for (int e = 0; e < 4; ++e) {
                 const float* v = p[m][2 * k + (e >> 1)];
                 uint32_t t[kWTerms];
-                split_pair<kWTerms, kFinite>(v[2 * (e & 1)], v[2 * (e & 1) + 1], t);
+                split_pair<kWTerms>(v[2 * (e & 1)], v[2 * (e & 1) + 1], t);
 #pragma unroll
                 for (int i = 0; i < kWTerms; ++i) fa[k][m][i][e] = t[i];
             }
@@ -329,6 +333,87 @@ __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const f
             for (int n = 0; n < kNC; ++n)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[m][n0 + n][i] += big[m][n][i] + small[m][n][i];
+    }
+}
+
+// ------------------------------------------------------------------------------------------ the same products on the values themselves
+// whether a thread's results (elements i0, i0 + 1 of its accumulator blocks: one row) ask for them: a NaN, or nothing but magnitudes
+// below 2^-100
+template <int kN>
+__device__ __forceinline__ bool asks_for_direct(const float (&acc)[kN][4], int i0) {
+    float most = 0.f;
+    bool nan = false;
+#pragma unroll
+    for (int n = 0; n < kN; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            nan |= acc[n][i0 + e] != acc[n][i0 + e];
+            most = fmaxf(most, fabsf(acc[n][i0 + e]));
+        }
+    return nan || (most > 0.f && most < 0x1p-100f);
+}
+// c[r][j] = row r of A (na of them valid) . row j of B (nb valid)
+template <typename T, int kR, int kC>
+__device__ __forceinline__ void direct_nt(float (&c)[kR][kC], const T* a, int64_t sa, int na, const T* b, int64_t sb, int nb, int D) {
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+#pragma unroll
+        for (int j = 0; j < kC; ++j) c[r][j] = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) {
+        float x[kR], y[kC];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) x[r] = r < na ? to_f32<T>(a[r * sa + d]) : 0.f;
+#pragma unroll
+        for (int j = 0; j < kC; ++j) y[j] = j < nb ? to_f32<T>(b[j * sb + d]) : 0.f;
+#pragma unroll
+        for (int r = 0; r < kR; ++r)
+#pragma unroll
+            for (int j = 0; j < kC; ++j) c[r][j] = fmaf(x[r], y[j], c[r][j]);
+    }
+}
+// scores of forward and dq: this lane's rows (r, r + 8) against its eight neighbouring keys
+template <typename T>
+__device__ __forceinline__ void direct_scores(float (&s)[1][4][4], const T* a, int64_t sa, int rows, const T* b, int64_t sb, int keys, int D) {
+    float c[2][8];
+    direct_nt<T>(c, a, 8 * sa, rows > 8 ? 2 : rows > 0, b, sb, keys, D);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[0][j >> 1][2 * r + (j & 1)] = c[r][j];
+}
+// scores of dk/dv: four neighbouring keys against this lane's two queries
+template <typename T>
+__device__ __forceinline__ void direct_scores_t(float (&s)[2][1][4], const T* a, int64_t sa, int keys, const T* b, int64_t sb, int rows, int D) {
+    float c[4][2];
+    direct_nt<T>(c, a, sa, keys, b, sb, rows, D);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) s[k >> 1][0][2 * (k & 1) + e] = c[k][e];
+}
+// acc += P * X over the 32 keys of a half, `keys` of them valid; P in registers as the forward and dq hold it
+template <typename T, int DP>
+__device__ __forceinline__ void direct_px(float (&acc)[1][DP / 8][4], const float (&p)[1][4][4], const T* x, int64_t st, int keys, int D, int lane) {
+    const int t = lane & 3;
+#pragma unroll 1
+    for (int from = 0; from < 4; ++from) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float p0 = __shfl_sync(0xffffffffu, p[0][j >> 1][j & 1], (lane & ~3) | from);
+            const float p1 = __shfl_sync(0xffffffffu, p[0][j >> 1][2 + (j & 1)], (lane & ~3) | from);
+            const int k = 8 * from + j;
+            if (k >= keys) continue;
+#pragma unroll
+            for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int d = 8 * n + 2 * t + e;
+                    const float v = d < D ? to_f32<T>(x[k * st + d]) : 0.f;
+                    acc[0][n][e] = fmaf(p0, v, acc[0][n][e]);
+                    acc[0][n][2 + e] = fmaf(p1, v, acc[0][n][2 + e]);
+                }
+        }
     }
 }
 
@@ -411,6 +496,11 @@ __device__ inline ItemCtx item_ctx(const int2* items, const SeqInfo* seqs, int i
     return ItemCtx{it.y, s.batch, s.start, s.len, s.slot_base};
 }
 __device__ inline ItemCtx item_ctx(const KArgs& a, int item) { return item_ctx(a.items, a.seqs, item); }
+// row `i` of the item's sequence
+template <typename T>
+__device__ __forceinline__ const T* row_of(const MatView& m, const ItemCtx& c, int h, int i) {
+    return (const T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + i) * m.st;
+}
 // Blocks in the order of the item table (heaviest first), the heads and the halves of a 128-row tile innermost: the hardware
 // deals blocks out in this order, so the heavy ones of all heads start first.
 struct BlockIdx {
@@ -426,33 +516,21 @@ __device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * b
 // ------------------------------------------------------------------------------------------ forward
 // Eight warps: four groups of 16 query rows x the two 32-key halves of a tile.  The halves exchange their products once per tile; o
 // is summed over the halves at the end.
-template <typename T, int DP>
-__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __grid_constant__ KArgs a) {
+// kDirect: the sums by multiply-adds on the values themselves.  Returns whether they have to be formed so (nothing is stored then).
+// xs: product of 1 - beta over a half, per row.
+template <typename T, int DP, bool kDirect>
+__device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, __nv_bfloat16* tiles, float (*xs)[kBM]) {
     constexpr int kT = 256, kN = Terms<T>::n;
-    constexpr bool kEarly = sizeof(T) == 2;  // loads a tile ahead; the 32 words of two float32 tiles cost more registers than they gain
-    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
-    __shared__ float xs[2][kBM];  // product of 1 - beta over a half, per row
+    constexpr bool kEarly = sizeof(T) == 2 && !kDirect;  // loads a tile ahead; the 32 words of two float32 tiles cost more registers than they gain
     __nv_bfloat16* sQ = tiles;
     __nv_bfloat16* sK = sQ + kTileElems<T, DP>;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
-    __shared__ OwnTables own;
-    pdl_wait();
-    if (a.own_tables) {
-        if (threadIdx.x < 32) build_own_tables(a, &own, threadIdx.x);
-        __syncthreads();
-    }
-    const int covered_end = a.own_tables ? own.covered_end : a.hdr->covered_end;
-    if (a.zero_tail && covered_end < a.tokens) zero_tail_rows<T>(a, covered_end, linear_thread(), all_threads());
-    const BlockIdx bi = block_idx(a.heads);
-    if (bi.item >= (a.own_tables ? own.n_items : a.hdr->n_items)) return;
-    const ItemCtx c = a.own_tables ? item_ctx(own.items, own.seqs, bi.item) : item_ctx(a, bi.item);
     const int h = bi.h, D = a.head_dim;
     const int row0 = c.qt * kTileQ + bi.part * kBM;
-    if (row0 >= c.len) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;  // hf 0: the left 32 keys, 1: the right
     const int rows_valid = min(kBM, c.len - row0);
-    load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+    if (!kDirect) load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
     const int wrow = 16 * rg + g;  // this lane's rows of the block: wrow, wrow + 8
     float W[2] = {1.f, 1.f};
     float o[1][DP / 8][4] = {};
@@ -477,7 +555,8 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        if (kEarly) {
+        if (kDirect) {
+        } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
             rv.template put<kKeyColumns>(sV, uv);
         } else {
@@ -486,7 +565,8 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
         }
         __syncthreads();
         float s[1][4][4], om[2][8], excl[2];
-        product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
+        if (kDirect) direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key0 + 32 * hf + 8 * t), a.k.st, keys_valid - 32 * hf - 8 * t, D);
+        else product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
         const bool edge = kh == last || keys_valid < kBN;  // some pair of the tile is not visible
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -523,9 +603,9 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
             W[r] = W[r] * right * left;
         }
         if (kEarly && kh > 0) fetch(kh - 1);
-        product_px<kN, DP, DP, 1, 4, true>(o, s, sV + 32 * hf * kPitch<DP>, lane);
+        if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.v, c, h, key0 + 32 * hf), a.v.st, keys_valid - 32 * hf, D, lane);
+        else product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
     }
-    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     float* x = (float*)tiles;
     __syncthreads();
     if (hf == 1) {
@@ -535,11 +615,18 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
     __syncthreads();
-    if (hf == 1) return;
+    bool again = false;
+    if (hf == 0) {
 #pragma unroll
-    for (int n = 0; n < DP / 8; ++n)
+        for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+            for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) again |= wrow + 8 * r < rows_valid && (asks_for_direct(o[0], 2 * r) || W[r] != W[r]);
+    }
+    if (!kDirect && __syncthreads_or(again)) return true;
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    if (hf == 1) return false;
     if (a.fused) {  // out = o + rem * v, each operation rounded by itself: the same bits as the expression outside for float32
         const T* v = (const T*)a.v.ptr + (int64_t)c.b * a.v.sb + (int64_t)h * a.v.sh + (int64_t)(c.start + row0) * a.v.st;
 #pragma unroll
@@ -558,33 +645,50 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
             ((float*)a.nla.ptr)[(int64_t)c.b * a.nla.sb + (int64_t)h * a.nla.sh + tok * a.nla.st] = log2f(W[r]);
         }
     }
+    return false;
+}
+template <typename T, int DP>
+__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __grid_constant__ KArgs a) {
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __shared__ float xs[2][kBM];
+    __shared__ OwnTables own;
+    pdl_wait();
+    if (a.own_tables) {
+        if (threadIdx.x < 32) build_own_tables(a, &own, threadIdx.x);
+        __syncthreads();
+    }
+    const int covered_end = a.own_tables ? own.covered_end : a.hdr->covered_end;
+    if (a.zero_tail && covered_end < a.tokens) zero_tail_rows<T>(a, covered_end, linear_thread(), all_threads());
+    const BlockIdx bi = block_idx(a.heads);
+    if (bi.item >= (a.own_tables ? own.n_items : a.hdr->n_items)) return;
+    const auto item = [&]() { return a.own_tables ? item_ctx(own.items, own.seqs, bi.item) : item_ctx(a, bi.item); };
+    const ItemCtx c = item();
+    if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
+    // (16-bit types look their item up again instead of keeping it: the loop has no register to spare for it.  35.8 -> 35.3 us on
+    // 4 x 8 heads x 500 tokens, head dim 50; float32 loses by it, 132 -> 137 us on 8 heads, 4096 tokens)
+    if (fwd_block<T, DP, false>(a, c, bi, tiles, xs)) fwd_block<T, DP, true>(a, sizeof(T) == 2 ? item() : c, bi, tiles, xs);
 }
 
 // ------------------------------------------------------------------------------------------ backward: dq
 // Warps as in the forward; W comes from the forward's carries, the halves exchange their sums of g.
-template <typename T, int DP>
-__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const __grid_constant__ KArgs a) {
+// xs: sum of g over a half, per row.
+template <typename T, int DP, bool kDirect>
+__device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, __nv_bfloat16* tiles, float (*xs)[kBM]) {
     constexpr int kT = 256, kN = Terms<T>::n;
-    constexpr bool kEarly = kN == 1 || (kN == 2 && DP < 64);  // loads a tile ahead, where registers allow
-    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
-    __shared__ float xs[2][kBM];  // sum of g over a half, per row
+    constexpr bool kEarly = (kN == 1 || (kN == 2 && DP < 64)) && !kDirect;  // loads a tile ahead, where registers allow
     __nv_bfloat16* sQ = tiles;
     __nv_bfloat16* sG = sQ + kTileElems<T, DP>;  // dO
     __nv_bfloat16* sK = sG + kTileElems<T, DP>;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
-    pdl_wait();
-    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
-    const BlockIdx bi = block_idx(a.heads);
-    if (bi.item >= a.hdr->n_items) return;
-    const ItemCtx c = item_ctx(a, bi.item);
     const int h = bi.h, D = a.head_dim;
     const int row0 = c.qt * kTileQ + bi.part * kBM;
-    if (row0 >= c.len) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;
     const int rows_valid = min(kBM, c.len - row0);
-    load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
-    load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+    if (!kDirect) {
+        load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
+        load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
+    }
     const int wrow = 16 * rg + g;
     float drem[2], prefix[2] = {0.f, 0.f};  // prefix: sum of g over all keys left of the current tile
 #pragma unroll
@@ -609,7 +713,8 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
         __syncthreads();
-        if (kEarly) {
+        if (kDirect) {
+        } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
             rv.template put<kKeyColumns>(sV, uv);
         } else {
@@ -622,8 +727,14 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
         for (int r = 0; r < 2; ++r) W[r] = wrow + 8 * r < rows_valid ? cw[slot + 8 * r] : 0.f;
         __syncthreads();
         float s[1][4][4], dp[1][4][4], excl[2];
-        product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
-        product_nt<kN, DP, 1, 4>(dp, sG + 16 * rg * kPitch<DP>, sV + 32 * hf * kPitch<DP>, D, lane);
+        if (kDirect) {
+            const int key = key0 + 32 * hf + 8 * t, keys = keys_valid - 32 * hf - 8 * t;
+            direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key), a.k.st, keys, D);
+            direct_scores<T>(dp, row_of<T>(a.d_o, c, h, row0 + wrow), a.d_o.st, rows_valid - wrow, row_of<T>(a.v, c, h, key), a.v.st, keys, D);
+        } else {
+            product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
+            product_nt<kN, DP, 1, 4>(dp, sG + 16 * rg * kPitch<DP>, sV + 32 * hf * kPitch<DP>, D, lane);
+        }
         const bool edge = kh == last || keys_valid < kBN;
         // right to left: s <- beta, dp <- g
 #pragma unroll
@@ -675,9 +786,9 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
             prefix[r] = prefix[r] + left + right;
         }
         if (kEarly && kh < last) fetch(kh + 1);
-        product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
+        if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.k, c, h, key0 + 32 * hf), a.k.st, keys_valid - 32 * hf, D, lane);
+        else product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
     }
-    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     float* x = (float*)tiles;
     __syncthreads();
     if (hf == 1) {
@@ -687,16 +798,36 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
     __syncthreads();
-    if (hf == 1) return;
+    bool again = false;
+    if (hf == 0) {
 #pragma unroll
-    for (int n = 0; n < DP / 8; ++n)
+        for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+            for (int e = 0; e < 4; ++e) o[0][n][e] += x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) again |= wrow + 8 * r < rows_valid && asks_for_direct(o[0], 2 * r);
+    }
+    if (!kDirect && __syncthreads_or(again)) return true;
+    pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
+    if (hf == 1) return false;
     const bool pairs = units_ok<T>(a.dq, D, 2);
     T* base = (T*)a.dq.ptr + (int64_t)c.b * a.dq.sb + (int64_t)h * a.dq.sh + (int64_t)(c.start + row0) * a.dq.st;
 #pragma unroll
     for (int r = 0; r < 2; ++r)
         if (wrow + 8 * r < rows_valid) store_row<T, DP>(o[0], 2 * r, a.inv_temp, a.dq, pairs, D, 0, base, wrow + 8 * r, t);
+    return false;
+}
+template <typename T, int DP>
+__global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const __grid_constant__ KArgs a) {
+    extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+    __shared__ float xs[2][kBM];
+    pdl_wait();
+    if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
+    const BlockIdx bi = block_idx(a.heads);
+    if (bi.item >= a.hdr->n_items) return;
+    const ItemCtx c = item_ctx(a, bi.item);
+    if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
+    if (dq_block<T, DP, false>(a, c, bi, tiles, xs)) dq_block<T, DP, true>(a, c, bi, tiles, xs);
 }
 
 // ------------------------------------------------------------------------------------------ backward: dk, dv
@@ -784,7 +915,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
     const int quarter = key0 / 32 + kq;            // of the sequence
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    float acc[kDC / 8][4] = {};
+    float acc[kDC / 8][4];
 
     const int uq = unit<T>(a.q, D), ug = unit<T>(a.d_o, D);
     Rows<kT, T, DP, kQ> rq, rg;
@@ -793,100 +924,142 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
         rq.fetch(a.q, uq, D, c.b, h, c.start + row0, n);
         rg.fetch(a.d_o, ug, D, c.b, h, c.start + row0, n);
     };
-    if (kEarly) fetch(key0);
-    if (kBuf == 2) {
-        rq.template put<kPlain>(sQ, uq);
-        rg.template put<kPlain>(sG, ug);
-    }
-    for (int row0 = key0; row0 < c.len; row0 += kQ) {
-        const int rows_valid = min(kQ, c.len - row0);
-        if (kBuf == 1) {
-            if (!kEarly) fetch(row0);
-            __syncthreads();
+    const auto sweep = [&](auto direct) {
+        constexpr bool kDirect = decltype(direct)::value;
+        float* const fP = (float*)sP;  // direct: P^T and dS^T as they are, one after the other
+        float* const fS = fP + kPPlane;
+        static_assert(2 * sizeof(float) * kPPlane <= 2 * kWTerms * sizeof(__nv_bfloat16) * kPPlane, "P^T and dS^T in the place of their terms");
+#pragma unroll
+        for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+        if (kEarly && !kDirect) fetch(key0);
+        if (kBuf == 2 && !kDirect) {
             rq.template put<kPlain>(sQ, uq);
             rg.template put<kPlain>(sG, ug);
         }
-        const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, quarter) * kTileQ + row0 % kTileQ;
-        float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int q = q0 + 2 * t + e;
-            if (q < rows_valid) {
-                W[e] = cw[slot + q];
-                cr[e] = cc[slot + q];
-                drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
+        for (int row0 = key0; row0 < c.len; row0 += kQ) {
+            const int rows_valid = min(kQ, c.len - row0);
+            if (kDirect) {
+                __syncthreads();
+            } else if (kBuf == 1) {
+                if (!kEarly) fetch(row0);
+                __syncthreads();
+                rq.template put<kPlain>(sQ, uq);
+                rg.template put<kPlain>(sG, ug);
             }
-        }
-        __syncthreads();
-        const bool edge = row0 < key0 + kBN || keys_valid < kBN || rows_valid < kQ;
-        if (q0 < kQ) {
-            float s[2][1][4], dp[2][1][4];
-            product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
-            product_nt<kN, DP, 2, 1, kQ>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+            const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, quarter) * kTileQ + row0 % kTileQ;
+            float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
-                float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
                 const int q = q0 + 2 * t + e;
-                // a query behind the end of the sequence sees no key: its zeros against an infinite or NaN key would make NaNs
-                const int lim = q < rows_valid ? min(keys_valid, row0 + q + a.attend_current - key0) : 0;
-                column(ps, pd, a.inv_temp, edge, lim - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
-            }
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    uint32_t tp[kWTerms], ts[kWTerms];
-                    split_pair<kWTerms, true>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
-                    split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
-                    const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
-#pragma unroll
-                    for (int i = 0; i < kWTerms; ++i) {
-                        *(uint32_t*)(sP + i * kPPlane + at) = tp[i];
-                        *(uint32_t*)(sS + i * kPPlane + at) = ts[i];
-                    }
+                if (q < rows_valid) {
+                    W[e] = cw[slot + q];
+                    cr[e] = cc[slot + q];
+                    drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
                 }
-        }
-        __syncthreads();
-        if (kEarly && row0 + kQ < c.len) fetch(row0 + kQ);
-        if (second) {
-            const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
-            const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
+            }
+            __syncthreads();
+            const bool edge = row0 < key0 + kBN || keys_valid < kBN || rows_valid < kQ;
+            if (q0 < kQ) {
+                float s[2][1][4], dp[2][1][4];
+                if (kDirect) {
+                    const int key = 32 * kq + 4 * g, q = q0 + 2 * t;
+                    direct_scores_t<T>(s, row_of<T>(a.k, c, h, key0 + key), a.k.st, keys_valid - key, row_of<T>(a.q, c, h, row0 + q), a.q.st, rows_valid - q, D);
+                    direct_scores_t<T>(dp, row_of<T>(a.v, c, h, key0 + key), a.v.st, keys_valid - key, row_of<T>(a.d_o, c, h, row0 + q), a.d_o.st, rows_valid - q, D);
+                } else {
+                    product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
+                    product_nt<kN, DP, 2, 1, kQ>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+                }
 #pragma unroll
-            for (int n0 = 0; n0 < kDC / 8; n0 += kNC) {
-                float big[kNC][4] = {}, small[kNC][4] = {};
+                for (int e = 0; e < 2; ++e) {
+                    float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
+                    float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
+                    const int q = q0 + 2 * t + e;
+                    // a query behind the end of the sequence sees no key: its zeros against an infinite or NaN key would make NaNs
+                    const int lim = q < rows_valid ? min(keys_valid, row0 + q + a.attend_current - key0) : 0;
+                    column(ps, pd, a.inv_temp, edge, lim - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
+                }
 #pragma unroll
-                for (int k = 0; k < kQ / 16; ++k) {
-                    uint32_t fa[kWTerms][4];
+                for (int m = 0; m < 2; ++m)
 #pragma unroll
-                    for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
-#pragma unroll
-                    for (int j = 0; j < kN; ++j) {
-                        uint32_t fb[kNC / 2][4];
-#pragma unroll
-                        for (int n2 = 0; n2 < kNC / 2; ++n2)
-                            ldsm4_t(fb[n2], px + j * kQ * kPitch<DP> + k * 16 * kPitch<DP> + n0 * 8 + n2 * 16);
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
+                        if (kDirect) {
+                            *(float2*)(fP + at) = make_float2(s[m][0][2 * hh], s[m][0][2 * hh + 1]);
+                            *(float2*)(fS + at) = make_float2(dp[m][0][2 * hh], dp[m][0][2 * hh + 1]);
+                            continue;
+                        }
+                        uint32_t tp[kWTerms], ts[kWTerms];
+                        split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
+                        split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
 #pragma unroll
                         for (int i = 0; i < kWTerms; ++i) {
-                            if (i + j > 2) continue;
-#pragma unroll
-                            for (int n = 0; n < kNC; ++n) mma(i + j == 0 ? big[n] : small[n], fa[i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                            *(uint32_t*)(sP + i * kPPlane + at) = tp[i];
+                            *(uint32_t*)(sS + i * kPPlane + at) = ts[i];
                         }
                     }
+            }
+            __syncthreads();
+            if (kEarly && !kDirect && row0 + kQ < c.len) fetch(row0 + kQ);
+            if (kDirect && second) {
+                const MatView& mx = is_dk ? a.q : a.d_o;
+                const T* x = row_of<T>(mx, c, h, row0) + col0 + 2 * t;
+                const float* pa = (is_dk ? fS : fP) + (16 * kg + g) * kPP;
+#pragma unroll 1
+                for (int q = 0; q < rows_valid; ++q) {
+                    const float p0 = pa[q], p1 = pa[8 * kPP + q];
+#pragma unroll
+                    for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float v = col0 + 8 * n + 2 * t + e < D ? to_f32<T>(x[(int64_t)q * mx.st + 8 * n + e]) : 0.f;
+                            acc[n][e] = fmaf(p0, v, acc[n][e]);
+                            acc[n][2 + e] = fmaf(p1, v, acc[n][2 + e]);
+                        }
                 }
+            }
+            if (!kDirect && second) {
+                const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
+                const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
 #pragma unroll
-                for (int n = 0; n < kNC; ++n)
+                for (int n0 = 0; n0 < kDC / 8; n0 += kNC) {
+                    float big[kNC][4] = {}, small[kNC][4] = {};
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[n0 + n][i] += big[n][i] + small[n][i];
+                    for (int k = 0; k < kQ / 16; ++k) {
+                        uint32_t fa[kWTerms][4];
+#pragma unroll
+                        for (int i = 0; i < kWTerms; ++i) ldsm4(fa[i], pa + i * kPPlane + 16 * k);
+#pragma unroll
+                        for (int j = 0; j < kN; ++j) {
+                            uint32_t fb[kNC / 2][4];
+#pragma unroll
+                            for (int n2 = 0; n2 < kNC / 2; ++n2)
+                                ldsm4_t(fb[n2], px + j * kQ * kPitch<DP> + k * 16 * kPitch<DP> + n0 * 8 + n2 * 16);
+#pragma unroll
+                            for (int i = 0; i < kWTerms; ++i) {
+                                if (i + j > 2) continue;
+#pragma unroll
+                                for (int n = 0; n < kNC; ++n) mma(i + j == 0 ? big[n] : small[n], fa[i], fb[n >> 1][2 * (n & 1)], fb[n >> 1][2 * (n & 1) + 1]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int n = 0; n < kNC; ++n)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[n0 + n][i] += big[n][i] + small[n][i];
+                }
+            }
+            if (kBuf == 2 && !kDirect && row0 + kQ < c.len) {
+                sQ = tiles_q + (sQ == tiles_q ? 2 * kQTile : 0);
+                sG = sQ + kQTile;
+                rq.template put<kPlain>(sQ, uq);
+                rg.template put<kPlain>(sG, ug);
             }
         }
-        if (kBuf == 2 && row0 + kQ < c.len) {
-            sQ = tiles_q + (sQ == tiles_q ? 2 * kQTile : 0);
-            sG = sQ + kQTile;
-            rq.template put<kPlain>(sQ, uq);
-            rg.template put<kPlain>(sG, ug);
-        }
-    }
+        return __syncthreads_or(asks_for_direct(acc, 0) || asks_for_direct(acc, 2));
+    };
+    if (sweep(std::false_type{})) sweep(std::true_type{});
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
     if (!second) return;
     if (a.fused && !is_dk) {  // dv += rem * do
