@@ -382,9 +382,12 @@ PYBIND11_MODULE(_binding, m) {
             torch::translate_exception_to_python(p);
         }
     });
-    m.def("attend", &attend);
-    m.def("fwd", &fwd);
-    m.def("bwd", &bwd);
-    m.def("seq_bounds", &seq_bounds);
-    m.def("status_word", &status_word);
+    // Without the interpreter lock: the calls may wait for the GPU (seq_bounds does, an allocation and the status check may), and what the
+    // GPU has queued may in turn wait for another Python thread.
+    const auto unlocked = py::call_guard<py::gil_scoped_release>();
+    m.def("attend", &attend, unlocked);
+    m.def("fwd", &fwd, unlocked);
+    m.def("bwd", &bwd, unlocked);
+    m.def("seq_bounds", &seq_bounds, unlocked);
+    m.def("status_word", &status_word, unlocked);
 }
