@@ -83,6 +83,12 @@ void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v, int ndim) {
     TORCH_CHECK_VALUE(k.device() == q.device() && v.device() == q.device(), "q, k, v must live on one device");
     TORCH_CHECK_VALUE(q.size(-1) <= 128, "head_dim above 128 is not supported");
 }
+// Forward-mode differentiation is not implemented.  Refused here, for calls whose inputs need no gradient too: these pass the autograd
+// node by, which would refuse it, and would drop the tangents without a word.
+void refuse_forward_mode(const Tensor& q, const Tensor& k, const Tensor& v) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!q._fw_grad(0).defined() && !k._fw_grad(0).defined() && !v._fw_grad(0).defined(),
+                                "stick-breaking attention does not implement forward mode AD");
+}
 void require_cuda(const Tensor& t) {
     TORCH_CHECK(t.is_cuda(), "stick-breaking attention runs on CUDA tensors only (there is no CPU implementation)");
 }
@@ -319,6 +325,7 @@ std::pair<Tensor, Tensor> attend(const Tensor& q, const Tensor& k, const Tensor&
                                  double scale, bool attend_current, bool fused, bool recompute, int path) {
     const bool batched = !cu_seqlens.has_value();
     check_qkv(q, k, v, batched ? 4 : 3);
+    refuse_forward_mode(q, k, v);
     Tensor cu;
     if (batched) max_seqlens = q.size(2);
     else cu = prep_cu(*cu_seqlens, q, max_seqlens);

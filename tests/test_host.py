@@ -100,6 +100,23 @@ def test_shape_and_dtype_validation():
         sb_attn_varlen(q, q, q, torch.tensor([4, 16]), 16, zero_start=True)
 
 
+@pytest.mark.parametrize("requires_grad", [False, True])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_forward_mode_is_refused(which, requires_grad):
+    """Dual tensors raise, also where no gradient is asked for (a call that passes the autograd node by would drop the tangents)."""
+    import torch.autograd.forward_ad as fw
+    from stickbreaking_attention_b200 import sb_attn, sb_attn_varlen
+    with fw.dual_level():
+        x = [torch.randn(2, 16, 8) for _ in range(3)]
+        x[which] = fw.make_dual(x[which].requires_grad_(requires_grad), torch.ones(2, 16, 8))
+        with pytest.raises(NotImplementedError):
+            sb_attn_varlen(*x, torch.tensor([0, 16]), 16)
+        with pytest.raises(NotImplementedError):
+            sb_attn(*(y[None] for y in x))
+        with torch.no_grad(), pytest.raises(NotImplementedError):
+            sb_attn_varlen(*x, torch.tensor([0, 16]), 16)
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "stickbreaking_attention_b200")
     for dirpath, _, files in os.walk(pkg):
