@@ -73,10 +73,10 @@ typedef struct SbVec {
  * reference computes next: tests/test_varlen.py:103, tests/test_attn.py:67, benchmarks/varlen.py:53), with rem rounded
  * to the output dtype first, as in that expression.  The backward then takes d_o = gradient of out and d_rem = gradient
  * of the separately returned rem, needs `rem` (the forward's output) and `v`, and returns dv including rem * d_o.
- * The backward takes it on the tensor-core path only (16-bit inputs, head_dim 32, 64 or 128): otherwise SBATTN_EUNSUPPORTED. */
+ * Tensor-core path only (16-bit inputs, head_dim 32, 64 or 128): otherwise SBATTN_EUNSUPPORTED, from forward and backward alike. */
 #define SBATTN_FLAG_FUSED_REMAINDER 1
-/* Backward on the kernels of float32 precision: d_rem already holds the whole gradient of rem (d_rem + sum over D of d_o * v); `rem` is
- * the forward's, and dv includes rem * d_o. */
+/* The same on the kernels of float32 precision (SBATTN_EUNSUPPORTED on the tensor-core path).  Forward: o + rem * v into `o`.  Backward:
+ * d_rem already holds the whole gradient of rem (d_rem + sum over D of d_o * v); `rem` is the forward's, and dv includes rem * d_o. */
 #define SBATTN_FLAG_REMAINDER_IN_DV 2
 
 typedef struct SbParams {

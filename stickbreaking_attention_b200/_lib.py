@@ -36,7 +36,7 @@ class SbParams(ctypes.Structure):
     ]
 
 
-FLAG_FUSED_REMAINDER = 1
+FLAG_FUSED_REMAINDER, FLAG_REMAINDER_IN_DV = 1, 2
 
 EXPORTS = ("sbattn_workspace_bytes", "sbattn_fwd", "sbattn_bwd", "sbattn_strerror", "sbattn_version",
            "sbattn_params_size", "sbattn_fwd_static", "sbattn_static_scratch_bytes", "sbattn_attention_weights",

@@ -154,7 +154,9 @@ extern "C" int sbattn_fwd(const SbParams* p) {
     if (((uintptr_t)p->fwd_workspace & 255) != 0) return SBATTN_EWORKSPACE;
     const int path = choose_path(*p, false);
     if (path < 0) return path;
-    if (p->flags & SBATTN_FLAG_REMAINDER_IN_DV) return SBATTN_EINVAL;  // a flag of the backward
+    // the fused remainder has one flag per kernel family: what the backward would refuse, the forward refuses already
+    if ((p->flags & SBATTN_FLAG_FUSED_REMAINDER) && path != 1) return SBATTN_EUNSUPPORTED;
+    if ((p->flags & SBATTN_FLAG_REMAINDER_IN_DV) && path != 0) return SBATTN_EUNSUPPORTED;
     cudaStream_t st = (cudaStream_t)p->stream;
     KArgs a = make_args(*p, L);
     a.own_tables = forward_builds_tables(*p, L, path == 1);

@@ -182,7 +182,7 @@ SbParams base_params(const Tensor& q, const Tensor& cu, const Opts& o, bool save
     p.attend_current = o.attend_current;
     p.inv_temp = (float)o.scale;
     p.save_carries = save;
-    p.flags = o.fused || o.f32_fused ? SBATTN_FLAG_FUSED_REMAINDER : 0;
+    p.flags = o.fused ? SBATTN_FLAG_FUSED_REMAINDER : o.f32_fused ? SBATTN_FLAG_REMAINDER_IN_DV : 0;
     p.status = status_ptr(q.get_device());
     p.stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
     return p;
@@ -268,10 +268,7 @@ std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Ten
     }
     SbParams p = base_params(q, cu, opt, true);
     p.bwd_phases = phases;
-    if (opt.f32_fused) {
-        p.flags = SBATTN_FLAG_REMAINDER_IN_DV;
-        d_rem = d_rem + (d_o * v).sum(-1);  // as autograd of o + rem * v forms it
-    }
+    if (opt.f32_fused) d_rem = d_rem + (d_o * v).sum(-1);  // as autograd of o + rem * v forms it
     size_t fb = 0, bb = 0;
     check(sbattn_workspace_bytes(&p, &fb, &bb), "sbattn_workspace_bytes");
     TORCH_CHECK_VALUE((size_t)ws.numel() >= fb, "the forward workspace does not belong to this problem (was the forward run with no_grad?)");

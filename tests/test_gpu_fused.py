@@ -137,6 +137,21 @@ def test_fused_falls_back_for_float32_inputs():
         assert torch.equal(a_, b_)
 
 
+@pytest.mark.parametrize("D,dtype", [(64, torch.float32), (50, torch.bfloat16)])
+def test_launchers_refuse_the_fused_sum_at_float32_precision_in_the_forward(D, dtype):
+    """Its backward does not exist there (sb_attn and sb_attn_varlen form the sum in another way), so the forward raises, not the
+    backward after a whole forward pass."""
+    from stickbreaking_attention_b200 import _lib, ops
+    from stickbreaking_attention_b200.sb_attn import StickBreakingAttention as Batched
+    from stickbreaking_attention_b200.sb_varlen import StickBreakingAttention as Packed
+    q = torch.randn(2, 256, D, device="cuda", dtype=dtype)
+    cu = torch.tensor([100, 256], device="cuda")
+    for call in (lambda: ops.varlen_fwd(q, q, q, cu, 256, 0.1, fuse_remainder=True), lambda: ops.attn_fwd(q[None], q[None], q[None], 0.1, fuse_remainder=True),
+                 lambda: Packed.apply(q, q, q, cu, 256, 0.1, False, True), lambda: Batched.apply(q[None], q[None], q[None], 0.1, False, True)):
+        with pytest.raises(_lib.SbAttnError, match="unsupported"):
+            call()
+
+
 @pytest.mark.parametrize("D,dtype", [(64, torch.float32), (128, torch.float32), (50, torch.bfloat16), (33, torch.float16), (16, torch.bfloat16)])
 @pytest.mark.parametrize("heads", [2, 30])
 def test_varlen_fused_at_float32_precision_against_oracle(D, dtype, heads):
