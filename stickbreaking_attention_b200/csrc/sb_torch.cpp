@@ -279,7 +279,7 @@ std::array<Tensor, 3> backward(Tensor d_o, Tensor d_rem, Tensor q, Tensor k, Ten
     p.v = mat(v, opt.batched);
     p.d_o = mat(d_o, opt.batched);
     p.d_rem = vec(d_rem, opt.batched);
-    if (opt.fused || opt.f32_fused) p.rem = vec(rem.defined() ? rem : d_rem, opt.batched);
+    if (opt.fused || opt.f32_fused) p.rem = vec(rem, opt.batched);
     p.dq = mat(g[0], opt.batched);
     p.dk = mat(g[1], opt.batched);
     p.dv = mat(g[2], opt.batched);
@@ -362,6 +362,8 @@ std::array<Tensor, 3> bwd(const Tensor& d_o, const Tensor& d_rem, const Tensor& 
     at::NoGradGuard guard;
     const bool batched = !cu_seqlens.has_value();
     check_qkv(q, k, v, batched ? 4 : 3);
+    TORCH_CHECK_VALUE(!fused || (rem && rem->sizes() == q.sizes().slice(0, q.dim() - 1) && rem->scalar_type() == q.scalar_type() && rem->device() == q.device()),
+                      "the backward of the fused sum needs the forward's rem: the leading sizes, dtype and device of q");
     Tensor cu;
     if (batched) max_seqlens = q.size(2);
     else cu = prep_cu(*cu_seqlens, q, max_seqlens);

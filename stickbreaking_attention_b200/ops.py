@@ -301,7 +301,9 @@ def _forward_traced(q, k, v, batched, cu_seqlens, max_seqlens, logit_scale, atte
 def _backward_traced(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logit_scale, attend_current, fused=False, rem=None):
     """The backward while torch.compile is tracing."""
     if rem is None:
-        rem = dr  # placeholder of the right shape: only read when fused
+        if fused:
+            raise ValueError("the backward of the fused sum needs the forward's rem")
+        rem = dr  # placeholder of the right shape: not read
     q, k, v, do = _unit_inner(q), _unit_inner(k), _unit_inner(v), _unit_inner(do)
     if do.dtype != q.dtype:
         do = do.to(q.dtype)

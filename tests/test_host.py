@@ -117,6 +117,18 @@ def test_forward_mode_is_refused(which, requires_grad):
             sb_attn_varlen(*x, torch.tensor([0, 16]), 16)
 
 
+def test_fused_backward_needs_the_forwards_rem():
+    from stickbreaking_attention_b200 import ops
+    q, rem, ws = torch.randn(2, 16, 32), torch.zeros(2, 16), torch.zeros(1, dtype=torch.uint8)
+    for bad in (None, rem[:, :8], rem.double(), q):
+        with pytest.raises(ValueError, match="rem"):
+            ops.varlen_bwd(q, rem, q, q, q, torch.tensor([16]), 16, ws, 0.1, fuse_remainder=True, rem=bad)
+        with pytest.raises(ValueError, match="rem"):
+            ops.attn_bwd(q[None], rem[None], q[None], q[None], q[None], ws, 0.1, fuse_remainder=True, rem=bad if bad is None else bad[None])
+    with pytest.raises(RuntimeError, match="CUDA"):  # the right one gets past the check
+        ops.varlen_bwd(q, rem, q, q, q, torch.tensor([16]), 16, ws, 0.1, fuse_remainder=True, rem=rem)
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "stickbreaking_attention_b200")
     for dirpath, _, files in os.walk(pkg):
