@@ -327,9 +327,14 @@ def _backward_traced(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logi
     return dq, dk, dv
 
 
+def _length(max_seqlens):
+    """What int() takes (a float, a 0-d tensor), not only what the binding would."""
+    return None if max_seqlens is None else int(max_seqlens)
+
+
 def attend(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, fuse_remainder):
     """(o, rem) with an autograd node, through the native host path; cu_seqlens None: batched layout."""
-    return _lib.binding().attend(q, k, v, cu_seqlens, max_seqlens, logit_scale, bool(attend_current), bool(fuse_remainder),
+    return _lib.binding().attend(q, k, v, cu_seqlens, _length(max_seqlens), float(logit_scale), bool(attend_current), bool(fuse_remainder),
                                  _carry_policy == "recompute", _PATHS[_forced_path])
 
 
@@ -384,7 +389,7 @@ def varlen_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current=Fal
         cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
         out = _forward_traced(q, k, v, False, cu_seqlens, max_seqlens, logit_scale, attend_current, no_grad, fuse_remainder)
     else:
-        out = _lib.binding().fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, bool(attend_current), bool(no_grad),
+        out = _lib.binding().fwd(q, k, v, cu_seqlens, _length(max_seqlens), float(logit_scale), bool(attend_current), bool(no_grad),
                                  bool(fuse_remainder), _PATHS[_forced_path])
     if return_attention:
         return out + (attention_weights(q, k, cu_seqlens, logit_scale, attend_current),)
@@ -401,7 +406,7 @@ def varlen_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, workspace, logit_scale,
         cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
         return _backward_traced(do, dr, q, k, v, False, cu_seqlens, max_seqlens, workspace, logit_scale, attend_current,
                                 fuse_remainder, rem)
-    return tuple(_lib.binding().bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, workspace, logit_scale, bool(attend_current), phases,
+    return tuple(_lib.binding().bwd(do, dr, q, k, v, cu_seqlens, _length(max_seqlens), workspace, float(logit_scale), bool(attend_current), phases,
                                     bool(fuse_remainder), rem, _PATHS[_forced_path], list(out) if out is not None else [], bwd_workspace))
 
 
@@ -412,7 +417,7 @@ def attn_fwd(q, k, v, logit_scale, attend_current=False, no_grad=False, fuse_rem
         _check_qkv(q, k, v, 4)
         out = _forward_traced(q, k, v, True, None, q.size(2), logit_scale, attend_current, no_grad, fuse_remainder)
     else:
-        out = _lib.binding().fwd(q, k, v, None, None, logit_scale, bool(attend_current), bool(no_grad), bool(fuse_remainder),
+        out = _lib.binding().fwd(q, k, v, None, None, float(logit_scale), bool(attend_current), bool(no_grad), bool(fuse_remainder),
                                  _PATHS[_forced_path])
     if return_attention:
         return out + (attention_weights(q, k, None, logit_scale, attend_current),)
@@ -424,5 +429,5 @@ def attn_bwd(do, dr, q, k, v, workspace, logit_scale, attend_current=False, fuse
     if torch.compiler.is_compiling():
         _check_qkv(q, k, v, 4)
         return _backward_traced(do, dr, q, k, v, True, None, q.size(2), workspace, logit_scale, attend_current, fuse_remainder, rem)
-    return tuple(_lib.binding().bwd(do, dr, q, k, v, None, None, workspace, logit_scale, bool(attend_current), 0, bool(fuse_remainder),
+    return tuple(_lib.binding().bwd(do, dr, q, k, v, None, None, workspace, float(logit_scale), bool(attend_current), 0, bool(fuse_remainder),
                                     rem, _PATHS[_forced_path], [], None))

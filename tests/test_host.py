@@ -4,6 +4,7 @@ import ctypes
 import os
 import re
 
+import numpy as np
 import pytest
 import torch
 
@@ -127,6 +128,20 @@ def test_fused_backward_needs_the_forwards_rem():
             ops.attn_bwd(q[None], rem[None], q[None], q[None], q[None], ws, 0.1, fuse_remainder=True, rem=bad if bad is None else bad[None])
     with pytest.raises(RuntimeError, match="CUDA"):  # the right one gets past the check
         ops.varlen_bwd(q, rem, q, q, q, torch.tensor([16]), 16, ws, 0.1, fuse_remainder=True, rem=rem)
+
+
+@pytest.mark.parametrize("number", [float, np.float64, np.int64, torch.tensor, str])
+def test_numbers_that_int_and_float_take_are_taken(number):
+    """max_seqlens and the scale come as whatever int() and float() accept (a float length was a float division's result): the calls
+    get as far as the missing GPU."""
+    from stickbreaking_attention_b200 import ops, sb_attn, sb_attn_varlen
+    q, cu, ws = torch.randn(2, 16, 32), torch.tensor([16]), torch.zeros(1, dtype=torch.uint8)
+    m, scale = number(16), 1.0 if number is np.int64 else number(0.5)
+    for call in (lambda: sb_attn_varlen(q, q, q, cu, m, scale, zero_start=False), lambda: sb_attn(q[None], q[None], q[None], scale),
+                 lambda: ops.varlen_fwd(q, q, q, cu, m, scale), lambda: ops.varlen_bwd(q, q[..., 0], q, q, q, cu, m, ws, scale),
+                 lambda: ops.attn_fwd(q[None], q[None], q[None], scale), lambda: ops.attn_bwd(q[None], q[None, ..., 0], q[None], q[None], q[None], ws, scale)):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            call()
 
 
 def test_product_never_imports_the_oracle():
