@@ -406,8 +406,11 @@ def varlen_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, workspace, logit_scale,
         cu_seqlens, max_seqlens = _prep_cu(cu_seqlens, q, max_seqlens)
         return _backward_traced(do, dr, q, k, v, False, cu_seqlens, max_seqlens, workspace, logit_scale, attend_current,
                                 fuse_remainder, rem)
+    if out is not None:
+        dq, dk, dv = out
+        out = [dq, dk, dv]
     return tuple(_lib.binding().bwd(do, dr, q, k, v, cu_seqlens, _length(max_seqlens), workspace, float(logit_scale), bool(attend_current), phases,
-                                    bool(fuse_remainder), rem, _PATHS[_forced_path], list(out) if out is not None else [], bwd_workspace))
+                                    bool(fuse_remainder), rem, _PATHS[_forced_path], out or [], bwd_workspace))
 
 
 def attn_fwd(q, k, v, logit_scale, attend_current=False, no_grad=False, fuse_remainder=False, return_attention=False):

@@ -144,6 +144,16 @@ def test_numbers_that_int_and_float_take_are_taken(number):
             call()
 
 
+def test_backward_into_given_tensors_takes_exactly_three():
+    from stickbreaking_attention_b200 import ops
+    q, ws = torch.randn(2, 16, 32), torch.zeros(1, dtype=torch.uint8)
+    for n in (0, 1, 2, 4):
+        with pytest.raises(ValueError):
+            ops.varlen_bwd(q, q[..., 0], q, q, q, torch.tensor([16]), 16, ws, 0.1, out=(torch.empty_like(q),) * n)
+    with pytest.raises(RuntimeError, match="CUDA"):
+        ops.varlen_bwd(q, q[..., 0], q, q, q, torch.tensor([16]), 16, ws, 0.1, out=iter([torch.empty_like(q)] * 3))
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "stickbreaking_attention_b200")
     for dirpath, _, files in os.walk(pkg):
