@@ -135,10 +135,16 @@ Tensor prep_cu(const Tensor& cu, const Tensor& q, std::optional<int64_t>& max_se
 }
 
 Tensor unit_inner(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
-// Allocations past the dispatcher (~0.5 us each less): the caching allocator's memory all the same
-Tensor empty_like_dtype(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype) { return at::detail::empty_cuda(sizes, dtype, t.device(), std::nullopt); }
+// Allocations past the dispatcher (~0.5 us each less): the caching allocator's memory all the same.  Not where torch fills new memory
+// (torch.use_deterministic_algorithms): the rows of o behind the last sequence stay as they were allocated.
+bool fills_memory() { return at::globalContext().deterministicAlgorithms() && at::globalContext().deterministicFillUninitializedMemory(); }
+Tensor empty_like_dtype(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype) {
+    return fills_memory() ? at::empty(sizes, t.options().dtype(dtype)) : at::detail::empty_cuda(sizes, dtype, t.device(), std::nullopt);
+}
 Tensor empty_rows(const Tensor& t) {
-    if (t.is_non_overlapping_and_dense() && t.stride(-1) == 1) return at::detail::empty_strided_cuda(t.sizes(), t.strides(), t.scalar_type(), t.device());
+    if (t.is_non_overlapping_and_dense() && t.stride(-1) == 1)
+        return fills_memory() ? at::empty_strided(t.sizes(), t.strides(), t.options())
+                              : at::detail::empty_strided_cuda(t.sizes(), t.strides(), t.scalar_type(), t.device());
     Tensor out = at::empty_like(t);
     return out.stride(-1) == 1 ? out : at::empty(t.sizes(), t.options());
 }

@@ -37,3 +37,22 @@ def test_other_threads_run_while_a_call_waits(max_seqlens):
     torch.cuda.synchronize()
     assert took > 0.05  # the call did wait
     assert advanced >= 10, (took, advanced)
+
+
+@pytest.mark.parametrize("token_major", [False, True])
+def test_rows_behind_the_last_sequence_are_filled_in_deterministic_mode(token_major):
+    """torch.use_deterministic_algorithms fills new memory with NaN; the rows of o that no kernel writes hold what was allocated."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    cu = torch.tensor([0, 100, 256], device="cuda")
+    q = torch.randn(2, 300, 64, device="cuda", dtype=torch.bfloat16)
+    if token_major:
+        q = q.transpose(0, 1).contiguous().transpose(0, 1)
+    torch.full((2, 300, 64), 7.0, device="cuda", dtype=torch.bfloat16)  # what the next allocation of this size would find
+    before = torch.are_deterministic_algorithms_enabled()
+    torch.use_deterministic_algorithms(True)
+    try:
+        for x in (q, q.clone().requires_grad_()):
+            o, _ = sb_attn_varlen(x, x, x, cu, 256)
+            assert torch.isnan(o[:, 256:]).all() and torch.isfinite(o[:, :256].float()).all()
+    finally:
+        torch.use_deterministic_algorithms(before)
