@@ -199,7 +199,8 @@ Tensor bytes(size_t n, const Tensor& like) { return empty_like_dtype(like, {(int
 struct FwdOut {
     Tensor o, rem, nla, ws;
 };
-// want_nla: neg_log_acc as a tensor of its own; otherwise it lies behind the workspace, where nobody reads it
+// want_nla: the caller reads neg_log_acc.  It is a tensor of its own then, and where the workspace is kept for the backward (it would be
+// kept with it); otherwise it lies behind the workspace, one allocation less, and goes with it.
 FwdOut forward(Tensor q, Tensor k, Tensor v, const Tensor& cu, const Opts& opt, bool save, bool want_nla) {
     require_cuda(q);
     c10::cuda::OptionalCUDAGuard guard(q.device());
@@ -211,17 +212,18 @@ FwdOut forward(Tensor q, Tensor k, Tensor v, const Tensor& cu, const Opts& opt, 
     const auto rows = q.sizes().slice(0, q.dim() - 1);
     // no zero-fill: the library writes every row of rem and neg_log_acc
     out.rem = empty_like_dtype(q, rows, q.scalar_type());
-    if (want_nla) out.nla = empty_like_dtype(q, rows, at::kFloat);
+    const bool own_nla = want_nla || save;
+    if (own_nla) out.nla = empty_like_dtype(q, rows, at::kFloat);
     SbParams p = base_params(q, cu, opt, save);
     size_t fb = 0;
     check(sbattn_workspace_bytes(&p, &fb, nullptr), "sbattn_workspace_bytes");
-    out.ws = bytes(fb + (want_nla ? 0 : 4 * (size_t)out.rem.numel()), q);  // fb is a multiple of 4
+    out.ws = bytes(fb + (own_nla ? 0 : 4 * (size_t)out.rem.numel()), q);  // fb is a multiple of 4
     p.q = mat(q, opt.batched);
     p.k = mat(k, opt.batched);
     p.v = mat(v, opt.batched);
     p.o = mat(out.o, opt.batched);
     p.rem = vec(out.rem, opt.batched);
-    if (want_nla) {
+    if (own_nla) {
         p.neg_log_acc = vec(out.nla, opt.batched);
     } else {
         p.neg_log_acc = vec(out.rem, opt.batched);  // same shape, contiguous as well

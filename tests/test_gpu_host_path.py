@@ -56,3 +56,21 @@ def test_rows_behind_the_last_sequence_are_filled_in_deterministic_mode(token_ma
             assert torch.isnan(o[:, 256:]).all() and torch.isfinite(o[:, :256].float()).all()
     finally:
         torch.use_deterministic_algorithms(before)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_memory_kept_for_the_backward(dtype):
+    """o, rem and the forward workspace, nothing else: not neg_log_acc, which no backward reads."""
+    from stickbreaking_attention_b200 import ops, sb_attn_varlen
+    H, T, D = 4, 2000, 64
+    x = torch.randn(H, T, D, device="cuda", dtype=dtype, requires_grad=True)
+    cu = torch.tensor([900, T], device="cuda")
+
+    def requested():
+        return torch.cuda.memory_stats()["requested_bytes.all.current"]
+
+    sb_attn_varlen(x, x, x, cu, 1100, zero_start=False)
+    before = requested()
+    out = sb_attn_varlen(x, x, x, cu, 1100, zero_start=False)
+    workspace, _ = ops.workspace_bytes(False, 2, H, T, 1100)
+    assert requested() - before == workspace + sum(y.numel() * y.element_size() for y in out)
