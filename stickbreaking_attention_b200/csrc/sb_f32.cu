@@ -502,16 +502,22 @@ __device__ __forceinline__ const T* row_of(const MatView& m, const ItemCtx& c, i
     return (const T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + i) * m.st;
 }
 // Blocks in the order of the item table (heaviest first), the heads and the halves of a 128-row tile innermost: the hardware
-// deals blocks out in this order, so the heavy ones of all heads start first.
+// deals blocks out in this order, so the heavy ones of all heads start first.  Items along y and z (together more than an axis takes,
+// and more blocks than x alone would).
 struct BlockIdx {
     int item, h, part;
 };
-__device__ __forceinline__ BlockIdx block_idx(int heads) {
-    const int per = heads * 2, item = (int)blockIdx.x / per, rest = (int)blockIdx.x - item * per;
-    return BlockIdx{item, rest >> 1, rest & 1};
+inline dim3 block_grid(int items, int heads) {
+    const unsigned y = items < 65535 ? items : 65535;
+    return dim3(2u * heads, y, (items + y - 1) / y);
 }
-__device__ __forceinline__ int64_t linear_thread() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
-__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * blockDim.x; }
+__device__ __forceinline__ BlockIdx block_idx() {
+    return BlockIdx{(int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu), (int)(blockIdx.x >> 1), (int)(blockIdx.x & 1)};
+}
+__device__ __forceinline__ int64_t linear_thread() {
+    return (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+}
+__device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x; }
 
 // ------------------------------------------------------------------------------------------ forward
 // Eight warps: four groups of 16 query rows x the two 32-key halves of a tile.  The halves exchange their products once per tile; o
@@ -659,7 +665,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
     }
     const int covered_end = a.own_tables ? own.covered_end : a.hdr->covered_end;
     if (a.zero_tail && covered_end < a.tokens) zero_tail_rows<T>(a, covered_end, linear_thread(), all_threads());
-    const BlockIdx bi = block_idx(a.heads);
+    const BlockIdx bi = block_idx();
     if (bi.item >= (a.own_tables ? own.n_items : a.hdr->n_items)) return;
     const auto item = [&]() { return a.own_tables ? item_ctx(own.items, own.seqs, bi.item) : item_ctx(a, bi.item); };
     const ItemCtx c = item();
@@ -823,7 +829,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
     __shared__ float xs[2][kBM];
     pdl_wait();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
-    const BlockIdx bi = block_idx(a.heads);
+    const BlockIdx bi = block_idx();
     if (bi.item >= a.hdr->n_items) return;
     const ItemCtx c = item_ctx(a, bi.item);
     if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
@@ -897,7 +903,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
     __nv_bfloat16* sP = sQ + 2 * kBuf * kQTile;
     __nv_bfloat16* sS = sP + kWTerms * kPPlane;
     pdl_wait();
-    const BlockIdx bi = block_idx(a.heads);
+    const BlockIdx bi = block_idx();
     const int n_items = a.hdr->n_items;
     if (bi.item >= n_items) return;
     // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
@@ -1086,7 +1092,7 @@ int launch_one(void (*kernel)(KArgs), int threads, int tiles, int more, const Ws
     const int smem = tiles * kTileElems<T, DP> * 2 + more;
     const int e = ensure_kernel_attrs((const void*)kernel, smem, true);
     if (e != 0) return e;
-    return launch_kernel(kernel, dim3((unsigned)L.max_items * a.heads * 2), dim3(threads), smem, st, a);
+    return launch_kernel(kernel, block_grid(L.max_items, a.heads), dim3(threads), smem, st, a);
 }
 template <typename T, int DP, int kQ, int kBuf>
 constexpr int dkdv_smem() {

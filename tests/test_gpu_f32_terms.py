@@ -115,3 +115,16 @@ def test_values_that_terms_do_not_hold(dtype, D, copies, what, value, checked):
         most = np.abs(w[finite]).max()
         err = np.abs(g[finite] - w[finite]).max() / most
         assert err <= (1e-5 if dtype == torch.float32 else 1e-2), (name, err)
+
+
+def test_more_blocks_than_one_grid_axis_takes():
+    """513 heads x 2^21 sequences (all but two of them empty): 2.15e9 blocks, more than 2^31 - 1."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    H, T, D, S = 513, 64, 16, 1 << 21
+    q = torch.randn(H, T, D, device="cuda", generator=torch.Generator("cuda").manual_seed(55))
+    cu = torch.full((S,), T, dtype=torch.int32, device="cuda")
+    cu[:4] = torch.tensor([0, 7, 7, T])
+    with torch.no_grad():
+        want = sb_attn_varlen(q, q, q, torch.tensor([7, T], device="cuda"), T, zero_start=False)
+        got = sb_attn_varlen(q, q, q, cu, T, zero_start=False)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
