@@ -29,37 +29,47 @@ def stale():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def built_for():
+    """What _binding.so depends on besides its sources: the PyTorch and Python it was compiled against (compiled into it)."""
+    import sysconfig
+    import torch
+    return f"sbattn binding for torch {torch.__version__}, python {sysconfig.get_config_var('SOABI')}, " \
+           f"cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}."
+
+
 def binding_stale():
     if not os.path.exists(BINDING):
         return True
+    with open(BINDING, "rb") as f:
+        if built_for().encode() not in f.read():
+            return True
     t = os.path.getmtime(BINDING)
     return any(os.path.getmtime(d) > t for d in [BINDING_SRC] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
 
 
-def start_binding():
-    """The compiler process of _binding.so; it refers to libsbattn.so by name and finds it beside itself ($ORIGIN)."""
+def build_binding():
+    """_binding.so refers to libsbattn.so by name, so that has been built before, and finds it beside itself ($ORIGIN)."""
     import sysconfig
     import torch
     from torch.utils.cpp_extension import CUDA_HOME, include_paths
     libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda = CUDA_HOME or "/usr/local/cuda"
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_binding",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DSBATTN_BUILT_FOR="{built_for()}"']
     cmd += [f"-isystem{d}" for d in include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]]
     cmd += [BINDING_SRC, "-o", BINDING, f"-L{libdir}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
             "-L" + HERE, "-l:libsbattn.so", "-Wl,-rpath,$ORIGIN"]
-    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    pr = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if pr.returncode != 0:
+        sys.stderr.write(pr.stdout)
+        raise RuntimeError("g++ failed")
 
 
 def build(force=False, verbose=False):
     if force or stale():
         build_library(verbose)
     if force or binding_stale():
-        pr = start_binding()
-        out, _ = pr.communicate()
-        if pr.returncode != 0:
-            sys.stderr.write(out)
-            raise RuntimeError("g++ failed")
+        build_binding()
     return LIB
 
 

@@ -382,6 +382,7 @@ std::array<Tensor, 3> bwd(const Tensor& d_o, const Tensor& d_rem, const Tensor& 
 
 PYBIND11_MODULE(_binding, m) {
     m.doc() = "Native host path of stickbreaking_attention_b200 (see csrc/sb_torch.cpp)";
+    m.attr("built_for") = SBATTN_BUILT_FOR;  // read by build.py
     py::register_exception_translator([](std::exception_ptr p) {
         try {
             if (p) std::rethrow_exception(p);

@@ -154,6 +154,13 @@ def test_backward_into_given_tensors_takes_exactly_three():
         ops.varlen_bwd(q, q[..., 0], q, q, q, torch.tensor([16]), 16, ws, 0.1, out=iter([torch.empty_like(q)] * 3))
 
 
+def test_a_binding_of_another_pytorch_is_built_again(lib, monkeypatch):
+    from stickbreaking_attention_b200 import _lib, build
+    assert not build.binding_stale() and _lib.binding().built_for == build.built_for()
+    monkeypatch.setattr(torch, "__version__", "1.0.0")
+    assert build.binding_stale()
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "stickbreaking_attention_b200")
     for dirpath, _, files in os.walk(pkg):
