@@ -1,4 +1,7 @@
 """What the native host path (csrc/sb_torch.cpp) owes its callers besides the numbers: the interpreter lock, memory, refusals."""
+import os
+import subprocess
+import sys
 import threading
 import time
 
@@ -74,3 +77,20 @@ def test_memory_kept_for_the_backward(dtype):
     out = sb_attn_varlen(x, x, x, cu, 1100, zero_start=False)
     workspace, _ = ops.workspace_bytes(False, 2, H, T, 1100)
     assert requested() - before == workspace + sum(y.numel() * y.element_size() for y in out)
+
+
+def test_first_backward_of_a_process_takes_the_tensor_core_kernels():
+    """The first backward runs on an autograd thread that has made no CUDA call yet; its tensor maps are encoded all the same.  (With the
+    tensor-core path asked for, a refused map is an error and not a quiet change of kernels.)"""
+    code = """
+import torch
+from stickbreaking_attention_b200 import sb_attn_varlen, set_path
+set_path("tensor")
+q = torch.randn(2, 300, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+o, rem = sb_attn_varlen(q, q, q, torch.tensor([0, 100, 300], device="cuda"), 200)
+g, = torch.autograd.grad(o, q, torch.ones_like(o))
+assert torch.isfinite(g.float()).all()
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]

@@ -67,3 +67,36 @@ def test_rows_behind_a_sequence_see_no_key(D, dtype, bad):
         results.append((o, rem, dk, dv))
     for name, want, got in zip(("o", "rem", "dk", "dv"), *results):
         assert torch.equal(got, want), name
+
+
+@pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (64, torch.float16), (32, torch.bfloat16)])
+@pytest.mark.parametrize("fused", [False, True])
+def test_blocks_go_from_item_to_item(D, dtype, fused):
+    """720 (sequence, head) items, so that every block works on four or five: tile slots, tensor memory and exchange slots are used again,
+    phases flip, items come from the counter.  Against the oracle; a second backward from the same workspace gives the same bits (the
+    counter starts over)."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    H = 8
+    lengths = [int(n) for n in np.random.default_rng(7).permutation(LENGTHS * 6)]
+    assert len(lengths) * H >= 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    ins = [rounded(x, dtype) for x in synth(H, sum(lengths), D, seed=34)]
+    q, k, v, do, dr = (to_dev(x, dtype) for x in ins)
+    for x in (q, k, v):
+        x.requires_grad_()
+    cu = torch.tensor(np.cumsum(lengths), dtype=torch.int32, device="cuda")
+    it = 1 / math.sqrt(D)
+    o, rem = sb_attn_varlen(q, k, v, cu, max(lengths), zero_start=False, inv_temp=it, fuse_remainder=fused)
+    grads = torch.autograd.grad([o, rem], [q, k, v], [do, dr], retain_graph=True)
+    again = torch.autograd.grad([o, rem], [q, k, v], [do, dr])
+    for x, y in zip(grads, again):
+        assert torch.equal(x, y)
+    qn, kn, vn, don, drn = ins
+    if fused:
+        drn = drn + (don.astype(np.float64) * vn).sum(-1)
+    want = list(oracle_varlen(qn, kn, vn, don, drn, lengths, it, False))
+    if fused:
+        want[0] = want[0] + want[1][..., None] * vn
+        want[4] = want[4] + want[1][..., None] * don
+    got = [x.detach().double().cpu().numpy() for x in (o, rem) + grads]
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_BF16, f"items in turn {D} {dtype} {fused}", out_half_ulp=half_ulp)

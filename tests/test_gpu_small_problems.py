@@ -46,6 +46,27 @@ def test_own_tables_give_the_same_bits(name, dtype, cu_dtype):
         assert torch.equal(a, b[:1])
 
 
+@pytest.mark.parametrize("name", sorted(set(PACKS) - {"too_many"}) + ["most_items"])
+def test_blocks_of_own_tables_take_items_in_turn(name):
+    """As many heads as still build their own table, on the tensor-core kernels up to two (item, head) pairs per SM: blocks then take a
+    second one without a counter.  The same bits as among one head more, where the table kernel and the counter do it.  Packs of up to
+    256 items: the most that the table in shared memory holds."""
+    lengths, pad, D, dtype = PACKS.get(name, [128 * 249 + 5] + [1] * 6), 7, 64, torch.bfloat16
+    T = sum(lengths) + pad
+    items = T // 128 + len(lengths)  # the bound that the rule goes by
+    assert items <= 256
+    H = 296 // items
+    q, k, v, do, dr = (torch.from_numpy(x).to("cuda", dtype) for x in synth(H + 1, T, D, 42))
+    cu = torch.tensor(np.cumsum(lengths), dtype=torch.int32, device="cuda")
+    n_all, want = _run(q, k, v, do, dr, cu, max(lengths))
+    n_own, got = _run(*(x[:H] for x in (q, k, v, do, dr)), cu, max(lengths))
+    assert n_all == 2 and n_own == 1
+    covered = T - pad
+    assert torch.equal(got[0][:, :covered], want[0][:H, :covered])
+    for a, b in zip(got[1:], want[1:]):
+        assert torch.equal(a, b[:H])
+
+
 def test_own_tables_report_bad_sequence_ends():
     import stickbreaking_attention_b200 as sb
     q = torch.randn(1, 256, 64, device="cuda", dtype=torch.bfloat16)
