@@ -49,7 +49,7 @@ extern "C" {
 
 /* kernel family */
 #define SBATTN_PATH_AUTO 0   /* tensor-core kernels when eligible (bf16/f16, head_dim 32, 64 or 128, aligned), else SIMT */
-#define SBATTN_PATH_SIMT 1   /* fp32-arithmetic kernels: any dtype, any head_dim <= 128, any strides     */
+#define SBATTN_PATH_SIMT 1   /* kernels of float32 precision: any dtype, any head_dim <= 128, any strides */
 #define SBATTN_PATH_TENSOR 2 /* tcgen05 kernels or SBATTN_EUNSUPPORTED / SBATTN_EALIGN                   */
 
 /* backward phases */

@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 #include <utility>
@@ -127,14 +128,9 @@ struct KArgs {
 };
 
 // Carries exist at every 32-key boundary.  carry_slot32: (128-row tile qt of a sequence, 32-key quarter kq in [0, 4*qt+3]),
-// the value at the quarter's right edge.  carry_slot: the same for the 64-key half kh in [0, 2*qt+1], i.e. its right quarter
-// (the fp32-arithmetic kernels work in 64-key halves and use these alone).  slot_base and WsLayout::slot_cap count
-// 64-key slots, KArgs::slot_cap 32-key slots.
+// the value at the quarter's right edge.  slot_base and WsLayout::slot_cap count 64-key slots, KArgs::slot_cap 32-key slots.
 __host__ __device__ inline int64_t carry_slot32(int32_t slot_base, int32_t qt, int32_t kq) {
     return 2 * ((int64_t)slot_base + (int64_t)qt * (qt + 1)) + kq;
-}
-__host__ __device__ inline int64_t carry_slot(int32_t slot_base, int32_t qt, int32_t kh) {
-    return carry_slot32(slot_base, qt, 2 * kh + 1);
 }
 
 template <typename T> __device__ inline float to_f32(T x);
@@ -171,6 +167,19 @@ inline int launch_kernel(void (*kernel)(KArgsT...), dim3 grid, dim3 block, size_
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<ArgsT>(args)...);
     count_launch();
     return (int)(e == cudaSuccess ? cudaGetLastError() : e);
+}
+
+// streaming multiprocessors of the current device
+inline int sm_count() {
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = cache[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cache[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 // Dynamic shared memory size (and the carve-out preference) of a kernel, set once per kernel and device instead of on

@@ -26,16 +26,15 @@
 // What bounds them: the latency of the chain load -> scores -> scan -> second product of a tile, with the issue slots of the per-score
 // arithmetic behind it.  (warp-level mma takes 1024 multiply-adds per clock and SM, measured: a 64 x 64 x 64 product costs 256
 // clocks for bf16 inputs, 768 where one side is float32 and 1536 where both are, against 2048 on the FMA pipes at their peak.
-// tcgen05 would take an eighth, but its operands would have to pass through shared memory, three tiles each, where here P and dS
-// stay in registers from the scores to the second product.)  So a block has eight warps where registers allow it, and the keys of
+// tcgen05 would take an eighth; its operands would be the term tiles in shared memory and, for P and dS, three 16-bit planes each in tensor
+// memory or, transposed, in shared memory.  Not built.)  So a block has eight warps where registers allow it, and the keys of
 // a tile are stored in an order that makes the keys of a thread neighbours: the scan along a row is a serial one in registers
 // and one over four lanes.
-// us per kernel, forward / dq / dk,dv:                          scalar FMA kernels   FMA register tiles   now
-//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    642 / 825 / 1028     201 / 297 / 363      143 / 193 / 282
-//   4 x 8 heads x 500 tokens, bf16, head dim 50:                 186 / 235 / 280       76 / 106 / 119       47 /  57 /  60
-//   4 heads, 512 float32 tokens, head dim 64:                     53 /  72 /  82       27 /  37 /  31       25 /  35 /  30
-// Back to back (no gaps between launches), before and after loads a tile ahead, two buffers in dk/dv and the cheaper split:
-// 137 / 171 / 265 -> 135 / 168 / 249; 44 / 46 / 48 -> 39 / 42 / 44; 18 / 22 / 25 -> 18 / 22 / 24.
+// us per kernel, forward / dq / dk,dv, each launched back to back:
+//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    134 / 165 / 246
+//   4 x 8 heads x 500 tokens, bf16, head dim 50:                  35 /  41 /  44
+//   4 heads, 512 float32 tokens, head dim 64:                     18 /  21 /  24
+// (the same on the FMA pipes with register tiles, single launches: 201 / 297 / 363, 76 / 106 / 119, 27 / 37 / 31)
 // 16 heads, 4096 float32 tokens: tensor pipe 49 %, issue slots 47 %, shared memory 56 % busy in dk/dv, 45 / 52 / 37 % in the forward.
 #include <type_traits>
 
@@ -1111,7 +1110,7 @@ int launch_d(bool backward, const WsLayout& L, const KArgs& a, int phases, cudaS
     }
     if (phases == SBATTN_BWD_DQ) return 0;
     if constexpr (DP <= 64) {  // six blocks for each SM: see the kernel
-        if ((int64_t)L.max_items * a.heads * 2 >= 6 * 148) return launch_dkdv<T, DP, 8, 32, 1>(L, a, st);
+        if ((int64_t)L.max_items * a.heads * 2 >= 6 * sm_count()) return launch_dkdv<T, DP, 8, 32, 1>(L, a, st);
     }
     constexpr int kQ = DP > 64 && Terms<T>::n == 3 ? 32 : 64;
     return launch_dkdv<T, DP, 16, kQ, dkdv_smem<T, DP, kQ, 2>() <= kMaxSmem ? 2 : 1>(L, a, st);

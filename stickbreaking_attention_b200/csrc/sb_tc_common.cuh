@@ -209,22 +209,9 @@ __device__ __forceinline__ void tc_teardown(volatile uint32_t* abort_flag, uint3
 }
 
 // persistent blocks for at most `n_work` items: one per SM
-inline int sm_count();
 inline int persistent_grid(int64_t n_work) {
     const int n = sm_count();
     return (int)(n_work < 1 ? 1 : (n_work < n ? n_work : n));
-}
-
-inline int sm_count() {
-    static int cache[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (cache[dev] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cache[dev] = n;
-    }
-    return cache[dev];
 }
 
 inline bool aligned_mat(const SbMat& m) {

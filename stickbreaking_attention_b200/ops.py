@@ -43,7 +43,7 @@ def get_carry_policy():
 
 
 def set_path(name):
-    """'auto' (default), 'simt' (fp32-arithmetic kernels) or 'tensor' (tcgen05 kernels or an error)."""
+    """'auto' (default), 'simt' (the kernels of float32 precision) or 'tensor' (tcgen05 kernels or an error)."""
     global _forced_path
     if name not in _PATHS:
         raise ValueError(name)
@@ -309,7 +309,7 @@ def _backward_traced(do, dr, q, k, v, batched, cu_seqlens, max_seqlens, ws, logi
         do = do.to(q.dtype)
     if dr.dtype != q.dtype:
         dr = dr.to(q.dtype)
-    # no zero-fill: the library writes every row (rows outside all sequences are cleared by a small kernel)
+    # no zero-fill: the library writes every row (the first backward kernel clears the rows outside all sequences)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     if dq.stride(-1) != 1:
         dq, dk, dv = (torch.empty(q.shape, dtype=q.dtype, device=q.device) for _ in range(3))

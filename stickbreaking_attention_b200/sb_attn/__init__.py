@@ -43,7 +43,7 @@ def sb_attn(q, k, v, inv_temp=None, zero_start=True, attend_current=False, fuse_
         inv_temp = 1 / math.sqrt(q.size(-1))
     if not torch.compiler.is_compiling():
         return attend(q, k, v, None, None, inv_temp, attend_current, fuse_remainder)
-    if fuse_remainder and not fusable(q, k, v):  # fp32-arithmetic kernels: the same sum, formed here
+    if fuse_remainder and not fusable(q, k, v):  # traced, on the kernels of float32 precision: the same sum, formed here
         o, rem = sb_attn_(q, k, v, inv_temp, attend_current=attend_current)
         return o + rem[..., None] * v, rem
     return sb_attn_(q, k, v, inv_temp, attend_current=attend_current, fuse_remainder=fuse_remainder)

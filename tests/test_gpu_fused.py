@@ -123,7 +123,7 @@ def test_batched_fused_matches_composed():
 
 
 def test_fused_falls_back_for_float32_inputs():
-    """The fp32-arithmetic kernels have no fused epilogue: the Python layer forms the sum itself, same results."""
+    """The kernels of float32 precision form the sum in their epilogues with the roundings of the expression outside: the same bits."""
     from stickbreaking_attention_b200 import sb_attn_varlen
     lengths = [100, 156]
     H, T, D = 2, 256, 64

@@ -248,7 +248,7 @@ def test_tensor_path_head_dim_32(D, dtype):
 
 def test_broadcast_head_falls_back():
     """k and v expanded over the heads (stride 0, multi-query attention): a tensor map cannot describe them, so the
-    fp32-arithmetic kernels take the call; same results as with materialised copies."""
+    kernels of float32 precision take the call; same results as with materialised copies."""
     from stickbreaking_attention_b200 import sb_attn_varlen
     lengths = [150, 106]
     H, T, D = 4, 256, 64
@@ -266,7 +266,7 @@ def test_broadcast_head_falls_back():
 
 def test_forward_after_fp32_path_feeds_tensor_backward():
     """The forward and the backward choose their kernels independently (by the alignment of their own operands): an
-    output buffer the tensor-core forward cannot write sends the forward to the fp32-arithmetic kernels, whose carries the
+    output buffer the tensor-core forward cannot write sends the forward to the kernels of float32 precision, whose carries the
     tensor-core backward must be able to use."""
     from stickbreaking_attention_b200 import ops
     lengths = [300, 212]
@@ -381,7 +381,7 @@ def test_tokens_outside_all_sequences_get_zero_gradients():
 @pytest.mark.parametrize("seed", [1, 2, 3])
 def test_tensor_path_agrees_with_fp32_arithmetic_path_on_random_packs(seed):
     """Random ragged packs (many short sequences next to long ones, both head dims, both 16-bit types, both
-    diagonal conventions): the tcgen05 kernels against the fp32-arithmetic kernels of the same library on the same
+    diagonal conventions): the tcgen05 kernels against the kernels of float32 precision of the same library on the same
     16-bit inputs.  Sized beyond what the numpy oracle finishes quickly; exercises item transitions of the
     persistent kernels (sequences of 1 ... 3 tiles) and several items per block."""
     from stickbreaking_attention_b200 import get_path, sb_attn_varlen, set_path
