@@ -79,17 +79,29 @@ def test_memory_kept_for_the_backward(dtype):
     assert requested() - before == workspace + sum(y.numel() * y.element_size() for y in out)
 
 
-def test_first_backward_of_a_process_takes_the_tensor_core_kernels():
-    """The first backward runs on an autograd thread that has made no CUDA call yet; its tensor maps are encoded all the same.  (With the
-    tensor-core path asked for, a refused map is an error and not a quiet change of kernels.)"""
+def test_threads_without_a_current_context_take_the_tensor_core_kernels():
+    """A thread whose first CUDA call is the operator's (its memory comes from the allocator's cache) has no current context when its
+    tensor maps are encoded: a fresh Python thread, and the autograd thread of a process's first backward.  With the tensor-core path
+    asked for, a refused map is an error and not a quiet change of kernels."""
     code = """
-import torch
+import threading, torch
 from stickbreaking_attention_b200 import sb_attn_varlen, set_path
 set_path("tensor")
 q = torch.randn(2, 300, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
-o, rem = sb_attn_varlen(q, q, q, torch.tensor([0, 100, 300], device="cuda"), 200)
-g, = torch.autograd.grad(o, q, torch.ones_like(o))
-assert torch.isfinite(g.float()).all()
+cu = torch.tensor([100, 300], device="cuda")
+results = []
+def forward():
+    o, rem = sb_attn_varlen(q, q, q, cu, 200, zero_start=False)
+    results.append(o)
+forward()
+torch.cuda.synchronize()
+x = [torch.empty(1 << 16, device="cuda") for _ in range(8)]  # for the cache
+del x
+thread = threading.Thread(target=forward)
+thread.start()
+thread.join()
+g, = torch.autograd.grad(results[1], q, torch.ones_like(results[1]))
+assert torch.equal(results[0], results[1]) and torch.isfinite(g.float()).all()
 """
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     run = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
