@@ -310,6 +310,7 @@ constexpr int kMapEncodeFailed = -1000;
 int launch_prep(const SbParams& p, const WsLayout& L, cudaStream_t st);
 int launch_drem(const SbParams& p, const KArgs& a, cudaStream_t st);
 int launch_f32_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
+int launch_f32tc(const SbParams& p, bool backward, const WsLayout& L, const KArgs& a, cudaStream_t st);  // head dims up to 64
 int launch_f32_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 bool tensor_path_eligible(const SbParams& p, bool backward, int* why);
 int launch_tensor_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
