@@ -30,6 +30,8 @@
 // terms do not fit shared memory in the backward.)  So a block has eight warps where registers allow it, and the keys of
 // a tile are stored in an order that makes the keys of a thread neighbours: the scan along a row is a serial one in registers
 // and one over four lanes.
+#include <type_traits>
+
 #include "sb_f32.cuh"
 
 namespace sb {
@@ -127,20 +129,25 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
         rq.fetch(a.q, uq, D, c.b, h, c.start + row0, n);
         rg.fetch(a.d_o, ug, D, c.b, h, c.start + row0, n);
     };
-    static_assert(2 * sizeof(float) * kPPlane <= 2 * kWTerms * sizeof(__nv_bfloat16) * kPPlane, "P^T and dS^T as they are in the place of their terms");
-    {
+    const auto sweep = [&](auto direct) {
+        constexpr bool kDirect = decltype(direct)::value;
+        float* const fP = (float*)sP;  // direct: P^T and dS^T as they are, one after the other
+        float* const fS = fP + kPPlane;
+        static_assert(2 * sizeof(float) * kPPlane <= 2 * kWTerms * sizeof(__nv_bfloat16) * kPPlane, "P^T and dS^T in the place of their terms");
 #pragma unroll
         for (int n = 0; n < kDC / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
-        if (kEarly) fetch(key0);
-        if (kBuf == 2) {
+        if (kEarly && !kDirect) fetch(key0);
+        if (kBuf == 2 && !kDirect) {
             rq.template put<kPlain>(sQ, uq);
             rg.template put<kPlain>(sG, ug);
         }
         for (int row0 = key0; row0 < c.len; row0 += kQ) {
             const int rows_valid = min(kQ, c.len - row0);
-            if (kBuf == 1) {
+            if (kDirect) {
+                __syncthreads();
+            } else if (kBuf == 1) {
                 if (!kEarly) fetch(row0);
                 __syncthreads();
                 rq.template put<kPlain>(sQ, uq);
@@ -161,8 +168,14 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
             const bool edge = row0 < key0 + kBN || keys_valid < kBN || rows_valid < kQ;
             if (q0 < kQ) {
                 float s[2][1][4], dp[2][1][4];
-                product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
-                product_nt<kN, DP, 2, 1, kQ>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+                if (kDirect) {
+                    const int key = 32 * kq + 4 * g, q = q0 + 2 * t;
+                    direct_scores_t<T>(s, row_of<T>(a.k, c, h, key0 + key), a.k.st, keys_valid - key, row_of<T>(a.q, c, h, row0 + q), a.q.st, rows_valid - q, D);
+                    direct_scores_t<T>(dp, row_of<T>(a.v, c, h, key0 + key), a.v.st, keys_valid - key, row_of<T>(a.d_o, c, h, row0 + q), a.d_o.st, rows_valid - q, D);
+                } else {
+                    product_nt<kN, DP, 2, 1, kQ>(s, sK + 32 * kq * kPitch<DP>, sQ + q0 * kPitch<DP>, D, lane);
+                    product_nt<kN, DP, 2, 1, kQ>(dp, sV + 32 * kq * kPitch<DP>, sG + q0 * kPitch<DP>, D, lane);
+                }
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
@@ -177,6 +190,11 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
                         const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
+                        if (kDirect) {
+                            *(float2*)(fP + at) = make_float2(s[m][0][2 * hh], s[m][0][2 * hh + 1]);
+                            *(float2*)(fS + at) = make_float2(dp[m][0][2 * hh], dp[m][0][2 * hh + 1]);
+                            continue;
+                        }
                         uint32_t tp[kWTerms], ts[kWTerms];
                         split_pair<kWTerms>(s[m][0][2 * hh], s[m][0][2 * hh + 1], tp);
                         split_pair<kWTerms>(dp[m][0][2 * hh], dp[m][0][2 * hh + 1], ts);
@@ -188,8 +206,25 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
                     }
             }
             __syncthreads();
-            if (kEarly && row0 + kQ < c.len) fetch(row0 + kQ);
-            if (second) {
+            if (kEarly && !kDirect && row0 + kQ < c.len) fetch(row0 + kQ);
+            if (kDirect && second) {
+                const MatView& mx = is_dk ? a.q : a.d_o;
+                const T* x = row_of<T>(mx, c, h, row0) + col0 + 2 * t;
+                const float* pa = (is_dk ? fS : fP) + (16 * kg + g) * kPP;
+#pragma unroll 1
+                for (int q = 0; q < rows_valid; ++q) {
+                    const float p0 = pa[q], p1 = pa[8 * kPP + q];
+#pragma unroll
+                    for (int n = 0; n < kDC / 8; ++n)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float v = col0 + 8 * n + 2 * t + e < D ? to_f32<T>(x[(int64_t)q * mx.st + 8 * n + e]) : 0.f;
+                            acc[n][e] = fmaf(p0, v, acc[n][e]);
+                            acc[n][2 + e] = fmaf(p1, v, acc[n][2 + e]);
+                        }
+                }
+            }
+            if (!kDirect && second) {
                 const __nv_bfloat16* pa = (is_dk ? sS : sP) + (16 * kg + (lane & 15)) * kPP + (lane >> 4) * 8;
                 const __nv_bfloat16* px = (is_dk ? sQ : sG) + ((lane & 7) + ((lane >> 3) & 1) * 8) * kPitch<DP> + (lane >> 4) * 8 + col0;
 #pragma unroll
@@ -220,18 +255,35 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(
                         for (int i = 0; i < 4; ++i) acc[n0 + n][i] += big[n][i] + small[n][i];
                 }
             }
-            if (kBuf == 2 && row0 + kQ < c.len) {
+            if (kBuf == 2 && !kDirect && row0 + kQ < c.len) {
                 sQ = tiles_q + (sQ == tiles_q ? 2 * kQTile : 0);
                 sG = sQ + kQTile;
                 rq.template put<kPlain>(sQ, uq);
                 rg.template put<kPlain>(sG, ug);
             }
         }
-    }
-    const bool again = __syncthreads_or(asks_for_direct(acc, 0) || asks_for_direct(acc, 2));
+        return __syncthreads_or(asks_for_direct(acc, 0) || asks_for_direct(acc, 2));
+    };
+    if (sweep(std::false_type{})) sweep(std::true_type{});
     pdl_launch_dependents();  // not earlier: waiting blocks would take the places of this kernel's own and spread unevenly
-    if (again) dkdv_direct<T, DP, kWarps, kQ>(a, c, bi, (float*)sP);
-    else dkdv_store<T, DP, kWarps>(a, c, bi, acc);
+    if (!second) return;
+    if (a.fused && !is_dk) {  // dv += rem * do
+        const T* d_o = (const T*)a.d_o.ptr + (int64_t)c.b * a.d_o.sb + (int64_t)h * a.d_o.sh + (int64_t)(c.start + key0) * a.d_o.st;
+        const T* rem = (const T*)a.rem.ptr + (int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0) * a.rem.st;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int row = 32 * (kg >> 1) + 4 * g + 2 * (kg & 1) + hh;
+            if (row < keys_valid) add_row<T, kDC>(acc, 2 * hh, to_f32<T>(rem[(int64_t)row * a.rem.st]), d_o + (int64_t)row * a.d_o.st, D, col0, t);
+        }
+    }
+    const MatView m = is_dk ? a.dk : a.dv;
+    const bool pairs = units_ok<T>(m, D, 2);
+    T* base = (T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + key0) * m.st;
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int row = 32 * (kg >> 1) + 4 * g + 2 * (kg & 1) + hh;
+        if (row < keys_valid) store_row<T, kDC>(acc, 2 * hh, is_dk ? a.inv_temp : 1.f, m, pairs, D, col0, base, row, t);
+    }
 }
 
 template <typename T, int DP>

@@ -449,10 +449,10 @@ constexpr int kQuadRight = 0x1c1f, kQuadLeft = 0x1c00, kWarpRight = 0x1f;
 
 // the two warps that share 16 query rows
 __device__ __forceinline__ void pair_sync(int group) { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); }
-// the 256 threads of a 64-row block: a thread block, or (direct form only) one of the two halves of a larger one
+// the 256 threads of a 64-row block: a thread block, or (direct form only) the first ones of a larger one
 template <bool kDirect>
-__device__ __forceinline__ void rows_sync(int half) {
-    if (kDirect) asm volatile("bar.sync %0, 256;" ::"r"(half + 9) : "memory");
+__device__ __forceinline__ void rows_sync() {
+    if (kDirect) asm volatile("bar.sync 9, 256;" ::: "memory");
     else __syncthreads();
 }
 
@@ -502,8 +502,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
     const int h = bi.h, D = a.head_dim;
     const int row0 = c.qt * kTileQ + bi.part * kBM;
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7, g = lane >> 2, t = lane & 3;
-    const int half = threadIdx.x >> 8;  // of the thread block: see rows_sync
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;  // hf 0: the left 32 keys, 1: the right
     const int rows_valid = min(kBM, c.len - row0);
     if (!kDirect) load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
@@ -530,7 +529,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
     for (int kh = last; kh >= 0; --kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
-        rows_sync<kDirect>(half);
+        rows_sync<kDirect>();
         if (kDirect) {
         } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
@@ -539,7 +538,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
             load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
             load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
         }
-        rows_sync<kDirect>(half);
+        rows_sync<kDirect>();
         float s[1][4][4], om[2][8], excl[2];
         if (kDirect) direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key0 + 32 * hf + 8 * t), a.k.st, keys_valid - 32 * hf - 8 * t, D);
         else product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
@@ -564,7 +563,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
             excl[r] = t == 3 ? 1.f : y;
             if (t == 0) xs[hf][wrow + 8 * r] = incl;  // over the whole half
         }
-        pair_sync(4 * half + rg);
+        pair_sync(rg);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float right = xs[1][wrow + 8 * r], left = xs[0][wrow + 8 * r];
@@ -583,14 +582,14 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
         else product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
     }
     float* x = (float*)tiles;
-    rows_sync<kDirect>(half);
+    rows_sync<kDirect>();
     if (hf == 1) {
 #pragma unroll
         for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
-    rows_sync<kDirect>(half);
+    rows_sync<kDirect>();
     bool again = false;
     if (hf == 0) {
 #pragma unroll
@@ -636,8 +635,7 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
     const int h = bi.h, D = a.head_dim;
     const int row0 = c.qt * kTileQ + bi.part * kBM;
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7, g = lane >> 2, t = lane & 3;
-    const int half = threadIdx.x >> 8;  // of the thread block: see rows_sync
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;
     const int rows_valid = min(kBM, c.len - row0);
     if (!kDirect) {
@@ -667,7 +665,7 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
     for (int kh = 0; kh <= last; ++kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
-        rows_sync<kDirect>(half);
+        rows_sync<kDirect>();
         if (kDirect) {
         } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
@@ -680,7 +678,7 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
         float W[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) W[r] = wrow + 8 * r < rows_valid ? cw[slot + 8 * r] : 0.f;
-        rows_sync<kDirect>(half);
+        rows_sync<kDirect>();
         float s[1][4][4], dp[1][4][4], excl[2];
         if (kDirect) {
             const int key = key0 + 32 * hf + 8 * t, keys = keys_valid - 32 * hf - 8 * t;
@@ -723,7 +721,7 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
             excl[r] = t == 0 ? 0.f : z;
             if (t == 3) xs[hf][wrow + 8 * r] = upto;  // over the whole half
         }
-        pair_sync(4 * half + rg);
+        pair_sync(rg);
         // left to right: s <- ds = g - beta * (prefix of g including the key)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -745,14 +743,14 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
         else product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
     }
     float* x = (float*)tiles;
-    rows_sync<kDirect>(half);
+    rows_sync<kDirect>();
     if (hf == 1) {
 #pragma unroll
         for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
-    rows_sync<kDirect>(half);
+    rows_sync<kDirect>();
     bool again = false;
     if (hf == 0) {
 #pragma unroll
@@ -808,117 +806,6 @@ __device__ __forceinline__ void column(float* const (&s)[4], float* const (&dp)[
         *dp[k] = gk[k] - beta[k] * cin;
         cin -= gk[k];
     }
-}
-
-// Which part of a step a warp of a dk/dv block (64 keys) takes.  First half: a 32-key quarter and 8 queries; second half: 16 keys, dk or dv, kDC
-// columns of it.
-template <int DP, int kWarps>
-struct KvWarp {
-    static constexpr int kDC = kWarps == 16 && DP >= 32 ? DP / 2 : DP;
-    int kq, q0, kg, col0;
-    bool is_dk, second;  // second: takes part in the second half (head dim 16: the columns are not split)
-    __device__ __forceinline__ explicit KvWarp(int warp)
-        : kq(warp & 1), q0(8 * (warp >> 1)), kg(warp & 3), col0((warp >> 3) * kDC), is_dk((warp >> 2) & 1), second((warp >> 3) * kDC < DP) {}
-};
-// dk and dv of a block out of its accumulators
-template <typename T, int DP, int kWarps>
-__device__ __forceinline__ void dkdv_store(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, float (&acc)[KvWarp<DP, kWarps>::kDC / 8][4]) {
-    constexpr int kDC = KvWarp<DP, kWarps>::kDC;
-    const int h = bi.h, D = a.head_dim, key0 = c.qt * kTileQ + bi.part * kBN, keys_valid = min(kBN, c.len - key0);
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const KvWarp<DP, kWarps> w(threadIdx.x >> 5);
-    if (!w.second) return;
-    if (a.fused && !w.is_dk) {  // dv += rem * do
-        const T* rem = (const T*)a.rem.ptr + (int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0) * a.rem.st;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int row = 32 * (w.kg >> 1) + 4 * g + 2 * (w.kg & 1) + hh;
-            if (row < keys_valid) add_row<T, kDC>(acc, 2 * hh, to_f32<T>(rem[(int64_t)row * a.rem.st]), row_of<T>(a.d_o, c, h, key0 + row), D, w.col0, t);
-        }
-    }
-    const MatView m = w.is_dk ? a.dk : a.dv;
-    const bool pairs = units_ok<T>(m, D, 2);
-    T* base = (T*)m.ptr + (int64_t)c.b * m.sb + (int64_t)h * m.sh + (int64_t)(c.start + key0) * m.st;
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-        const int row = 32 * (w.kg >> 1) + 4 * g + 2 * (w.kg & 1) + hh;
-        if (row < keys_valid) store_row<T, kDC>(acc, 2 * hh, w.is_dk ? a.inv_temp : 1.f, m, pairs, D, w.col0, base, row, t);
-    }
-}
-// dk and dv of a block by multiply-adds on the values themselves, kQ queries per step; fP: 2 x 64 x (kQ + 8) floats of shared memory.  For 32 kWarps
-// threads (warps 0 ... of the thread block); stores them.
-template <typename T, int DP, int kWarps, int kQ>
-__device__ __noinline__ void dkdv_direct(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, float* fP) {
-    constexpr int kDC = KvWarp<DP, kWarps>::kDC, kPP = kQ + 8;
-    float* const fS = fP + 64 * kPP;
-    float acc[kDC / 8][4];
-    const int h = bi.h, D = a.head_dim, key0 = c.qt * kTileQ + bi.part * kBN, keys_valid = min(kBN, c.len - key0);
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const KvWarp<DP, kWarps> w(threadIdx.x >> 5);
-    const int kq = w.kq, q0 = w.q0, kg = w.kg, col0 = w.col0, quarter = key0 / 32 + kq;
-    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
-    const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
-    const auto sync = [&]() { asm volatile("bar.sync 9, %0;" ::"n"(32 * kWarps) : "memory"); };
-#pragma unroll
-    for (int n = 0; n < kDC / 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
-    for (int row0 = key0; row0 < c.len; row0 += kQ) {
-        const int rows_valid = min(kQ, c.len - row0);
-        const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, quarter) * kTileQ + row0 % kTileQ;
-        float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int q = q0 + 2 * t + e;
-            if (q < rows_valid) {
-                W[e] = cw[slot + q];
-                cr[e] = cc[slot + q];
-                drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
-            }
-        }
-        sync();
-        if (q0 < kQ) {
-            float s[2][1][4], dp[2][1][4];
-            const int key = 32 * kq + 4 * g, qq = q0 + 2 * t;
-            direct_scores_t<T>(s, row_of<T>(a.k, c, h, key0 + key), a.k.st, keys_valid - key, row_of<T>(a.q, c, h, row0 + qq), a.q.st, rows_valid - qq, D);
-            direct_scores_t<T>(dp, row_of<T>(a.v, c, h, key0 + key), a.v.st, keys_valid - key, row_of<T>(a.d_o, c, h, row0 + qq), a.d_o.st, rows_valid - qq, D);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
-                float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
-                const int q = qq + e;
-                const int lim = q < rows_valid ? min(keys_valid, row0 + q + a.attend_current - key0) : 0;
-                column(ps, pd, a.inv_temp, true, lim - 32 * kq - 4 * g, W[e], cr[e], drem[e], g);
-            }
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
-                    *(float2*)(fP + at) = make_float2(s[m][0][2 * hh], s[m][0][2 * hh + 1]);
-                    *(float2*)(fS + at) = make_float2(dp[m][0][2 * hh], dp[m][0][2 * hh + 1]);
-                }
-        }
-        sync();
-        if (w.second) {
-            const MatView& mx = w.is_dk ? a.q : a.d_o;
-            const T* x = row_of<T>(mx, c, h, row0) + col0 + 2 * t;
-            const float* pa = (w.is_dk ? fS : fP) + (16 * kg + g) * kPP;
-#pragma unroll 1
-            for (int q = 0; q < rows_valid; ++q) {
-                const float p0 = pa[q], p1 = pa[8 * kPP + q];
-#pragma unroll
-                for (int n = 0; n < kDC / 8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float v = col0 + 8 * n + 2 * t + e < D ? to_f32<T>(x[(int64_t)q * mx.st + 8 * n + e]) : 0.f;
-                        acc[n][e] = fmaf(p0, v, acc[n][e]);
-                        acc[n][2 + e] = fmaf(p1, v, acc[n][2 + e]);
-                    }
-            }
-        }
-    }
-    dkdv_store<T, DP, kWarps>(a, c, bi, acc);
 }
 
 }  // namespace

@@ -361,6 +361,85 @@ __device__ __noinline__ void direct_dq(const KArgs& a, const ItemCtx c, const Bl
     dq_block<T, 64, true>(a, c, bi, (__nv_bfloat16*)tiles, xs);
 }
 
+// dk and dv of a 64-key tile by the eight row warps, 32 queries per step; stores them.  tiles: 2 x 64 x kPP floats of shared memory.
+template <typename T>
+__device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const BlockIdx bi, float* tiles) {
+    constexpr int DP = 64, kQ = 32, kPP = kQ + 8;
+    float *const fP = tiles, *const fS = tiles + 64 * kPP;  // weights and score gradients, [64 keys][kQ queries]
+    const int h = bi.h, D = a.head_dim, key0 = c.qt * kTileQ + bi.part * kBN, keys_valid = min(kBN, c.len - key0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int kq = warp & 1, q0 = 8 * (warp >> 1);  // first half of a step: 32 keys and 8 queries
+    const int kg = warp & 3;                        // second half: 16 keys of dk or dv
+    const bool is_dk = warp >> 2;
+    const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
+    const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
+    float acc[DP / 8][4] = {};
+    for (int row0 = key0; row0 < c.len; row0 += kQ) {
+        const int rows_valid = min(kQ, c.len - row0);
+        const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, key0 / 32 + kq) * kTileQ + row0 % kTileQ;
+        float W[2] = {0.f, 0.f}, cr[2] = {0.f, 0.f}, drem[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int q = q0 + 2 * t + e;
+            if (q < rows_valid) {
+                W[e] = cw[slot + q];
+                cr[e] = cc[slot + q];
+                drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
+            }
+        }
+        rows_sync<true>();
+        {
+            float s[2][1][4], dp[2][1][4];
+            const int key = 32 * kq + 4 * g, qq = q0 + 2 * t;
+            direct_scores_t<T>(s, row_of<T>(a.k, c, h, key0 + key), a.k.st, keys_valid - key, row_of<T>(a.q, c, h, row0 + qq), a.q.st, rows_valid - qq, D);
+            direct_scores_t<T>(dp, row_of<T>(a.v, c, h, key0 + key), a.v.st, keys_valid - key, row_of<T>(a.d_o, c, h, row0 + qq), a.d_o.st, rows_valid - qq, D);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
+                float* const pd[4] = {&dp[0][0][e], &dp[0][0][2 + e], &dp[1][0][e], &dp[1][0][2 + e]};
+                const int q = qq + e;
+                const int lim = q < rows_valid ? min(keys_valid, row0 + q + a.attend_current - key0) : 0;
+                column(ps, pd, a.inv_temp, true, lim - key, W[e], cr[e], drem[e], g);
+            }
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int at = (32 * kq + 16 * m + 8 * hh + g) * kPP + q0 + 2 * t;
+                    *(float2*)(fP + at) = make_float2(s[m][0][2 * hh], s[m][0][2 * hh + 1]);
+                    *(float2*)(fS + at) = make_float2(dp[m][0][2 * hh], dp[m][0][2 * hh + 1]);
+                }
+        }
+        rows_sync<true>();
+        const MatView& mx = is_dk ? a.q : a.d_o;
+        const T* x = row_of<T>(mx, c, h, row0) + 2 * t;
+        const float* pa = (is_dk ? fS : fP) + (16 * kg + g) * kPP;
+#pragma unroll 1
+        for (int q = 0; q < rows_valid; ++q) {
+            const float p0 = pa[q], p1 = pa[8 * kPP + q];
+#pragma unroll
+            for (int n = 0; n < DP / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float v = 8 * n + 2 * t + e < D ? to_f32<T>(x[(int64_t)q * mx.st + 8 * n + e]) : 0.f;
+                    acc[n][e] = fmaf(p0, v, acc[n][e]);
+                    acc[n][2 + e] = fmaf(p1, v, acc[n][2 + e]);
+                }
+        }
+    }
+    const MatView m = is_dk ? a.dk : a.dv;
+    const bool pairs = units_ok<T>(m, D, 2);
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int row = 32 * (kg >> 1) + 4 * g + 2 * (kg & 1) + hh;
+        if (row >= keys_valid) continue;
+        if (a.fused && !is_dk)  // dv += rem * do
+            add_row<T, DP>(acc, 2 * hh, to_f32<T>(((const T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0 + row) * a.rem.st]),
+                           row_of<T>(a.d_o, c, h, key0 + row), D, 0, t);
+        store_row<T, DP>(acc, 2 * hh, is_dk ? a.inv_temp : 1.f, m, pairs, D, 0, (T*)row_of<T>(m, c, h, key0), row, t);
+    }
+}
+
 // start and end common to the kernels
 struct Shared {
     uint32_t tmem, abort;
@@ -972,7 +1051,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dkdv_kernel(const __gri
             pdl_launch_dependents();
             if (*abort_flag) {
             } else if (again) {
-                dkdv_direct<T, 64, 8, 32>(a, c, BlockIdx{item, h, part}, (float*)smem);
+                direct_dkdv<T>(a, c, BlockIdx{item, h, part}, (float*)smem);
             } else if (key_ok && cols > 0) {
                 if (a.fused && !is_dk)  // dv += rem * do
                     add32<T>(acc, to_f32<T>(((const T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0 + key) * a.rem.st]),

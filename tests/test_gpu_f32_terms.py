@@ -1,5 +1,6 @@
 """The kernels of float32 precision at head dims and lengths where their tiles end: rows read in units of one, two or four
-elements, head dims on both sides of the tile widths, sequence ends on both sides of 32 and 64."""
+elements, head dims on both sides of the tile widths, sequence ends on both sides of 32 and 64; and values that do not divide into terms.
+LONG brings head dims up to 64 to the kernels on tcgen05, shorter packs to those on warp-level matrix instructions."""
 import math
 
 import numpy as np
@@ -10,6 +11,7 @@ from util import TOL_BF16, TOL_F32, assert_close, oracle_varlen, rounded, run_va
 
 pytestmark = pytest.mark.gpu
 
+LONG = [900, 700, 810]  # 803 on average; last tiles of 4, 60 and 42 rows
 
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 33), (torch.float32, 8), (torch.float32, 100), (torch.float32, 128), (torch.bfloat16, 33),
                                      (torch.bfloat16, 17), (torch.float16, 100), (torch.float16, 66)])
@@ -34,14 +36,14 @@ def test_many_blocks_against_oracle(dtype, D):
 
 
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 100), (torch.bfloat16, 50), (torch.float16, 16)])
-@pytest.mark.parametrize("copies", [1, 24])
+@pytest.mark.parametrize("pack", [[1, 31, 33, 63, 65, 100, 129], [1, 31, 33, 63, 65, 100, 129] * 24, [897, 800, 961, 1000]])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
-def test_rows_behind_a_sequence_see_no_key(dtype, D, copies, bad):
+def test_rows_behind_a_sequence_see_no_key(dtype, D, pack, bad):
     """The last key of every sequence is visible to no query: whatever its k holds, o, rem and dv are the same bits, in both forms of
-    dk/dv (`copies`: enough blocks for the one with two blocks per SM), and dk the same but for the rounding of the prefix sums that the
+    dk/dv on warp-level instructions (the second pack: enough blocks for the one with two blocks per SM) and on tcgen05, and dk the same but for the rounding of the prefix sums that the
     dq kernel leaves it (dq itself is NaN, zero times k, and formed again by multiply-adds)."""
     from stickbreaking_attention_b200 import sb_attn_varlen
-    lengths = [1, 31, 33, 63, 65, 100, 129] * copies
+    lengths = pack
     ends = np.cumsum(lengths)
     ins = [to_dev(rounded(x, dtype), dtype) for x in synth(2, ends[-1], D, seed=53)]
     cu = torch.tensor(ends, dtype=torch.int32, device="cuda")
@@ -82,24 +84,25 @@ def _dense(q, k, v, do, dr, lengths, scale):
 
 
 @pytest.mark.parametrize("dtype,D", [(torch.float32, 64), (torch.float32, 100), (torch.float32, 16), (torch.float16, 50), (torch.bfloat16, 50)])
-@pytest.mark.parametrize("copies", [1, 24])
+@pytest.mark.parametrize("pack", [[150, 40], [150, 40] * 24, LONG])
 @pytest.mark.parametrize("what,value,checked", [
     ("k", np.inf, "o rem dk dv"), ("q", -np.inf, "o rem dq dv"), ("v", np.inf, "o rem dv"), ("do", -np.inf, "o rem dv"),  # one element
     ("v", np.finfo(np.float32).max, "o rem dv"), ("k", np.finfo(np.float32).min, "o rem dk dv"),
     ("v", None, "o rem"), ("do", None, "dq dk dv"),  # the whole tensor (and dr with do) times 1e-36
 ])
-def test_values_that_terms_do_not_hold(dtype, D, copies, what, value, checked):
+def test_values_that_terms_do_not_hold(dtype, D, pack, what, value, checked):
     """Infinities, float32's largest values (beyond bf16's) and magnitudes whose later terms would lie below bf16's smallest, against
-    dense float64 sums: finite where those are, the same infinities, no bits lost (`copies`: both forms of dk/dv)."""
+    dense float64 sums: finite where those are, the same infinities, no bits lost (the packs: both forms of dk/dv on
+    warp-level instructions, and the kernels on tcgen05, with a bad element in each half of a 128-row tile and in a last tile of 4 rows)."""
     if dtype == torch.float16 and (value is None or np.isfinite(value)):
         pytest.skip("beyond the range of float16")
-    lengths = [150, 40] * copies
+    lengths = pack
     q, k, v, do, dr = synth(2, sum(lengths), D, seed=54)
     if value is None:
         for x in {"v": [v], "do": [do, dr]}[what]:
             x *= np.float32(1e-36)
     else:
-        for pos in (40, 130):
+        for pos in (40, 130, 200, 898) if pack == LONG else (40, 130):
             {"q": q, "k": k, "v": v, "do": do}[what][0, pos, 3] = value
     ins = [rounded(x, dtype) for x in (q, k, v, do, dr)]
     scale = 1 / math.sqrt(D)
@@ -111,7 +114,7 @@ def test_values_that_terms_do_not_hold(dtype, D, copies, what, value, checked):
         finite, inf = np.isfinite(w), np.isinf(w)
         assert np.isfinite(g[finite]).all(), name
         assert np.array_equal(g[inf], w[inf]), name
-        # relative to the largest result (float32: sums of up to 150 products; 16-bit types: rounding of the result)
+        # relative to the largest result (float32: sums of up to 900 products, whose errors grow with the root of their number; 16-bit types: rounding of the result)
         most = np.abs(w[finite]).max()
         err = np.abs(g[finite] - w[finite]).max() / most
         assert err <= (1e-5 if dtype == torch.float32 else 1e-2), (name, err)
