@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
     if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
     // (16-bit types look their item up again instead of keeping it: the loop has no register to spare for it.  35.8 -> 35.3 us on
     // 4 x 8 heads x 500 tokens, head dim 50; float32 loses by it, 132 -> 137 us on 8 heads, 4096 tokens)
-    if (fwd_block<T, DP, false>(a, c, bi, tiles, xs)) fwd_block<T, DP, true>(a, sizeof(T) == 2 ? item() : c, bi, tiles, xs);
+    if (fwd_block<T, DP, kTerms>(a, c, bi, tiles, xs)) fwd_block<T, DP, kValuesInPlace>(a, sizeof(T) == 2 ? item() : c, bi, tiles, xs);
 }
 
 template <typename T, int DP>
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
     if (bi.item >= a.hdr->n_items) return;
     const ItemCtx c = item_ctx(a, bi.item);
     if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
-    if (dq_block<T, DP, false>(a, c, bi, tiles, xs)) dq_block<T, DP, true>(a, c, bi, tiles, xs);
+    if (dq_block<T, DP, kTerms>(a, c, bi, tiles, xs)) dq_block<T, DP, kValuesInPlace>(a, c, bi, tiles, xs);
 }
 
 // Scores transposed (rows = keys).  kQ queries per step.  First half of a step: two 32-key quarters (each entered with its own carries) x

@@ -380,6 +380,85 @@ __device__ __forceinline__ void direct_px(float (&acc)[1][DP / 8][4], const floa
     }
 }
 
+// The same three on tiles of float32 values in shared memory: rows of DP columns, 16 bytes longer, with zeros behind the valid rows and columns.  Four
+// columns at a time; sums in the same order.
+template <int DP> constexpr int kValuePitch = DP + 4;
+template <int DP> constexpr int kValues = 64 * kValuePitch<DP>;  // of a tile
+template <typename T, int DP, int kRows>
+__device__ __forceinline__ void stage_values(float* dst, const T* src, int64_t st, int D, int rows_valid) {  // 256 threads
+    constexpr int kStep = 256 / DP, kPasses = kRows / kStep, kBatch = kPasses < 8 ? kPasses : 8;  // loads under way at a time: the stores may alias them
+    const int d = threadIdx.x % DP, r0 = threadIdx.x / DP, left = d < D ? rows_valid - r0 : 0;
+    src += r0 * st + d;
+    dst += r0 * kValuePitch<DP> + d;
+#pragma unroll
+    for (int i0 = 0; i0 < kPasses; i0 += kBatch) {
+        float v[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) v[i] = (i0 + i) * kStep < left ? to_f32<T>(src[(i0 + i) * kStep * st]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) dst[(i0 + i) * kStep * kValuePitch<DP>] = v[i];
+    }
+}
+template <int DP, int kR, int kC>
+__device__ __forceinline__ void values_nt(float (&c)[kR][kC], const float* a, int sa, const float* b, int sb, int D) {
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+#pragma unroll
+        for (int j = 0; j < kC; ++j) c[r][j] = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; d += 4) {
+        float4 x[kR], y[kC];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) x[r] = *(const float4*)(a + r * sa + d);
+#pragma unroll
+        for (int j = 0; j < kC; ++j) y[j] = *(const float4*)(b + j * sb + d);
+#pragma unroll
+        for (int r = 0; r < kR; ++r)
+#pragma unroll
+            for (int j = 0; j < kC; ++j) c[r][j] = fmaf(x[r].w, y[j].w, fmaf(x[r].z, y[j].z, fmaf(x[r].y, y[j].y, fmaf(x[r].x, y[j].x, c[r][j]))));
+    }
+}
+template <int DP>
+__device__ __forceinline__ void values_scores(float (&s)[1][4][4], const float* a, const float* b, int D) {
+    float c[2][8];
+    values_nt<DP>(c, a, 8 * kValuePitch<DP>, b, kValuePitch<DP>, D);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[0][j >> 1][2 * r + (j & 1)] = c[r][j];
+}
+template <int DP>
+__device__ __forceinline__ void values_scores_t(float (&s)[2][1][4], const float* a, const float* b, int D) {
+    float c[4][2];
+    values_nt<DP>(c, a, kValuePitch<DP>, b, kValuePitch<DP>, D);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) s[k >> 1][0][2 * (k & 1) + e] = c[k][e];
+}
+template <int DP>
+__device__ __forceinline__ void values_px(float (&acc)[1][DP / 8][4], const float (&p)[1][4][4], const float* x, int keys, int lane) {
+    const int t = lane & 3;
+#pragma unroll 1
+    for (int from = 0; from < 4; ++from) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float p0 = __shfl_sync(0xffffffffu, p[0][j >> 1][j & 1], (lane & ~3) | from);
+            const float p1 = __shfl_sync(0xffffffffu, p[0][j >> 1][2 + (j & 1)], (lane & ~3) | from);
+            const int k = 8 * from + j;
+            if (k >= keys) continue;
+#pragma unroll
+            for (int n = 0; n < DP / 8; ++n) {
+                const float2 v = *(const float2*)(x + k * kValuePitch<DP> + 8 * n + 2 * t);
+                acc[0][n][0] = fmaf(p0, v.x, acc[0][n][0]);
+                acc[0][n][1] = fmaf(p0, v.y, acc[0][n][1]);
+                acc[0][n][2] = fmaf(p1, v.x, acc[0][n][2]);
+                acc[0][n][3] = fmaf(p1, v.y, acc[0][n][3]);
+            }
+        }
+    }
+}
+
 // a row of accumulator blocks (elements i0, i0 + 1 of each) into row `row` of a [.., T, D] tensor
 template <typename T, int DC>
 __device__ __forceinline__ void store_row(const float (&acc)[DC / 8][4], int i0, float scale, const MatView& m, bool pairs, int D, int col0, T* base,
@@ -449,10 +528,13 @@ constexpr int kQuadRight = 0x1c1f, kQuadLeft = 0x1c00, kWarpRight = 0x1f;
 
 // the two warps that share 16 query rows
 __device__ __forceinline__ void pair_sync(int group) { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); }
-// the 256 threads of a 64-row block: a thread block, or (direct form only) the first ones of a larger one
-template <bool kDirect>
+// How a 64-row block forms its sums: of terms; by multiply-adds on the values where they lie; or on copies of them in shared memory (blocks that have an SM
+// to themselves: room for the copies, and too few warps for the latency of the loads)
+enum Sums { kTerms, kValuesInPlace, kStaged };
+// the 256 threads of a 64-row block: a thread block, or (kStaged) the first ones of a larger one
+template <int kSums>
 __device__ __forceinline__ void rows_sync() {
-    if (kDirect) asm volatile("bar.sync 9, 256;" ::: "memory");
+    if (kSums == kStaged) asm volatile("bar.sync 9, 256;" ::: "memory");
     else __syncthreads();
 }
 
@@ -491,12 +573,15 @@ __device__ __forceinline__ int64_t all_threads() { return (int64_t)gridDim.x * g
 // ------------------------------------------------------------------------------------------ forward
 // Eight warps: four groups of 16 query rows x the two 32-key halves of a tile.  The halves exchange their products once per tile; o
 // is summed over the halves at the end.
-// kDirect: the sums by multiply-adds on the values themselves.  Returns whether they have to be formed so (nothing is stored then).
+// kSums: how the sums are formed; returns whether multiply-adds have to (nothing is stored then).
 // xs: product of 1 - beta over a half, per row.
-template <typename T, int DP, bool kDirect>
+template <typename T, int DP, int kSums>
 __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, __nv_bfloat16* tiles, float (*xs)[kBM]) {
     constexpr int kT = 256, kN = Terms<T>::n;
+    constexpr bool kDirect = kSums != kTerms;
     constexpr bool kEarly = sizeof(T) == 2 && !kDirect;  // loads a tile ahead; the 32 words of two float32 tiles cost more registers than they gain
+    float* const vQ = (float*)tiles;  // kStaged
+    float *const vK = vQ + kValues<DP>, *const vV = vK + kValues<DP>;
     __nv_bfloat16* sQ = tiles;
     __nv_bfloat16* sK = sQ + kTileElems<T, DP>;
     __nv_bfloat16* sV = sK + kTileElems<T, DP>;
@@ -505,6 +590,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;  // hf 0: the left 32 keys, 1: the right
     const int rows_valid = min(kBM, c.len - row0);
+    if (kSums == kStaged) stage_values<T, DP, kBM>(vQ, row_of<T>(a.q, c, h, row0), a.q.st, D, rows_valid);
     if (!kDirect) load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
     const int wrow = 16 * rg + g;  // this lane's rows of the block: wrow, wrow + 8
     float W[2] = {1.f, 1.f};
@@ -529,8 +615,11 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
     for (int kh = last; kh >= 0; --kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
-        rows_sync<kDirect>();
-        if (kDirect) {
+        rows_sync<kSums>();
+        if (kSums == kStaged) {
+            stage_values<T, DP, kBN>(vK, row_of<T>(a.k, c, h, key0), a.k.st, D, keys_valid);
+            stage_values<T, DP, kBN>(vV, row_of<T>(a.v, c, h, key0), a.v.st, D, keys_valid);
+        } else if (kDirect) {
         } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
             rv.template put<kKeyColumns>(sV, uv);
@@ -538,9 +627,10 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
             load_tile<kT, T, DP, kKeyColumns>(sK, a.k, D, c.b, h, c.start + key0, keys_valid);
             load_tile<kT, T, DP, kKeyColumns>(sV, a.v, D, c.b, h, c.start + key0, keys_valid);
         }
-        rows_sync<kDirect>();
+        rows_sync<kSums>();
         float s[1][4][4], om[2][8], excl[2];
-        if (kDirect) direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key0 + 32 * hf + 8 * t), a.k.st, keys_valid - 32 * hf - 8 * t, D);
+        if (kSums == kStaged) values_scores<DP>(s, vQ + wrow * kValuePitch<DP>, vK + (32 * hf + 8 * t) * kValuePitch<DP>, D);
+        else if (kDirect) direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key0 + 32 * hf + 8 * t), a.k.st, keys_valid - 32 * hf - 8 * t, D);
         else product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
         const bool edge = kh == last || keys_valid < kBN;  // some pair of the tile is not visible
 #pragma unroll
@@ -578,18 +668,19 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
             W[r] = W[r] * right * left;
         }
         if (kEarly && kh > 0) fetch(kh - 1);
-        if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.v, c, h, key0 + 32 * hf), a.v.st, keys_valid - 32 * hf, D, lane);
+        if (kSums == kStaged) values_px<DP>(o, s, vV + 32 * hf * kValuePitch<DP>, keys_valid - 32 * hf, lane);
+        else if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.v, c, h, key0 + 32 * hf), a.v.st, keys_valid - 32 * hf, D, lane);
         else product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
     }
     float* x = (float*)tiles;
-    rows_sync<kDirect>();
+    rows_sync<kSums>();
     if (hf == 1) {
 #pragma unroll
         for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
-    rows_sync<kDirect>();
+    rows_sync<kSums>();
     bool again = false;
     if (hf == 0) {
 #pragma unroll
@@ -625,10 +716,13 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
 // ------------------------------------------------------------------------------------------ backward: dq
 // Warps as in the forward; W comes from the forward's carries, the halves exchange their sums of g.
 // xs: sum of g over a half, per row.
-template <typename T, int DP, bool kDirect>
+template <typename T, int DP, int kSums>
 __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, __nv_bfloat16* tiles, float (*xs)[kBM]) {
     constexpr int kT = 256, kN = Terms<T>::n;
+    constexpr bool kDirect = kSums != kTerms;
     constexpr bool kEarly = (kN == 1 || (kN == 2 && DP < 64)) && !kDirect;  // loads a tile ahead, where registers allow
+    float* const vQ = (float*)tiles;  // kStaged
+    float *const vG = vQ + kValues<DP>, *const vK = vG + kValues<DP>, *const vV = vK + kValues<DP>;
     __nv_bfloat16* sQ = tiles;
     __nv_bfloat16* sG = sQ + kTileElems<T, DP>;  // dO
     __nv_bfloat16* sK = sG + kTileElems<T, DP>;
@@ -638,6 +732,10 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int rg = warp & 3, hf = warp >> 2;
     const int rows_valid = min(kBM, c.len - row0);
+    if (kSums == kStaged) {
+        stage_values<T, DP, kBM>(vQ, row_of<T>(a.q, c, h, row0), a.q.st, D, rows_valid);
+        stage_values<T, DP, kBM>(vG, row_of<T>(a.d_o, c, h, row0), a.d_o.st, D, rows_valid);
+    }
     if (!kDirect) {
         load_tile<kT, T, DP, kPlain>(sQ, a.q, D, c.b, h, c.start + row0, rows_valid);
         load_tile<kT, T, DP, kPlain>(sG, a.d_o, D, c.b, h, c.start + row0, rows_valid);
@@ -665,8 +763,11 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
     for (int kh = 0; kh <= last; ++kh) {
         const int key0 = kh * kBN;
         const int keys_valid = min(kBN, c.len - key0);
-        rows_sync<kDirect>();
-        if (kDirect) {
+        rows_sync<kSums>();
+        if (kSums == kStaged) {
+            stage_values<T, DP, kBN>(vK, row_of<T>(a.k, c, h, key0), a.k.st, D, keys_valid);
+            stage_values<T, DP, kBN>(vV, row_of<T>(a.v, c, h, key0), a.v.st, D, keys_valid);
+        } else if (kDirect) {
         } else if (kEarly) {
             rk.template put<kKeyColumns>(sK, uk);
             rv.template put<kKeyColumns>(sV, uv);
@@ -678,9 +779,12 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
         float W[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) W[r] = wrow + 8 * r < rows_valid ? cw[slot + 8 * r] : 0.f;
-        rows_sync<kDirect>();
+        rows_sync<kSums>();
         float s[1][4][4], dp[1][4][4], excl[2];
-        if (kDirect) {
+        if (kSums == kStaged) {
+            values_scores<DP>(s, vQ + wrow * kValuePitch<DP>, vK + (32 * hf + 8 * t) * kValuePitch<DP>, D);
+            values_scores<DP>(dp, vG + wrow * kValuePitch<DP>, vV + (32 * hf + 8 * t) * kValuePitch<DP>, D);
+        } else if (kDirect) {
             const int key = key0 + 32 * hf + 8 * t, keys = keys_valid - 32 * hf - 8 * t;
             direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key), a.k.st, keys, D);
             direct_scores<T>(dp, row_of<T>(a.d_o, c, h, row0 + wrow), a.d_o.st, rows_valid - wrow, row_of<T>(a.v, c, h, key), a.v.st, keys, D);
@@ -739,18 +843,19 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
             prefix[r] = prefix[r] + left + right;
         }
         if (kEarly && kh < last) fetch(kh + 1);
-        if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.k, c, h, key0 + 32 * hf), a.k.st, keys_valid - 32 * hf, D, lane);
+        if (kSums == kStaged) values_px<DP>(o, s, vK + 32 * hf * kValuePitch<DP>, keys_valid - 32 * hf, lane);
+        else if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.k, c, h, key0 + 32 * hf), a.k.st, keys_valid - 32 * hf, D, lane);
         else product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
     }
     float* x = (float*)tiles;
-    rows_sync<kDirect>();
+    rows_sync<kSums>();
     if (hf == 1) {
 #pragma unroll
         for (int n = 0; n < DP / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[((rg * (DP / 8) + n) * 4 + e) * 32 + lane] = o[0][n][e];
     }
-    rows_sync<kDirect>();
+    rows_sync<kSums>();
     bool again = false;
     if (hf == 0) {
 #pragma unroll

@@ -52,6 +52,10 @@ __device__ __forceinline__ bool any_row_thread(bool x) {
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 11, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(y) : "r"((int)x), "n"(kRowThreads) : "memory");
     return y != 0;
 }
+// the halves of a tile (bit 0: rows 0-63, bit 1: 64-127) in which a row thread says so
+__device__ __forceinline__ int halves_where(bool x, int row) {
+    return any_row_thread(x) ? (int)any_row_thread(x && row < 64) | (int)any_row_thread(x && row >= 64) << 1 : 0;
+}
 
 // ------------------------------------------------------------------------------------------ operand tiles
 // loads without branches; zeros where ok is 0
@@ -352,20 +356,50 @@ __device__ __forceinline__ bool row_asks_for_direct(const float (&x)[32], int n)
         }
     return nan || (most > 0.f && most < 0x1p-100f);
 }
-template <typename T>
-__device__ __noinline__ void direct_fwd(const KArgs& a, const ItemCtx c, const BlockIdx bi, uint8_t* tiles, float (*xs)[kBM]) {
-    fwd_block<T, 64, true>(a, c, bi, (__nv_bfloat16*)tiles, xs);
+// this block's work item
+__device__ __forceinline__ int block_item() { return (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu); }
+// Sums by multiply-adds, by the eight row warps.  Forward and dq redo the 64-row halves of a tile that ask for it (bits of `halves`), one after the other;
+// they look up again what they need instead of having the kernels keep it (registers).
+template <typename T, int DP>
+__device__ __forceinline__ void direct_fwd_halves(const KArgs& a, const ItemCtx& c, int halves, uint8_t* tiles, float (*xs)[kBM]) {
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part)
+        if (halves >> part & 1) {
+            rows_sync<kStaged>();  // the half before has read its tiles
+            fwd_block<T, DP, kStaged>(a, c, BlockIdx{0, (int)blockIdx.x, part}, (__nv_bfloat16*)tiles, xs);
+        }
 }
 template <typename T>
-__device__ __noinline__ void direct_dq(const KArgs& a, const ItemCtx c, const BlockIdx bi, uint8_t* tiles, float (*xs)[kBM]) {
-    dq_block<T, 64, true>(a, c, bi, (__nv_bfloat16*)tiles, xs);
+__device__ __noinline__ void direct_fwd(const KArgs& a, const OwnTables& own, int halves, uint8_t* tiles, float (*xs)[kBM]) {
+    const ItemCtx c = a.own_tables ? item_ctx(own.items, own.seqs, block_item()) : item_ctx(a, block_item());
+    if (a.head_dim > 32) direct_fwd_halves<T, 64>(a, c, halves, tiles, xs);
+    else if (a.head_dim > 16) direct_fwd_halves<T, 32>(a, c, halves, tiles, xs);
+    else direct_fwd_halves<T, 16>(a, c, halves, tiles, xs);
 }
-
-// dk and dv of a 64-key tile by the eight row warps, 32 queries per step; stores them.  tiles: 2 x 64 x kPP floats of shared memory.
+template <typename T, int DP>
+__device__ __forceinline__ void direct_dq_halves(const KArgs& a, const ItemCtx& c, int halves, uint8_t* tiles, float (*xs)[kBM]) {
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part)
+        if (halves >> part & 1) {
+            rows_sync<kStaged>();  // the half before has read its tiles
+            dq_block<T, DP, kStaged>(a, c, BlockIdx{0, (int)blockIdx.x, part}, (__nv_bfloat16*)tiles, xs);
+        }
+}
 template <typename T>
-__device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const BlockIdx bi, float* tiles) {
-    constexpr int DP = 64, kQ = 32, kPP = kQ + 8;
-    float *const fP = tiles, *const fS = tiles + 64 * kPP;  // weights and score gradients, [64 keys][kQ queries]
+__device__ __noinline__ void direct_dq(const KArgs& a, int halves, uint8_t* tiles, float (*xs)[kBM]) {
+    const ItemCtx c = item_ctx(a, block_item());
+    if (a.head_dim > 32) direct_dq_halves<T, 64>(a, c, halves, tiles, xs);
+    else if (a.head_dim > 16) direct_dq_halves<T, 32>(a, c, halves, tiles, xs);
+    else direct_dq_halves<T, 16>(a, c, halves, tiles, xs);
+}
+// dk and dv of a 64-key tile, 32 queries per step
+constexpr int kDirectQ = 32, kDirectP = kDirectQ + 8;
+template <int DP> constexpr int kDirectKv = 3 * kValues<DP> + 2 * 64 * kDirectP;  // floats
+template <typename T, int DP>
+__device__ __forceinline__ void direct_dkdv_tile(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, float* tiles) {
+    constexpr int kQ = kDirectQ, kPP = kDirectP, kVP = kValuePitch<DP>;
+    float *const vK = tiles, *const vV = vK + kValues<DP>, *const vQ = vV + kValues<DP>, *const vG = vQ + kQ * kVP;
+    float *const fP = vG + kQ * kVP, *const fS = fP + 64 * kPP;  // weights and score gradients, [64 keys][kQ queries]
     const int h = bi.h, D = a.head_dim, key0 = c.qt * kTileQ + bi.part * kBN, keys_valid = min(kBN, c.len - key0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int kq = warp & 1, q0 = 8 * (warp >> 1);  // first half of a step: 32 keys and 8 queries
@@ -374,6 +408,8 @@ __device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const 
     const float* cw = a.carry_w + ((int64_t)h * a.slot_cap) * kTileQ;
     const float* cc = a.carry_c + ((int64_t)h * a.slot_cap) * kTileQ;
     float acc[DP / 8][4] = {};
+    stage_values<T, DP, kBN>(vK, row_of<T>(a.k, c, h, key0), a.k.st, D, keys_valid);
+    stage_values<T, DP, kBN>(vV, row_of<T>(a.v, c, h, key0), a.v.st, D, keys_valid);
     for (int row0 = key0; row0 < c.len; row0 += kQ) {
         const int rows_valid = min(kQ, c.len - row0);
         const int64_t slot = carry_slot32(c.slot_base, row0 / kTileQ, key0 / 32 + kq) * kTileQ + row0 % kTileQ;
@@ -387,12 +423,15 @@ __device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const 
                 drem[e] = to_f32<T>(((const T*)a.d_rem.ptr)[(int64_t)c.b * a.d_rem.sb + (int64_t)h * a.d_rem.sh + (int64_t)(c.start + row0 + q) * a.d_rem.st]);
             }
         }
-        rows_sync<true>();
+        rows_sync<kStaged>();
+        stage_values<T, DP, kQ>(vQ, row_of<T>(a.q, c, h, row0), a.q.st, D, rows_valid);
+        stage_values<T, DP, kQ>(vG, row_of<T>(a.d_o, c, h, row0), a.d_o.st, D, rows_valid);
+        rows_sync<kStaged>();
         {
             float s[2][1][4], dp[2][1][4];
             const int key = 32 * kq + 4 * g, qq = q0 + 2 * t;
-            direct_scores_t<T>(s, row_of<T>(a.k, c, h, key0 + key), a.k.st, keys_valid - key, row_of<T>(a.q, c, h, row0 + qq), a.q.st, rows_valid - qq, D);
-            direct_scores_t<T>(dp, row_of<T>(a.v, c, h, key0 + key), a.v.st, keys_valid - key, row_of<T>(a.d_o, c, h, row0 + qq), a.d_o.st, rows_valid - qq, D);
+            values_scores_t<DP>(s, vK + key * kVP, vQ + qq * kVP, D);
+            values_scores_t<DP>(dp, vV + key * kVP, vG + qq * kVP, D);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
@@ -410,21 +449,20 @@ __device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const 
                     *(float2*)(fS + at) = make_float2(dp[m][0][2 * hh], dp[m][0][2 * hh + 1]);
                 }
         }
-        rows_sync<true>();
-        const MatView& mx = is_dk ? a.q : a.d_o;
-        const T* x = row_of<T>(mx, c, h, row0) + 2 * t;
+        rows_sync<kStaged>();
+        const float* x = (is_dk ? vQ : vG) + 2 * t;
         const float* pa = (is_dk ? fS : fP) + (16 * kg + g) * kPP;
-#pragma unroll 1
+#pragma unroll 2
         for (int q = 0; q < rows_valid; ++q) {
             const float p0 = pa[q], p1 = pa[8 * kPP + q];
 #pragma unroll
-            for (int n = 0; n < DP / 8; ++n)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const float v = 8 * n + 2 * t + e < D ? to_f32<T>(x[(int64_t)q * mx.st + 8 * n + e]) : 0.f;
-                    acc[n][e] = fmaf(p0, v, acc[n][e]);
-                    acc[n][2 + e] = fmaf(p1, v, acc[n][2 + e]);
-                }
+            for (int n = 0; n < DP / 8; ++n) {
+                const float2 v = *(const float2*)(x + q * kVP + 8 * n);
+                acc[n][0] = fmaf(p0, v.x, acc[n][0]);
+                acc[n][1] = fmaf(p0, v.y, acc[n][1]);
+                acc[n][2] = fmaf(p1, v.x, acc[n][2]);
+                acc[n][3] = fmaf(p1, v.y, acc[n][3]);
+            }
         }
     }
     const MatView m = is_dk ? a.dk : a.dv;
@@ -440,6 +478,17 @@ __device__ __noinline__ void direct_dkdv(const KArgs& a, const ItemCtx c, const 
     }
 }
 
+template <typename T>
+__device__ __noinline__ void direct_dkdv(const KArgs& a, uint8_t* tiles) {
+    const ItemCtx c = item_ctx(a, a.hdr->n_items - 1 - block_item());
+    const BlockIdx bi{0, (int)(blockIdx.x >> 1), (int)(blockIdx.x & 1)};
+    if (a.head_dim > 32) direct_dkdv_tile<T, 64>(a, c, bi, (float*)tiles);
+    else if (a.head_dim > 16) direct_dkdv_tile<T, 32>(a, c, bi, (float*)tiles);
+    else direct_dkdv_tile<T, 16>(a, c, bi, (float*)tiles);
+}
+
+// bytes of a kernel's tiles, which share their place with the float32 values of the direct forms
+constexpr int tiles_size(int bytes, int values) { return bytes > 4 * values ? bytes : 4 * values; }
 // start and end common to the kernels
 struct Shared {
     uint32_t tmem, abort;
@@ -463,7 +512,9 @@ struct FwdShared : Shared {
     OwnTables own;
 };
 template <typename T, int kU>
-constexpr int fwd_smem() { return Terms<T>::n * (kQPlane + 2 * kKPlane) + 2 * Staged<T, kU>::kBytes + (int)sizeof(FwdShared) + 1024; }
+constexpr int kFwdTiles = tiles_size(Terms<T>::n * (kQPlane + 2 * kKPlane) + 2 * Staged<T, kU>::kBytes, 3 * kValues<64>);
+template <typename T, int kU>
+constexpr int fwd_smem() { return kFwdTiles<T, kU> + (int)sizeof(FwdShared) + 1024; }
 
 template <typename T, int kU>
 __global__ void __launch_bounds__(kThreads, 1) f32tc_fwd_kernel(const __grid_constant__ KArgs a) {
@@ -475,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_fwd_kernel(const __grid_con
     uint8_t* sV = sK + kN * kKPlane;
     uint8_t* stage_k = sV + kN * kKPlane;
     uint8_t* stage_v = stage_k + Staged<T, kU>::kBytes;
-    FwdShared& sh = *(FwdShared*)(stage_v + Staged<T, kU>::kBytes);
+    FwdShared& sh = *(FwdShared*)(smem + kFwdTiles<T, kU>);
     uint64_t* bars = sh.bars;
     volatile uint32_t* abort_flag = &sh.abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -490,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_fwd_kernel(const __grid_con
     const uint32_t tmem = sh.tmem;
     const int covered_end = a.own_tables ? sh.own.covered_end : a.hdr->covered_end;
     if (a.zero_tail && covered_end < a.tokens) zero_tail_rows<T>(a, covered_end, linear_thread(), all_threads());
-    const int item = (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu), h = blockIdx.x, D = a.head_dim;
+    const int item = block_item(), h = blockIdx.x, D = a.head_dim;
     const bool mine = item < (a.own_tables ? sh.own.n_items : a.hdr->n_items) && !*abort_flag;
     const ItemCtx c = !mine ? ItemCtx{} : a.own_tables ? item_ctx(sh.own.items, sh.own.seqs, item) : item_ctx(a, item);
     const int row0 = c.qt * kTileQ, rows_valid = min(kTileQ, c.len - row0);
@@ -619,12 +670,9 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_fwd_kernel(const __grid_con
             }
             const int cols = D - 32 * q;  // of this thread's 32, that exist
             const bool in_rows = r < rows_valid;
-            const bool again = any_row_thread(in_rows && (row_asks_for_direct(o, cols) || W != W));
+            const int again = halves_where(in_rows && (row_asks_for_direct(o, cols) || W != W), r);
             pdl_launch_dependents();
-            if (*abort_flag) {
-            } else if (again) {
-                for (int part = 0; part * kBM < rows_valid; ++part) direct_fwd<T>(a, c, BlockIdx{item, h, part}, smem, (float(*)[kBM])sh.xs);
-            } else if (in_rows) {
+            if (!*abort_flag && in_rows && !(again >> (r >> 6) & 1)) {
                 // out = o + rem * v: the same bits as the expression outside for float32
                 if (a.fused) add32<T>(o, to_f32<T>(from_f32<T>(W)), row_of<T>(a.v, c, h, row0 + r) + 32 * q, cols);
                 if (cols > 0) store32<T>(o, 1.f, (T*)row_of<T>(a.o, c, h, row0 + r) + 32 * q, unit<T>(a.o, D), cols);
@@ -634,6 +682,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_fwd_kernel(const __grid_con
                     ((float*)a.nla.ptr)[(int64_t)c.b * a.nla.sb + (int64_t)h * a.nla.sh + tok * a.nla.st] = log2f(W);
                 }
             }
+            if (again && !*abort_flag) direct_fwd<T>(a, sh.own, again, smem, (float(*)[kBM])sh.xs);
         }
     }
     tc_teardown(abort_flag, a.status, tmem, 512, 8);
@@ -646,7 +695,9 @@ struct DqShared : Shared {
     float xg[2][2][128];  // [step parity][half][row]: sum of g over 32 keys
 };
 template <typename T, int kU>
-constexpr int dq_smem() { return Terms<T>::n * (2 * kQPlane + 3 * kKPlane) + 2 * Staged<T, kU>::kBytes + (int)sizeof(DqShared) + 1024; }
+constexpr int kDqTiles = tiles_size(Terms<T>::n * (2 * kQPlane + 3 * kKPlane) + 2 * Staged<T, kU>::kBytes, 4 * kValues<64>);
+template <typename T, int kU>
+constexpr int dq_smem() { return kDqTiles<T, kU> + (int)sizeof(DqShared) + 1024; }
 
 template <typename T, int kU>
 __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dq_kernel(const __grid_constant__ KArgs a) {
@@ -659,7 +710,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dq_kernel(const __grid_
     uint8_t* sV = sK + 2 * kN * kKPlane;
     uint8_t* stage_k = sV + kN * kKPlane;
     uint8_t* stage_v = stage_k + Staged<T, kU>::kBytes;
-    DqShared& sh = *(DqShared*)(stage_v + Staged<T, kU>::kBytes);
+    DqShared& sh = *(DqShared*)(smem + kDqTiles<T, kU>);
     uint64_t* bars = sh.bars;
     volatile uint32_t* abort_flag = &sh.abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -672,7 +723,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dq_kernel(const __grid_
     const uint32_t tmem = sh.tmem;
     pdl_wait();
     if (a.zero_tail && a.hdr->covered_end < a.tokens) zero_tail_grads<T>(a, a.hdr->covered_end, linear_thread(), all_threads());
-    const int item = (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu), h = blockIdx.x, D = a.head_dim;
+    const int item = block_item(), h = blockIdx.x, D = a.head_dim;
     const bool mine = item < a.hdr->n_items && !*abort_flag;
     const ItemCtx c = !mine ? ItemCtx{} : item_ctx(a, item);
     const int row0 = c.qt * kTileQ, rows_valid = min(kTileQ, c.len - row0);
@@ -823,14 +874,11 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dq_kernel(const __grid_
             }
             const int cols = D - 32 * q;
             const bool in_rows = r < rows_valid;
-            const bool again = any_row_thread(in_rows && row_asks_for_direct(acc, cols));
+            const int again = halves_where(in_rows && row_asks_for_direct(acc, cols), r);
             pdl_launch_dependents();
-            if (*abort_flag) {
-            } else if (again) {
-                for (int part = 0; part * kBM < rows_valid; ++part) direct_dq<T>(a, c, BlockIdx{item, h, part}, smem, (float(*)[kBM])sh.xg);
-            } else if (in_rows && cols > 0) {
+            if (!*abort_flag && in_rows && cols > 0 && !(again >> (r >> 6) & 1))
                 store32<T>(acc, a.inv_temp, (T*)row_of<T>(a.dq, c, h, row0 + r) + 32 * q, unit<T>(a.dq, D), cols);
-            }
+            if (again && !*abort_flag) direct_dq<T>(a, again, smem, (float(*)[kBM])sh.xg);
         }
     }
     tc_teardown(abort_flag, a.status, tmem, 512, 8);
@@ -843,7 +891,9 @@ struct KvShared : Shared {
 };
 constexpr int kChunk = kWTerms * 2 * 32 * 128;  // 32 queries: terms of [weights | ds], 64 keys each
 template <typename T>
-constexpr int kv_smem() { return Terms<T>::n * (2 * kQPlane + 2 * kKPlane) + 3 * kChunk + (int)sizeof(KvShared) + 1024; }
+constexpr int kKvTiles = tiles_size(Terms<T>::n * (2 * kQPlane + 2 * kKPlane) + 3 * kChunk, kDirectKv<64>);
+template <typename T>
+constexpr int kv_smem() { return kKvTiles<T> + (int)sizeof(KvShared) + 1024; }
 
 template <typename T, int kU>
 __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
@@ -855,7 +905,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dkdv_kernel(const __gri
     uint8_t* sG = sV + kN * kKPlane;  // dO
     uint8_t* sQ = sG + kN * kQPlane;
     uint8_t* sW = sQ + kN * kQPlane;  // three chunks
-    KvShared& sh = *(KvShared*)(sW + 3 * kChunk);
+    KvShared& sh = *(KvShared*)(smem + kKvTiles<T>);
     uint64_t* bars = sh.bars;
     volatile uint32_t* abort_flag = &sh.abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -867,7 +917,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dkdv_kernel(const __gri
     tc_fence_after();
     const uint32_t tmem = sh.tmem;
     pdl_wait();
-    const int item = (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu), h = blockIdx.x >> 1, part = blockIdx.x & 1, D = a.head_dim;
+    const int item = block_item(), h = blockIdx.x >> 1, part = blockIdx.x & 1, D = a.head_dim;
     const int n_items = a.hdr->n_items;
     bool mine = item < n_items && !*abort_flag;
     // the table is heaviest-first for query tiles; key tiles are heaviest at the other end
@@ -1051,7 +1101,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32tc_bwd_dkdv_kernel(const __gri
             pdl_launch_dependents();
             if (*abort_flag) {
             } else if (again) {
-                direct_dkdv<T>(a, c, BlockIdx{item, h, part}, (float*)smem);
+                direct_dkdv<T>(a, smem);
             } else if (key_ok && cols > 0) {
                 if (a.fused && !is_dk)  // dv += rem * do
                     add32<T>(acc, to_f32<T>(((const T*)a.rem.ptr)[(int64_t)c.b * a.rem.sb + (int64_t)h * a.rem.sh + (int64_t)(c.start + key0 + key) * a.rem.st]),
