@@ -344,17 +344,14 @@ __device__ __forceinline__ void add32(float (&x)[32], float f, const T* y, int n
     for (int i = 0; i < 32; ++i)
         if (i < n) x[i] = __fadd_rn(x[i], __fmul_rn(f, to_f32<T>(y[i])));
 }
-// see asks_for_direct
+// whether these results ask for multiply-adds: a NaN, or a magnitude below 2^-100 other than zero.  (asks_for_direct wants all of a thread's to be small.  Here
+// a thread has 32 neighbouring columns, and a tiny column among ordinary ones would lose its later terms.)
 __device__ __forceinline__ bool row_asks_for_direct(const float (&x)[32], int n) {
-    float most = 0.f;
-    bool nan = false;
+    bool asks = false;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-        if (i < n) {
-            nan |= x[i] != x[i];
-            most = fmaxf(most, fabsf(x[i]));
-        }
-    return nan || (most > 0.f && most < 0x1p-100f);
+        if (i < n) asks |= !(fabsf(x[i]) >= 0x1p-100f || x[i] == 0.f);
+    return asks;
 }
 // this block's work item
 __device__ __forceinline__ int block_item() { return (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu); }

@@ -120,6 +120,23 @@ def test_values_that_terms_do_not_hold(dtype, D, pack, what, value, checked):
         assert err <= (1e-5 if dtype == torch.float32 else 1e-2), (name, err)
 
 
+@pytest.mark.parametrize("pack", [[150, 40], LONG])
+@pytest.mark.parametrize("D", [64, 40, 16])
+@pytest.mark.parametrize("what,result", [("v", "o"), ("k", "dq"), ("q", "dk"), ("do", "dv")])
+def test_tiny_columns_among_ordinary_ones(pack, D, what, result):
+    """Two of every eight columns times 1e-36: results below 2^-100 beside ordinary ones lose no bits either."""
+    names = ("o", "rem", "dq", "dk", "dv")
+    ins = dict(zip(("q", "k", "v", "do", "dr"), synth(2, sum(pack), D, seed=56)))
+    tiny = np.arange(D) % 8 < 2
+    ins[what][..., tiny] *= np.float32(1e-36)
+    scale = 1 / math.sqrt(D)
+    got = dict(zip(names, run_varlen(*ins.values(), pack, scale, False, torch.float32)))[result]
+    want = dict(zip(names, _dense(*ins.values(), pack, scale)))[result]
+    for columns in (tiny, ~tiny):
+        g, w = got[..., columns], want[..., columns]
+        assert np.abs(g - w).max() <= 1e-5 * np.abs(w).max()  # as above
+
+
 def test_more_blocks_than_one_grid_axis_takes():
     """513 heads x 2^21 sequences (all but two of them empty): 2.15e9 blocks, more than 2^31 - 1."""
     from stickbreaking_attention_b200 import sb_attn_varlen
