@@ -380,23 +380,25 @@ __device__ __forceinline__ void direct_px(float (&acc)[1][DP / 8][4], const floa
     }
 }
 
-// The same three on tiles of float32 values in shared memory: rows of DP columns, 16 bytes longer, with zeros behind the valid rows and columns.  Four
-// columns at a time; sums in the same order.
-template <int DP> constexpr int kValuePitch = DP + 4;
-template <int DP> constexpr int kValues = 64 * kValuePitch<DP>;  // of a tile
+// The same three on tiles of float32 values in shared memory: rows of DP columns, 16 bytes longer, and 16 more after every eighth, so that rows next to each other
+// and rows eight apart start in different banks; zeros behind the valid rows and columns.  Four columns at a time; sums in the same order.
+template <int DP> constexpr int kValuePitch = DP + 4;               // inside eight rows
+template <int DP> constexpr int kValueEight = 8 * kValuePitch<DP> + 4;
+template <int DP> constexpr int kValues = 8 * kValueEight<DP>;  // of a tile
+template <int DP>
+__device__ __forceinline__ int value_row(int r) { return (r >> 3) * kValueEight<DP> + (r & 7) * kValuePitch<DP>; }
 template <typename T, int DP, int kRows>
 __device__ __forceinline__ void stage_values(float* dst, const T* src, int64_t st, int D, int rows_valid) {  // 256 threads
     constexpr int kStep = 256 / DP, kPasses = kRows / kStep, kBatch = kPasses < 8 ? kPasses : 8;  // loads under way at a time: the stores may alias them
     const int d = threadIdx.x % DP, r0 = threadIdx.x / DP, left = d < D ? rows_valid - r0 : 0;
     src += r0 * st + d;
-    dst += r0 * kValuePitch<DP> + d;
 #pragma unroll
     for (int i0 = 0; i0 < kPasses; i0 += kBatch) {
         float v[kBatch];
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) v[i] = (i0 + i) * kStep < left ? to_f32<T>(src[(i0 + i) * kStep * st]) : 0.f;
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) dst[(i0 + i) * kStep * kValuePitch<DP>] = v[i];
+        for (int i = 0; i < kBatch; ++i) dst[value_row<DP>(r0 + (i0 + i) * kStep) + d] = v[i];
     }
 }
 template <int DP, int kR, int kC>
@@ -421,7 +423,7 @@ __device__ __forceinline__ void values_nt(float (&c)[kR][kC], const float* a, in
 template <int DP>
 __device__ __forceinline__ void values_scores(float (&s)[1][4][4], const float* a, const float* b, int D) {
     float c[2][8];
-    values_nt<DP>(c, a, 8 * kValuePitch<DP>, b, kValuePitch<DP>, D);
+    values_nt<DP>(c, a, kValueEight<DP>, b, kValuePitch<DP>, D);
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
@@ -449,7 +451,7 @@ __device__ __forceinline__ void values_px(float (&acc)[1][DP / 8][4], const floa
             if (k >= keys) continue;
 #pragma unroll
             for (int n = 0; n < DP / 8; ++n) {
-                const float2 v = *(const float2*)(x + k * kValuePitch<DP> + 8 * n + 2 * t);
+                const float2 v = *(const float2*)(x + from * kValueEight<DP> + j * kValuePitch<DP> + 8 * n + 2 * t);
                 acc[0][n][0] = fmaf(p0, v.x, acc[0][n][0]);
                 acc[0][n][1] = fmaf(p0, v.y, acc[0][n][1]);
                 acc[0][n][2] = fmaf(p1, v.x, acc[0][n][2]);
@@ -629,7 +631,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
         }
         rows_sync<kSums>();
         float s[1][4][4], om[2][8], excl[2];
-        if (kSums == kStaged) values_scores<DP>(s, vQ + wrow * kValuePitch<DP>, vK + (32 * hf + 8 * t) * kValuePitch<DP>, D);
+        if (kSums == kStaged) values_scores<DP>(s, vQ + value_row<DP>(wrow), vK + (4 * hf + t) * kValueEight<DP>, D);
         else if (kDirect) direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key0 + 32 * hf + 8 * t), a.k.st, keys_valid - 32 * hf - 8 * t, D);
         else product_nt<kN, DP, 1, 4>(s, sQ + 16 * rg * kPitch<DP>, sK + 32 * hf * kPitch<DP>, D, lane);
         const bool edge = kh == last || keys_valid < kBN;  // some pair of the tile is not visible
@@ -668,7 +670,7 @@ __device__ __forceinline__ bool fwd_block(const KArgs& a, const ItemCtx& c, cons
             W[r] = W[r] * right * left;
         }
         if (kEarly && kh > 0) fetch(kh - 1);
-        if (kSums == kStaged) values_px<DP>(o, s, vV + 32 * hf * kValuePitch<DP>, keys_valid - 32 * hf, lane);
+        if (kSums == kStaged) values_px<DP>(o, s, vV + 4 * hf * kValueEight<DP>, keys_valid - 32 * hf, lane);
         else if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.v, c, h, key0 + 32 * hf), a.v.st, keys_valid - 32 * hf, D, lane);
         else product_px<kN, DP, DP, 1, 4>(o, s, sV + 32 * hf * kPitch<DP>, lane);
     }
@@ -782,8 +784,8 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
         rows_sync<kSums>();
         float s[1][4][4], dp[1][4][4], excl[2];
         if (kSums == kStaged) {
-            values_scores<DP>(s, vQ + wrow * kValuePitch<DP>, vK + (32 * hf + 8 * t) * kValuePitch<DP>, D);
-            values_scores<DP>(dp, vG + wrow * kValuePitch<DP>, vV + (32 * hf + 8 * t) * kValuePitch<DP>, D);
+            values_scores<DP>(s, vQ + value_row<DP>(wrow), vK + (4 * hf + t) * kValueEight<DP>, D);
+            values_scores<DP>(dp, vG + value_row<DP>(wrow), vV + (4 * hf + t) * kValueEight<DP>, D);
         } else if (kDirect) {
             const int key = key0 + 32 * hf + 8 * t, keys = keys_valid - 32 * hf - 8 * t;
             direct_scores<T>(s, row_of<T>(a.q, c, h, row0 + wrow), a.q.st, rows_valid - wrow, row_of<T>(a.k, c, h, key), a.k.st, keys, D);
@@ -843,7 +845,7 @@ __device__ __forceinline__ bool dq_block(const KArgs& a, const ItemCtx& c, const
             prefix[r] = prefix[r] + left + right;
         }
         if (kEarly && kh < last) fetch(kh + 1);
-        if (kSums == kStaged) values_px<DP>(o, s, vK + 32 * hf * kValuePitch<DP>, keys_valid - 32 * hf, lane);
+        if (kSums == kStaged) values_px<DP>(o, s, vK + 4 * hf * kValueEight<DP>, keys_valid - 32 * hf, lane);
         else if (kDirect) direct_px<T, DP>(o, s, row_of<T>(a.k, c, h, key0 + 32 * hf), a.k.st, keys_valid - 32 * hf, D, lane);
         else product_px<kN, DP, DP, 1, 4>(o, s, sK + 32 * hf * kPitch<DP>, lane);
     }

@@ -394,9 +394,9 @@ constexpr int kDirectQ = 32, kDirectP = kDirectQ + 8;
 template <int DP> constexpr int kDirectKv = 3 * kValues<DP> + 2 * 64 * kDirectP;  // floats
 template <typename T, int DP>
 __device__ __forceinline__ void direct_dkdv_tile(const KArgs& a, const ItemCtx& c, const BlockIdx& bi, float* tiles) {
-    constexpr int kQ = kDirectQ, kPP = kDirectP, kVP = kValuePitch<DP>;
-    float *const vK = tiles, *const vV = vK + kValues<DP>, *const vQ = vV + kValues<DP>, *const vG = vQ + kQ * kVP;
-    float *const fP = vG + kQ * kVP, *const fS = fP + 64 * kPP;  // weights and score gradients, [64 keys][kQ queries]
+    constexpr int kQ = kDirectQ, kPP = kDirectP;
+    float *const vK = tiles, *const vV = vK + kValues<DP>, *const vQ = vV + kValues<DP>, *const vG = vQ + kValues<DP> / 2;
+    float *const fP = vG + kValues<DP> / 2, *const fS = fP + 64 * kPP;  // weights and score gradients, [64 keys][kQ queries]
     const int h = bi.h, D = a.head_dim, key0 = c.qt * kTileQ + bi.part * kBN, keys_valid = min(kBN, c.len - key0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int kq = warp & 1, q0 = 8 * (warp >> 1);  // first half of a step: 32 keys and 8 queries
@@ -427,8 +427,8 @@ __device__ __forceinline__ void direct_dkdv_tile(const KArgs& a, const ItemCtx& 
         {
             float s[2][1][4], dp[2][1][4];
             const int key = 32 * kq + 4 * g, qq = q0 + 2 * t;
-            values_scores_t<DP>(s, vK + key * kVP, vQ + qq * kVP, D);
-            values_scores_t<DP>(dp, vV + key * kVP, vG + qq * kVP, D);
+            values_scores_t<DP>(s, vK + value_row<DP>(key), vQ + value_row<DP>(qq), D);
+            values_scores_t<DP>(dp, vV + value_row<DP>(key), vG + value_row<DP>(qq), D);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 float* const ps[4] = {&s[0][0][e], &s[0][0][2 + e], &s[1][0][e], &s[1][0][2 + e]};
@@ -454,7 +454,7 @@ __device__ __forceinline__ void direct_dkdv_tile(const KArgs& a, const ItemCtx& 
             const float p0 = pa[q], p1 = pa[8 * kPP + q];
 #pragma unroll
             for (int n = 0; n < DP / 8; ++n) {
-                const float2 v = *(const float2*)(x + q * kVP + 8 * n);
+                const float2 v = *(const float2*)(x + value_row<DP>(q) + 8 * n);
                 acc[n][0] = fmaf(p0, v.x, acc[n][0]);
                 acc[n][1] = fmaf(p0, v.y, acc[n][1]);
                 acc[n][2] = fmaf(p1, v.x, acc[n][2]);
