@@ -332,26 +332,44 @@ int launch_any(const SbParams& p, bool backward, const WsLayout& L, const KArgs&
 
 }  // namespace
 
-// Whether the kernels on tcgen05 (sb_f32_tc.cu) take a call.  They work on 128-row tiles, a block per SM, with ~6 us around an item's steps, and on
-// 64 columns whatever the head dim: long sequences.  The host knows the average length only.  Forward + backward in us, warp-level / tcgen05 kernels, 8 heads,
+// Whether the kernels on tcgen05 (sb_f32_tc.cu) take a pass.  They work on 128-row tiles, a block per SM, with ~6 us around an item's steps, and on
+// 64 columns whatever the head dim: long sequences, by the average length of a pack.  Forward + backward in us, warp-level / tcgen05 kernels, 8 heads,
 // 8192 tokens in sequences of equal length:
-//   head dim 64, float32:  64 each 176 / 236, 128: 229 / 201, 129: 338 / 340, 256: 324 / 239, 1024: 901 / 457, 4096: 3267 / 1348
-//   head dim 50, bf16:     192: 180 / 195, 256: 217 / 183, 1024: 577 / 353, 4096: 2049 / 1047
+//   head dim 64, float32:  64 each 176 / 236, 128: 229 / 201, 256: 324 / 239, 1024: 901 / 457, 4096: 3267 / 1348
+//   head dim 50, bf16:     192: 180 / 195, 1024: 577 / 353, 4096: 2049 / 1047
 //   head dim 32, float32:  192: 178 / 213, 256: 216 / 200, 384: 274 / 226, 4096: 2137 / 1275;   18, bf16: 256: 164 / 162, 384: 208 / 183, 4096: 1555 / 1007
 //   head dim 16, float32:  384: 215 / 220, 512: 264 / 256, 1024: 457 / 396, 4096: 1644 / 1240;  16, bf16: 512: 209 / 205, 1024: 358 / 312, 4096: 1261 / 958
+// The bounds lie above some lengths at which they gain up to 10 % with 8 heads: with 32 they do not.
+// Lengths around the average (log-normal, sigma 0.7) only help, since the long ones have the work: at the bounds forward 1.0 ... 1.6 and backward 1.0 ... 1.7 times
+// as fast.  Sequences of nearly equal length, though, all have a last tile as full as the average says, and where that is half a tile or less the rows
+// that do not exist cost more than the units gain up to a second bound, as soon as three blocks and more follow one another on an SM (up to there the shorter
+// chain of a block counts: 1.05 ... 1.5 times as fast).  Warp-level / tcgen05 there, forward and backward apart, 8 heads (32 alike):
+//   float32, head dim 64: 140 each forward 90.8 / 83.5, backward 227 / 244;  161: 80.3 / 73.3, 228 / 221
+//   bf16, 50:             257: 78.8 / 73.8, 190 / 193;   300: 70.7 / 64.5, 183 / 173;   f16: 257: 103 / 82, 248 / 229
+//   float32, 32:          320: 65.7 / 63.8, 171 / 183;   385: 91.9 / 80.0, 240 / 238
+//   bf16, 18:             320: 52.9 / 55.4, 128 / 145;   385: 72.6 / 69.0, 175 / 189;   448: 64.0 / 58.3, 163 / 161;  f16, 20: 320: 59.7 / 59.2, 152 / 165
+//   float32, 16:          800: 102 / 90, 276 / 284;      bf16, 16: 1.05 and 0.97 times as fast at 800, 1.10 and 1.01 at 897
+//   bf16, 9:              800: 86.4 / 91.5, 235 / 253;   897: 99.7 / 101, 277 / 287;    1000: 99.6 / 95.3, 287 / 268
 // (A form of theirs in which one block per SM draws item after item, and with 32 columns, gains up to 25 % below these lines, where it still loses, and
-// costs 9-20 % above them: a drawn item is bound to its block, a block that the hardware starts is not.)  Not by the number of heads: a head's bits do not
-// depend on how many there are.
-bool on_tcgen05(const SbParams& p) {
-    if (p.head_dim > 64) return false;
-    const int64_t seqs = p.batch > 0 ? 1 : (p.num_seqs > 0 ? p.num_seqs : 1);
-    return p.tokens / seqs >= (p.head_dim > 32 ? (p.dtype == SBATTN_F32 ? 128 : 224) : p.head_dim > 16 ? 320 : 768);
+// costs 9-20 % above them: a drawn item is bound to its block, a block that the hardware starts is not.)
+// A sequence's last bits depend on its pack thereby: the average, the longest length and, between the two bounds, the number of blocks choose the family.
+bool on_tcgen05(const SbParams& p, const WsLayout& L, bool backward) {
+    const int D = p.head_dim;
+    if (D > 64) return false;
+    const int64_t seqs = p.batch > 0 ? 1 : (p.num_seqs > 0 ? p.num_seqs : 1), average = p.tokens / seqs;
+    const bool f32 = p.dtype == SBATTN_F32, bf16 = p.dtype == SBATTN_BF16;
+    const int bound = D > 32 ? (f32 ? 128 : 224) : D > 16 ? 320 : 768;
+    if (average < bound) return false;
+    const int64_t longest = p.batch == 0 && p.max_seqlen > 0 && p.max_seqlen < p.tokens ? p.max_seqlen : p.tokens;
+    if (longest > average + average / 16 || (average - 1) % kTileQ >= kTileQ / 2 || (int64_t)L.max_items * p.heads <= 3 * sm_count()) return true;
+    if (backward) return average >= (D > 32 ? (f32 ? 160 : bf16 ? 288 : 224) : D > 16 ? 416 : 961);
+    return !bf16 || D > 32 || average >= (D > 16 ? 384 : D % 2 == 0 ? 768 : 961);  // odd head dims: rows are loaded one element at a time
 }
 int launch_f32_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    return on_tcgen05(p) ? launch_f32tc(p, false, L, a, st) : launch_any(p, false, L, a, st);
+    return on_tcgen05(p, L, false) ? launch_f32tc(p, false, L, a, st) : launch_any(p, false, L, a, st);
 }
 int launch_f32_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {
-    return on_tcgen05(p) ? launch_f32tc(p, true, L, a, st) : launch_any(p, true, L, a, st);
+    return on_tcgen05(p, L, true) ? launch_f32tc(p, true, L, a, st) : launch_any(p, true, L, a, st);
 }
 
 }  // namespace sb

@@ -62,6 +62,30 @@ def test_rows_behind_a_sequence_see_no_key(dtype, D, pack, bad):
     assert (got - want).abs().max() <= (1e-6 if dtype == torch.float32 else 1e-2) * want.abs().max()
 
 
+@pytest.mark.parametrize("dtype,D,length", [(torch.float32, 64, 140), (torch.bfloat16, 50, 257), (torch.float16, 20, 320), (torch.bfloat16, 18, 385),
+                                            (torch.float32, 16, 800), (torch.bfloat16, 9, 800), (torch.bfloat16, 18, 320)])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_forward_and_backward_choose_apart(dtype, D, length, ragged):
+    """Equal lengths whose last tile is at most half full, more than three blocks per SM: the forward mostly runs on tcgen05 there and the backward on
+    warp-level instructions, over the carries that the forward has left.  `ragged`: the same average, on tcgen05 both ways."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    lengths = [length - 100, length + 101, length] if ragged else [length] * 3
+    ins = [rounded(x, dtype) for x in synth(2, sum(lengths), D, seed=57)]
+    heads = 148 * 3 // 6 + 1  # the two heads again and again: three sequences of at least two tiles each
+    tensors = [to_dev(x, dtype).repeat(heads, *[1] * (x.ndim - 1)) for x in ins]
+    for x in tensors[:3]:
+        x.requires_grad_()
+    q, k, v, do, dr = tensors
+    o, rem = sb_attn_varlen(q, k, v, torch.tensor(np.cumsum(lengths), device="cuda"), max(lengths), zero_start=False)
+    results = (o, rem, *torch.autograd.grad([o, rem], [q, k, v], [do, dr]))
+    for x in results:
+        assert torch.equal(x[:-2], x[2:])  # whatever block a head's tile got
+    got = [x[:2].detach().double().cpu().numpy() for x in results]
+    want = oracle_varlen(*ins, lengths, 1 / math.sqrt(D), False)
+    half_ulp = {torch.float32: 0.0, torch.float16: 2**-11, torch.bfloat16: 2**-8}[dtype]  # of the results, which are float32 sums rounded once
+    assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_F32, f"{dtype} {D}", out_half_ulp=half_ulp)
+
+
 def _dense(q, k, v, do, dr, lengths, scale):
     """The operator and its gradients as dense float64 sums in which an infinity is an infinity (products of 1 - beta, no logarithms)."""
     out = [np.zeros(x, np.float64) for x in (q.shape, dr.shape, q.shape, q.shape, q.shape)]
