@@ -12,6 +12,7 @@ from oracle import sb_oracle as orc
 
 pytestmark = pytest.mark.gpu
 NAMES = ("out", "rem", "dq", "dk", "dv")
+SHORT = [300, 1, 129, 31, 77, 128, 65, 33]
 
 
 def _close(got, want):
@@ -153,11 +154,11 @@ def test_launchers_refuse_the_fused_sum_at_float32_precision_in_the_forward(D, d
 
 
 @pytest.mark.parametrize("D,dtype", [(64, torch.float32), (128, torch.float32), (50, torch.bfloat16), (33, torch.float16), (16, torch.bfloat16)])
-@pytest.mark.parametrize("heads", [2, 30])
-def test_varlen_fused_at_float32_precision_against_oracle(D, dtype, heads):
-    """out = o + rem * v in the epilogues of the kernels of float32 precision (both forms of dk/dv), tokens behind the last sequence."""
+@pytest.mark.parametrize("heads,lengths", [(2, SHORT), (30, SHORT), (2, [700, 1, 1729, 1057, 865, 833])])
+def test_varlen_fused_at_float32_precision_against_oracle(D, dtype, heads, lengths):
+    """out = o + rem * v in the epilogues of the kernels of float32 precision (both forms of dk/dv on warp-level instructions; head dims up to 64
+    on tcgen05 with the last pack, 864 on average), tokens behind the last sequence."""
     from stickbreaking_attention_b200 import check_status, sb_attn_varlen
-    lengths = [300, 1, 129, 31, 77, 128, 65, 33]
     T, used = sum(lengths) + 20, sum(lengths)
     ins = [rounded(x, dtype) for x in synth(heads, T, D, 22)]
     q, k, v, dout, dr = (torch.from_numpy(x).to("cuda", dtype) for x in ins)
