@@ -12,7 +12,7 @@ BINDING = os.path.join(HERE, "_binding.so")
 BINDING_SRC = os.path.join(HERE, "csrc", "sb_torch.cpp")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
          "-Xcompiler", "-fPIC"]
-# files that must keep IEEE division/exp (the kernels of float32 precision): compiled without --use_fast_math
+# the kernels of float32 precision, which need accurate exponentials, denormal numbers and IEEE division: compiled without --use_fast_math
 PRECISE = {"sb_f32.cu", "sb_f32_tc.cu", "sb_weights.cu"}
 
 

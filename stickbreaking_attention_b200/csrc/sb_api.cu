@@ -90,8 +90,9 @@ KArgs make_args(const SbParams& p, const WsLayout& L) {
 
 // Small forwards do without the prep kernel: its launch costs the host ~2.5 us and the GPU ~3 us of the 13 us of a forward over a
 // few short sequences.  Tensor-core kernel: up to two items per SM, which then are dealt out in turn: beyond that the blocks
-// should draw their items from the counter, which only a kernel before this one can set to zero.  Float32-precision kernel: each of its
-// blocks (two per item) pays for a table, so up to two blocks per SM; up to head dim 64 these are resident at once, above it one is.
+// should draw their items from the counter, which only a kernel before this one can set to zero.  Float32-precision kernels: each of their
+// blocks (one per item on tcgen05, else two) pays for a table, so up to one item per SM; two blocks are resident at once on warp-level instructions up to head
+// dim 64, else one.
 bool forward_builds_tables(const SbParams& p, const WsLayout& L, bool tensor) {
     return L.n_seqs <= kOwnSeqs && L.max_items <= kOwnItems && (int64_t)L.max_items * p.heads <= (tensor ? 2 : 1) * sm_count();
 }

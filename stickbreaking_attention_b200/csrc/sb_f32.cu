@@ -17,10 +17,11 @@
 // One term holds a bf16 value, two an f16 value, three the 24 bits of a float32, all exactly.  Every product runs on the tensor
 // cores as the sum of the term products x_i y_j with i + j <= 2, accumulated in float32: what is left out, x1 y2 and smaller, is
 // below 2^-25 |x y|, a unit of which float32 multiply-adds lose as much in every addition.  Weights and score gradients are
-// float32 values and enter the second products in three terms.  exp and division are the accurate ones (no fast math here).
+// float32 values and enter the second products in three terms.  exp and division are the accurate ones (no fast math here; on tcgen05 the division
+// is an approximate reciprocal and a step of Newton's method, as accurate).
 // Three kinds of values do not divide into terms: infinities, magnitudes that round to one in bf16, and magnitudes below 2^-100, whose
 // later terms lie below the smallest bf16.  They show in a block's results, which then are NaN (terms of the first two kinds are), or
-// all tiny: such a block starts over and forms its sums with ordinary multiply-adds on the values as they are ("direct" below;
+// tiny: such a block starts over and forms its sums with ordinary multiply-adds on the values as they are ("direct" below;
 // several times slower; a block that does not need it looks at its results and no more).
 //
 // This file: head dims above 64 and short sequences, on warp-level mma.  (The others: sb_f32_tc.cu; the rule is on_tcgen05 below.)
@@ -55,8 +56,8 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_fwd_kernel(const __g
     const auto item = [&]() { return a.own_tables ? item_ctx(own.items, own.seqs, bi.item) : item_ctx(a, bi.item); };
     const ItemCtx c = item();
     if (c.qt * kTileQ + bi.part * kBM >= c.len) return;
-    // (16-bit types look their item up again instead of keeping it: the loop has no register to spare for it.  35.8 -> 35.3 us on
-    // 4 x 8 heads x 500 tokens, head dim 50; float32 loses by it, 132 -> 137 us on 8 heads, 4096 tokens)
+    // (16-bit types look their item up again instead of keeping it: the loop has no register to spare for it.  At sizes that take tcgen05 by now,
+    // 35.8 -> 35.3 us on 4 x 8 heads x 500 tokens, head dim 50; float32 loses by it, 132 -> 137 us on 8 heads, 4096 tokens, head dim 64)
     if (fwd_block<T, DP, kTerms>(a, c, bi, tiles, xs)) fwd_block<T, DP, kValuesInPlace>(a, sizeof(T) == 2 ? item() : c, bi, tiles, xs);
 }
 
@@ -76,16 +77,16 @@ __global__ void __launch_bounds__(256, DP > 64 ? 1 : 2) f32_bwd_dq_kernel(const 
 // Scores transposed (rows = keys).  kQ queries per step.  First half of a step: two 32-key quarters (each entered with its own carries) x
 // groups of 8 queries; P^T and dS^T go to shared memory as three terms each.  Second half: four groups of 16 keys x {dv, dk} (x the
 // two halves of the columns with sixteen warps, so that a thread accumulates 16 or 32 values only).  (With P^T and dS^T kept in
-// registers four warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 311 and 107 us in the first two
-// lines at the top.)
+// registers four warps had to hold dk and dv of 32 keys each, 255 registers and 8 warps per SM: 311 against 255 us on 8 heads, 4096 float32 tokens, head dim
+// 64, which take tcgen05 by now.)
 // Sixteen warps, one block per SM, take steps of 64 queries, or of 32 where the tiles would not fit otherwise (float32 at D > 64; eight
 // of the warps then sit out the first half; forward + backward of 8 heads, 4096 tokens, head dim 128: 1638 us with four warps
 // that kept P^T and dS^T in registers, 1163 us so).  kBuf = 2, where shared memory has the room: the next step's Q and dO travel during
-// the second half and go to the other buffer at its end, which takes a barrier and the whole load out of the step (265 -> 255 us in the first
-// line at the top).
-// Eight warps, two blocks per SM, take steps of 32: one block's loads and scans run under the other's products.  Better from six blocks
-// for each SM on, where a short last wave does not matter (64 sequences of 64 float32 tokens, 8 heads: 42 -> 36 us), worse below (4 x 8 heads x
-// 500 tokens: 45 -> 61 us).
+// the second half and go to the other buffer at its end, which takes a barrier and the whole load out of the step (265 -> 255 us on the same).
+// Eight warps, two blocks per SM, take steps of 32: one block's loads and scans run under the other's products.  From six blocks for each SM on, where a short
+// last wave does not matter (64 sequences of 64 float32 tokens, 8 heads: 42 -> 36 us).  Over the lengths that these kernels still take (head dims up to 64,
+// all types, 40 to 700 tokens each) the whole backward takes 1.01 to 1.24 times as long with sixteen warps at 6 to 24 blocks per SM, 1.01 to 1.2 at 3 to 5, and 0.78
+// to 0.94 at one and less; in between it goes by the last wave, 0.81 to 1.1: a line at three blocks would serve these lengths better.
 template <typename T, int DP, int kWarps, int kQ, int kBuf>
 __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) f32_bwd_dkdv_kernel(const __grid_constant__ KArgs a) {
     constexpr int kT = 32 * kWarps, kN = Terms<T>::n;

@@ -300,8 +300,8 @@ __device__ __forceinline__ void product_px(float (&acc)[kMB][DC / 8][4], const f
 }
 
 // ------------------------------------------------------------------------------------------ the same products on the values themselves
-// whether a thread's results (elements i0, i0 + 1 of its accumulator blocks: one row) ask for them: a NaN, or nothing but magnitudes
-// below 2^-100
+// whether a thread's results (elements i0, i0 + 1 of its accumulator blocks: one row, every fourth pair of columns) ask for them: a NaN, or nothing but
+// magnitudes below 2^-100
 template <int kN>
 __device__ __forceinline__ bool asks_for_direct(const float (&acc)[kN][4], int i0) {
     float most = 0.f;

@@ -18,13 +18,15 @@
 // Errors against float64 sums (norm of the difference / norm, 8 heads, 4096 float32 tokens; warp-level kernels before): o 8.3e-8 (9.2e-8), dq 1.4e-7
 // (1.5e-7), dk 1.6e-7 (3.6e-7), dv 1.0e-7 (1.0e-7).
 //
-// us per kernel, forward / dq / dk,dv (the warp-level kernels of sb_f32.cu before):
-//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    57 /  78 / 133 (134 / 173 / 250)
-//   4 x 8 heads x 500 tokens, bf16, head dim 50:                  23 /  27 /  34 (36 / 43 / 45)
-//   4 heads, 512 float32 tokens, head dim 64:                     13 /  17 /  18 (18 / 23 / 25)
-// What bounds them: the row threads.  A forward step takes 4 150 cycles (float32): 1 650 the weights (25 instructions per score, issue-bound), 800 splitting
-// the next K and V, 570 splitting the weights, 450 sums of accumulators, the rest barriers (~100 each); the tensor pipe is busy for half of it.  dk/dv:
-// 10 700 for twice the scores, 4 900 of them in the tensor pipe, which it partly waits for: shared memory has no room for a second tile of Q and dO.
+// us per kernel, forward / dq / dk,dv (the warp-level kernels of sb_f32.cu before); medians of 30 training calls in a row under the PyTorch profiler, where
+// kernels do not overlap as they do in a stream (the first call takes 264 us without it):
+//   8 heads, 4096 float32 tokens in 4 sequences, head dim 64:    56 /  75 / 134 (134 / 174 / 251)
+//   4 x 8 heads x 500 tokens, bf16, head dim 50:                  24 /  27 /  35 (36 / 43 / 45)
+//   4 heads, 512 float32 tokens, head dim 64:                     13 /  17 /  18 (19 / 23 / 25)
+// What bounds them: the row threads.  A forward step takes 4 150 cycles (float32; clock readings around its parts): 1 650 the weights (25 instructions per
+// score, issue-bound), 800 splitting the next K and V, 570 splitting the weights, 450 sums of accumulators, the rest barriers (~100 each).  dk/dv: 10 700 for
+// twice the scores, 4 900 of them until its products are there: shared memory has no room for a second tile of Q and dO.  Counters (16 heads): tensor
+// pipe 27 / 31 / 32 % active, issue slots 46 / 42 / 33 %.
 // Sixteen row warps of 16 keys per thread were slower (56 / 90 / 168 us): 96 registers a thread, and with 28 KB left for the L1 every spilled
 // value came back from the L2 at ~300 cycles.  Hence eight warps, and the registers that the last group of warps does without.
 #include "sb_f32.cuh"
@@ -356,7 +358,10 @@ __device__ __forceinline__ bool row_asks_for_direct(const float (&x)[32], int n)
 // this block's work item
 __device__ __forceinline__ int block_item() { return (int)min(blockIdx.z * gridDim.y + blockIdx.y, 0x7fffffffu); }
 // Sums by multiply-adds, by the eight row warps.  Forward and dq redo the 64-row halves of a tile that ask for it (bits of `halves`), one after the other;
-// they look up again what they need instead of having the kernels keep it (registers).
+// they look up again what they need instead of having the kernels keep it (registers).  One block has the SM, and was bound by the latency of its loads where it read
+// the values in place, so they are copied to shared memory as float32 first.  8 heads, four sequences of 1024 tokens, one infinite value per head, forward /
+// backward in us, in place, here and on the warp-level kernels: float32 head dim 64 863 / 2388, 342 / 741, 514 / 2163; bf16 50 977 / 2583, 343 / 697, 513 / 2150;
+// float32 16 456 / 1010, 184 / 385, 235 / 672.  (Four loads of the values in place at a time: 772 / 2508 and 1242 / 2956 for the first two.)
 template <typename T, int DP>
 __device__ __forceinline__ void direct_fwd_halves(const KArgs& a, const ItemCtx& c, int halves, uint8_t* tiles, float (*xs)[kBM]) {
 #pragma unroll 1
