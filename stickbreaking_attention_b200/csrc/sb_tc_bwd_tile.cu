@@ -7,8 +7,10 @@
 //
 // What bounds it is memory: seven matrices per item, 224 KB at head dim 128, ~10 000 cycles of the SM's share of the DRAM
 // bandwidth.  Contractions, arithmetic, read-out and stores of an item take about as long one after the other, so the loads,
-// S and dP of the next item run while the results of this one are stored.  32 heads, 512 sequences of 128 tokens, bf16, head dim 128: forward
-// + backward 1.76 ms with the two kernels, 1.30 ms with this one.
+// S and dP of the next item run while the results of this one are stored, and the row threads read the next item and its scalars (the carry, drem)
+// before these stores: at the item's start the ring, the table entry and two dependent loads cost 3 000 of 14 000 cycles.  32 heads, 512 sequences of
+// 128 tokens, bf16, head dim 128: 757 -> 640 us for this kernel (575 at the copy bandwidth), forward + backward 1.32 -> 1.23 ms (1.76 ms with the two
+// kernels).  Two slots for q and k, with p in the place of v, were slower (757 -> 833, with the early reads 640 -> 665).
 //
 // One persistent block of 576 threads per SM: warps 0-15 row warps (a thread owns one query row and 32 keys, warps 0-3 the
 // rightmost quarter ... 12-15 the leftmost), warp 16 TMA producer, warp 17 issues tcgen05.mma.
@@ -278,25 +280,35 @@ tc_bwd_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         bool ok = true;
         SchedConsumer sched;
         int w;
-        KvWork wk;
-        for (uint32_t i = 0; ok && (w = sched.next(ring, &bars[T_WORK_FULL0], &bars[T_WORK_EMPTY0], abort_flag, wk, lane == 0, true)) >= 0; ++i) {
+        KvWork wk, nx;
+        // The next item and its scalars are fetched as soon as this one's gradients of the scores are out, and arrive under its stores
+        float W = 0.f;
+        uint32_t drem_raw = 0u;  // drem stays as it was loaded until it is used: a conversion behind the load would wait for it
+        const auto next_item = [&]() {
+            w = sched.next(ring, &bars[T_WORK_FULL0], &bars[T_WORK_EMPTY0], abort_flag, nx, false, true);
+            W = 0.f;
+            drem_raw = 0u;
+            if (w < 0 || r >= nx.len) return;
+            // a quarter behind the end of the sequence (in a half whose carry slots do not exist) has no visible key: any W does
+            if (64 * hf < nx.len) W = __ldg(a.carry_w + ((int64_t)nx.h * a.slot_cap + carry_slot32(nx.slot_base, 0, kq)) * kTileQ + r);
+            const int64_t tok = nx.start + r;
+            if (kFused) {  // drem + do . v
+                drem_raw = __ldg((const uint32_t*)a.drem_eff + (int64_t)nx.h * a.drem_rows + (int64_t)nx.b * a.tokens + tok);
+            } else {
+                const char* dp = a.d_rem.ptr + 2 * ((int64_t)nx.b * a.d_rem.sb + (int64_t)nx.h * a.d_rem.sh + tok * a.d_rem.st);
+                drem_raw = __ldg((const unsigned short*)dp);
+            }
+        };
+        next_item();
+        for (uint32_t i = 0; ok && w >= 0; ++i) {
             const uint32_t ph = i & 1;
+            wk = nx;
+            if (lane == 0) sched.release(&bars[T_WORK_EMPTY0]);
             const bool row_ok = r < wk.len;
             const int64_t tok = wk.start + r;
             // Columns < lim of the quarter are visible.  None to a row behind the end of the sequence: its zero query against an infinite
             // or NaN key would make a NaN of every weight to the left, and dk, dv contract over such rows up to a multiple of 16.
             const int lim = row_ok ? r + a.attend_current - 32 * kq : 0;
-            float W = 0.f, drem = 0.f;
-            if (row_ok) {
-                // a quarter behind the end of the sequence (in a half whose carry slots do not exist) has no visible key: any W does
-                if (64 * hf < wk.len) W = __ldg(a.carry_w + ((int64_t)wk.h * a.slot_cap + carry_slot32(wk.slot_base, 0, kq)) * kTileQ + r);
-                if (kFused) {  // drem + do . v
-                    drem = __ldg(a.drem_eff + (int64_t)wk.h * a.drem_rows + (int64_t)wk.b * a.tokens + tok);
-                } else {
-                    const char* dp = a.d_rem.ptr + 2 * ((int64_t)wk.b * a.d_rem.sb + (int64_t)wk.h * a.d_rem.sh + tok * a.d_rem.st);
-                    drem = kF16 ? __half2float(*(const __half*)dp) : __bfloat162float(*(const __nv_bfloat16*)dp);
-                }
-            }
             ok = mbar_wait(&bars[T_SDP_READY], ph, abort_flag);
             if (!ok) break;
             tc_fence_after();
@@ -305,6 +317,7 @@ tc_bwd_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tmem_ld32(lane_base + kColDP + 32 * kq, gv);
             tmem_wait_ld(om, gv);
             tc_fence_before();
+            const float drem = kFused ? __uint_as_float(drem_raw) : kF16 ? __half2float(__ushort_as_half((unsigned short)drem_raw)) : __uint_as_float(drem_raw << 16);
             float tot;
             {
                 uint32_t pp[16];
@@ -335,6 +348,7 @@ tc_bwd_tile_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 fence_async_smem();
                 mbar_arrive(&bars[T_DS_READY]);
             }
+            next_item();
             // dq: a quarter of the columns per thread; then the next item's dP may overwrite it
             ok = mbar_wait(&bars[T_DQ_READY], ph, abort_flag);
             if (!ok) break;

@@ -178,6 +178,9 @@ struct SchedConsumer {
         if (arrive) sm100::mbar_arrive(&empty[sl]);
         return w;
     }
+    // For a consumer that reads the next item ahead of time (arrive = false): the slot is released when the item begins, so that items
+    // are not drawn earlier than they would be otherwise.
+    __device__ __forceinline__ void release(uint64_t* empty) { sm100::mbar_arrive(&empty[(i - 1) & (kRing - 1)]); }
 };
 // the last block to finish re-arms the counters for the next launch
 __device__ __forceinline__ void sched_finish(int32_t* counter) {
