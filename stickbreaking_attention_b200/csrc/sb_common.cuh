@@ -314,6 +314,7 @@ int launch_f32tc(const SbParams& p, bool backward, const WsLayout& L, const KArg
 int launch_f32_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 bool tensor_path_eligible(const SbParams& p, bool backward, int* why);
 int launch_tensor_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
+int launch_tensor_fwd_pair(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);  // two query tiles at a time
 int launch_tensor_bwd_tile(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);  // sequences of one tile
 int launch_tensor_bwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st);
 int launch_weights(const SbParams& p, float* w, int64_t stride_b, int64_t stride_h, int64_t stride_m, cudaStream_t st);

@@ -83,13 +83,19 @@ __device__ __forceinline__ void store_row32_pairs(char* dst, const uint32_t (&v)
     if (ok_other) put(oth, s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]);
 }
 
-// 32 16-bit values at `src` as fp32
+// 32 16-bit values at `src`, and as fp32: apart, so that the loads can travel across a wait
+struct Row32 {
+    uint4 u[4];
+    __device__ __forceinline__ void load(const char* src) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) u[h] = __ldg((const uint4*)(src + 16 * h));
+    }
+};
 template <bool kF16>
-__device__ __forceinline__ void load_row32(const char* src, float (&x)[32]) {
+__device__ __forceinline__ void unpack_row32(const Row32& row, float (&x)[32]) {
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-        const uint4 u = __ldg((const uint4*)(src + 16 * h));
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        const uint32_t w[4] = {row.u[h].x, row.u[h].y, row.u[h].z, row.u[h].w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (kF16) {
@@ -102,6 +108,12 @@ __device__ __forceinline__ void load_row32(const char* src, float (&x)[32]) {
             }
         }
     }
+}
+template <bool kF16>
+__device__ __forceinline__ void load_row32(const char* src, float (&x)[32]) {
+    Row32 row;
+    row.load(src);
+    unpack_row32<kF16>(row, x);
 }
 template <bool kF16>
 __device__ __forceinline__ float round16(float x) {
