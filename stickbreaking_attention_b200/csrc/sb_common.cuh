@@ -115,7 +115,6 @@ struct KArgs {
     float* drem_eff;        // [heads][drem_rows]: drem + do . v (fused-remainder backward)
     int64_t drem_rows;      // batch * tokens (tokens for the packed layout)
     int32_t head_group;     // heads whose work is interleaved (sized so that their K and V stay in L2)
-    int32_t defer_fwd, defer_dq, defer_dkdv;  // tensor-core kernels: store an item's result one step into the next item
     int32_t zero_tail;      // packed layout: clear the result rows of tokens behind the last sequence
     // forward of small problems: every block builds the work-item table itself (no prep kernel)
     int32_t own_tables, cu_width, n_seqs, batch, max_len, n_max, max_items;

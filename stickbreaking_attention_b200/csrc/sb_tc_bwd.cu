@@ -102,7 +102,7 @@ __device__ __forceinline__ void dq_half_finish(const uint32_t (&beta)[32], const
 
 // kFused (both backward kernels): d_o is the gradient of out = o + rem * v; separate instantiations, the plain ones stay
 // as they are
-template <int D, bool kF16, bool kFused, bool kDefer>
+template <int D, bool kF16, bool kFused>
 __global__ void __launch_bounds__(kDqThreads, 1)
 tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do, const KArgs a) {
@@ -129,7 +129,7 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             uint32_t cnt = 1;
             if (i >= A_X_G0) cnt = 32;
             if (i == A_LOADED || i == A_DQ_FREE) cnt = 512;
-            if (i >= A_DS_READY0 && i <= A_DS_READY3) cnt = kDefer ? 512 : 128;  // one per 32-key quarter of the step, or one for all
+            if (i >= A_DS_READY0 && i <= A_DS_READY3) cnt = 128;  // one per 32-key quarter of the step
             if (i == A_WORK_EMPTY0 || i == A_WORK_EMPTY1) cnt = 514;  // MMA warp (one lane), V producer, 512 row threads
             mbar_init(&bars[i], cnt);
         }
@@ -287,15 +287,12 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     // dQ += dS K in slices of 32 keys, each as soon as that quarter's dS exists: the quarters finish one after
                     // the other (leftmost first, the prefix chain), and the tensor pipe does not wait for the last one before
                     // it starts on the first
-                    // (-1.5 % on long sequences; on packs of short ones, the kDefer instantiation, one barrier for all four
-                    // quarters is 3 % faster)
+                    // (-1.5 % on long sequences)
 #pragma unroll
                     for (int qq = 0; qq < 4; ++qq) {
-                        if (!kDefer || qq == 0) {
-                            ok = mbar_wait(&bars[A_DS_READY0 + qq], g & 1, abort_flag);
-                            if (!ok) break;
-                            tc_fence_after();
-                        }
+                        ok = mbar_wait(&bars[A_DS_READY0 + qq], g & 1, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
                         if (qq == 0) mma_ts_dyn(leader, tmem + kColDQ, a_ds, dkmn, 0, idesc_dq, j > 0);
                         else mma_ts<true>(leader, tmem + kColDQ, a_ds + qq * 32, dkmn, 2 * qq * 2048, idesc_dq);
                         mma_ts<true>(leader, tmem + kColDQ, a_ds + qq * 32 + 8, dkmn, (2 * qq + 1) * 2048, idesc_dq);
@@ -319,10 +316,6 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const float scale = a.inv_temp * kLog2e;
         uint32_t G = 0, items = 0;
         bool ok = true;
-        // With kDefer (chosen by the host for packs of short sequences) a finished item's dq leaves tensor memory one step
-        // late: its last contraction needs a while to complete, and waiting for it at the end of the item idles the row
-        // threads.  They work on the first step of the next item instead (whose S and dP exist already) and store dq then;
-        // the first dQ contraction of the next item waits for A_DQ_FREE, i.e. for this store.
         struct PendingItem {
             int b, h;
             int64_t tok;
@@ -342,10 +335,7 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 uint32_t v[32];
                 tmem_ld32(lane_base + kColDQ + d0, v);
                 tmem_wait_ld(v);
-                const bool wr = pend.row_ok && (D == 128 || a.head_dim > d0);  // D == 64 serves head dim 32 too
-                // two rows per lane pair where items are long (-0.8 %); on packs of short sequences it costs 3-5 %
-                if (!kDefer) store_row32_pairs<kF16>(orow, v, a.inv_temp, (int64_t)a.dq.st * 2, wr, lane);
-                else if (wr) store_row32<kF16>(orow, v, a.inv_temp);
+                store_row32_pairs<kF16>(orow, v, a.inv_temp, (int64_t)a.dq.st * 2, pend.row_ok && (D == 128 || a.head_dim > d0), lane);  // D == 64 serves head dim 32 too
             }
             tc_fence_before();
             mbar_arrive(&bars[A_DQ_FREE]);
@@ -356,6 +346,8 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         // The next item and its drem are fetched before an item's result is stored, and arrive meanwhile (drem stays as it was loaded until it is
         // used: a conversion behind the load would wait for it).  32 heads, 16 384 tokens in 7 sequences: 701 -> 679 us.  The ring's slot is given
         // back when the item begins, as before: given back here, items are drawn earlier and blocks with five items each end further apart (+4 %).
+        // (An instantiation that stored dq a step into the next item, for packs of short sequences, loses 4 ... 20 % of the kernel against this at
+        // average lengths of 58 ... 1024 tokens; one of dk/dv 0 ... 13 %.)
         uint32_t drem_raw = 0u;
         const auto next_item = [&]() {
             w = sched.next(ring, &bars[A_WORK_FULL0], &bars[A_WORK_EMPTY0], abort_flag, wk, false);
@@ -372,7 +364,7 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         };
         while (ok) {
             next_item();
-            if (!kDefer && have_pend) store_item();
+            if (have_pend) store_item();
             if (!ok || w < 0) break;
             sched.release(&bars[A_WORK_EMPTY0]);
             const int n = wk.qt + 1;
@@ -438,11 +430,7 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 tmem_st16(lane_base + kColS + 128 * buf + 32 * kq, packed);
                 tmem_wait_st();
                 tc_fence_before();
-                mbar_arrive(&bars[A_DS_READY0 + (kDefer ? 0 : kq)]);
-                if (kDefer && j == 0 && have_pend) {
-                    store_item();
-                    if (!ok) break;
-                }
+                mbar_arrive(&bars[A_DS_READY0 + kq]);
             }
             if (!ok) break;
             pend = PendingItem{wk.b, wk.h, tok, items, row_ok};
@@ -450,7 +438,6 @@ tc_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             G += n;
             ++items;
         }
-        if (kDefer && ok && have_pend) store_item();  // the block's last item
     }
     tc_teardown(abort_flag, a.status, tmem, kCols, 17);
     sched_finish(a.sched + 2);
@@ -513,7 +500,7 @@ __device__ __forceinline__ void kv_chunk(const uint32_t (&s)[32], const uint32_t
     }
 }
 
-template <int D, bool kF16, bool kFused, bool kDefer>
+template <int D, bool kF16, bool kFused>
 __global__ void __launch_bounds__(kKvThreads, 1)
 tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -774,16 +761,12 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         auto store_dkdv = [&](const KvWork& e, uint32_t item) {
             ok = mbar_wait(&bars[B_DKV_READY], item & 1, abort_flag);
             if (!ok) return;
-            if (kDefer) kv_store_rows_inl<D, kF16, kFused>(a, sub == 1, e, r, lane_base + (sub == 0 ? kColDK : kColDV), hf * (D / 64), kv_chunks);
-            else kv_store_rows<D, kF16, kFused>(a, sub == 1, e, r, lane_base + (sub == 0 ? kColDK : kColDV), hf * (D / 64), kv_chunks);
+            kv_store_rows<D, kF16, kFused>(a, sub == 1, e, r, lane_base + (sub == 0 ? kColDK : kColDV), hf * (D / 64), kv_chunks);
             mbar_arrive(&bars[B_DKV_FREE]);
         };
         SchedConsumer sched;
         int w;
         KvWork wk;
-        // With kDefer (packs of sequences of one tile) dk, dv of a finished item are stored inside the first step of the next
-        // item: the item's last contractions need a while to complete; the first contraction of the next item waits for
-        // B_DKV_FREE, i.e. for this store
         KvWork pend{};
         uint32_t pend_item = 0;
         bool have_pend = false;
@@ -823,7 +806,7 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         };
         while (ok) {
             next_item();
-            if (!kDefer && have_pend) store_dkdv(pend, pend_item);
+            if (have_pend) store_dkdv(pend, pend_item);
             if (!ok || w < 0) break;
             sched.release(&bars[B_WORK_EMPTY0]);
             const int n = wk.n_qt - wk.kt;
@@ -850,13 +833,6 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     else kv_chunk<false, kF16>(s1, d1, scale, 32 * sub, lim, drem, c, W, pp, ps);
                 }
                 if (j + 1 < n) load_scalars(wk, i + 1);
-                if (kDefer && j == 0 && have_pend) {
-                    // Here and not after this step's p / ds have been written: the second row half can write only when the
-                    // first half's contraction of this step is complete, and that contraction waits for B_DKV_FREE.
-                    store_dkdv(pend, pend_item);
-                    have_pend = false;
-                    if (!ok) break;
-                }
                 // The 64-row p / ds buffers are two regions of 32 rows, each used by one warp quartet of either row half
                 // in turn (rows 0-31 and 64-95 the first region, 32-63 and 96-127 the second).  A region is free once the
                 // contractions of its previous use are complete: the other half's, of the previous step for half 0 and of
@@ -883,7 +859,6 @@ tc_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             G += n;
             ++items;
         }
-        if (kDefer && ok && have_pend) store_dkdv(pend, pend_item);  // the block's last item
     }
     tc_teardown(abort_flag, a.status, tmem, kCols, 17);
     sched_finish(a.sched + 4);
@@ -908,12 +883,11 @@ int launch_bwd_kernels(const SbParams& p, const KArgs& a, cudaStream_t st, const
             const int e = launch_drem(p, a, st);
             if (e != 0) return e;
         }
-        const int e = a.defer_dq ? launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, true>) : launch_dq(tc_bwd_dq_kernel<D, kF16, kFused, false>);
+        const int e = launch_dq(tc_bwd_dq_kernel<D, kF16, kFused>);
         if (e != 0) return e;
     }
     if (p.bwd_phases != SBATTN_BWD_DQ) {
-        const int e = a.defer_dkdv ? launch_dkdv(tc_bwd_dkdv_kernel<D, kF16, kFused, true>)
-                                   : launch_dkdv(tc_bwd_dkdv_kernel<D, kF16, kFused, false>);
+        const int e = launch_dkdv(tc_bwd_dkdv_kernel<D, kF16, kFused>);
         if (e != 0) return e;
     }
     return 0;

@@ -43,9 +43,7 @@ enum FwdBar { Q_FULL, Q_EMPTY, K_FULL0, K_FULL1, K_FULL2, K_EMPTY0, K_EMPTY1, K_
               kNumBars = X_W0 + 32 };
 
 // kFused: out = o + rem * v is formed in the epilogue (a separate instantiation: the plain one stays as it is)
-// kDefer: an item's output is stored after the first step of the next item instead of at the item's end (chosen by the
-// host for packs of short sequences, where the wait for the item's last contraction is a large share of the item)
-template <int D, bool kF16, bool kFused, bool kDefer>
+template <int D, bool kF16, bool kFused>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const KArgs a) {
@@ -260,11 +258,6 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         const float scale = a.inv_temp * kLog2e;
         uint32_t ph_o = 0, items = 0;
         bool ok = true;
-        // With kDefer a finished item's output leaves tensor memory one step late: its last contraction needs a while to
-        // complete, and waiting for it at the end of the item idles the row threads.  They sweep the first tile of the
-        // next item instead (whose scores exist already) and store the output then; the first P V contraction of the next
-        // item waits for O_FREE, i.e. for this store.  It pays for short items only: for long ones the few registers that
-        // carry the pending item through the loop cost more than the wait.
         struct PendingItem {
             int b, h, tok, item;
             bool row_ok;
@@ -301,7 +294,13 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         SchedConsumer sched;
         int w;
         Work wk;
-        while (ok && (w = sched.next(ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, wk)) >= 0) {
+        while (ok) {
+            // The next item is read from the ring before the item before is stored.  (Instantiations that stored it a step into the next item,
+            // for packs of short sequences, lose against this: 0 ... 12 % of the forward at average lengths of 58 ... 3276 tokens.)
+            w = sched.next(ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, wk, false);
+            if (have_pend) store_item();
+            if (!ok || w < 0) break;
+            sched.release(&bars[WORK_EMPTY0]);
             const int n = wk.qt + 1;
             const int qi = wk.qt * kBM + r;
             const bool row_ok = qi < wk.len;
@@ -349,19 +348,11 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 tmem_wait_st();
                 tc_fence_before();
                 mbar_arrive(&bars[P_READY0 + sb]);
-                if (kDefer && j == 0 && have_pend) {
-                    store_item();
-                    if (!ok) break;
-                }
             }
             if (!ok) break;
             step += n;
             pend = PendingItem{wk.b, wk.h, wk.start + qi, (int)items, row_ok};
             have_pend = true;
-            if (!kDefer) {
-                store_item();
-                if (!ok) break;
-            }
             ++items;
             if (row_ok && kq == 0) {  // this thread swept the leftmost quarter: W is the remainder of the row
                 const int64_t t = wk.start + qi;
@@ -371,7 +362,6 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 ((float*)a.nla.ptr)[(int64_t)wk.b * a.nla.sb + (int64_t)wk.h * a.nla.sh + t * a.nla.st] = lg2_approx(W);
             }
         }
-        if (kDefer && ok && have_pend) store_item();  // the block's last item
     }
     tc_teardown(abort_flag, a.status, tmem, kTmemCols, 17);
     if (!a.own_tables) sched_finish(a.sched + 0);
@@ -396,8 +386,7 @@ int launch_fwd_t(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStrea
         if (e != 0) return e;
         return launch_kernel(kernel, dim3(persistent_grid((int64_t)L.max_items * p.heads)), dim3(kFwdThreads), smem, st, mq, mk, mv, a);
     };
-    if (a.fused) return a.defer_fwd ? launch(tc_fwd_kernel<D, kF16, true, true>) : launch(tc_fwd_kernel<D, kF16, true, false>);
-    return a.defer_fwd ? launch(tc_fwd_kernel<D, kF16, false, true>) : launch(tc_fwd_kernel<D, kF16, false, false>);
+    return a.fused ? launch(tc_fwd_kernel<D, kF16, true>) : launch(tc_fwd_kernel<D, kF16, false>);
 }
 
 }  // namespace
