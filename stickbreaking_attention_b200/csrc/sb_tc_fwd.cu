@@ -411,9 +411,9 @@ bool tensor_path_eligible(const SbParams& p, bool backward, int* why) {
     return true;
 }
 
-// Two query tiles at a time (sb_tc_fwd_pair.cu), from two tiles per sequence on.  Measured back to back, bf16, without / with carries:
-//   enough work to spread pairs: 32 heads x 16 384 tokens in sequences of 256 ... 8192 (28 tiles per SM) 1.01 ... 1.10 / 1.02 ... 1.09 times as fast, of
-//   16 384 1.0 / 1.02; 14 tiles per SM 0.97 ... 1.07 / 1.0 ... 1.09; 12 heads x 4 x 4000 (ten tiles) 0.96 / 0.98; 3 heads x 16 384 (2.6 tiles) 0.79 / 0.82;
+// Two query tiles at a time (sb_tc_fwd_pair.cu), from two tiles per sequence on.  Against one at a time, back to back, bf16, without / with carries:
+//   enough work to spread pairs: 32 heads x 16 384 tokens in sequences of 256 ... 16 384 (28 tiles per SM) 0.97 ... 1.09 / 0.99 ... 1.11 times as fast;
+//   14 ... 16 tiles per SM 0.95 ... 1.08 / 1.0 ... 1.11; 12 heads x 4 x 4000 (ten tiles) 0.96 / 0.98; 3 heads x 16 384 (2.6 tiles) 0.79 / 0.82;
 //   lengths that differ little: log-normal ones (28 tiles per SM) 0.96 ... 0.99 / 0.98 ... 1.0 (odd tiles alone, uneven ends);
 //   head dim 128: with 64 0.93 ... 1.02 (its contractions, which the pair overlaps better, are half as long).
 // Blocks that build their own tables (few tiles per SM) deal them out one by one.
