@@ -98,7 +98,7 @@ __device__ __forceinline__ void kv_store_rows_inl(const KArgs& a, bool is_dv, co
         tmem_ld32(taddr + cidx * 32, v);
         tmem_wait_ld(v);
         if (!(kFused && is_dv)) {  // two rows per lane pair: -7 % on a pack of 128-token sequences, -0.6 % on long ones
-            // (the same in the forward and the dq kernel, whose threads store half as much, cost 1-5 %)
+            // (in the forward, whose threads store half as much, it gains at head dim 64 only)
             store_row32_pairs<kF16>(orow + cidx * 64, v, sc, (int64_t)m.st * 2, key_ok && (D == 128 || cc < n_chunks), (int)(threadIdx.x & 31));
         } else if (key_ok && (D == 128 || cc < n_chunks)) {  // D == 64 serves head dim 32 as well: then fewer chunks exist
             if (kFused && add) {

@@ -276,7 +276,11 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 uint32_t v[32];
                 tmem_ld32(lane_base + kColO + d0, v);
                 tmem_wait_ld(v);
-                if (pend.row_ok && (D == 128 || a.head_dim > d0)) {  // D == 64 serves head dim 32 as well
+                const bool wr = pend.row_ok && (D == 128 || a.head_dim > d0);  // D == 64 serves head dim 32 as well
+                // two rows per lane pair at head dim 64 (0 ... 5 % of the forward, 8 and 32 heads, average lengths 58 ... 4096; nothing clear at 128)
+                if (!kFused && D == 64) {
+                    store_row32_pairs<kF16>(orow, v, 1.f, (int64_t)a.o.st * 2, wr, lane);
+                } else if (wr) {
                     if (kFused) {  // out = o + rem * v, rem rounded to the output type first
                         const float remf = round16<kF16>(wfin[(pend.item % 3) * 128 + r]);
                         float x[32];
