@@ -121,18 +121,20 @@ __device__ __forceinline__ float round16(float x) {
 }
 
 // (head, sequence, 128-row tile) of a flat work index.  Order: groups of `head_group` heads; inside a group the
-// items heaviest first, the heads of the group innermost.
+// items heaviest first, the heads of the group innermost.  Heads that do not fill the groups make the last group smaller, or the first
+// one if `missing` says how many it lacks.
 struct Work {
     int h, b, start, len, qt, slot_base;
 };
-__device__ __forceinline__ Work fetch_work(const KArgs& a, const int2* items, const SeqInfo* seqs, int n_items, int w) {
-    const int per_group = n_items * a.head_group;
-    const int g = w / per_group, rest = w - g * per_group;
-    const int hg = min(a.head_group, a.heads - g * a.head_group);
+__device__ __forceinline__ Work fetch_work(const KArgs& a, const int2* items, const SeqInfo* seqs, int n_items, int w, int missing = 0) {
+    const int g = (w + missing * n_items) / (n_items * a.head_group);
+    const int h0 = max(g * a.head_group - missing, 0);
+    const int hg = min((g + 1) * a.head_group - missing, a.heads) - h0;
+    const int rest = w - h0 * n_items;
     const int item = rest / hg;
     const int2 it = items[item];
     const SeqInfo s = seqs[it.x];
-    return Work{g * a.head_group + rest - item * hg, s.batch, s.start, s.len, it.y, s.slot_base};
+    return Work{h0 + rest - item * hg, s.batch, s.start, s.len, it.y, s.slot_base};
 }
 __device__ __forceinline__ Work fetch_work(const KArgs& a, int n_items, int w) { return fetch_work(a, a.items, a.seqs, n_items, w); }
 

@@ -159,6 +159,10 @@ tc_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             uint32_t kv = 0;
             bool ok = true, first = true;
             uint32_t ph_we = 3, ri = 0;
+            // Heads that do not fill the groups go first: the longest pair of a last group that is too small for all SMs would end the kernel
+            // alone.  One sequence of 16 384 tokens, 16 heads (groups of five), against one tile at a time: 9 % slower with the
+            // one head of the remainder last, 8 % faster with it first; 17 heads 10 % slower and 2 % faster.
+            const int missing = (a.head_group - a.heads % a.head_group) % a.head_group;
             const auto wait_q_slot = [&]() {
                 ok = mbar_wait_idle(&bars[Q_EMPTY0 + qs], (ph_qe >> qs) & 1, abort_flag);
                 ph_qe ^= 1u << qs;
@@ -177,7 +181,7 @@ tc_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     w = first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(a.sched + 0, 1);
                     first = false;
                     if (w >= n_work) { w = -1; break; }
-                    wk = fetch_work(a, n_items, w);
+                    wk = fetch_work(a, a.items, a.seqs, n_items, w, missing);
                     if (((((wk.len + kBM - 1) / kBM) - 1 - wk.qt) & 1) == 0) break;
                 }
                 if (w >= 0) ring->work[sl] = wk;

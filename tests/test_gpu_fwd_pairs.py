@@ -52,3 +52,59 @@ def test_pairs_of_tiles_against_oracle(lengths, dtype, attend_current, fused):
     got = [x[heads, :T].detach().double().cpu().numpy() for x in (o, rem) + grads]
     half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11  # what storing the exact result in the output type costs
     assert_close(("o", "rem", "dq", "dk", "dv"), got, want, TOL_BF16, f"pairs {lengths} {dtype} {fused}", out_half_ulp=half_ulp)
+
+
+def forward_kernels(call):
+    """Names of the forward kernels that `call` launches."""
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return {name for e in prof.events() for name in ("tc_fwd_pair_kernel", "tc_fwd_kernel") if name in e.name}
+
+
+@pytest.mark.parametrize("heads,tokens", [(16, 16384), (33, 8192), (7, 32768)])  # groups of 5, 8 and 2 heads, one head in the first group
+def test_heads_that_do_not_fill_their_groups(heads, tokens):
+    """Every head is worked on once: each against the same head in a call of few heads, which works on single tiles; both round their
+    16-bit weights and results from the same float32 sums, so they differ by a unit in the last place of results and the error of the weights
+    (2^-8 of each, in a weighted mean of N(0, 1) values: far below the bar)."""
+    from stickbreaking_attention_b200 import sb_attn
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    q, k, v = (torch.randn(1, heads, tokens, 128, generator=g, device="cuda").bfloat16() for _ in range(3))
+    with torch.no_grad():
+        assert forward_kernels(lambda: sb_attn(q, k, v)) == {"tc_fwd_pair_kernel"}
+        o, rem = sb_attn(q, k, v)
+        few = max(1, 8 * torch.cuda.get_device_properties(0).multi_processor_count * 128 // tokens // 2)
+        for h in range(0, heads, few):
+            part = [x[:, h:h + few] for x in (q, k, v)]
+            assert forward_kernels(lambda: sb_attn(*part)) == {"tc_fwd_kernel"}
+            want_o, want_rem = sb_attn(*part)
+            assert torch.all((o[:, h:h + few] - want_o).abs() <= 2.0 ** -7 * want_o.abs() + TOL_BF16)
+            assert torch.all((rem[:, h:h + few].float() - want_rem.float()).abs() <= 2.0 ** -7 * want_rem.float().abs() + 1e-6)
+
+
+def test_a_head_more_costs_a_head_more():
+    """Sixteen heads of 16 384 tokens go as groups of 1, 5, 5 and 5.  With the single head last, its longest pair (two rows of 128 tiles, about
+    4.5 times a head's share of all SMs) ends the kernel alone: 1.25 times the time of fifteen heads.  With it first the ratio is about 16 / 15;
+    the bar lies between the two."""
+    from stickbreaking_attention_b200 import sb_attn
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(1, 16, 16384, 128, generator=g, device="cuda").bfloat16() for _ in range(3))
+
+    def fastest(heads):
+        part = [x[:, :heads] for x in (q, k, v)]
+        times = []
+        with torch.no_grad():
+            for i in range(8):
+                start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                start.record()
+                for _ in range(3):
+                    sb_attn(*part)
+                end.record()
+                end.synchronize()
+                times.append(start.elapsed_time(end))
+        return min(times[2:])
+    fifteen, sixteen = fastest(15), fastest(16)
+    assert sixteen <= 1.18 * fifteen, (fifteen, sixteen)
