@@ -415,16 +415,27 @@ bool tensor_path_eligible(const SbParams& p, bool backward, int* why) {
     return true;
 }
 
-// Two query tiles at a time (sb_tc_fwd_pair.cu), from two tiles per sequence on.  Against one at a time, back to back, bf16, without / with carries:
-//   enough work to spread pairs: 32 heads x 16 384 tokens in sequences of 256 ... 16 384 (28 tiles per SM) 0.97 ... 1.09 / 0.99 ... 1.11 times as fast;
-//   14 ... 16 tiles per SM 0.95 ... 1.08 / 1.0 ... 1.11; 12 heads x 4 x 4000 (ten tiles) 0.96 / 0.98; 3 heads x 16 384 (2.6 tiles) 0.79 / 0.82;
-//   lengths that differ little: log-normal ones (28 tiles per SM) 0.96 ... 0.99 / 0.98 ... 1.0 (odd tiles alone, uneven ends);
-//   head dim 128: with 64 0.93 ... 1.02 (its contractions, which the pair overlaps better, are half as long).
-// Blocks that build their own tables (few tiles per SM) deal them out one by one.
+// Two query tiles at a time (sb_tc_fwd_pair.cu) or one.  How many times as fast two are, bf16, means of runs with and without carries, back to back and
+// alone, which scatter by 0.015; o / out = o + rem v:
+//   Sequences of one length, 12 ... 65 tiles per SM, 3 ... 128 heads: 256 tokens 0.995 ... 1.06 / 1.04 ... 1.08, 300 ... 768 0.99 ... 1.07 / 0.99 ... 1.09,
+//   900 ... 2048 0.985 ... 1.04 / 0.99 ... 1.05, 3000 ... 65 536 0.985 ... 1.09 / 0.985 ... 1.06; at multiples of 128 tokens 0.995 and more.
+//   257 tokens, of whose last tile one row is used: 0.98 ... 1.02 / 1.03.  The tiles have to be used to three quarters.
+//   Lengths 5, 15, 25 % around 280 ... 3500 tokens: 0.97 ... 1.04, 0.96 ... 1.02, 0.965 ... 1.015 / 0.98 ... 1.06, 0.97 ... 1.04, 0.97 ... 1.01; around 4096 ... 6000
+//   0.99 ... 1.04 / 0.98 ... 1.015.  The longest may exceed the average by a 64th.
+//   Below twelve tiles per SM: 3 heads x 16 384 tokens (2.6 tiles) 0.8, 16 x 3 x 4096 (10.4) 0.99.
+//   Head dim 64: 0.93 ... 1.02 (its contractions, which the pair overlaps better, are half as long): not taken.
+// Few long items per group of heads: items are dealt group by group, so while the longest pair of the last group is worked on, only that group's other
+// items are left for the SMs.  A group's time, in steps of 128 x 128 scores: 0.94 per step and 1.72 per tile; the longest pair's: 1.88 per step.  What the
+// longest pair takes beyond its group's share may be a twentieth of the whole: at 6 ... 16 % one sequence of 1024 ... 4096 tokens and 56 ... 260 heads 0.92 ... 1.01
+// (56 x 4096 0.92, 128 x 2048 0.945; 65 and 66 x 4096 1.04 ... 1.07).
 static bool use_pairs(const SbParams& p, const WsLayout& L, const KArgs& a) {
-    const int64_t total = (int64_t)p.tokens * (p.batch > 0 ? p.batch : 1);
-    return p.head_dim > 64 && !a.own_tables && (int64_t)L.max_items * p.heads >= 12ll * sm_count() && total >= 256ll * L.n_seqs &&
-           4ll * a.max_len * L.n_seqs <= 5 * total;
+    const int64_t total = (int64_t)p.tokens * (p.batch > 0 ? p.batch : 1), longest = (a.max_len + kBM - 1) / kBM;
+    if (p.head_dim <= 64 || a.own_tables || total < 256ll * L.n_seqs || 64ll * a.max_len * L.n_seqs > 65 * total ||
+        4 * total < 3 * longest * kBM * L.n_seqs || longest * L.n_seqs * p.heads < 12ll * sm_count())
+        return false;
+    const double tiles = (double)total / ((double)kBM * L.n_seqs);
+    const double head = L.n_seqs * tiles * (0.47 * (tiles + 1) + 1.72) / sm_count();
+    return 1.88 * longest <= ((p.heads < a.head_group ? p.heads : a.head_group) + 0.05 * p.heads) * head;
 }
 
 int launch_tensor_fwd(const SbParams& p, const WsLayout& L, const KArgs& a, cudaStream_t st) {

@@ -108,3 +108,31 @@ def test_a_head_more_costs_a_head_more():
         return min(times[2:])
     fifteen, sixteen = fastest(15), fastest(16)
     assert sixteen <= 1.18 * fifteen, (fifteen, sixteen)
+
+
+@pytest.mark.parametrize("heads,lengths,pairs", [
+    (32, [8192], True),
+    (12, [8192] * 4, True),
+    (8, [65536], True),
+    (17, [16384], True),
+    (16, [256] * 64, True),
+    (16, [1020, 1030, 1024, 1015] * 4, True),  # within 1/64 of the average
+    (6, [8192], False),                         # 2.6 tiles per SM
+    (10, [256] * 64, False),                    # 8.6 tiles per SM
+    (20, [870, 1130, 1000, 1100, 900] * 3, False),   # lengths that differ: 0.97 ... 1.0 times as fast in pairs
+    (32, [2943, 3503, 2192, 1807, 3696, 649, 1594], False),
+    (28, [257] * 31, False),                    # 0.99: a row in the last tile of three
+    (128, [2048], False),                       # 0.945: eight heads have too few long pairs for all SMs
+    (56, [4096], False),                        # 0.92
+])
+def test_calls_that_go_in_pairs(heads, lengths, pairs):
+    """The rule takes what two query tiles at a time are faster at, and nothing that they are slower at."""
+    from stickbreaking_attention_b200 import sb_attn_varlen
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the cases are those of 148 SMs")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(heads, sum(lengths), 128, generator=g, device="cuda").bfloat16() for _ in range(3))
+    cu = torch.tensor(np.cumsum(lengths), device="cuda")
+    with torch.no_grad():
+        ran = forward_kernels(lambda: sb_attn_varlen(q, k, v, cu, max(lengths), zero_start=False))
+    assert ran == {"tc_fwd_pair_kernel" if pairs else "tc_fwd_kernel"}
