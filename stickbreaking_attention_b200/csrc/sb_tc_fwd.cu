@@ -60,7 +60,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     volatile uint32_t* abort_flag = tmem_slot + 1;
     float* xw = (float*)(tmem_slot + 4);  // [quarter][128 rows]: carry leaving the quarter its thread has just swept
     OwnTables* own = (OwnTables*)(xw + 512 + 384);
-    float* wfin = xw + 512;               // [item mod 3][128 rows]: remainder of the row, for the fused epilogue (read one item late)
+    // [item mod 3][128 rows]: remainder of the row, for the fused epilogue, which reads it at the item's end.  Two slots would do (a thread that writes
+    // item i + 2 has stored item i + 1, whose first P V waited for O_FREE, until everybody had read item i), and measured the same or
+    // slower: 32 heads, 128-token sequences, head dim 128 127.5 -> 130.5 us, 64 84.2 -> 83.3.
+    float* wfin = xw + 512;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
@@ -277,7 +280,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 tmem_ld32(lane_base + kColO + d0, v);
                 tmem_wait_ld(v);
                 const bool wr = pend.row_ok && (D == 128 || a.head_dim > d0);  // D == 64 serves head dim 32 as well
-                // two rows per lane pair at head dim 64 (0 ... 5 % of the forward, 8 and 32 heads, average lengths 58 ... 4096; nothing clear at 128)
+                // two rows per lane pair at head dim 64 (0 ... 5 % of the forward, 8 and 32 heads, average lengths 58 ... 4096; nothing clear at 128; in the
+                // fused epilogue 0 ... 5 % slower at 64: average lengths 58 ... 256 129 -> 136 us, 85 -> 88, 2340 354 -> 356)
                 if (!kFused && D == 64) {
                     store_row32_pairs<kF16>(orow, v, 1.f, (int64_t)a.o.st * 2, wr, lane);
                 } else if (wr) {
@@ -299,8 +303,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         int w;
         Work wk;
         while (ok) {
-            // The next item is read from the ring before the item before is stored.  (Instantiations that stored it a step into the next item,
-            // for packs of short sequences, lose against this: 0 ... 12 % of the forward at average lengths of 58 ... 3276 tokens.)
+            // The next item is read from the ring before the item before is stored; read at its start, the forward takes 1 ... 12 % longer (32 heads,
+            // 512 x 128 tokens, head dim 128 357 -> 401 us; 1 % from a few thousand tokens on).  Instantiations that stored an item's result a step into
+            // the next item, for packs of short sequences, take 0 ... 5 % longer than this (fused 6 ... 26 %), average lengths 58 ... 2340.
             w = sched.next(ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, wk, false);
             if (have_pend) store_item();
             if (!ok || w < 0) break;
