@@ -281,7 +281,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 tmem_wait_ld(v);
                 const bool wr = pend.row_ok && (D == 128 || a.head_dim > d0);  // D == 64 serves head dim 32 as well
                 // two rows per lane pair at head dim 64 (0 ... 5 % of the forward, 8 and 32 heads, average lengths 58 ... 4096; nothing clear at 128; in the
-                // fused epilogue 0 ... 5 % slower at 64: average lengths 58 ... 256 129 -> 136 us, 85 -> 88, 2340 354 -> 356)
+                // fused epilogue up to 5 % slower at 64: 32 heads, 16 384 tokens, log-normal lengths around 100 128 -> 134 us, 128 tokens 84 -> 86, around 2340 362 -> 364)
                 if (!kFused && D == 64) {
                     store_row32_pairs<kF16>(orow, v, 1.f, (int64_t)a.o.st * 2, wr, lane);
                 } else if (wr) {
@@ -303,9 +303,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         int w;
         Work wk;
         while (ok) {
-            // The next item is read from the ring before the item before is stored; read at its start, the forward takes 1 ... 12 % longer (32 heads,
-            // 512 x 128 tokens, head dim 128 357 -> 401 us; 1 % from a few thousand tokens on).  Instantiations that stored an item's result a step into
-            // the next item, for packs of short sequences, take 0 ... 5 % longer than this (fused 6 ... 26 %), average lengths 58 ... 2340.
+            // The next item is read from the ring before the item before is stored; read at its start, the forward takes up to 17 % longer (32 heads,
+            // 512 x 128 tokens, head dim 128 348 -> 406 us; 1 % at 8192 tokens).  Instantiations that stored an item's result a step into
+            // the next item, for packs of short sequences, take up to 6 % longer than this (fused 3 ... 27 %), average lengths 58 ... 2340.
             w = sched.next(ring, &bars[WORK_FULL0], &bars[WORK_EMPTY0], abort_flag, wk, false);
             if (have_pend) store_item();
             if (!ok || w < 0) break;

@@ -1,6 +1,7 @@
-// Tensor-core forward (sm_100a), two query tiles of a sequence at a time: head dim 128, packs of sequences of about the same length with enough
-// work for every SM (use_pairs in sb_tc_fwd.cu).  Same results and carries as sb_tc_fwd.cu (the reference's _forward_one_row,
-// stickbreaking_attention/sb_varlen/sb_varlen_fwd.py:155-193).
+// Tensor-core forward (sm_100a), two query tiles of a sequence at a time: head dim 128, sequences of one length with enough work for every SM
+// (use_pairs in sb_tc_fwd.cu).  The results and carries of sb_tc_fwd.cu to rounding (the reference's _forward_one_row,
+// stickbreaking_attention/sb_varlen/sb_varlen_fwd.py:155-193): here the carry enters a chunk's chain of reciprocals at its start, there it is multiplied in at
+// the end, and here P V sums the right half of a tile first.
 //
 // One work item = (head, sequence, pair of neighbouring 128-row query tiles); the lowest tile of an odd number stands alone.  The pair
 // walks the key tiles right to left together, so a K or V tile is loaded once for both.  Each tile has its own row warps, scores and
@@ -20,8 +21,9 @@
 // What bounds it: power, then the row threads.  A step of one tile takes 3 190 cycles (clock readings around its parts), 1 910 of them row work
 // (1 152 of the special-function unit) and 1 280 between P and the next S, in which the other tile has the scheduler to itself: 1 595
 // cycles for 128 x 128 scores against 2 100 in sb_tc_fwd.cu.  In back-to-back calls the SM clock falls to about 1.7 GHz with either kernel.
-// Forward of 32 heads, 8192 tokens in one sequence, bf16, calls back to back: 557 -> 520 us (cuBLAS at its sustained rate would need 397 us
-// for the same operations); as single launches 484 -> 475 us.  With P V in parts of 96 and 32 keys 528 us.
+// Forward of 32 heads, 8192 tokens in one sequence, bf16, calls back to back: 557 -> 520 us when written (cuBLAS at its sustained rate would need 397 us
+// for the same operations), 535 -> 534 us against sb_tc_fwd.cu with its early reads of items; 8 heads, 65 536 tokens 7 920 -> 7 640 us.  With P V in parts
+// of 96 and 32 keys 528 us.
 #include "sb_tc_fwd_common.cuh"
 
 namespace sb {
