@@ -64,7 +64,10 @@ def forward_kernels(call):
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         call()
         torch.cuda.synchronize()
-    return {name for e in prof.events() for name in ("tc_fwd_pair_kernel", "tc_fwd_kernel") if name in e.name}
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    if not names:
+        pytest.skip("the profiler records no kernels here")
+    return {kernel for kernel in ("tc_fwd_pair_kernel", "tc_fwd_kernel") if any(kernel in name for name in names)}
 
 
 @pytest.mark.parametrize("heads,tokens", [(16, 16384), (33, 8192), (7, 32768)])  # groups of 5, 8 and 2 heads, one head in the first group
